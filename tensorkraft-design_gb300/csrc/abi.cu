@@ -159,6 +159,7 @@ void tk_ctx_destroy(tk_ctx* ctx) {
         if (ctx->stream) cudaStreamSynchronize((cudaStream_t)ctx->stream);
         if (ctx->dev_scratch) cudaFree(ctx->dev_scratch);
         if (ctx->host_stage) cudaFreeHost(ctx->host_stage);
+        for (auto& b : ctx->gemm_free) cudaFree(b.first);
         if (ctx->stream) cudaStreamDestroy((cudaStream_t)ctx->stream);
     }
     delete ctx;

@@ -1,0 +1,730 @@
+// digit_gemm.cu -- FP64 products on the fp16 tensor cores.
+//
+// This GPU does 1.2 TFLOP/s in FP64 and 1.9 PFLOP/s in fp16, so an FP64
+// product is cheaper as 28 exact fp16 ones.  The error-free splitting is the
+// published one of Ozaki, Ogita, Oishi and Rump (Numer. Algorithms 59, 2012):
+// every operand row becomes seven integer digits (digit_gemm.cuh), and
+//   sum_k x_k y_k = 2^(ea + eb - 66) sum_s 2^(8 (6 - s)) v_s,
+//   v_s = sum over i + j = s <= 6 of sum_k d_i d'_j.
+// Every v_s is an integer below 2^24 over 64 k (level s holds two products
+// with a leading digit, at most 2^16 each, and s - 1 of at most 2^14; level 0
+// one of 2^18), so fp32 accumulation is exact; after 64 k the seven sums are
+// added to an integer sum per output, and the result is rounded to FP64
+// once.  What is left out (levels 7 and up, at most 2^-64 of row maximum times
+// column maximum per k) lies three bits below the result's own rounding, and
+// each digit sum is that much finer than an FP64 element of the row's largest
+// magnitude: see the accuracy test for the error against exact sums.
+//
+// The kernel is persistent and warp-specialised, one CTA per SM: one thread
+// moves operands by TMA (32 k of all digits of 128 + 64 rows: 84 KB, a ring of
+// two), one issues tcgen05.mma, eight warps drain the accumulators.  The
+// digits of 32 B rows lie one after the other in shared memory and the levels
+// 32 columns apart in TMEM, so digit i of A meets digits 0 .. 6 - i of B in
+// ONE instruction (N = 32 (7 - i)) that lands on levels i .. 6: seven
+// instructions per 16 k, and A is read once for each.  A tile's two column
+// halves have accumulators of their own (2 x 224 columns): one is drained
+// while the other is summed.
+//
+// Measured (2048^3, N(0, 1) operands): digits 0.06 ms and product 0.50 ms (960
+// TFLOP/s of fp16, 0.50 of the measured peak), against 15.0 ms for the FP64
+// kernel, whose pipe is at its limit; relative error 4.9e-17 against 5.8e-16
+// at K = 300.  4096^3: 3.6 ms against 110 ms.  What bounds it now is the
+// operand traffic from L2: 168 KB for 64 k of a tile, 6.5 TB/s.
+#include "digit_gemm.cuh"
+
+#include <cudaTypedefs.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstdlib>
+#include <cstring>
+
+#include "tk_plan.cuh"
+
+namespace tk {
+namespace {
+
+constexpr int KW = 32;                                // K of one ring stage
+constexpr int HN = 32;                                // columns of a tile half
+constexpr int A_BYTES = kDigits * kTcBM * KW * 2;     // 57344
+constexpr int H_BYTES = kDigits * HN * KW * 2;        // 14336
+constexpr int STAGE_BYTES = A_BYTES + 2 * H_BYTES;    // 86016
+constexpr int EPI_WARPS = 16;
+constexpr int WCOLS = 16;                             // columns a drain warp holds: half a tile half
+constexpr int NTHREADS = 32 * (EPI_WARPS + 2);
+constexpr int SCOLS = 8;                              // columns staged at a time for the stores
+constexpr int ST_LD = SCOLS + 1;
+constexpr int STORE_BYTES = 32 * ST_LD * 8;           // per drain warp
+constexpr int SMEM_BYTES = 1024 + kDigitRing * STAGE_BYTES + EPI_WARPS * STORE_BYTES + 256;
+constexpr int TMEM_ALLOC = 512, TMEM_HALF = 256;
+constexpr long WAIT_LIMIT = 1L << 24;
+constexpr int kExBias = 2110;  // 2 * 1022 + 114 - 48: V * 2^(exa + exb - kExBias)
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t n) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(n) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* b) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
+}
+__device__ __forceinline__ bool mbar_test(uint64_t* b, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(b)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// Bounded wait.  Once one wait of the CTA has run out (*stop), every later one
+// returns at once, so that all roles leave together.
+__device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, volatile int* stop, int* redo) {
+    for (long i = 0; i < WAIT_LIMIT; ++i) {
+        if (mbar_test(b, parity)) return true;
+        if (*stop) return false;
+    }
+    *stop = 1;
+    atomicExch(redo, kDigitWait);
+    return false;
+}
+// Bounded wait for work already issued, whatever else went wrong.
+__device__ __forceinline__ void mbar_drain(uint64_t* b, uint32_t parity) {
+    for (long i = 0; i < WAIT_LIMIT; ++i)
+        if (mbar_test(b, parity)) return;
+}
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::
+            "r"(smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(0), "r"(smem_u32(bar))
+        : "memory");
+}
+// K-major rows of 64 bytes, 64-byte swizzle, 8-row groups 512 bytes apart.
+__device__ __forceinline__ uint64_t sw64_desc(uint32_t saddr) {
+    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(512u >> 4) << 32) |
+           ((uint64_t)1 << 46) | ((uint64_t)4 << 61);
+}
+// kind::f16: fp32 accumulate, fp16 A and B, both K-major, M = 128.
+__device__ __forceinline__ uint32_t idesc_f16(int n) {
+    return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTcBM >> 4) << 24);
+}
+__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accum)
+        : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tmem_ld4(uint32_t t, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(t));
+}
+
+// One output's sum: s 2^24 + l, in units of 2^8 of level 6.
+struct Sum {
+    int64_t s;
+    int32_t l;
+    // += the seven level sums of 64 k.  An int32 conversion runs at a sixteenth
+    // of the rate of an fp32 operation here, so levels 3 and 4 first hand
+    // their upper parts to the level above (adding 1.5 * 2^23 leaves a rounded
+    // integer in the low mantissa bits; every step is exact) and four
+    // conversions are left.  The last one rounds at 2^-58 of row maximum times
+    // column maximum.
+    __device__ __forceinline__ void add(float v0, float v1, float v2, float v3, float v4, float v5, float v6) {
+        const float M = 12582912.0f;
+        const float h4 = fmaf(v4, 0x1p-8f, M) - M;
+        const float l4 = fmaf(h4, -256.0f, v4);
+        const float w3 = v3 + h4;
+        const float h3 = fmaf(w3, 0x1p-8f, M) - M;
+        const float l3 = fmaf(h3, -256.0f, w3);
+        l += __float2int_rn(fmaf(l3, 65536.0f, fmaf(l4, 256.0f, fmaf(v6, 0x1p-8f, v5))));
+        mad(__float2int_rz(v2 + h3), 1);
+        mad(__float2int_rz(v1), 256);
+        mad(__float2int_rz(v0), 65536);
+    }
+    // s += a * b as one wide multiply-add (a shift and a 64-bit addition take four instructions)
+    __device__ __forceinline__ void mad(int a, int b) { asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(s) : "r"(a), "r"(b)); }
+    __device__ __forceinline__ void carry() {  // l back to 24 bits
+        s += l >> 24;
+        l &= 0xFFFFFF;
+    }
+    // (s 2^24 + l) 2^-u with m = 2^(24 - u)
+    __device__ __forceinline__ int64_t whole(uint32_t m, int u) const {
+        int64_t r = l >> u;
+        asm("mad.wide.u32 %0, %1, %2, %0;" : "+l"(r) : "r"((uint32_t)s), "r"(m));
+        return r + ((int64_t)(uint64_t)((uint32_t)((uint64_t)s >> 32) * m) << 32);
+    }
+};
+constexpr int kCarryChunks = 64;  // chunks after which l is near its range
+
+// x * 2^t rounded to nearest even, on the integer pipes (the FP64 pipe does
+// two operations a clock).  Free of branches, so that the columns of a row
+// overlap; *off is set where |x| < 2^32 or the result is subnormal or
+// overflows, which to_double_slow computes.
+__device__ __forceinline__ double to_double(int64_t x, int t, bool* off) {
+    const int32_t neg = (int32_t)((uint64_t)x >> 32) >> 31;
+    const uint64_t u = (uint64_t)((x ^ (int64_t)neg) - (int64_t)neg);
+    const uint32_t h = (uint32_t)(u >> 32), l = (uint32_t)u;
+    // the leading bit to bit 62, so that rounding at bit 10 cannot carry out
+    const int z = __clz(h) - 1;
+    uint64_t q = ((uint64_t)__funnelshift_l(l, h, z) << 32) | (l << (z & 31));
+    q = (q + 0x1FFu + ((uint32_t)(q >> 10) & 1u)) >> 10;
+    const int e = t + 10 - z;  // the value is q * 2^e
+    const bool fast = h != 0 && (uint32_t)(e + 1073) < 2045u;
+    *off |= !fast && u != 0;
+    const uint32_t rh = ((uint32_t)(q >> 32) + ((uint32_t)(e + 1074) << 20)) | ((uint32_t)neg & 0x80000000u);
+    return fast ? __hiloint2double((int)rh, (int)(uint32_t)q) : 0.0;
+}
+__device__ __noinline__ double to_double_slow(int64_t x, int t) {
+    uint64_t u = x < 0 ? 0 - (uint64_t)x : (uint64_t)x;
+    if (u == 0) return 0.0;
+    // drop the bits below the result's last place, 2^-1074 at the least
+    const int drop = max(11 - __clzll((long long)u), -1074 - t);
+    if (drop > 0) {
+        const int d = min(drop, 63);
+        const uint64_t half = 1ull << (d - 1), rest = u & ((1ull << d) - 1);
+        u = drop > 64 ? 0 : (u >> d) + (rest + ((u >> d) & 1) > half);
+        t += drop;
+    }
+    const double r = u == 0 ? 0.0 : t > 1000 ? INFINITY : ldexp((double)(long long)u, t);
+    return x < 0 ? -r : r;
+}
+
+// Tile ti of a launch: from the table, or (mode 0) of the C grid, columns first.
+template <int MODE>
+__device__ __forceinline__ TcTile tile_of(const TcTile* __restrict__ tiles, const DigitOut& om, int ti) {
+    if (MODE != 0) return tiles[ti];
+    TcTile t;
+    const int ntn = (om.n + kTcBN - 1) / kTcBN, m0 = ti / ntn * kTcBM, n0 = ti % ntn * kTcBN;
+    t.a_row = t.ldc = m0;
+    t.a_cs = om.m;
+    t.b_row = t.n0 = n0;
+    t.b_cs = om.n;
+    t.k_valid = om.k;
+    t.m_valid = min(kTcBM, om.m - m0);
+    t.n_valid = min(kTcBN, om.n - n0);
+    return t;
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* __restrict__ tiles, int n_tiles,
+                                                                 const __grid_constant__ DigitMaps maps,
+                                                                 const int32_t* __restrict__ exa,
+                                                                 const int32_t* __restrict__ exb, const DigitOut om,
+                                                                 int* redo) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    double* store = (double*)(smem + kDigitRing * STAGE_BYTES);
+    uint64_t* full = (uint64_t*)(smem + kDigitRing * STAGE_BYTES + EPI_WARPS * STORE_BYTES);
+    uint64_t* empty = full + kDigitRing;
+    uint64_t* acc_full = empty + kDigitRing;
+    uint64_t* acc_empty = acc_full + 2;
+    uint64_t* done = acc_empty + 2;
+    uint32_t* tslot = (uint32_t*)(done + 1);
+    volatile int* stop = (volatile int*)(tslot + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        *stop = *(volatile int*)redo;  // an operand held an infinity or a NaN: another kernel computes this product
+        for (int i = 0; i < kDigitRing; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&acc_full[i], 1);
+            mbar_init(&acc_empty[i], EPI_WARPS / 2);
+        }
+        mbar_init(done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == EPI_WARPS) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
+                     "r"(TMEM_ALLOC)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = *tslot;
+    const bool run = *stop == 0;  // written before the barrier; a wait can only run out after it
+    __syncthreads();
+
+    if (warp == EPI_WARPS) {
+        if (lane == 0) {
+            int it = 0;
+            bool ok = run;
+            for (int ti = blockIdx.x; ti < n_tiles && ok; ti += gridDim.x) {
+                const TcTile t = tile_of<MODE>(tiles, om, ti);
+                const int halves = t.n_valid > HN ? 2 : 1;
+                const int box = (t.m_valid + 31) >> 5;
+                const uint32_t bytes = kDigits * KW * 2 * (32 * box + HN * halves);
+                const int steps = (t.k_valid + KW - 1) / KW;
+                for (int q = 0; q < steps && ok; ++q, ++it) {
+                    const int st = it % kDigitRing;
+                    uint8_t* base = smem + st * STAGE_BYTES;
+                    if (it >= kDigitRing) ok = mbar_wait(&empty[st], (it / kDigitRing - 1) & 1, stop, redo);
+                    if (!ok) break;
+                    mbar_expect_tx(&full[st], bytes);
+                    const int x = (q & 1) * KW, c = q >> 1;
+                    tma_load_3d(base, &maps.a[box - 1], x, t.a_row + c * t.a_cs, &full[st]);
+                    for (int h = 0; h < halves; ++h)
+                        tma_load_3d(base + A_BYTES + h * H_BYTES, &maps.b, x, t.b_row + c * t.b_cs + HN * h, &full[st]);
+                }
+            }
+            // the loads in flight land before the CTA's shared memory goes
+            for (int i = max(0, it - kDigitRing); i < it; ++i) mbar_drain(&full[i % kDigitRing], (i / kDigitRing) & 1);
+        }
+    } else if (warp == EPI_WARPS + 1) {
+        if (lane == 0) {
+            int it = 0, unit = 0;
+            int drains[2] = {0, 0};
+            bool ok = run;
+            for (int ti = blockIdx.x; ti < n_tiles && ok; ti += gridDim.x) {
+                const TcTile t = tile_of<MODE>(tiles, om, ti);
+                const int halves = t.n_valid > HN ? 2 : 1;
+                const uint32_t astep = (uint32_t)((((t.m_valid + 31) >> 5) * 32) * KW * 2);
+                const int steps = (t.k_valid + KW - 1) / KW;
+                for (int q = 0; q < steps && ok; ++q, ++it) {
+                    const int st = it % kDigitRing;
+                    const bool first = (q & 1) == 0, last = (q & 1) == 1 || q == steps - 1;
+                    ok = mbar_wait(&full[st], (it / kDigitRing) & 1, stop, redo);
+                    const uint32_t sa = smem_u32(smem + st * STAGE_BYTES);
+                    const int ks = min(KW / 16, (t.k_valid - q * KW + 15) / 16);
+                    for (int h = 0; h < halves && ok; ++h) {
+                        const int buf = (unit + h) & 1;
+                        if (first && drains[buf] > 0) ok = mbar_wait(&acc_empty[buf], (drains[buf] - 1) & 1, stop, redo);
+                        if (!ok) break;
+                        fence_after();
+                        const uint64_t b0 = sw64_desc(sa + A_BYTES + h * H_BYTES);
+                        const uint32_t d0 = tmem + buf * TMEM_HALF;
+                        for (int kk = 0; kk < ks; ++kk) {
+                            const uint64_t adv = (uint64_t)((kk * 32) >> 4);
+#pragma unroll
+                            for (int i = 0; i < kDigits; ++i)
+                                mma_f16(d0 + i * HN, sw64_desc(sa + i * astep) + adv, b0 + adv,
+                                        idesc_f16((kDigits - i) * HN), !(first && kk == 0 && i == 0));
+                        }
+                        if (last) {
+                            mma_commit(&acc_full[buf]);
+                            ++drains[buf];
+                        }
+                    }
+                    mma_commit(&empty[st]);
+                }
+                unit += halves;
+            }
+            // no instruction is in flight when the accumulators are given back
+            mma_commit(done);
+            mbar_drain(done, 0);
+        }
+    } else {
+        // warps 0-7 drain accumulator 0, warps 8-15 accumulator 1; warp % 4 is
+        // the TMEM lane quarter, (warp / 4) % 2 the 16 of the half's 32 columns:
+        // a thread holds one row of 16 columns
+        const int buf = warp >> 3, row0 = (warp & 3) * 32, col0 = ((warp >> 2) & 1) * WCOLS;
+        const uint32_t tbase = tmem + buf * TMEM_HALF + col0 + ((uint32_t)row0 << 16);
+        double* sw = store + warp * (STORE_BYTES / 8);
+        int drains = 0, unit = 0;
+        bool ok = run;
+        for (int ti = blockIdx.x; ti < n_tiles && ok; ti += gridDim.x) {
+            const TcTile t = tile_of<MODE>(tiles, om, ti);
+            const int halves = t.n_valid > HN ? 2 : 1;
+            const int h = (buf - unit) & 1;
+            unit += halves;
+            if (h >= halves) continue;
+            const int nc = min(WCOLS, t.n_valid - h * HN - col0);  // columns of this warp's that the tile has
+            const bool mine = row0 < t.m_valid && nc > 0;
+            Sum acc[WCOLS];
+#pragma unroll
+            for (int i = 0; i < WCOLS; ++i) acc[i] = {0, 0};
+            const int chunks = (t.k_valid + kTcBK - 1) / kTcBK;
+            for (int c = 0; c < chunks && ok; ++c) {
+                ok = mbar_wait(&acc_full[buf], drains & 1, stop, redo);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                ++drains;
+                fence_after();
+                if (mine) {
+#pragma unroll
+                    for (int g = 0; g < WCOLS / 4; ++g) {
+                        uint32_t v[kDigits][4];
+#pragma unroll
+                        for (int s = 0; s < kDigits; ++s) tmem_ld4(tbase + s * HN + g * 4, v[s]);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            auto f = [&](int s) { return __uint_as_float(v[s][i]); };
+                            acc[g * 4 + i].add(f(0), f(1), f(2), f(3), f(4), f(5), f(6));
+                        }
+                    }
+                    if (c % kCarryChunks == kCarryChunks - 1) {
+#pragma unroll
+                        for (int i = 0; i < WCOLS; ++i) acc[i].carry();
+                    }
+                }
+                fence_before();
+                if (lane == 0) mbar_arrive(&acc_empty[buf]);
+            }
+            if (!ok || !mine) continue;
+            // s 2^24 + l in 64 bits, for the whole row less the u low bits that the
+            // row's largest sum leaves no room for (it then has 62 of its own)
+            uint32_t bits = 0;
+#pragma unroll
+            for (int i = 0; i < WCOLS; ++i) {
+                const int32_t hi = (int32_t)(acc[i].s >> 32);
+                bits |= (uint32_t)(hi ^ (hi >> 31));
+            }
+            const int u = max(0, 26 - __clz((int)bits));
+            const uint32_t um = 1u << (24 - u);
+            // exponents: a row of this thread, a column per lane
+            const int ea = (row0 + lane < t.m_valid ? exa[t.a_row + row0 + lane] : 1) - kExBias + 8 + u;
+            const int eb = lane < nc ? exb[t.b_row + h * HN + col0 + lane] : 1;
+            // eight columns at a time through shared memory: consecutive lanes
+            // store consecutive columns
+            const int cl = lane & (SCOLS - 1);
+#pragma unroll
+            for (int g = 0; g < WCOLS / SCOLS; ++g) {
+                if (g * SCOLS >= nc) break;
+                bool off = false;
+                double val[SCOLS];
+#pragma unroll
+                for (int i = 0; i < SCOLS; ++i)
+                    val[i] = to_double(acc[g * SCOLS + i].whole(um, u), ea + __shfl_sync(0xffffffffu, eb, g * SCOLS + i), &off);
+                if (__any_sync(0xffffffffu, off && row0 + lane < t.m_valid)) {
+#pragma unroll
+                    for (int i = 0; i < SCOLS; ++i)
+                        val[i] = to_double_slow(acc[g * SCOLS + i].whole(um, u), ea + __shfl_sync(0xffffffffu, eb, g * SCOLS + i));
+                }
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < SCOLS; ++i) sw[lane * ST_LD + i] = val[i];
+                __syncwarp();
+                const int col = h * HN + col0 + g * SCOLS + cl;
+                if (g * SCOLS + cl >= nc) continue;
+                const int r0 = lane / SCOLS;
+                double* o;
+                int64_t step = 0;
+                if (MODE == 2) {
+                    step = om.colstride[t.out_off + col];
+                    o = om.out + om.colbase[t.out_off + col] + (int64_t)(t.ldc + row0 + r0) * step;
+                } else if (MODE == 1) {
+                    o = om.out + t.n0 + col;
+                } else {
+                    step = om.c_rs;
+                    o = om.out + (int64_t)(t.n0 + col) * om.c_cs + (int64_t)(t.ldc + row0 + r0) * step;
+                }
+                step *= 32 / SCOLS;
+                const int last = t.m_valid - row0 - r0;  // rows of this lane's are 4 v < last
+                if (MODE == 0 && (om.alpha != 1.0 || om.beta != 0.0)) {
+                    for (int v = 0; v < SCOLS && v * (32 / SCOLS) < last; ++v, o += step) {
+                        double x = om.alpha * sw[(v * (32 / SCOLS) + r0) * ST_LD + cl];
+                        if (om.beta != 0.0) x += om.beta * *o;
+                        *o = x;
+                    }
+                } else {
+#pragma unroll
+                    for (int v = 0; v < SCOLS; ++v, o += step) {
+                        if (v * (32 / SCOLS) >= last) break;
+                        const double x = sw[(v * (32 / SCOLS) + r0) * ST_LD + cl];
+                        *(MODE == 1 ? o + om.rowtab[t.out_off + row0 + v * (32 / SCOLS) + r0] : o) = x;
+                    }
+                }
+            }
+        }
+    }
+    fence_before();
+    __syncthreads();
+    if (warp == EPI_WARPS) {
+        fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_ALLOC) : "memory");
+    }
+}
+
+// ---------------------------------------------------------------- digits
+
+__device__ __forceinline__ uint32_t abs_hi(double x) { return (uint32_t)__double2hiint(x) & 0x7FFFFFFFu; }
+// Biased exponent of a row whose largest element has these high bits (below 1
+// for a row of subnormals).
+__device__ __forceinline__ int row_exponent(uint32_t max_hi, int* redo) {
+    const int e = (int)(max_hi >> 20);
+    if (e == 2047) atomicExch(redo, kDigitValue);
+    return e > 0 ? e : 12 - __clz((int)(max_hi | 1));
+}
+// x on its row's grid, rounded to nearest, plus 128 in each of the six low
+// bytes: byte j is then digit 6 - j plus 128, the upper 16 bits digit 0.
+__device__ __forceinline__ uint64_t on_grid(double x, int ex) {
+    const uint64_t b = (uint64_t)__double_as_longlong(x);
+    const int e = (int)(b >> 52) & 0x7FF;
+    uint64_t m = (b & 0xFFFFFFFFFFFFFull) << 4;
+    if (e) m |= 1ull << 56;
+    const int s = min(ex - max(e, 1), 62);
+    m = s >= 0 ? (m + ((1ull << s) >> 1)) >> s : m << -s;
+    if ((int64_t)b < 0) m = 0 - m;
+    return m + 0x0000808080808080ull;
+}
+// The digits of two neighbouring elements, as pairs of fp16.
+__device__ __forceinline__ void digits2(double x, double y, int ex, uint32_t* d) {
+    const uint64_t a = on_grid(x, ex), b = on_grid(y, ex);
+    const uint32_t al = (uint32_t)a, ah = (uint32_t)(a >> 32), bl = (uint32_t)b, bh = (uint32_t)(b >> 32);
+    // 0x6400 | n is fp16 1024 + n
+    auto half_of = [](uint32_t v, uint32_t bias) {
+        const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&bias));
+        return *reinterpret_cast<const uint32_t*>(&h);
+    };
+    auto bytes = [&](uint32_t u, uint32_t v, uint32_t sel) {
+        return half_of((__byte_perm(u, v, sel) & 0x00FF00FFu) | 0x64006400u, 0x64806480u);  // minus 1152
+    };
+    d[6] = bytes(al, bl, 0x4400);
+    d[5] = bytes(al, bl, 0x5511);
+    d[4] = bytes(al, bl, 0x6622);
+    d[3] = bytes(al, bl, 0x7733);
+    d[2] = bytes(ah, bh, 0x4400);
+    d[1] = bytes(ah, bh, 0x5511);
+    const uint32_t top = ((uint32_t)((int)ah >> 16) + 512u) | (((uint32_t)((int)bh >> 16) + 512u) << 16);
+    d[0] = half_of(top + 0x64006400u, 0x66006600u);  // minus 1536
+}
+__device__ __forceinline__ void put_digits(const DigitStack& o, int64_t row, int k, const uint32_t* d) {
+    uint32_t* p = reinterpret_cast<uint32_t*>(o.q) + (row << 5) + (k >> 1);
+#pragma unroll
+    for (int j = 0; j < kDigits; ++j) p[j * (o.rows << 5)] = d[j];
+}
+
+// One warp per row of an FP64 stack (K-major 64-wide chunks): the row's
+// largest exponent, then its digits; the first kKeep chunks stay in registers
+// in between, the others are read again (from L1 or L2).
+constexpr int kKeep = 4;
+__global__ void __launch_bounds__(32 * kDigitRowsPerCta) digit_rows_kernel(const DigitRows* __restrict__ jobs,
+                                                                           const double* __restrict__ q64,
+                                                                           const DigitStack out, int* redo) {
+    const DigitRows j = jobs[blockIdx.x];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (w >= j.n) return;
+    const int64_t row = (int64_t)j.row + w;
+    auto at = [&](int c) { return reinterpret_cast<const double2*>(q64 + ((row + (int64_t)c * j.cs) << 6))[lane]; };
+    double2 v[kKeep];
+    uint32_t mx = 0;
+#pragma unroll
+    for (int c = 0; c < kKeep; ++c) {
+        v[c] = c < j.kch ? at(c) : make_double2(0.0, 0.0);
+        mx = max(mx, max(abs_hi(v[c].x), abs_hi(v[c].y)));
+    }
+#pragma unroll 4
+    for (int c = kKeep; c < j.kch; ++c) {
+        const double2 u = at(c);
+        mx = max(mx, max(abs_hi(u.x), abs_hi(u.y)));
+    }
+    const int ex = row_exponent(__reduce_max_sync(0xffffffffu, mx), redo);
+    if (lane == 0) out.ex[row] = ex;
+    uint32_t d[kDigits];
+#pragma unroll
+    for (int c = 0; c < kKeep; ++c)
+        if (c < j.kch) {
+            digits2(v[c].x, v[c].y, ex, d);
+            put_digits(out, row + (int64_t)c * j.cs, 2 * lane, d);
+        }
+#pragma unroll 2
+    for (int c = kKeep; c < j.kch; ++c) {
+        const double2 u = at(c);
+        digits2(u.x, u.y, ex, d);
+        put_digits(out, row + (int64_t)c * j.cs, 2 * lane, d);
+    }
+}
+
+// psi sub-blocks: 32 columns x all K rows by one CTA, lanes along the columns;
+// each 64-wide chunk is turned in shared memory.
+constexpr int BT = 256;
+__global__ void __launch_bounds__(BT) digit_psi_kernel(const TcSplitJob* __restrict__ jobs, const double* __restrict__ x,
+                                                       const DigitStack out, int* redo) {
+    __shared__ uint32_t smax[32];
+    __shared__ double tile[32][kTcBK + 1];
+    const TcSplitJob j = jobs[blockIdx.x];
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const int nr = min(32, j.cols - j.b0), K = j.rows;
+    const double* src = x + j.src + j.b0 + lane;
+    const int64_t row = (int64_t)j.xrow + j.b0;
+    if (tid < 32) smax[tid] = 0;
+    __syncthreads();
+    uint32_t mx = 0;
+#pragma unroll 4
+    for (int k = w; k < K; k += BT / 32) mx = max(mx, lane < nr ? abs_hi(src[(int64_t)k * j.cols]) : 0u);
+    atomicMax(&smax[lane], mx);
+    __syncthreads();
+    if (tid < nr) {
+        const int ex = row_exponent(smax[tid], redo);
+        out.ex[row + tid] = ex;
+        smax[tid] = (uint32_t)ex;
+    }
+    for (int c = 0; c * kTcBK < K; ++c) {
+        const int k0 = c * kTcBK;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kTcBK / (BT / 32); ++i) {
+            const int k = k0 + w + i * (BT / 32);
+            tile[lane][k - k0] = lane < nr && k < K ? src[(int64_t)k * j.cols] : 0.0;
+        }
+        __syncthreads();
+        const int kv = (min(kTcBK, K - k0) + 15) & ~15;  // whole 16-wide steps are multiplied
+        for (int r = w; r < nr; r += BT / 32)
+            if (2 * lane < kv) {
+                uint32_t d[kDigits];
+                digits2(tile[r][2 * lane], tile[r][2 * lane + 1], (int)smax[r], d);
+                put_digits(out, row + r + (int64_t)c * j.cstride, 2 * lane, d);
+            }
+    }
+}
+
+// The two operands of a dense product, 32 rows x 64 k a CTA (the rows of A,
+// then those of B).  PASS 0 leaves every row's largest high word in ex (zeroed
+// before), PASS 1 writes the digits; lanes walk along the shorter stride.
+template <int PASS>
+__global__ void __launch_bounds__(BT) digit_matrix_kernel(const DigitMatrix A, const DigitMatrix B, int K, int* redo) {
+    __shared__ double tile[32][kTcBK + 1];
+    __shared__ int sex[32];
+    const int na = (A.rows + 31) / 32;
+    const bool first = (int)blockIdx.x < na;
+    const DigitMatrix& m = first ? A : B;
+    const int r0 = ((int)blockIdx.x - (first ? 0 : na)) * 32, nr = min(32, m.rows - r0), k0 = (int)blockIdx.y * kTcBK;
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const double* x = m.x + r0 * m.rs + k0 * m.ks;
+    auto fetch = [&](int r, int k) { return r < nr && k0 + k < K ? x[r * m.rs + k * m.ks] : 0.0; };
+    if (PASS == 1 && tid < nr) {
+        sex[tid] = row_exponent((uint32_t)m.out.ex[r0 + tid], redo);
+    }
+    if ((m.rs < 0 ? -m.rs : m.rs) < (m.ks < 0 ? -m.ks : m.ks)) {
+#pragma unroll
+        for (int i = 0; i < kTcBK / (BT / 32); ++i) tile[lane][w + i * (BT / 32)] = fetch(lane, w + i * (BT / 32));
+    } else {
+#pragma unroll
+        for (int i = 0; i < 32 / (BT / 64); ++i) {
+            const int r = (tid >> 6) + i * (BT / 64), k = tid & 63;
+            tile[r][k] = fetch(r, k);
+        }
+    }
+    __syncthreads();
+    for (int r = w; r < nr; r += BT / 32) {
+        if (PASS == 0) {
+            const uint32_t mx = __reduce_max_sync(0xffffffffu, max(abs_hi(tile[r][lane]), abs_hi(tile[r][lane + 32])));
+            if (lane == 0) atomicMax(m.out.ex + r0 + r, (int)mx);
+        } else {
+            const double u = tile[r][2 * lane], v = tile[r][2 * lane + 1];
+            uint32_t d[kDigits];
+            digits2(u, v, sex[r], d);
+            put_digits(m.out, r0 + r + (int64_t)blockIdx.y * m.rows, 2 * lane, d);
+            // the row's squares, its largest element counting at most 1
+            const float a = (float)(int)(on_grid(u, sex[r]) >> 32) * 0x1p-25f, b = (float)(int)(on_grid(v, sex[r]) >> 32) * 0x1p-25f;
+            float sq = fmaf(a, a, b * b);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+            if (lane == 0) atomicAdd(m.square + r0 + r, sq);
+        }
+    }
+}
+// The largest high word of every row becomes its exponent.  A row far from
+// flat has no place on one grid: with P = K 2^(2 e) / sum x^2, the digits' error
+// is about 2^-59 sqrt(P_a P_b / K) of ||a|| ||b||, an FP64 chain's 2^-53
+// sqrt(K / 12) of sqrt(sum a^2 b^2), about ||a|| ||b|| / sqrt(K); so a row whose P
+// exceeds 64 sqrt(K / 12) (a normal one has up to 110, and P <= 4 K) sends the
+// product to the FP64 pipe.
+__global__ void digit_exponent_kernel(const DigitMatrix A, const DigitMatrix B, float least, int* redo) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int o = 0; o < 2; ++o) {
+        const DigitMatrix& m = o ? B : A;
+        if (i >= m.rows) continue;
+        const uint32_t hi = (uint32_t)m.out.ex[i];
+        m.out.ex[i] = row_exponent(hi, redo);
+        if (hi != 0 && m.square[i] < least) atomicExch(redo, kDigitValue);
+    }
+}
+
+}  // namespace
+
+bool digit_maps(DigitMaps& m, const DigitStack& a, const DigitStack& b, std::string& err) {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess || !fn) {
+        err = "cuTensorMapEncodeTiled entry point unavailable";
+        return false;
+    }
+    std::memset(&m, 0, sizeof(m));
+    auto make = [&](CUtensorMap* map, const DigitStack& s, int box_rows) {
+        if (s.rows <= 0) return true;
+        cuuint64_t dims[3] = {(cuuint64_t)kTcBK, (cuuint64_t)s.rows, (cuuint64_t)kDigits};
+        cuuint64_t strides[2] = {(cuuint64_t)kTcBK * 2, (cuuint64_t)s.rows * kTcBK * 2};
+        cuuint32_t box[3] = {(cuuint32_t)KW, (cuuint32_t)box_rows, (cuuint32_t)kDigits};
+        cuuint32_t estr[3] = {1, 1, 1};
+        CUresult r = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn)(
+            map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, s.q, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) err = "cuTensorMapEncodeTiled failed with CUresult " + std::to_string((int)r);
+        return r == CUDA_SUCCESS;
+    };
+    for (int i = 0; i < 4; ++i)
+        if (!make(&m.a[i], a, 32 * (i + 1))) return false;
+    return make(&m.b, b, HN);
+}
+
+cudaError_t digit_setup() {
+    cudaError_t e = cudaSuccess;
+    for (const void* k : {(const void*)digit_gemm_kernel<0>, (const void*)digit_gemm_kernel<1>, (const void*)digit_gemm_kernel<2>})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    return e;
+}
+
+cudaError_t launch_digit_gemm(int mode, const TcTile* tiles, int n_tiles, const DigitMaps& maps, const int32_t* exa,
+                              const int32_t* exb, const DigitOut& out, int* redo, int sms, cudaStream_t s) {
+    if (n_tiles <= 0) return cudaSuccess;
+    const int grid = std::min(n_tiles, sms);
+    if (mode == 0)
+        digit_gemm_kernel<0><<<grid, NTHREADS, SMEM_BYTES, s>>>(tiles, n_tiles, maps, exa, exb, out, redo);
+    else if (mode == 1)
+        digit_gemm_kernel<1><<<grid, NTHREADS, SMEM_BYTES, s>>>(tiles, n_tiles, maps, exa, exb, out, redo);
+    else
+        digit_gemm_kernel<2><<<grid, NTHREADS, SMEM_BYTES, s>>>(tiles, n_tiles, maps, exa, exb, out, redo);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_digit_rows(const DigitRows* jobs, int n_jobs, const double* q64, const DigitStack& out, int* redo,
+                              cudaStream_t s) {
+    if (n_jobs <= 0) return cudaSuccess;
+    digit_rows_kernel<<<n_jobs, 32 * kDigitRowsPerCta, 0, s>>>(jobs, q64, out, redo);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_digit_matrices(const DigitMatrix& a, const DigitMatrix& b, int K, int* redo, cudaStream_t s) {
+    const dim3 grid((unsigned)((a.rows + 31) / 32 + (b.rows + 31) / 32), (unsigned)((K + kTcBK - 1) / kTcBK));
+    cudaError_t e;
+    if ((e = cudaMemsetAsync(a.out.ex, 0, sizeof(int32_t) * a.rows, s)) != cudaSuccess ||
+        (e = cudaMemsetAsync(b.out.ex, 0, sizeof(int32_t) * b.rows, s)) != cudaSuccess ||
+        (e = cudaMemsetAsync(a.square, 0, sizeof(float) * a.rows, s)) != cudaSuccess ||
+        (e = cudaMemsetAsync(b.square, 0, sizeof(float) * b.rows, s)) != cudaSuccess)
+        return e;
+    digit_matrix_kernel<0><<<grid, BT, 0, s>>>(a, b, K, redo);
+    digit_matrix_kernel<1><<<grid, BT, 0, s>>>(a, b, K, redo);
+    digit_exponent_kernel<<<(std::max(a.rows, b.rows) + 255) / 256, 256, 0, s>>>(
+        a, b, std::sqrt(12.0f * (float)K) / 64.0f, redo);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_digit_psi(const TcSplitJob* jobs, int n_jobs, const double* x, const DigitStack& out, int* redo,
+                             cudaStream_t s) {
+    if (n_jobs <= 0) return cudaSuccess;
+    digit_psi_kernel<<<n_jobs, BT, 0, s>>>(jobs, x, out, redo);
+    return cudaGetLastError();
+}
+
+}  // namespace tk

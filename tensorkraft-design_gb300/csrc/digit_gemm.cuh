@@ -1,0 +1,86 @@
+// digit_gemm.cuh -- FP64 products on the fp16 tensor cores (digit_gemm.cu).
+#pragma once
+#include <cuda.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <string>
+
+#include "tk_internal.hpp"
+
+namespace tk {
+
+// An operand row x is held as seven fp16 integer digits on a grid of its own,
+//   x = 2^(e - 57) * sum_j d_j 2^(8 (6 - j)),  |d_0| <= 2^9, |d_j| <= 2^7,
+// e the exponent of the row's largest element (all |x| < 2^e): every element
+// to 2^(e - 58), five bits below the last place of the largest one.
+constexpr int kDigits = 7;
+constexpr int kDigitValue = 1, kDigitWait = 2;  // *redo: an operand's values / a wait that ran out
+constexpr int kDigitRing = 2;  // shared-memory stages of 32 K of a product
+
+// A digit operand in the operand-stack layout (K-major 64-wide chunks, see
+// TcTables): plane j of `rows` rows of 64, and the biased exponent of every
+// row of chunk 0.
+struct DigitStack {
+    __half* q = nullptr;
+    int32_t* ex = nullptr;
+    int64_t rows = 0;
+};
+inline size_t digit_stack_bytes(int64_t rows) { return (size_t)rows * kTcBK * kDigits * sizeof(__half); }
+
+// Rows [row, row + n) of a stack whose chunks are `cs` rows apart.
+struct DigitRows {
+    int32_t row, n, cs, kch;
+};
+constexpr int kDigitRowsPerCta = 8;
+
+// Tensor maps of one product's operands: A in boxes of 32, 64, 96 or 128 rows
+// x 32 k x all digits, B in boxes of 32 rows.
+struct DigitMaps {
+    CUtensorMap a[4], b;
+};
+bool digit_maps(DigitMaps& m, const DigitStack& a, const DigitStack& b, std::string& err);
+
+// Where a product goes: rows through a row table (TcTile mode 1), columns
+// through column tables (mode 2), or C = alpha A B + beta C with strides
+// (mode 0: a
+// single product whose tiles need no table).
+struct DigitOut {
+    double* out;
+    const int64_t* rowtab;
+    const int64_t* colbase;
+    const int32_t* colstride;
+    int64_t c_rs, c_cs;
+    double alpha, beta;
+    int m, n, k;  // mode 0: the product's size (its operands' stacks have m and n rows a chunk)
+};
+
+// Once per process and device before the first launch.
+cudaError_t digit_setup();
+// Runs the tiles' products on at most `sms` SMs.  Nothing is written once
+// *redo is non-zero (an operand row held an infinity or a NaN); a bounded
+// wait that ran out sets it too.  Whoever launches this computes the product
+// in another way when it ends up non-zero.
+cudaError_t launch_digit_gemm(int mode, const TcTile* tiles, int n_tiles, const DigitMaps& maps, const int32_t* exa,
+                              const int32_t* exb, const DigitOut& out, int* redo, int sms, cudaStream_t s);
+
+// Digits of FP64 operand stacks (rows of 64 doubles per chunk).
+cudaError_t launch_digit_rows(const DigitRows* jobs, int n_jobs, const double* q64, const DigitStack& out, int* redo,
+                              cudaStream_t s);
+// Digits of both operands of a dense product (*redo is set for operands that
+// one grid per row would hold less exactly than FP64): row r, k of K at
+// x[r * rs + k * ks], into stacks whose chunks are `rows` rows apart.
+struct DigitMatrix {
+    const double* x;
+    int64_t rs, ks;
+    int rows;
+    DigitStack out;
+    float* square;  // a scratch value per row
+};
+cudaError_t launch_digit_matrices(const DigitMatrix& a, const DigitMatrix& b, int K, int* redo, cudaStream_t s);
+// Digits of the psi sub-blocks of TcSplitJob lists (jobs with a0 == 0 alone:
+// 32 columns of a sub-block each, all its rows).
+cudaError_t launch_digit_psi(const TcSplitJob* jobs, int n_jobs, const double* x, const DigitStack& out, int* redo,
+                             cudaStream_t s);
+
+}  // namespace tk

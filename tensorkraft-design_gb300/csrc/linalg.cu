@@ -12,12 +12,16 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
+#include "digit_gemm.cuh"
 #include "kernels.cuh"
 #include "tk_bsgemm.hpp"
 #include "tk_internal.hpp"
@@ -75,6 +79,136 @@ struct Scratch {
 
 void tiles_for(GemmTable& g, int task) { bsgemm_tiles_for(g, task); }
 
+// A device buffer for one tk_gemm_f64 call.  The call waits for its stream
+// before it gives the buffer back, so any thread's next call on the context
+// may take it; at most kGemmKeep bytes stay with the context.
+constexpr size_t kGemmKeep = (size_t)1 << 30;
+struct GemmBuffer {
+    tk_ctx* ctx;
+    void* p = nullptr;
+    size_t n = 0;
+    GemmBuffer(tk_ctx* c, size_t bytes) : ctx(c) {
+        if (ctx) {
+            std::lock_guard<std::mutex> lock(ctx->gemm_mutex);
+            auto best = ctx->gemm_free.end();
+            for (auto it = ctx->gemm_free.begin(); it != ctx->gemm_free.end(); ++it)
+                if (it->second >= bytes && (best == ctx->gemm_free.end() || it->second < best->second)) best = it;
+            if (best != ctx->gemm_free.end()) {
+                p = best->first;
+                n = best->second;
+                ctx->gemm_free.erase(best);
+                return;
+            }
+        }
+        if (cudaMalloc(&p, bytes) != cudaSuccess) {
+            cudaGetLastError();  // the caller takes another path
+            p = nullptr;
+        }
+        n = bytes;
+    }
+    ~GemmBuffer() {
+        if (!p) return;
+        if (ctx) {
+            std::lock_guard<std::mutex> lock(ctx->gemm_mutex);
+            size_t kept = n;
+            for (auto& b : ctx->gemm_free) kept += b.second;
+            try {
+                // the smaller ones make room: the largest serves every call
+                std::sort(ctx->gemm_free.begin(), ctx->gemm_free.end(),
+                          [](const auto& a, const auto& b) { return a.second < b.second; });
+                while (kept > kGemmKeep && !ctx->gemm_free.empty() && ctx->gemm_free.front().second < n) {
+                    kept -= ctx->gemm_free.front().second;
+                    cudaFree(ctx->gemm_free.front().first);
+                    ctx->gemm_free.erase(ctx->gemm_free.begin());
+                }
+                if (kept <= kGemmKeep) {
+                    ctx->gemm_free.push_back({p, n});
+                    return;
+                }
+            } catch (const std::bad_alloc&) {
+            }
+        }
+        cudaFree(p);
+    }
+};
+
+// The dense product on the fp16 tensor cores (digit_gemm.cu).  *done is left
+// false where the FP64 kernel is to run instead: operands that one grid per
+// row would hold less exactly, and no memory for the digits.
+tk_status gemm_digits(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* b, double beta, tk_mat_mut* c,
+                      cudaStream_t s, bool* done) {
+    *done = false;
+    const int64_t M = a->rows, N = b->cols, K = a->cols, kch = (K + kTcBK - 1) / kTcBK;
+    DigitMatrix A{a->data, a->row_stride, a->col_stride, (int)M, {}, nullptr};
+    DigitMatrix B{b->data, b->col_stride, b->row_stride, (int)N, {}, nullptr};
+    A.out.rows = M * kch;
+    B.out.rows = N * kch;
+    size_t total = 256;
+    auto take = [&](size_t n) {
+        const size_t at = total;
+        total += (n + 255) & ~(size_t)255;
+        return at;
+    };
+    const size_t qa = take(digit_stack_bytes(A.out.rows)), qb = take(digit_stack_bytes(B.out.rows));
+    const size_t ea = take(sizeof(int32_t) * M), eb = take(sizeof(int32_t) * N);
+    const size_t sa = take(sizeof(float) * M), sb = take(sizeof(float) * N);
+    GemmBuffer buf(ctx, total);
+    if (!buf.p) return TK_OK;
+    unsigned char* p = static_cast<unsigned char*>(buf.p);
+    int* redo = reinterpret_cast<int*>(p);
+    A.out.q = reinterpret_cast<__half*>(p + qa);
+    B.out.q = reinterpret_cast<__half*>(p + qb);
+    A.out.ex = reinterpret_cast<int32_t*>(p + ea);
+    B.out.ex = reinterpret_cast<int32_t*>(p + eb);
+    A.square = reinterpret_cast<float*>(p + sa);
+    B.square = reinterpret_cast<float*>(p + sb);
+    DigitMaps maps;
+    std::string err;
+    if (!digit_maps(maps, A.out, B.out, err)) {
+        set_error("tk_gemm_f64: " + err);
+        return TK_ERR_CUDA;
+    }
+    DigitOut o{};
+    o.out = c->data;
+    o.c_rs = c->row_stride;
+    o.c_cs = c->col_stride;
+    o.alpha = alpha;
+    o.beta = beta;
+    o.m = (int)M;
+    o.n = (int)N;
+    o.k = (int)K;
+    const int64_t tiles = ((M + kTcBM - 1) / kTcBM) * ((N + kTcBN - 1) / kTcBN);
+    int state = 0;
+    cudaError_t e = digit_setup();
+    if (e == cudaSuccess) e = cudaMemsetAsync(redo, 0, sizeof(int), s);
+    if (e == cudaSuccess) e = launch_digit_matrices(A, B, (int)K, redo, s);
+    if (e == cudaSuccess) e = launch_digit_gemm(0, nullptr, (int)tiles, maps, A.out.ex, B.out.ex, o, redo, 152, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&state, redo, sizeof(int), cudaMemcpyDeviceToHost, s);
+    // the buffer goes back when the stream is done with it, whatever failed
+    const cudaError_t w = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = w;
+    if (e != cudaSuccess) return fail("tk_gemm_f64", e);
+    if (state == kDigitWait && beta != 0.0) {  // part of C is written: it cannot be computed again
+        set_error("tk_gemm_f64: a bounded wait of the tensor-core kernel ran out");
+        return TK_ERR_TIMEOUT;
+    }
+    *done = state == 0;
+    return TK_OK;
+}
+
+// The faster of the two kernels for a product.  The digits cost 45 us however
+// small it is (128^3: 33 us against 15 for the FP64 kernel, 256^3: 40 against
+// 42), then 4 us for 64 k of as many 128 x 64 tiles as there are SMs and 6 us
+// for the tiles' ends (100 x 100 x 2000: 145 us against 158); the FP64 kernel
+// runs near its pipe's 1.2 TFLOP/s when it is large (2048^3: 15 ms against
+// 0.56 ms).  Digits of more than 2 GB are not laid out.
+bool gemm_on_digits(int64_t M, int64_t N, int64_t K) {
+    if (K <= 0 || (double)(M + N) * (K + kTcBK) * kDigits * 2.0 > 2147483648.0) return false;
+    const double tiles = (double)((M + kTcBM - 1) / kTcBM) * ((N + kTcBN - 1) / kTcBN);
+    const double waves = std::ceil(tiles / 152.0), kch = (double)((K + kTcBK - 1) / kTcBK);
+    return 45e-6 + waves * (6e-6 + 4e-6 * kch) < 2.0 * M * N * K / 1.2e12;
+}
+
 }  // namespace
 
 extern "C" {
@@ -98,6 +232,15 @@ tk_status tk_gemm_f64(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* 
         set_error("tk_gemm_f64: dimensions or strides exceed 32 bits");
         return TK_ERR_UNSUPPORTED;
     }
+    int dev = 0;
+    if (ctx) dev = ctx->device;
+    Guard gd(dev);
+    cudaStream_t s = (cudaStream_t)stream;
+    if (gemm_on_digits(a->rows, b->cols, a->cols)) {
+        bool done = false;
+        const tk_status st = gemm_digits(ctx, alpha, a, b, beta, c, s, &done);
+        if (st != TK_OK || done) return st;
+    }
     GemmTable g;
     GemmTask t{};
     t.M = (int32_t)a->rows;
@@ -118,15 +261,11 @@ tk_status tk_gemm_f64(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* 
     }
     g.tasks.push_back(t);
     tiles_for(g, 0);
-    int dev = 0;
-    if (ctx) dev = ctx->device;
-    Guard gd(dev);
     Scratch sc;
     GemmTask* dt; GemmSeg* ds; GemmTile* dl;
     CK(sc.put(g.tasks, &dt));
     CK(sc.put(g.segs, &ds));
     CK(sc.put(g.tiles, &dl));
-    cudaStream_t s = (cudaStream_t)stream;
     CK(launch_gemm_f64(dl, (int)g.tiles.size(), dt, ds, a->data, b->data, c->data, s));
     // The task tables are freed on return; finish the launch first.
     CK(cudaStreamSynchronize(s));

@@ -6,9 +6,11 @@
 #include <cstdint>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <new>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/tk_heff.h"
@@ -26,6 +28,9 @@ struct tk_ctx {
     void* host_stage = nullptr;
     size_t host_stage_bytes = 0;
     void* stream = nullptr;  // cudaStream_t
+    // device buffers of finished tk_gemm_f64 calls, for the next ones (linalg.cu)
+    std::mutex gemm_mutex;
+    std::vector<std::pair<void*, size_t>> gemm_free;
 };
 
 namespace tk {
