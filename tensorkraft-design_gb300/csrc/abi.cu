@@ -16,6 +16,7 @@
 #include <string>
 #include <vector>
 
+#include "digit_gemm.cuh"
 #include "kernels.cuh"
 #include "tc_gemm.cuh"
 #include "tk_internal.hpp"
@@ -207,6 +208,14 @@ tk_status tk_heff2_plan_footprint(const tk_env* env_l, const tk_env* env_r, cons
              8.0 * std::max<int64_t>(C.t1_total, 1) + 2.0 * (vb(C.tiles1) + vb(C.tiles3)) + vb(C.jobs) +
              vb(C.terms) + 8.0 * C.terms.size() + vb(C.yrow) + vb(C.t1col_base) + vb(C.t1col_stride) + vb(C.xsrc) +
              vb(C.xstride);
+        if (f64stack_on_digits(C)) {
+            // the same stacks and a psi copy as digits, an exponent a row
+            double xrows = 0.0;
+            for (const std::vector<TcTile>* v : {&C.tiles1, &C.tiles1x})
+                for (const TcTile& t : *v)
+                    if (t.ldc == 0) xrows += (double)t.n_valid * t.kch;
+            b += (double)(digit_stack_bytes(1) + sizeof(int32_t)) * ((double)C.lq_rows + C.rq_rows + C.t2q_rows + xrows);
+        }
     }
     if (precision == TK_PREC_BF16X3) {
         const TcTables& C = H.tc;

@@ -464,21 +464,21 @@ __device__ __forceinline__ int row_exponent(uint32_t max_hi, int* redo) {
     if (e == 2047) atomicExch(redo, kDigitValue);
     return e > 0 ? e : 12 - __clz((int)(max_hi | 1));
 }
-// x on its row's grid, rounded to nearest, plus 128 in each of the six low
-// bytes: byte j is then digit 6 - j plus 128, the upper 16 bits digit 0.
-__device__ __forceinline__ uint64_t on_grid(double x, int ex) {
+// x 2^k on its row's grid, rounded to nearest, plus 128 in each of the six
+// low bytes: byte j is then digit 6 - j plus 128, the upper 16 bits digit 0.
+__device__ __forceinline__ uint64_t on_grid(double x, int ex, int k = 0) {
     const uint64_t b = (uint64_t)__double_as_longlong(x);
     const int e = (int)(b >> 52) & 0x7FF;
     uint64_t m = (b & 0xFFFFFFFFFFFFFull) << 4;
     if (e) m |= 1ull << 56;
-    const int s = min(ex - max(e, 1), 62);
+    const int s = min(ex - max(e, 1) - k, 62);
     m = s >= 0 ? (m + ((1ull << s) >> 1)) >> s : m << -s;
     if ((int64_t)b < 0) m = 0 - m;
     return m + 0x0000808080808080ull;
 }
 // The digits of two neighbouring elements, as pairs of fp16.
-__device__ __forceinline__ void digits2(double x, double y, int ex, uint32_t* d) {
-    const uint64_t a = on_grid(x, ex), b = on_grid(y, ex);
+__device__ __forceinline__ void digits2(double x, double y, int ex, uint32_t* d, int kx = 0, int ky = 0) {
+    const uint64_t a = on_grid(x, ex, kx), b = on_grid(y, ex, ky);
     const uint32_t al = (uint32_t)a, ah = (uint32_t)(a >> 32), bl = (uint32_t)b, bh = (uint32_t)(b >> 32);
     // 0x6400 | n is fp16 1024 + n
     auto half_of = [](uint32_t v, uint32_t bias) {
@@ -503,45 +503,82 @@ __device__ __forceinline__ void put_digits(const DigitStack& o, int64_t row, int
     for (int j = 0; j < kDigits; ++j) p[j * (o.rows << 5)] = d[j];
 }
 
+// Exponent of x 2^k (below 1 for subnormals), kNoExponent for zero.
+constexpr int kNoExponent = -(1 << 20);
+__device__ __forceinline__ int exponent_of(double x, int k) {
+    const uint32_t hi = abs_hi(x);
+    const int e = (int)(hi >> 20);
+    const bool zero = (hi | (uint32_t)__double2loint(x)) == 0;
+    return zero ? kNoExponent : (e > 0 ? e : 12 - __clz((int)(hi | 1))) + k;
+}
+
+// One CTA per 64-wide chunk of a stack: the columns' exponents.
+__global__ void __launch_bounds__(256) digit_columns_kernel(const DigitRows* __restrict__ jobs,
+                                                            const double* __restrict__ q64, int32_t* __restrict__ kx) {
+    __shared__ uint32_t top[4][kTcBK];
+    const DigitRows j = jobs[blockIdx.x];
+    const int k = threadIdx.x & 63, w = threadIdx.x >> 6;
+    for (int c = 0; c < j.kch; ++c) {
+        uint32_t mx = 0;
+        for (int r = w; r < j.n; r += 4) mx = max(mx, abs_hi(q64[(((int64_t)j.row + (int64_t)c * j.cs + r) << 6) + k]));
+        top[w][k] = mx;
+        __syncthreads();
+        if (w == 0) {
+            mx = max(max(top[0][k], top[1][k]), max(top[2][k], top[3][k]));
+            kx[j.kx + c * kTcBK + k] = mx >> 20 ? (int)(mx >> 20) - 1023 : 0;
+        }
+        __syncthreads();
+    }
+}
+
 // One warp per row of an FP64 stack (K-major 64-wide chunks): the row's
 // largest exponent, then its digits; the first kKeep chunks stay in registers
 // in between, the others are read again (from L1 or L2).
-constexpr int kKeep = 4;
+constexpr int kKeep = 3;
 __global__ void __launch_bounds__(32 * kDigitRowsPerCta) digit_rows_kernel(const DigitRows* __restrict__ jobs,
                                                                            const double* __restrict__ q64,
+                                                                           const int32_t* __restrict__ kx, int sign,
                                                                            const DigitStack out, int* redo) {
     const DigitRows j = jobs[blockIdx.x];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (w >= j.n) return;
     const int64_t row = (int64_t)j.row + w;
     auto at = [&](int c) { return reinterpret_cast<const double2*>(q64 + ((row + (int64_t)c * j.cs) << 6))[lane]; };
+    auto scale = [&](int c) {
+        if (j.kx < 0) return make_int2(0, 0);
+        const int2 k = reinterpret_cast<const int2*>(kx + j.kx + c * kTcBK)[lane];
+        return make_int2(sign * k.x, sign * k.y);
+    };
     double2 v[kKeep];
-    uint32_t mx = 0;
-#pragma unroll
-    for (int c = 0; c < kKeep; ++c) {
-        v[c] = c < j.kch ? at(c) : make_double2(0.0, 0.0);
-        mx = max(mx, max(abs_hi(v[c].x), abs_hi(v[c].y)));
-    }
-#pragma unroll 4
-    for (int c = kKeep; c < j.kch; ++c) {
-        const double2 u = at(c);
-        mx = max(mx, max(abs_hi(u.x), abs_hi(u.y)));
-    }
-    const int ex = row_exponent(__reduce_max_sync(0xffffffffu, mx), redo);
-    if (lane == 0) out.ex[row] = ex;
-    uint32_t d[kDigits];
+    int mx = kNoExponent;
+    uint32_t hi = 0;
+    auto top = [&](const double2& u, const int2& k) {
+        hi = max(hi, max(abs_hi(u.x), abs_hi(u.y)));
+        mx = max(mx, max(exponent_of(u.x, k.x), exponent_of(u.y, k.y)));
+    };
 #pragma unroll
     for (int c = 0; c < kKeep; ++c)
         if (c < j.kch) {
-            digits2(v[c].x, v[c].y, ex, d);
-            put_digits(out, row + (int64_t)c * j.cs, 2 * lane, d);
+            v[c] = at(c);
+            top(v[c], scale(c));
         }
-#pragma unroll 2
-    for (int c = kKeep; c < j.kch; ++c) {
-        const double2 u = at(c);
-        digits2(u.x, u.y, ex, d);
+#pragma unroll 4
+    for (int c = kKeep; c < j.kch; ++c) top(at(c), scale(c));
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (hi >= 0x7FF00000u) atomicExch(redo, kDigitValue);
+    const int ex = mx == kNoExponent ? 1 : mx;
+    if (lane == 0) out.ex[row] = ex;
+    auto put = [&](int c, const double2& u) {
+        const int2 k = scale(c);
+        uint32_t d[kDigits];
+        digits2(u.x, u.y, ex, d, k.x, k.y);
         put_digits(out, row + (int64_t)c * j.cs, 2 * lane, d);
-    }
+    };
+#pragma unroll
+    for (int c = 0; c < kKeep; ++c)
+        if (c < j.kch) put(c, v[c]);
+#pragma unroll 2
+    for (int c = kKeep; c < j.kch; ++c) put(c, at(c));
 }
 
 // psi sub-blocks: 32 columns x all K rows by one CTA, lanes along the columns;
@@ -698,10 +735,16 @@ cudaError_t launch_digit_gemm(int mode, const TcTile* tiles, int n_tiles, const 
     return cudaGetLastError();
 }
 
-cudaError_t launch_digit_rows(const DigitRows* jobs, int n_jobs, const double* q64, const DigitStack& out, int* redo,
-                              cudaStream_t s) {
+cudaError_t launch_digit_columns(const DigitRows* jobs, int n_jobs, const double* q64, int32_t* kx, cudaStream_t s) {
     if (n_jobs <= 0) return cudaSuccess;
-    digit_rows_kernel<<<n_jobs, 32 * kDigitRowsPerCta, 0, s>>>(jobs, q64, out, redo);
+    digit_columns_kernel<<<n_jobs, 256, 0, s>>>(jobs, q64, kx);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_digit_rows(const DigitRows* jobs, int n_jobs, const double* q64, const int32_t* kx, int sign,
+                              const DigitStack& out, int* redo, cudaStream_t s) {
+    if (n_jobs <= 0) return cudaSuccess;
+    digit_rows_kernel<<<n_jobs, 32 * kDigitRowsPerCta, 0, s>>>(jobs, q64, kx, sign, out, redo);
     return cudaGetLastError();
 }
 

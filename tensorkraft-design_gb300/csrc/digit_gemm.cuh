@@ -28,9 +28,10 @@ struct DigitStack {
 };
 inline size_t digit_stack_bytes(int64_t rows) { return (size_t)rows * kTcBK * kDigits * sizeof(__half); }
 
-// Rows [row, row + n) of a stack whose chunks are `cs` rows apart.
+// Rows [row, row + n) of a stack whose chunks are `cs` rows apart; `kx` >= 0:
+// the index of the power-of-two scales of its k (launch_digit_columns).
 struct DigitRows {
-    int32_t row, n, cs, kch;
+    int32_t row, n, cs, kch, kx, pad;
 };
 constexpr int kDigitRowsPerCta = 8;
 
@@ -64,9 +65,13 @@ cudaError_t digit_setup();
 cudaError_t launch_digit_gemm(int mode, const TcTile* tiles, int n_tiles, const DigitMaps& maps, const int32_t* exa,
                               const int32_t* exb, const DigitOut& out, int* redo, int sms, cudaStream_t s);
 
-// Digits of FP64 operand stacks (rows of 64 doubles per chunk).
-cudaError_t launch_digit_rows(const DigitRows* jobs, int n_jobs, const double* q64, const DigitStack& out, int* redo,
-                              cudaStream_t s);
+// Exponents of a stack's columns: kx[j.kx + k] = floor(log2 max |x|) over the
+// rows [row, row + n) of job j at k, 0 for a column of zeros.
+cudaError_t launch_digit_columns(const DigitRows* jobs, int n_jobs, const double* q64, int32_t* kx, cudaStream_t s);
+// Digits of FP64 operand stacks (rows of 64 doubles per chunk), of
+// x 2^(sign * kx) where the job has scales.
+cudaError_t launch_digit_rows(const DigitRows* jobs, int n_jobs, const double* q64, const int32_t* kx, int sign,
+                              const DigitStack& out, int* redo, cudaStream_t s);
 // Digits of both operands of a dense product (*redo is set for operands that
 // one grid per row would hold less exactly than FP64): row r, k of K at
 // x[r * rs + k * ks], into stacks whose chunks are `rows` rows apart.

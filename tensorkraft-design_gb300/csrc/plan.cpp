@@ -1340,8 +1340,8 @@ tk_status build_f64_stacks(Heff2Tables& T, std::string& err, const double* lbuf_
     }
     return guard_host("stacked FP64 tables", err, [&]() -> tk_status {
         TcOptions o;
-        o.tall_max_mtiles = 1 << 30;  // every stage-1 column read from psi through its table
-        o.fuse_max_ntiles = 0;        // every stage-3 stack reads a combined T2
+        o.tall_max_mtiles = 0;  // every stage-1 stack with the layout of a psi copy (the digit path's operand)
+        o.fuse_max_ntiles = 0;  // every stage-3 stack reads a combined T2
         TcTables C;
         tk_status st = build_tc_tables(T, *T.tcsrc, o, C, true, err, lbuf_im, rbuf_im);
         if (st == TK_OK && !validate_tc(T, C, err)) {

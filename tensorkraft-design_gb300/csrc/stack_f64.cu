@@ -29,13 +29,21 @@
 //   - pieces are cut so that each holds at most a share of the stage's
 //     FMAs, and go out longest first.
 // Every output sums its k in ascending order.
+//
+// Large real plans run the same stacks on the fp16 tensor cores instead
+// (digit_gemm.cu): digits of psi, T1 by digit products, the same combine,
+// digits of T2, y by digit products.  Hubbard D = 2048: 701 -> 184 us; cylinder
+// D = 2048: 40.9 -> 1.88 ms, relative error 2.6e-15 -> 1.5e-15.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
+#include <map>
+#include <memory>
 #include <set>
 #include <string>
 
+#include "digit_gemm.cuh"
 #include "tk_plan.cuh"
 
 namespace tk {
@@ -132,22 +140,26 @@ __device__ __forceinline__ void load_op_b(double (*S)[SBN + 1], const double* __
     }
 }
 
+// Shared memory of one piece.
+template <bool CPLX>
+struct PieceTiles {
+    double Ar[SBK][SBM + 1], Br[SBK][SBN + 1];
+    double Ai[CPLX ? SBK : 1][SBM + 1], Bi[CPLX ? SBK : 1][SBN + 1];
+};
+
 // Stage 1: T1 = L stacks * psi (CPLX: both complex, planar).
 template <bool CPLX>
-__global__ void __launch_bounds__(ST, 4) stack_gemm1_f64_kernel(const F64Piece* __restrict__ pieces,
-                                                                const KSeg* __restrict__ segs,
-                                                                const double* __restrict__ lq,
-                                                                const double* __restrict__ lq_im,
-                                                                const double* __restrict__ x,
-                                                                const double* __restrict__ x_im,
-                                                                const int64_t* __restrict__ xsrc,
-                                                                const int32_t* __restrict__ xstride,
-                                                                const int64_t* __restrict__ colbase,
-                                                                const int32_t* __restrict__ colstride,
-                                                                double* __restrict__ t1, double* __restrict__ t1_im) {
-    __shared__ double Ar[SBK][SBM + 1], Br[SBK][SBN + 1];
-    __shared__ double Ai[CPLX ? SBK : 1][SBM + 1], Bi[CPLX ? SBK : 1][SBN + 1];
-    const F64Piece t = pieces[blockIdx.x];
+__device__ __forceinline__ void stack_piece1(const F64Piece t, PieceTiles<CPLX>& sm, const KSeg* __restrict__ segs,
+                                             const double* __restrict__ lq, const double* __restrict__ lq_im,
+                                             const double* __restrict__ x, const double* __restrict__ x_im,
+                                             const int64_t* __restrict__ xsrc, const int32_t* __restrict__ xstride,
+                                             const int64_t* __restrict__ colbase,
+                                             const int32_t* __restrict__ colstride, double* __restrict__ t1,
+                                             double* __restrict__ t1_im) {
+    auto& Ar = sm.Ar;
+    auto& Br = sm.Br;
+    auto& Ai = sm.Ai;
+    auto& Bi = sm.Bi;
     const int tid = threadIdx.x;
     const int ln = tid & 63;  // the B column this thread loads
     const bool lv = ln < t.n_valid;
@@ -187,19 +199,33 @@ __global__ void __launch_bounds__(ST, 4) stack_gemm1_f64_kernel(const F64Piece* 
     }
 }
 
+template <bool CPLX>
+__global__ void __launch_bounds__(ST, 4) stack_gemm1_f64_kernel(const F64Piece* __restrict__ pieces,
+                                                                const KSeg* __restrict__ segs,
+                                                                const double* __restrict__ lq,
+                                                                const double* __restrict__ lq_im,
+                                                                const double* __restrict__ x,
+                                                                const double* __restrict__ x_im,
+                                                                const int64_t* __restrict__ xsrc,
+                                                                const int32_t* __restrict__ xstride,
+                                                                const int64_t* __restrict__ colbase,
+                                                                const int32_t* __restrict__ colstride,
+                                                                double* __restrict__ t1, double* __restrict__ t1_im) {
+    __shared__ PieceTiles<CPLX> sm;
+    stack_piece1<CPLX>(pieces[blockIdx.x], sm, segs, lq, lq_im, x, x_im, xsrc, xstride, colbase, colstride, t1, t1_im);
+}
+
 // Stage 3: y = T2 stacks * R stacks^T (CPLX: both complex, planar).
 template <bool CPLX>
-__global__ void __launch_bounds__(ST, 4) stack_gemm3_f64_kernel(const F64Piece* __restrict__ pieces,
-                                                                const KSeg* __restrict__ segs,
-                                                                const double* __restrict__ t2,
-                                                                const double* __restrict__ t2_im,
-                                                                const double* __restrict__ rq,
-                                                                const double* __restrict__ rq_im,
-                                                                const int64_t* __restrict__ yrow,
-                                                                double* __restrict__ y, double* __restrict__ y_im) {
-    __shared__ double Ar[SBK][SBM + 1], Br[SBK][SBN + 1];
-    __shared__ double Ai[CPLX ? SBK : 1][SBM + 1], Bi[CPLX ? SBK : 1][SBN + 1];
-    const F64Piece t = pieces[blockIdx.x];
+__device__ __forceinline__ void stack_piece3(const F64Piece t, PieceTiles<CPLX>& sm, const KSeg* __restrict__ segs,
+                                             const double* __restrict__ t2, const double* __restrict__ t2_im,
+                                             const double* __restrict__ rq, const double* __restrict__ rq_im,
+                                             const int64_t* __restrict__ yrow, double* __restrict__ y,
+                                             double* __restrict__ y_im) {
+    auto& Ar = sm.Ar;
+    auto& Br = sm.Br;
+    auto& Ai = sm.Ai;
+    auto& Bi = sm.Bi;
     const int tid = threadIdx.x;
     const DenseMap d(t.m_valid, t.n_valid, tid >> 5);
     double accr[RPT], acci[RPT];
@@ -232,14 +258,24 @@ __global__ void __launch_bounds__(ST, 4) stack_gemm3_f64_kernel(const F64Piece* 
     }
 }
 
+template <bool CPLX>
+__global__ void __launch_bounds__(ST, 4) stack_gemm3_f64_kernel(const F64Piece* __restrict__ pieces,
+                                                                const KSeg* __restrict__ segs,
+                                                                const double* __restrict__ t2,
+                                                                const double* __restrict__ t2_im,
+                                                                const double* __restrict__ rq,
+                                                                const double* __restrict__ rq_im,
+                                                                const int64_t* __restrict__ yrow,
+                                                                double* __restrict__ y, double* __restrict__ y_im) {
+    __shared__ PieceTiles<CPLX> sm;
+    stack_piece3<CPLX>(pieces[blockIdx.x], sm, segs, t2, t2_im, rq, rq_im, yrow, y, y_im);
+}
+
 // T2 = sum coef * T1 for one combine job (rows r0 .. r0 + rows of a slab),
 // written into the chunked stage-3 operand layout.
-__global__ void __launch_bounds__(128) stack_combine_f64_kernel(const TcCombJob* __restrict__ jobs,
-                                                                const TcCombTerm* __restrict__ terms,
-                                                                const double* __restrict__ coef,
-                                                                const double* __restrict__ t1,
-                                                                double* __restrict__ t2) {
-    const TcCombJob j = jobs[blockIdx.x];
+__device__ __forceinline__ void stack_combine_job(const TcCombJob& j, const TcCombTerm* __restrict__ terms,
+                                                  const double* __restrict__ coef, const double* __restrict__ t1,
+                                                  double* __restrict__ t2) {
     const int n = j.rows * j.cols;
     for (int e = threadIdx.x; e < n; e += blockDim.x) {
         const int rl = e / j.cols, c = e - rl * j.cols, r = j.r0 + rl;
@@ -249,6 +285,54 @@ __global__ void __launch_bounds__(128) stack_combine_f64_kernel(const TcCombJob*
         const int k = j.k0 + c;
         t2[(((int64_t)j.t2row + (int64_t)(k >> 6) * j.cstride + r) << 6) + (k & 63)] = acc;
     }
+}
+
+__global__ void __launch_bounds__(128) stack_combine_f64_kernel(const TcCombJob* __restrict__ jobs,
+                                                                const TcCombTerm* __restrict__ terms,
+                                                                const double* __restrict__ coef,
+                                                                const double* __restrict__ t1,
+                                                                double* __restrict__ t2) {
+    stack_combine_job(jobs[blockIdx.x], terms, coef, t1, t2);
+}
+
+// The whole FP64 matvec in one launch, after a digit matvec that could not
+// stand: *redo set by an operand with infinities or NaNs, or by a bounded wait
+// that ran out.  One cluster of eight CTAs, so that its stages can wait for one
+// another; otherwise it ends at once (launched behind every digit matvec).
+constexpr int kRedoCtas = 8;
+struct RedoArgs {
+    const F64Piece *pieces1, *pieces3;
+    const KSeg* segs;
+    const TcCombJob* jobs;
+    const TcCombTerm* terms;
+    const double *coef, *lq, *rq;
+    const int64_t *xsrc, *colbase, *yrow;
+    const int32_t *xstride, *colstride;
+    double *t1, *t2;
+    int n1, n3, njobs;
+};
+__device__ __forceinline__ void cluster_barrier() {
+    __threadfence();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__global__ void __cluster_dims__(kRedoCtas, 1, 1) __launch_bounds__(ST)
+    stack_redo_f64_kernel(const RedoArgs a, const double* __restrict__ x, double* __restrict__ y, int* redo) {
+    __shared__ PieceTiles<false> sm;
+    if (*(volatile int*)redo == 0) return;
+    for (int i = blockIdx.x; i < a.n1; i += kRedoCtas) {
+        __syncthreads();
+        stack_piece1<false>(a.pieces1[i], sm, a.segs, a.lq, nullptr, x, nullptr, a.xsrc, a.xstride, a.colbase,
+                            a.colstride, a.t1, nullptr);
+    }
+    cluster_barrier();
+    for (int i = blockIdx.x; i < a.njobs; i += kRedoCtas) stack_combine_job(a.jobs[i], a.terms, a.coef, a.t1, a.t2);
+    cluster_barrier();
+    for (int i = blockIdx.x; i < a.n3; i += kRedoCtas) {
+        __syncthreads();
+        stack_piece3<false>(a.pieces3[i], sm, a.segs, a.t2, nullptr, a.rq, nullptr, a.yrow, y, nullptr);
+    }
+    cluster_barrier();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *redo = 0;
 }
 
 double seg_len(const std::vector<KSeg>& segs, int32_t s0, int32_t n) {
@@ -368,7 +452,23 @@ bool stage3_pieces(const TcTables& C, std::vector<F64Piece>& out, std::vector<KS
 
 }  // namespace
 
+// The digit form of a stacked plan (digit_gemm.cu): the operand stacks as
+// digits, their tiles, and the rows to turn into digits on every matvec.
+struct F64Digits {
+    DevBuf<__half> lq, rq, t2, xq;
+    DevBuf<int32_t> lx, rx, tx, xx;  // exponents of their rows
+    DevBuf<int32_t> kx;              // scales of the R stacks' columns
+    DevBuf<TcTile> tiles1, tiles3;
+    DevBuf<TcSplitJob> psi;
+    DevBuf<DigitRows> rows;          // of T2
+    DevBuf<int> redo;
+    DigitMaps m1, m3;
+    int n1 = 0, n3 = 0, npsi = 0, nrows = 0, sms = 0;
+    DigitStack stack(const DevBuf<__half>& q, const DevBuf<int32_t>& x) const { return {q.p, x.p, (int64_t)x.n}; }
+};
+
 struct F64Stack {
+    std::unique_ptr<F64Digits> dg;  // null: the FP64 kernels run
     DevBuf<double> lq, rq, t1, t2, coef;
     DevBuf<double> lq_im, rq_im, t1_im, t2_im;  // complex environments only
     bool cplx = false;
@@ -384,12 +484,96 @@ struct F64Stack {
 
 void F64StackDeleter::operator()(F64Stack* p) const { delete p; }
 
+// The rows of a stack, kDigitRowsPerCta a job.
+static void digit_rows_of(std::vector<DigitRows>& out, int32_t row, int n, int32_t cs, int32_t kch, int32_t kx) {
+    for (int r = 0; r < n; r += kDigitRowsPerCta)
+        out.push_back({row + r, std::min(kDigitRowsPerCta, n - r), cs, kch, kx, 0});
+}
+
+// Whether a plan's FP64 matvec runs on digits: from 8 million multiply-adds in
+// stage 1.  Below, the FP64 kernels finish before the digit kernels' latencies
+// add up (Heisenberg D = 256, 3 million: 52 us against 59; Hubbard D = 512,
+// 3.6 million: 56 against 59; cylinder D = 128, 2 million: 60 against 73);
+// above, their pipe is the limit (Heisenberg D = 512, 25 million: 150 against
+// 75 us; Hubbard D = 1024, 25 million: 130 against 89; Hubbard D = 2048, 230
+// million: 701 against 184; cylinder D = 2048, 13 billion: 40.9 ms against 1.9).
+bool f64stack_on_digits(const TcTables& C) {
+    double f = 0.0;
+    for (const std::vector<TcTile>* v : {&C.tiles1, &C.tiles1x})
+        for (const TcTile& t : *v) f += (double)t.m_valid * t.n_valid * t.k_valid;
+    return f >= 8e6;
+}
+
+// Builds the digit form of p; left out (dg null) where the constant operands
+// hold infinities or NaNs.
+static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& err) {
+    std::unique_ptr<F64Digits> d(new F64Digits);
+    std::vector<DigitRows> lrows, rrows, trows, rcols;
+    std::vector<TcSplitJob> psi;
+    for (const TcSplitJob& j : C.split)
+        if (j.a0 == 0) psi.push_back(j);
+    std::set<int32_t> seen;
+    for (const TcTile& t : C.tiles1x)
+        if (seen.insert(t.a_row).second) digit_rows_of(lrows, t.a_row, t.m_valid, t.a_cs, t.kch, -1);
+    // stage 3: the columns of R on scales of their own, which T2 takes up, so
+    // that no channel's magnitude (an energy against an identity) costs the
+    // others digits
+    std::map<int32_t, int32_t> kx;  // stack (row of its first R row) -> scales
+    int32_t nk = 0;
+    for (const TcTile& t : C.tiles3) {
+        const int32_t base = t.b_row - t.n0;
+        if (kx.insert({base, nk}).second) {
+            rcols.push_back({base, t.b_cs, t.b_cs, t.kch, nk, 0});
+            nk += t.kch * kTcBK;
+        }
+        if (seen.insert(-1 - t.b_row).second) digit_rows_of(rrows, t.b_row, t.n_valid, t.b_cs, t.kch, kx[base]);
+        if (t.n0 == 0) digit_rows_of(trows, t.a_row, t.m_valid, t.a_cs, t.kch, kx[base]);
+    }
+    auto stack = [](DevBuf<__half>& q, DevBuf<int32_t>& x, int64_t rows) {
+        const size_t n = (size_t)std::max<int64_t>(rows, 1);
+        cudaError_t e = q.alloc(n * kTcBK * kDigits);
+        if (e == cudaSuccess) e = x.alloc(n);
+        if (e == cudaSuccess) e = cudaMemset(q.p, 0, sizeof(__half) * q.n);
+        if (e == cudaSuccess) e = cudaMemset(x.p, 0, sizeof(int32_t) * x.n);
+        return e;
+    };
+    DevBuf<DigitRows> dl, dr, dc;
+    cudaError_t e;
+    int redo = 0, dev = 0;
+    if ((e = stack(d->lq, d->lx, C.lq_rows)) != cudaSuccess || (e = stack(d->rq, d->rx, C.rq_rows)) != cudaSuccess ||
+        (e = stack(d->t2, d->tx, C.t2q_rows)) != cudaSuccess || (e = stack(d->xq, d->xx, C.xq_rows)) != cudaSuccess ||
+        (e = d->kx.alloc((size_t)std::max(nk, 1))) != cudaSuccess || (e = d->tiles1.upload(C.tiles1x)) != cudaSuccess ||
+        (e = d->tiles3.upload(C.tiles3)) != cudaSuccess || (e = d->psi.upload(psi)) != cudaSuccess ||
+        (e = d->rows.upload(trows)) != cudaSuccess || (e = d->redo.alloc(1)) != cudaSuccess ||
+        (e = cudaMemset(d->redo.p, 0, sizeof(int))) != cudaSuccess || (e = dl.upload(lrows)) != cudaSuccess ||
+        (e = dr.upload(rrows)) != cudaSuccess || (e = dc.upload(rcols)) != cudaSuccess || (e = digit_setup()) != cudaSuccess ||
+        (e = cudaGetDevice(&dev)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+        return e;
+    if (!digit_maps(d->m1, d->stack(d->lq, d->lx), d->stack(d->xq, d->xx), err) ||
+        !digit_maps(d->m3, d->stack(d->t2, d->tx), d->stack(d->rq, d->rx), err))
+        return cudaErrorInvalidValue;
+    if ((e = launch_digit_rows(dl.p, (int)lrows.size(), p.lq.p, nullptr, 1, d->stack(d->lq, d->lx), d->redo.p, 0)) !=
+            cudaSuccess ||
+        (e = launch_digit_columns(dc.p, (int)rcols.size(), p.rq.p, d->kx.p, 0)) != cudaSuccess ||
+        (e = launch_digit_rows(dr.p, (int)rrows.size(), p.rq.p, d->kx.p, -1, d->stack(d->rq, d->rx), d->redo.p, 0)) !=
+            cudaSuccess ||
+        (e = cudaMemcpy(&redo, d->redo.p, sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess)
+        return e;
+    d->n1 = (int)C.tiles1x.size();
+    d->n3 = (int)C.tiles3.size();
+    d->npsi = (int)psi.size();
+    d->nrows = (int)trows.size();
+    if (redo == 0) p.dg = std::move(d);
+    return cudaSuccess;
+}
+
 tk_status f64stack_create(const TcTables& C, std::unique_ptr<F64Stack, F64StackDeleter>& out, std::string& err) {
-    if (!C.tiles1x.empty() || !C.tiles3f.empty()) {
-        err = "stacked FP64 tables with split-copy or fused tiles";
+    if (!C.tiles1.empty() || !C.tiles3f.empty()) {
+        err = "stacked FP64 tables without a psi copy's layout, or with fused tiles";
         return TK_ERR_INVALID_ARG;
     }
-    for (const std::vector<TcTile>* v : {&C.tiles1, &C.tiles3})
+    for (const std::vector<TcTile>* v : {&C.tiles1x, &C.tiles3})
         for (const TcTile& t : *v)
             if (t.m_valid <= 0 || t.m_valid > kTcBM || t.n_valid <= 0 || t.n_valid > SBN) {
                 err = "stacked FP64 tile shape";
@@ -397,7 +581,7 @@ tk_status f64stack_create(const TcTables& C, std::unique_ptr<F64Stack, F64StackD
             }
     std::vector<KSeg> segs;
     std::vector<F64Piece> p1, p3;
-    stage1_pieces(C.tiles1, p1, segs);
+    stage1_pieces(C.tiles1x, p1, segs);
     if (!stage3_pieces(C, p3, segs, err)) return TK_ERR_INVALID_ARG;
     std::unique_ptr<F64Stack, F64StackDeleter> p(new F64Stack);
     cudaError_t e = cudaSuccess;
@@ -446,11 +630,42 @@ tk_status f64stack_create(const TcTables& C, std::unique_ptr<F64Stack, F64StackD
     p->n1 = (int)p1.size();
     p->n3 = (int)p3.size();
     p->njobs = (int)C.jobs.size();
+    if (!p->cplx && f64stack_on_digits(C) && (e = digits_create(C, *p, err)) != cudaSuccess) {
+        if (err.empty()) err = std::string("digit operands: ") + cudaGetErrorString(e);
+        return e == cudaErrorMemoryAllocation ? TK_ERR_OOM : TK_ERR_CUDA;
+    }
     out = std::move(p);
     return TK_OK;
 }
 
+// One stage of the digit matvec.
+static cudaError_t digits_stage(F64Stack& p, const double* x, double* y, cudaStream_t s, int stage) {
+    F64Digits& d = *p.dg;
+    cudaError_t e;
+    DigitOut o{};
+    if (stage == 0) {
+        if ((e = launch_digit_psi(d.psi.p, d.npsi, x, d.stack(d.xq, d.xx), d.redo.p, s)) != cudaSuccess) return e;
+        o.out = p.t1.p;
+        o.colbase = p.colbase.p;
+        o.colstride = p.colstride.p;
+        return launch_digit_gemm(2, d.tiles1.p, d.n1, d.m1, d.lx.p, d.xx.p, o, d.redo.p, d.sms, s);
+    }
+    if (stage == 1) {
+        if (p.njobs > 0) stack_combine_f64_kernel<<<p.njobs, 128, 0, s>>>(p.jobs.p, p.terms.p, p.coef.p, p.t1.p, p.t2.p);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        return launch_digit_rows(d.rows.p, d.nrows, p.t2.p, d.kx.p, 1, d.stack(d.t2, d.tx), d.redo.p, s);
+    }
+    o.out = y;
+    o.rowtab = p.yrow.p;
+    if ((e = launch_digit_gemm(1, d.tiles3.p, d.n3, d.m3, d.tx.p, d.rx.p, o, d.redo.p, d.sms, s)) != cudaSuccess) return e;
+    const RedoArgs a{p.pieces1.p, p.pieces3.p, p.segs.p, p.jobs.p, p.terms.p, p.coef.p,     p.lq.p, p.rq.p, p.xsrc.p,
+                     p.colbase.p, p.yrow.p,    p.xstride.p, p.colstride.p, p.t1.p, p.t2.p, p.n1,   p.n3,   p.njobs};
+    stack_redo_f64_kernel<<<kRedoCtas, ST, 0, s>>>(a, x, y, d.redo.p);
+    return cudaGetLastError();
+}
+
 cudaError_t f64stack_stage(F64Stack& p, const double* x, double* y, cudaStream_t s, int stage) {
+    if (p.dg) return digits_stage(p, x, y, s, stage);
     if (stage == 0 && p.n1 > 0)
         stack_gemm1_f64_kernel<false><<<p.n1, ST, 0, s>>>(p.pieces1.p, p.segs.p, p.lq.p, nullptr, x, nullptr,
                                                           p.xsrc.p, p.xstride.p, p.colbase.p, p.colstride.p, p.t1.p,
@@ -488,7 +703,10 @@ cudaError_t f64stack_apply_complex(F64Stack& p, const double* xr, const double* 
     return cudaGetLastError();
 }
 
-int f64stack_launches(const F64Stack& p) { return (p.n1 > 0) + (p.njobs > 0) + (p.n3 > 0); }
+int f64stack_launches(const F64Stack& p) {
+    const int n = (p.n1 > 0) + (p.njobs > 0) + (p.n3 > 0);
+    return p.dg ? n + (p.dg->npsi > 0) + (p.dg->nrows > 0) + 1 : n;
+}
 
 void f64stack_bytes(const F64Stack& p, double out[3]) {
     for (int i = 0; i < 3; ++i) out[i] = p.bytes[i];
