@@ -100,16 +100,6 @@ __global__ void reduce_partial_kernel(const double* __restrict__ partial, double
     }
 }
 
-// w[i] -= sum_j c[j] V_j[i]
-__global__ void gemv_sub_kernel(const double* __restrict__ V, int64_t ldv, int m, const double* __restrict__ c,
-                                double* __restrict__ w, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double s = w[i];
-        for (int j = 0; j < m; ++j) s = fma(-c[j], V[(int64_t)j * ldv + i], s);
-        w[i] = s;
-    }
-}
-
 // x[i] = sum_j z[j] V_j[i]
 __global__ void gemv_kernel(const double* __restrict__ V, int64_t ldv, int m, const double* __restrict__ z,
                             double* __restrict__ x, int64_t n) {
@@ -117,18 +107,6 @@ __global__ void gemv_kernel(const double* __restrict__ V, int64_t ldv, int m, co
         double s = 0.0;
         for (int j = 0; j < m; ++j) s = fma(z[j], V[(int64_t)j * ldv + i], s);
         x[i] = s;
-    }
-}
-
-// w -= a*x + b*y with a, b read from device memory (b may be null).
-__global__ void axpy2_kernel(double* __restrict__ w, const double* __restrict__ x, const double* pa,
-                             const double* __restrict__ y, const double* pb, int64_t n) {
-    const double a = *pa;
-    const double b = pb ? *pb : 0.0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double s = fma(-a, x[i], w[i]);
-        if (pb) s = fma(-b, y[i], s);
-        w[i] = s;
     }
 }
 
@@ -147,16 +125,290 @@ __global__ void axpby_kernel(double* __restrict__ y, const double* __restrict__ 
         y[i] = fma(a, x[i], b * y[i]);
 }
 
+// ---- one launch per orthogonalisation ---------------------------------------
+//
+// A step of the solvers below orthogonalises a new vector against its basis:
+// dot products, updates and a norm, each of which needs the sums before it.
+// Here one cooperative launch of at most one CTA per SM runs them all, with a
+// barrier of the grid where a sum is needed:
+//   ritz: x = sum c_j V_j, hx = sum c_j HV_j, r = hx - theta x, *rnorm = |r|,
+//     w = r, or DavidsonSolver's r / (theta - d) where
+//     |theta - d| > 1e-14 (eigensolver/mod.rs:427-437);
+//   three-term: *alpha = va . w, w -= alpha va + beta vb;
+//   `passes` times: c_j = V_j . w for all j < m, w -= sum c_j V_j;
+//   *norm = |w|, out = w / |w| (zeros below 1e-15);
+//   dots: dots[j] = V_j . w for all j < m.
+// |w| after a pass comes from the sums of that pass, |w|^2 = w . w - sum c_j^2,
+// unless the c_j took more than 2^-20 of it (then from a sum of its own), and
+// the residual's norm is summed with the first pass: one barrier a pass.
+// An element belongs to one thread from first to last.  Sums go through
+// partial[j * RG + region + block], the two regions in turn: a CTA may write its
+// next sums while others still read the last ones.  Every CTA adds the partial
+// sums in the same order, so all hold the same bits.
+// Bound by the FP64 pipe (two operations a clock and SM) for long vectors and
+// by the barriers' latencies for short ones; a block's sums go through shared
+// memory, 24 warp instructions a dot where shuffles from registers take 40 a
+// warp.  Measured: a Lanczos step's part at n = 398 thousand 23 us and 2.0 us a
+// basis vector (the pipe alone 1.4), 44 us on average over 20 steps, against 98
+// us as nine launches (dots and their sums apart); n = 61 thousand, two passes,
+// a Ritz pair and a norm: 31 us against 103 us as fifteen.
+struct OrthArgs {
+    int64_t n = 0, ldv = 0;
+    const double* V = nullptr;
+    int m = 0, passes = 0;
+    double* w = nullptr;
+    const double *va = nullptr, *vb = nullptr, *beta = nullptr;
+    double* alpha = nullptr;
+    const double *HV = nullptr, *c = nullptr, *diag = nullptr;  // HV: the ritz part is wanted
+    double theta = 0.0;
+    double *x = nullptr, *hx = nullptr, *r = nullptr, *rnorm = nullptr;
+    double *norm = nullptr, *out = nullptr, *dots = nullptr;
+    double* partial = nullptr;
+    unsigned* bar = nullptr;  // [0] arrivals, [1] CTAs done, [2] set when a wait ran out
+};
+constexpr int KT = 512;
+constexpr long kBarrierPolls = 1L << 22;
+
+// acc[j] = sum over i of V_j[i] w[i], j < MJ; with W also *ww = sum of w[i]^2.
+// MJ is exact: a multiply-add that is predicated off holds the FP64 pipe as long.
+template <int MJ, bool W>
+__device__ __forceinline__ void dot_chunk(const double* __restrict__ V, int64_t ldv, const double* w, int64_t first,
+                                          int64_t step, int64_t n, double* acc, double* ww) {
+#pragma unroll 2
+    for (int64_t i = first; i < n; i += step) {
+        const double wi = w[i];
+#pragma unroll
+        for (int j = 0; j < MJ; ++j) acc[j] = fma(V[(int64_t)j * ldv + i], wi, acc[j]);
+        if (W) *ww = fma(wi, wi, *ww);
+    }
+}
+template <bool W>
+__device__ __forceinline__ void dot_chunk_of(int mj, const double* V, int64_t ldv, const double* w, int64_t first,
+                                             int64_t step, int64_t n, double* acc, double* ww) {
+    switch (mj) {
+    case 1: dot_chunk<1, W>(V, ldv, w, first, step, n, acc, ww); break;
+    case 2: dot_chunk<2, W>(V, ldv, w, first, step, n, acc, ww); break;
+    case 3: dot_chunk<3, W>(V, ldv, w, first, step, n, acc, ww); break;
+    case 4: dot_chunk<4, W>(V, ldv, w, first, step, n, acc, ww); break;
+    case 5: dot_chunk<5, W>(V, ldv, w, first, step, n, acc, ww); break;
+    case 6: dot_chunk<6, W>(V, ldv, w, first, step, n, acc, ww); break;
+    case 7: dot_chunk<7, W>(V, ldv, w, first, step, n, acc, ww); break;
+    default: dot_chunk<8, W>(V, ldv, w, first, step, n, acc, ww); break;
+    }
+}
+
+// (Two CTAs fit an SM, so that two solvers on two streams can run at once.)
+__global__ void __launch_bounds__(KT, 2) orthogonalise_kernel(const OrthArgs a) {
+    extern __shared__ double sm[];
+    double* red = sm;                 // [MCH][KT]
+    double* coef = sm + MCH * KT;     // the sums of a phase
+    __shared__ int good;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int G = gridDim.x;
+    const int64_t first = (int64_t)blockIdx.x * KT + tid, step = (int64_t)G * KT;
+    int phase = 0;
+    if (tid == 0) good = 1;
+
+    // per-thread sums of mj <= MCH dots -> this block's partial sums j0 ..
+    auto put = [&](const double* acc, int j0, int mj) {
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < MCH; ++j)
+            if (j < mj) red[j * KT + tid] = acc[j];
+        __syncthreads();
+        if (warp < mj) {
+            double s[4] = {};
+#pragma unroll
+            for (int i = 0; i < KT / 32; ++i) s[i & 3] += red[warp * KT + lane + 32 * i];
+            double t = (s[0] + s[1]) + (s[2] + s[3]);
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+            if (lane == 0) a.partial[(int64_t)(j0 + warp) * RG + (phase & 1) * (RG / 2) + blockIdx.x] = t;
+        }
+    };
+    // the grid's sums of this phase into coef[0 .. k); false when a wait ran out
+    auto sums = [&](int k) -> bool {
+        __syncthreads();
+        ++phase;
+        if (G > 1) {
+            if (tid == 0) {
+                __threadfence();
+                atomicAdd(a.bar, 1u);
+                const unsigned want = (unsigned)(phase * G);
+                long i = 0;
+                unsigned seen;
+                do {
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.bar) : "memory");
+                } while (seen < want && ++i < kBarrierPolls);
+                if (seen < want) {
+                    good = 0;
+                    atomicExch(a.bar + 2, 1u);
+                }
+            }
+            __syncthreads();
+        }
+        if (!good) return false;
+        for (int j = warp; j < k; j += KT / 32) {
+            const double* p = a.partial + (int64_t)j * RG + ((phase - 1) & 1) * (RG / 2);
+            double s = 0.0;
+#pragma unroll
+            for (int i = 0; i < (RG / 2 + 31) / 32; ++i)
+                if (lane + 32 * i < G) s += __ldcg(p + lane + 32 * i);
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+            if (lane == 0) coef[j] = s;
+        }
+        __syncthreads();
+        return true;
+    };
+    const bool writer = blockIdx.x == 0 && tid == 0;
+
+    bool ok = true;
+    double rr = 0.0;
+    if (a.HV) {
+        for (int j = tid; j < a.m; j += KT) coef[j] = a.c[j];
+        __syncthreads();
+        for (int64_t i = first; i < a.n; i += step) {
+            double x = 0.0, h = 0.0;
+#pragma unroll 4
+            for (int j = 0; j < a.m; ++j) {
+                x = fma(coef[j], a.V[(int64_t)j * a.ldv + i], x);
+                h = fma(coef[j], a.HV[(int64_t)j * a.ldv + i], h);
+            }
+            const double r = fma(-a.theta, x, h);
+            a.x[i] = x;
+            a.hx[i] = h;
+            a.r[i] = r;
+            double t = r;
+            if (a.diag) {
+                const double den = a.theta - a.diag[i];
+                if (fabs(den) > 1e-14) t = r / den;
+            }
+            if (a.w) a.w[i] = t;
+            rr = fma(r, r, rr);
+        }
+        if (a.passes == 0) {
+            const double acc[MCH] = {rr};
+            put(acc, 0, 1);
+            ok = sums(1);
+            if (ok && writer) *a.rnorm = sqrt(fmax(coef[0], 0.0));
+        }
+    }
+    if (a.va) {
+        double acc[MCH] = {};
+        for (int64_t i = first; i < a.n; i += step) acc[0] = fma(a.va[i], a.w[i], acc[0]);
+        put(acc, 0, 1);
+        ok = sums(1);
+        if (ok) {
+            const double al = coef[0], be = a.vb ? *a.beta : 0.0;
+            if (writer) *a.alpha = al;
+            if (a.vb) {
+                for (int64_t i = first; i < a.n; i += step) a.w[i] = fma(-be, a.vb[i], fma(-al, a.va[i], a.w[i]));
+            } else {
+                for (int64_t i = first; i < a.n; i += step) a.w[i] = fma(-al, a.va[i], a.w[i]);
+            }
+        }
+    }
+    const int rounds = a.dots ? 1 : a.passes;
+    for (int pass = 0; pass < rounds && ok; ++pass) {
+        const bool last = pass + 1 == a.passes && a.norm;
+        double ww = 0.0;
+        for (int j0 = 0; j0 < a.m; j0 += MCH) {
+            const int mj = min(MCH, a.m - j0);
+            double acc[MCH] = {};
+            const double* v0 = a.V + (int64_t)j0 * a.ldv;
+            if (last && j0 == 0)
+                dot_chunk_of<true>(mj, v0, a.ldv, a.w, first, step, a.n, acc, &ww);
+            else
+                dot_chunk_of<false>(mj, v0, a.ldv, a.w, first, step, a.n, acc, &ww);
+            put(acc, j0, mj);
+        }
+        const bool res = a.HV && pass == 0;
+        if (last || res) {
+            const double acc[MCH] = {ww, rr};
+            put(acc, a.m, 2);
+        }
+        ok = sums(a.m + (last || res ? 2 : 0));
+        if (!ok) break;
+        if (res && writer) *a.rnorm = sqrt(fmax(coef[a.m + 1], 0.0));
+        if (a.dots) {
+            if (blockIdx.x == 0)
+                for (int j = tid; j < a.m; j += KT) a.dots[j] = coef[j];
+            break;
+        }
+        // the norm that the update will leave
+        double nv = 0.0, inv = 0.0;
+        bool known = false;
+        if (last) {
+            double cc = 0.0;
+            for (int j = 0; j < a.m; ++j) cc = fma(coef[j], coef[j], cc);
+            known = cc <= 0x1p-20 * coef[a.m];
+            nv = sqrt(fmax(coef[a.m] - cc, 0.0));
+            inv = nv < 1e-15 ? 0.0 : 1.0 / nv;
+        }
+        double nn = 0.0;
+        auto update = [&](int64_t i) {
+            double s = a.w[i];
+#pragma unroll 8
+            for (int j = 0; j < a.m; ++j) s = fma(-coef[j], a.V[(int64_t)j * a.ldv + i], s);
+            a.w[i] = s;
+            return s;
+        };
+        if (known && a.out) {
+            for (int64_t i = first; i < a.n; i += step) a.out[i] = update(i) * inv;
+        } else if (last && !known) {
+            for (int64_t i = first; i < a.n; i += step) {
+                const double s = update(i);
+                nn = fma(s, s, nn);
+            }
+        } else {
+            for (int64_t i = first; i < a.n; i += step) update(i);
+        }
+        if (!last) continue;
+        if (!known) {
+            const double acc[MCH] = {nn};
+            put(acc, 0, 1);
+            ok = sums(1);
+            if (!ok) break;
+            nv = sqrt(fmax(coef[0], 0.0));
+            inv = nv < 1e-15 ? 0.0 : 1.0 / nv;
+            if (a.out)
+                for (int64_t i = first; i < a.n; i += step) a.out[i] = a.w[i] * inv;
+        }
+        if (writer) *a.norm = nv;
+    }
+    // the last CTA leaves the counters as it found them
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        if (atomicAdd(a.bar + 1, 1u) == (unsigned)G - 1) {
+            a.bar[0] = 0;
+            a.bar[1] = 0;
+        }
+    }
+}
+
+cudaError_t launch_orthogonalise(OrthArgs a, cudaStream_t s) {
+    int dev = 0, sms = 0;
+    cudaError_t e;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+        return e;
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((a.n + KT - 1) / KT, std::min(sms, RG / 2)));
+    void* args[] = {&a};
+    return cudaLaunchCooperativeKernel((const void*)orthogonalise_kernel, dim3(grid), dim3(KT), args,
+                                       sizeof(double) * (MCH * KT + a.m + 2), s);
+}
+
 inline int vgrid(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 16)); }
 
 struct Ws {
     double* V;      // k+1 vectors of length n
     double* w;      // work vector
     double* scal;   // alpha[0..K), beta[K..2K), c[2K..3K+1), misc
-    double* part;   // RG * (K+1)
+    double* part;   // RG * (K+2)
     double* vec;    // x / r / CG vectors: 4 * n
     int64_t n;
     int K;
+    unsigned* bar;  // barrier words of orthogonalise_kernel
 };
 
 inline double* ALPHA(const Ws& s) { return s.scal; }
@@ -172,6 +424,43 @@ cudaError_t multidot(const Ws& ws, const double* V, int64_t ldv, int m, const do
     return cudaGetLastError();
 }
 
+// Step j of a Lanczos recurrence on ws.w = H V_j.
+OrthArgs three_term(const Ws& ws, int j, int passes, bool next) {
+    OrthArgs a;
+    a.n = a.ldv = ws.n;
+    a.V = ws.V;
+    a.m = j + 1;
+    a.passes = passes;
+    a.w = ws.w;
+    a.va = ws.V + (int64_t)j * ws.n;
+    a.alpha = ALPHA(ws) + j;
+    if (j > 0) {
+        a.vb = ws.V + (int64_t)(j - 1) * ws.n;
+        a.beta = BETA(ws) + (j - 1);
+    }
+    a.norm = BETA(ws) + j;
+    a.out = next ? ws.V + (int64_t)(j + 1) * ws.n : nullptr;
+    a.partial = ws.part;
+    a.bar = ws.bar;
+    return a;
+}
+
+// Zeroes the barrier words before a solver's first use of them.
+tk_status reset_barrier(const Ws& ws, cudaStream_t s) {
+    const cudaError_t e = cudaMemsetAsync(ws.bar, 0, 4 * sizeof(unsigned), s);
+    return e == cudaSuccess ? TK_OK : cuda_fail("barrier words", e);
+}
+// After a synchronisation: TK_ERR_TIMEOUT when a barrier's wait ran out.
+tk_status check_barrier(const Ws& ws, cudaStream_t s) {
+    unsigned late = 0;
+    cudaError_t e = cudaMemcpyAsync(&late, ws.bar + 2, sizeof(late), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return cuda_fail("barrier words", e);
+    if (late == 0) return TK_OK;
+    set_error("eigensolver: a bounded wait of the vector kernel ran out");
+    return TK_ERR_TIMEOUT;
+}
+
 // Enqueues k Lanczos steps starting from the normalised V_0 already in place.
 tk_status enqueue_steps(tk_heff2_plan* p, const Ws& ws, int k, int precision, cudaStream_t s) {
     const int64_t n = ws.n;
@@ -179,16 +468,9 @@ tk_status enqueue_steps(tk_heff2_plan* p, const Ws& ws, int k, int precision, cu
         double* vj = ws.V + (int64_t)j * n;
         tk_status st = tk_heff2_apply_prec(p, vj, ws.w, s, precision);
         if (st != TK_OK) return st;
-        cudaError_t e;
-        if ((e = multidot(ws, vj, n, 1, ws.w, ALPHA(ws) + j, 0, s)) != cudaSuccess) return cuda_fail("multidot", e);
-        axpy2_kernel<<<vgrid(n), 256, 0, s>>>(ws.w, vj, ALPHA(ws) + j, j > 0 ? ws.V + (int64_t)(j - 1) * n : nullptr,
-                                               j > 0 ? BETA(ws) + (j - 1) : nullptr, n);
         // full re-orthogonalisation against V_0..V_j (blocked classical Gram-Schmidt)
-        if ((e = multidot(ws, ws.V, n, j + 1, ws.w, COEF(ws), 0, s)) != cudaSuccess) return cuda_fail("multidot", e);
-        gemv_sub_kernel<<<vgrid(n), 256, 0, s>>>(ws.V, n, j + 1, COEF(ws), ws.w, n);
-        if ((e = multidot(ws, ws.w, n, 1, ws.w, BETA(ws) + j, 1, s)) != cudaSuccess) return cuda_fail("multidot", e);
-        if (j + 1 < k) normalize_kernel<<<vgrid(n), 256, 0, s>>>(ws.V + (int64_t)(j + 1) * n, ws.w, BETA(ws) + j, n);
-        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail("lanczos step", e);
+        const cudaError_t e = launch_orthogonalise(three_term(ws, j, 1, j + 1 < k), s);
+        if (e != cudaSuccess) return cuda_fail("lanczos step", e);
     }
     return TK_OK;
 }
@@ -519,16 +801,6 @@ double small_sym_lowest(const std::vector<double>& g, int m, int ld, std::vector
     return rq;
 }
 
-// DavidsonSolver's diagonal preconditioner (eigensolver/mod.rs:427-437):
-// t_i = r_i / (theta - d_i) where |theta - d_i| > 1e-14, else t_i = r_i.
-__global__ void precondition_kernel(double* __restrict__ t, const double* __restrict__ r,
-                                    const double* __restrict__ d, double theta, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double den = theta - d[i];
-        t[i] = fabs(den) > 1e-14 ? r[i] / den : r[i];
-    }
-}
-
 // Search space of the FP64 subspace solver: V (orthonormal directions), HV
 // (their FP64 images), host-visible scalars sc and reduction partials.
 struct Subspace {
@@ -584,8 +856,16 @@ tk_status subspace_solve(tk_heff2_plan* p, const Ws& ws, Subspace& sp, const Sub
         ++sp.fp64_matvecs;
     }
     auto add_column = [&](int j) -> tk_status {  // G[i][j] = G[j][i] = V_i . HV_j, i <= j
-        cudaError_t e2 = multidot(ws, sp.V, n, j + 1, sp.HV + (int64_t)j * n, sc, 0, s);
-        if (e2 != cudaSuccess) return cuda_fail("multidot", e2);
+        OrthArgs d;
+        d.n = d.ldv = n;
+        d.V = sp.V;
+        d.m = j + 1;
+        d.w = sp.HV + (int64_t)j * n;
+        d.dots = sc;
+        d.partial = ws.part;
+        d.bar = ws.bar;
+        cudaError_t e2 = launch_orthogonalise(d, s);
+        if (e2 != cudaSuccess) return cuda_fail("subspace step", e2);
         if ((e2 = cudaMemcpyAsync(col.data(), sc, sizeof(double) * (j + 1), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
             return cuda_fail("cudaMemcpyAsync", e2);
         if ((e2 = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_fail("subspace step", e2);
@@ -601,13 +881,39 @@ tk_status subspace_solve(tk_heff2_plan* p, const Ws& ws, Subspace& sp, const Sub
         theta = small_sym_lowest(G, m, M, cvec);
         if ((e = cudaMemcpyAsync(sc, cvec.data(), sizeof(double) * m, cudaMemcpyHostToDevice, s)) != cudaSuccess)
             return cuda_fail("cudaMemcpyAsync", e);
-        gemv_kernel<<<vgrid(n), 256, 0, s>>>(sp.V, n, m, sc, x, n);
-        gemv_kernel<<<vgrid(n), 256, 0, s>>>(sp.HV, n, m, sc, hx, n);
-        if ((e = cudaMemcpyAsync(r, hx, sizeof(double) * n, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
-            return cuda_fail("cudaMemcpyAsync", e);
-        axpby_kernel<<<vgrid(n), 256, 0, s>>>(r, x, -theta, 1.0, n);
-        if ((e = multidot(ws, r, n, 1, r, sc + M, 1, s)) != cudaSuccess) return cuda_fail("multidot", e);
-        if ((st = read_scalar(sc + M, rn, s)) != TK_OK) return st;
+        OrthArgs o;  // x, hx, r and, unless an inner solve makes the correction, the new direction
+        o.n = o.ldv = n;
+        o.V = sp.V;
+        o.HV = sp.HV;
+        o.m = m;
+        o.c = sc;
+        o.theta = theta;
+        o.x = x;
+        o.hx = hx;
+        o.r = r;
+        o.rnorm = sc + M + 1;
+        o.partial = ws.part;
+        o.bar = ws.bar;
+        auto with_direction = [&](OrthArgs v) {
+            v.w = t;
+            v.passes = 2;
+            v.norm = sc + M;
+            v.out = m < M ? sp.V + (int64_t)m * n : nullptr;
+            return v;
+        };
+        OrthArgs again = with_direction(o);  // the same for a vector already in t
+        again.HV = nullptr;
+        if (cfg.inner <= 0) {
+            o = with_direction(o);
+            o.diag = cfg.diag;
+        }
+        if ((e = launch_orthogonalise(o, s)) != cudaSuccess) return cuda_fail("subspace step", e);
+        double norms[2] = {0.0, 0.0};  // of the correction and of the residual
+        if ((e = cudaMemcpyAsync(norms, sc + M, sizeof(norms), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+            (e = cudaStreamSynchronize(s)) != cudaSuccess)
+            return cuda_fail("subspace step", e);
+        double cnorm = norms[0];
+        *rn = norms[1];
         *E = theta;
         if (*rn < cfg.tol) {
             *converged = true;
@@ -622,25 +928,18 @@ tk_status subspace_solve(tk_heff2_plan* p, const Ws& ws, Subspace& sp, const Sub
                                          s, &used)) != TK_OK)
                 return st;
             sp.matvecs += used;
-        } else if (cfg.diag) {
-            precondition_kernel<<<vgrid(n), 256, 0, s>>>(t, r, cfg.diag, theta, n);
-        } else if ((e = cudaMemcpyAsync(t, r, sizeof(double) * n, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) {
-            return cuda_fail("cudaMemcpyAsync", e);
-        }
-        double cnorm = 0.0;
-        for (int attempt = 0; attempt < 2; ++attempt) {
-            for (int pass = 0; pass < 2; ++pass) {
-                if ((e = multidot(ws, sp.V, n, m, t, sc, 0, s)) != cudaSuccess) return cuda_fail("multidot", e);
-                gemv_sub_kernel<<<vgrid(n), 256, 0, s>>>(sp.V, n, m, sc, t, n);
-            }
-            if ((e = multidot(ws, t, n, 1, t, sc + M, 1, s)) != cudaSuccess) return cuda_fail("multidot", e);
+            if ((e = launch_orthogonalise(again, s)) != cudaSuccess) return cuda_fail("subspace step", e);
             if ((st = read_scalar(sc + M, &cnorm, s)) != TK_OK) return st;
-            if (cnorm >= 1e-14 || attempt == 1) break;
+        }
+        if (!(cnorm >= 1e-14) && (cfg.inner > 0 || cfg.diag)) {
             // the correction collapsed into span(V): use the raw residual
             if ((e = cudaMemcpyAsync(t, r, sizeof(double) * n, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
                 return cuda_fail("cudaMemcpyAsync", e);
+            if ((e = launch_orthogonalise(again, s)) != cudaSuccess) return cuda_fail("subspace step", e);
+            if ((st = read_scalar(sc + M, &cnorm, s)) != TK_OK) return st;
         }
         if (cnorm < 1e-14) break;  // converged or stagnated
+        const double* placed = again.out;  // where the new direction already is
         if (m >= M) {
             if (m >= n) break;  // the space is complete
             if ((e = cudaMemcpyAsync(sp.V, x, sizeof(double) * n, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
@@ -660,7 +959,7 @@ tk_status subspace_solve(tk_heff2_plan* p, const Ws& ws, Subspace& sp, const Sub
             // t is orthogonal to the old span, which contains y: append it below
         }
         double* vm = sp.V + (int64_t)m * n;
-        normalize_kernel<<<vgrid(n), 256, 0, s>>>(vm, t, sc + M, n);
+        if (vm != placed) normalize_kernel<<<vgrid(n), 256, 0, s>>>(vm, t, sc + M, n);
         if ((st = tk_heff2_apply_prec(p, vm, sp.HV + (int64_t)m * n, s, TK_PREC_FP64)) != TK_OK) return st;
         ++sp.matvecs;
         ++sp.fp64_matvecs;
@@ -685,11 +984,12 @@ tk_status ensure_lanczos_ws(tk_heff2_plan* p, int k, int64_t n, Ws* ws) {
         if ((e = p->lz_basis.alloc((size_t)(kk + 1) * n)) != cudaSuccess) return cuda_fail("alloc basis", e);
         if ((e = p->lz_w.alloc((size_t)n)) != cudaSuccess) return cuda_fail("alloc w", e);
         if ((e = p->lz_scal.alloc((size_t)(4 * kk + 16))) != cudaSuccess) return cuda_fail("alloc scal", e);
-        if ((e = p->lz_part.alloc((size_t)RG * (kk + 1))) != cudaSuccess) return cuda_fail("alloc part", e);
+        if ((e = p->lz_part.alloc((size_t)RG * (kk + 2))) != cudaSuccess) return cuda_fail("alloc part", e);
         if ((e = p->lz_vec.alloc((size_t)4 * n)) != cudaSuccess) return cuda_fail("alloc vec", e);
         p->lz_cap_k = k;
     }
-    *ws = Ws{p->lz_basis.p, p->lz_w.p, p->lz_scal.p, p->lz_part.p, p->lz_vec.p, n, std::max(p->lz_cap_k, 2)};
+    if (!p->kry_bar.p && (e = p->kry_bar.alloc(4)) != cudaSuccess) return cuda_fail("alloc barrier words", e);
+    *ws = Ws{p->lz_basis.p, p->lz_w.p, p->lz_scal.p, p->lz_part.p, p->lz_vec.p, n, std::max(p->lz_cap_k, 2), p->kry_bar.p};
     return TK_OK;
 }
 
@@ -701,7 +1001,7 @@ tk_status ensure_subspace(tk_heff2_plan* p, int M, int64_t n, Ws* ws, Subspace* 
         if ((e = p->sub_v.alloc((size_t)M * n)) != cudaSuccess) return cuda_fail("alloc search space", e);
         if ((e = p->sub_hv.alloc((size_t)M * n)) != cudaSuccess) return cuda_fail("alloc search space", e);
         if ((e = p->sub_sc.alloc((size_t)M + 32)) != cudaSuccess) return cuda_fail("alloc search space", e);
-        if ((e = p->sub_part.alloc((size_t)RG * (M + 1))) != cudaSuccess) return cuda_fail("alloc search space", e);
+        if ((e = p->sub_part.alloc((size_t)RG * (M + 2))) != cudaSuccess) return cuda_fail("alloc search space", e);
         p->sub_cap = M;
     }
     ws->part = p->sub_part.p;
@@ -776,15 +1076,8 @@ tk_status expm_run(tk_heff2_plan* p, const Ws& ws, int nc, int64_t n, int m, dou
                 if ((st = tk_heff2_apply_prec(p, vj + h * n, ws.w + h * n, s, p->precision)) != TK_OK) return st;
             res->matvec_count += nc;
         }
-        if ((e = multidot(ws, vj, nn, 1, ws.w, ALPHA(ws) + j, 0, s)) != cudaSuccess) return cuda_fail("multidot", e);
-        axpy2_kernel<<<vgrid(nn), 256, 0, s>>>(ws.w, vj, ALPHA(ws) + j, j > 0 ? ws.V + (int64_t)(j - 1) * nn : nullptr,
-                                                j > 0 ? BETA(ws) + (j - 1) : nullptr, nn);
-        for (int pass = 0; pass < 2; ++pass) {
-            if ((e = multidot(ws, ws.V, nn, j + 1, ws.w, COEF(ws), 0, s)) != cudaSuccess) return cuda_fail("multidot", e);
-            gemv_sub_kernel<<<vgrid(nn), 256, 0, s>>>(ws.V, nn, j + 1, COEF(ws), ws.w, nn);
-        }
-        if ((e = multidot(ws, ws.w, nn, 1, ws.w, BETA(ws) + j, 1, s)) != cudaSuccess) return cuda_fail("multidot", e);
-        if (j + 1 < m) normalize_kernel<<<vgrid(nn), 256, 0, s>>>(ws.V + (int64_t)(j + 1) * nn, ws.w, BETA(ws) + j, nn);
+        if ((e = launch_orthogonalise(three_term(ws, j, 2, j + 1 < m), s)) != cudaSuccess)
+            return cuda_fail("krylov exponential step", e);
     }
     std::vector<double> ab(2 * (size_t)ws.K);
     if ((e = cudaMemcpyAsync(ab.data(), ws.scal, sizeof(double) * 2 * ws.K, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
@@ -865,15 +1158,18 @@ extern "C" tk_status tk_expm_krylov(tk_heff2_plan* p, const tk_expm_cfg* cfg, do
         if ((e = p->ex_w.alloc((size_t)nmax)) != cudaSuccess) return cuda_fail("alloc krylov", e);
         if ((e = p->ex_x2.alloc((size_t)nmax)) != cudaSuccess) return cuda_fail("alloc krylov", e);
         if ((e = p->ex_scal.alloc((size_t)(4 * (mm + 2) + 16))) != cudaSuccess) return cuda_fail("alloc krylov", e);
-        if ((e = p->ex_part.alloc((size_t)RG * (mm + 1))) != cudaSuccess) return cuda_fail("alloc krylov", e);
+        if ((e = p->ex_part.alloc((size_t)RG * (mm + 2))) != cudaSuccess) return cuda_fail("alloc krylov", e);
         p->ex_cap_m = mm;
         p->ex_cap_n = nmax;
     }
-    Ws ws{p->ex_basis.p, p->ex_w.p, p->ex_scal.p, p->ex_part.p, nullptr, nn, std::max(p->ex_cap_m, 2)};
-    tk_status st = expm_run(p, ws, nc, n, m, cfg->tol, alpha_re, alpha_im, v_re, v_im, out_re, out_im, p->ex_x2.p,
+    if (!p->kry_bar.p && (e = p->kry_bar.alloc(4)) != cudaSuccess) return cuda_fail("alloc barrier words", e);
+    Ws ws{p->ex_basis.p, p->ex_w.p, p->ex_scal.p, p->ex_part.p, nullptr, nn, std::max(p->ex_cap_m, 2), p->kry_bar.p};
+    tk_status st = reset_barrier(ws, s);
+    if (st != TK_OK) return st;
+    st = expm_run(p, ws, nc, n, m, cfg->tol, alpha_re, alpha_im, v_re, v_im, out_re, out_im, p->ex_x2.p,
                             res, s);
     if (st != TK_OK) return st;
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_fail("krylov exponential", e);
+    if ((st = check_barrier(ws, s)) != TK_OK) return st;
     if (p->tc && (st = tc_check_error(*p->tc, s)) != TK_OK) return st;
     return TK_OK;
 }
@@ -901,6 +1197,7 @@ extern "C" tk_status tk_lanczos_lowest(tk_heff2_plan* p, const tk_lanczos_cfg* c
     Ws ws;
     tk_status st = ensure_lanczos_ws(p, k, n, &ws);
     if (st != TK_OK) return st;
+    if ((st = reset_barrier(ws, s)) != TK_OK) return st;
     double* x = evec_dev;
     double* hx = ws.vec;
     double* r = ws.vec + n;
@@ -988,6 +1285,7 @@ extern "C" tk_status tk_lanczos_lowest(tk_heff2_plan* p, const tk_lanczos_cfg* c
         if (rn <= cfg->tol || restarts >= cfg->max_restarts) break;
         ++restarts;
     }
+    if ((st = check_barrier(ws, s)) != TK_OK) return st;
     if (p->tc && (st = tc_check_error(*p->tc, s)) != TK_OK) return st;
     out->eigenvalue = E;
     out->residual_norm = rn;
@@ -1024,6 +1322,7 @@ extern "C" tk_status tk_davidson_lowest(tk_heff2_plan* p, const tk_davidson_cfg*
     const int M = (int)std::min<int64_t>(cfg->max_subspace, n);
     Subspace sp;
     if ((st = ensure_subspace(p, M, n, &ws, &sp)) != TK_OK) return st;
+    if ((st = reset_barrier(ws, s)) != TK_OK) return st;
     double* x = evec_dev;
     if (x0_dev) {
         if (x0_dev != x && (e = cudaMemcpyAsync(x, x0_dev, sizeof(double) * n, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
@@ -1036,7 +1335,7 @@ extern "C" tk_status tk_davidson_lowest(tk_heff2_plan* p, const tk_davidson_cfg*
     double E = 0.0, rn = INFINITY;
     bool conv = false;
     if ((st = subspace_solve(p, ws, sp, sc, x, ws.vec, ws.vec + n, &E, &rn, &conv, s)) != TK_OK) return st;
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_fail("davidson", e);
+    if ((st = check_barrier(ws, s)) != TK_OK) return st;
     if (p->tc && (st = tc_check_error(*p->tc, s)) != TK_OK) return st;
     out->eigenvalue = E;
     out->residual_norm = rn;

@@ -151,6 +151,7 @@ struct tk_heff2_plan {
     int sub_cap = 0;
     // Krylov-exponential workspace (allocated on first use)
     tk::DevBuf<double> ex_basis, ex_w, ex_x2, ex_scal, ex_part;
+    tk::DevBuf<unsigned> kry_bar;  // barrier words of the solvers' vector kernel
     int ex_cap_m = 0;
     int64_t ex_cap_n = 0;
     int lz_cap_k = 0;
