@@ -38,6 +38,10 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
+#include <queue>
+#include <utility>
+#include <vector>
 
 #include "tk_plan.cuh"
 
@@ -58,6 +62,7 @@ constexpr int STORE_BYTES = 32 * ST_LD * 8;           // per drain warp
 constexpr int SMEM_BYTES = 1024 + kDigitRing * STAGE_BYTES + EPI_WARPS * STORE_BYTES + 256;
 constexpr int TMEM_ALLOC = 512, TMEM_HALF = 256;
 constexpr long WAIT_LIMIT = 1L << 24;
+
 constexpr int kExBias = 2110;  // 2 * 1022 + 114 - 48: V * 2^(exa + exb - kExBias)
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -220,7 +225,8 @@ __device__ __forceinline__ TcTile tile_of(const TcTile* __restrict__ tiles, cons
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* __restrict__ tiles, int n_tiles,
+__global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* __restrict__ tiles,
+                                                                 const int32_t* __restrict__ begin,
                                                                  const __grid_constant__ DigitMaps maps,
                                                                  const int32_t* __restrict__ exa,
                                                                  const int32_t* __restrict__ exb, const DigitOut om,
@@ -237,8 +243,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
     volatile int* stop = (volatile int*)(tslot + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+    dep_launch();
     if (threadIdx.x == 0) {
-        *stop = *(volatile int*)redo;  // an operand held an infinity or a NaN: another kernel computes this product
         for (int i = 0; i < kDigitRing; ++i) {
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 1);
@@ -256,18 +262,24 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    dep_wait();
+    if (threadIdx.x == 0) *stop = *(volatile int*)redo;  // an operand held an infinity or a NaN: another kernel computes this product
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tslot;
     const bool run = *stop == 0;  // written before the barrier; a wait can only run out after it
     __syncthreads();
+    // this CTA's tiles: a run of the table, or every gridDim.x-th of the C grid
+    const int t_begin = MODE == 0 ? (int)blockIdx.x : begin[blockIdx.x];
+    const int t_end = MODE == 0 ? om.tiles : begin[blockIdx.x + 1];
+    const int t_step = MODE == 0 ? (int)gridDim.x : 1;
 
     if (warp == EPI_WARPS) {
         if (lane == 0) {
             int it = 0;
             bool ok = run;
-            for (int ti = blockIdx.x; ti < n_tiles && ok; ti += gridDim.x) {
+            for (int ti = t_begin; ti < t_end && ok; ti += t_step) {
                 const TcTile t = tile_of<MODE>(tiles, om, ti);
                 const int halves = t.n_valid > HN ? 2 : 1;
                 const int box = (t.m_valid + 31) >> 5;
@@ -293,7 +305,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
             int it = 0, unit = 0;
             int drains[2] = {0, 0};
             bool ok = run;
-            for (int ti = blockIdx.x; ti < n_tiles && ok; ti += gridDim.x) {
+            for (int ti = t_begin; ti < t_end && ok; ti += t_step) {
                 const TcTile t = tile_of<MODE>(tiles, om, ti);
                 const int halves = t.n_valid > HN ? 2 : 1;
                 const uint32_t astep = (uint32_t)((((t.m_valid + 31) >> 5) * 32) * KW * 2);
@@ -340,7 +352,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
         double* sw = store + warp * (STORE_BYTES / 8);
         int drains = 0, unit = 0;
         bool ok = run;
-        for (int ti = blockIdx.x; ti < n_tiles && ok; ti += gridDim.x) {
+        for (int ti = t_begin; ti < t_end && ok; ti += t_step) {
             const TcTile t = tile_of<MODE>(tiles, om, ti);
             const int halves = t.n_valid > HN ? 2 : 1;
             const int h = (buf - unit) & 1;
@@ -348,6 +360,26 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
             if (h >= halves) continue;
             const int nc = min(WCOLS, t.n_valid - h * HN - col0);  // columns of this warp's that the tile has
             const bool mine = row0 < t.m_valid && nc > 0;
+            // what the stores will need, on its way while the sums are drained:
+            // exponents (a row of this thread, a column per lane), output offsets
+            const int cl = lane & (SCOLS - 1), r0 = lane / SCOLS;
+            int ea = 1, eb = 1;
+            int64_t place[WCOLS / SCOLS] = {}, rows = 0;
+            int32_t pitch[WCOLS / SCOLS] = {};
+            if (mine) {
+                if (row0 + lane < t.m_valid) {
+                    ea = exa[t.a_row + row0 + lane];
+                    if (MODE == 1) rows = om.rowtab[t.out_off + row0 + lane];
+                }
+                if (lane < nc) eb = exb[t.b_row + h * HN + col0 + lane];
+                if (MODE == 2)
+#pragma unroll
+                    for (int g = 0; g < WCOLS / SCOLS; ++g)
+                        if (g * SCOLS + cl < nc) {
+                            place[g] = om.colbase[t.out_off + h * HN + col0 + g * SCOLS + cl];
+                            pitch[g] = om.colstride[t.out_off + h * HN + col0 + g * SCOLS + cl];
+                        }
+            }
             Sum acc[WCOLS];
 #pragma unroll
             for (int i = 0; i < WCOLS; ++i) acc[i] = {0, 0};
@@ -390,12 +422,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
             }
             const int u = max(0, 26 - __clz((int)bits));
             const uint32_t um = 1u << (24 - u);
-            // exponents: a row of this thread, a column per lane
-            const int ea = (row0 + lane < t.m_valid ? exa[t.a_row + row0 + lane] : 1) - kExBias + 8 + u;
-            const int eb = lane < nc ? exb[t.b_row + h * HN + col0 + lane] : 1;
+            ea += u + 8 - kExBias;
             // eight columns at a time through shared memory: consecutive lanes
             // store consecutive columns
-            const int cl = lane & (SCOLS - 1);
 #pragma unroll
             for (int g = 0; g < WCOLS / SCOLS; ++g) {
                 if (g * SCOLS >= nc) break;
@@ -414,13 +443,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
                 for (int i = 0; i < SCOLS; ++i) sw[lane * ST_LD + i] = val[i];
                 __syncwarp();
                 const int col = h * HN + col0 + g * SCOLS + cl;
-                if (g * SCOLS + cl >= nc) continue;
-                const int r0 = lane / SCOLS;
+                if (MODE != 1 && g * SCOLS + cl >= nc) continue;
                 double* o;
                 int64_t step = 0;
                 if (MODE == 2) {
-                    step = om.colstride[t.out_off + col];
-                    o = om.out + om.colbase[t.out_off + col] + (int64_t)(t.ldc + row0 + r0) * step;
+                    step = pitch[g];
+                    o = om.out + place[g] + (int64_t)(t.ldc + row0 + r0) * step;
                 } else if (MODE == 1) {
                     o = om.out + t.n0 + col;
                 } else {
@@ -435,12 +463,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
                         if (om.beta != 0.0) x += om.beta * *o;
                         *o = x;
                     }
+                } else if (MODE == 1) {
+#pragma unroll
+                    for (int v = 0; v < SCOLS; ++v) {
+                        const int64_t row = __shfl_sync(0xffffffffu, rows, v * (32 / SCOLS) + r0);
+                        if (v * (32 / SCOLS) < last && g * SCOLS + cl < nc) o[row] = sw[(v * (32 / SCOLS) + r0) * ST_LD + cl];
+                    }
                 } else {
 #pragma unroll
                     for (int v = 0; v < SCOLS; ++v, o += step) {
                         if (v * (32 / SCOLS) >= last) break;
-                        const double x = sw[(v * (32 / SCOLS) + r0) * ST_LD + cl];
-                        *(MODE == 1 ? o + om.rowtab[t.out_off + row0 + v * (32 / SCOLS) + r0] : o) = x;
+                        *o = sw[(v * (32 / SCOLS) + r0) * ST_LD + cl];
                     }
                 }
             }
@@ -541,7 +574,9 @@ __global__ void __launch_bounds__(32 * kDigitRowsPerCta) digit_rows_kernel(const
                                                                            const DigitStack out, int* redo) {
     const DigitRows j = jobs[blockIdx.x];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    dep_launch();
     if (w >= j.n) return;
+    dep_wait();
     const int64_t row = (int64_t)j.row + w;
     auto at = [&](int c) { return reinterpret_cast<const double2*>(q64 + ((row + (int64_t)c * j.cs) << 6))[lane]; };
     auto scale = [&](int c) {
@@ -593,8 +628,10 @@ __global__ void __launch_bounds__(BT) digit_psi_kernel(const TcSplitJob* __restr
     const int nr = min(32, j.cols - j.b0), K = j.rows;
     const double* src = x + j.src + j.b0 + lane;
     const int64_t row = (int64_t)j.xrow + j.b0;
+    dep_launch();
     if (tid < 32) smax[tid] = 0;
     __syncthreads();
+    dep_wait();
     uint32_t mx = 0;
 #pragma unroll 4
     for (int k = w; k < K; k += BT / 32) mx = max(mx, lane < nr ? abs_hi(src[(int64_t)k * j.cols]) : 0u);
@@ -722,17 +759,63 @@ cudaError_t digit_setup() {
     return e;
 }
 
-cudaError_t launch_digit_gemm(int mode, const TcTile* tiles, int n_tiles, const DigitMaps& maps, const int32_t* exa,
-                              const int32_t* exb, const DigitOut& out, int* redo, int sms, cudaStream_t s) {
-    if (n_tiles <= 0) return cudaSuccess;
-    const int grid = std::min(n_tiles, sms);
-    if (mode == 0)
-        digit_gemm_kernel<0><<<grid, NTHREADS, SMEM_BYTES, s>>>(tiles, n_tiles, maps, exa, exb, out, redo);
-    else if (mode == 1)
-        digit_gemm_kernel<1><<<grid, NTHREADS, SMEM_BYTES, s>>>(tiles, n_tiles, maps, exa, exb, out, redo);
-    else
-        digit_gemm_kernel<2><<<grid, NTHREADS, SMEM_BYTES, s>>>(tiles, n_tiles, maps, exa, exb, out, redo);
-    return cudaGetLastError();
+cudaError_t launch_digit_gemm(int mode, const TcTile* tiles, const int32_t* begin, int ctas, const DigitMaps& maps,
+                              const int32_t* exa, const int32_t* exb, const DigitOut& out, int* redo, cudaStream_t s) {
+    if (ctas <= 0) return cudaSuccess;
+    if (mode == 0) return launch_dependent(digit_gemm_kernel<0>, ctas, NTHREADS, SMEM_BYTES, s, tiles, begin, maps, exa, exb, out, redo);
+    if (mode == 1) return launch_dependent(digit_gemm_kernel<1>, ctas, NTHREADS, SMEM_BYTES, s, tiles, begin, maps, exa, exb, out, redo);
+    return launch_dependent(digit_gemm_kernel<2>, ctas, NTHREADS, SMEM_BYTES, s, tiles, begin, maps, exa, exb, out, redo);
+}
+
+void digit_schedule(const std::vector<TcTile>& in, int ctas, std::vector<TcTile>& out, std::vector<int32_t>& begin) {
+    // microseconds a tile holds its SM: the product per 64 k, then the ends
+    // (measured on Hubbard D = 2048 and on dense products)
+    auto cost = [](const TcTile& t) {
+        const double halves = t.n_valid > HN ? 2.0 : 1.0, k = std::ceil(t.k_valid / (double)KW) * 0.5;
+        return 1.0 + k * (0.8 + 1.4 * halves) + 4.0 * t.m_valid * t.n_valid / (kTcBM * (double)kTcBN);
+    };
+    auto pack = [&](const std::vector<TcTile>& v, std::vector<int>& cta) {
+        std::vector<int> order(v.size());
+        for (size_t i = 0; i < v.size(); ++i) order[i] = (int)i;
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost(v[a]) > cost(v[b]); });
+        std::priority_queue<std::pair<double, int>, std::vector<std::pair<double, int>>, std::greater<>> load;
+        for (int c = 0; c < ctas; ++c) load.push({0.0, c});
+        cta.assign(v.size(), 0);
+        double top = 0.0;
+        for (int i : order) {
+            auto [t, c] = load.top();
+            load.pop();
+            cta[(size_t)i] = c;
+            t += cost(v[(size_t)i]);
+            top = std::max(top, t);
+            load.push({t, c});
+        }
+        return top;
+    };
+    // half-wide tiles read A twice, but two SMs share what one would do
+    std::vector<TcTile> halves;
+    for (const TcTile& t : in)
+        for (int n = 0; n < t.n_valid; n += HN) {
+            TcTile q = t;
+            q.b_row += n;
+            q.n_valid = std::min(HN, t.n_valid - n);
+            if (t.mode == 2) q.out_off += n;
+            q.n0 += n;
+            halves.push_back(q);
+        }
+    std::vector<int> whole_cta, half_cta;
+    const double whole = pack(in, whole_cta), half = pack(halves, half_cta);
+    const std::vector<TcTile>& v = half < whole ? halves : in;
+    const std::vector<int>& cta = half < whole ? half_cta : whole_cta;
+    std::vector<std::vector<int>> of((size_t)ctas);
+    for (size_t i = 0; i < v.size(); ++i) of[(size_t)cta[i]].push_back((int)i);
+    out.clear();
+    begin.assign(1, 0);
+    for (std::vector<int>& l : of) {
+        std::stable_sort(l.begin(), l.end(), [&](int a, int b) { return cost(v[(size_t)a]) > cost(v[(size_t)b]); });
+        for (int i : l) out.push_back(v[(size_t)i]);
+        begin.push_back((int32_t)out.size());
+    }
 }
 
 cudaError_t launch_digit_columns(const DigitRows* jobs, int n_jobs, const double* q64, int32_t* kx, cudaStream_t s) {
@@ -744,8 +827,7 @@ cudaError_t launch_digit_columns(const DigitRows* jobs, int n_jobs, const double
 cudaError_t launch_digit_rows(const DigitRows* jobs, int n_jobs, const double* q64, const int32_t* kx, int sign,
                               const DigitStack& out, int* redo, cudaStream_t s) {
     if (n_jobs <= 0) return cudaSuccess;
-    digit_rows_kernel<<<n_jobs, 32 * kDigitRowsPerCta, 0, s>>>(jobs, q64, kx, sign, out, redo);
-    return cudaGetLastError();
+    return launch_dependent(digit_rows_kernel, n_jobs, 32 * kDigitRowsPerCta, 0, s, jobs, q64, kx, sign, out, redo);
 }
 
 cudaError_t launch_digit_matrices(const DigitMatrix& a, const DigitMatrix& b, int K, int* redo, cudaStream_t s) {
@@ -766,8 +848,7 @@ cudaError_t launch_digit_matrices(const DigitMatrix& a, const DigitMatrix& b, in
 cudaError_t launch_digit_psi(const TcSplitJob* jobs, int n_jobs, const double* x, const DigitStack& out, int* redo,
                              cudaStream_t s) {
     if (n_jobs <= 0) return cudaSuccess;
-    digit_psi_kernel<<<n_jobs, BT, 0, s>>>(jobs, x, out, redo);
-    return cudaGetLastError();
+    return launch_dependent(digit_psi_kernel, n_jobs, BT, 0, s, jobs, x, out, redo);
 }
 
 }  // namespace tk

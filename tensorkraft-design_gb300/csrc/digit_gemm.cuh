@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <string>
+#include <vector>
 
 #include "tk_internal.hpp"
 
@@ -17,6 +18,28 @@ namespace tk {
 constexpr int kDigits = 7;
 constexpr int kDigitValue = 1, kDigitWait = 2;  // *redo: an operand's values / a wait that ran out
 constexpr int kDigitRing = 2;  // shared-memory stages of 32 K of a product
+
+// Programmatic dependent launch: a kernel's prologue overlaps the tail of the
+// one before it; it touches nothing another kernel writes before dep_wait(),
+// which returns once the previous kernel is complete and its memory visible.
+#ifdef __CUDACC__
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... A>
+cudaError_t launch_dependent(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, k, P(args)...);
+}
+#endif
 
 // A digit operand in the operand-stack layout (K-major 64-wide chunks, see
 // TcTables): plane j of `rows` rows of 64, and the biased exponent of every
@@ -53,17 +76,24 @@ struct DigitOut {
     const int32_t* colstride;
     int64_t c_rs, c_cs;
     double alpha, beta;
+    int tiles;    // mode 0: tiles of the C grid
     int m, n, k;  // mode 0: the product's size (its operands' stacks have m and n rows a chunk)
 };
 
 // Once per process and device before the first launch.
 cudaError_t digit_setup();
-// Runs the tiles' products on at most `sms` SMs.  Nothing is written once
-// *redo is non-zero (an operand row held an infinity or a NaN); a bounded
-// wait that ran out sets it too.  Whoever launches this computes the product
-// in another way when it ends up non-zero.
-cudaError_t launch_digit_gemm(int mode, const TcTile* tiles, int n_tiles, const DigitMaps& maps, const int32_t* exa,
-                              const int32_t* exb, const DigitOut& out, int* redo, int sms, cudaStream_t s);
+// Deals the tiles of a product out to `ctas` CTAs: CTA c runs out[begin[c] ..
+// begin[c + 1]), heaviest first, the sums of the estimated times as equal as
+// longest-first dealing makes them; in 32-wide halves where that ends sooner
+// (fewer tiles than SMs).
+void digit_schedule(const std::vector<TcTile>& in, int ctas, std::vector<TcTile>& out, std::vector<int32_t>& begin);
+
+// Runs the tiles' products (mode 0: the C grid's, dealt in turn).  Nothing is
+// written once *redo is non-zero (an operand row held an infinity or a NaN); a
+// bounded wait that ran out sets it too.  Whoever launches this computes the
+// product in another way when it ends up non-zero.
+cudaError_t launch_digit_gemm(int mode, const TcTile* tiles, const int32_t* begin, int ctas, const DigitMaps& maps,
+                              const int32_t* exa, const int32_t* exb, const DigitOut& out, int* redo, cudaStream_t s);
 
 // Exponents of a stack's columns: kx[j.kx + k] = floor(log2 max |x|) over the
 // rows [row, row + n) of job j at k, 0 for a column of zeros.

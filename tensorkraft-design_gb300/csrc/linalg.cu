@@ -177,12 +177,12 @@ tk_status gemm_digits(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* 
     o.m = (int)M;
     o.n = (int)N;
     o.k = (int)K;
-    const int64_t tiles = ((M + kTcBM - 1) / kTcBM) * ((N + kTcBN - 1) / kTcBN);
+    o.tiles = (int)(((M + kTcBM - 1) / kTcBM) * ((N + kTcBN - 1) / kTcBN));
     int state = 0;
     cudaError_t e = digit_setup();
     if (e == cudaSuccess) e = cudaMemsetAsync(redo, 0, sizeof(int), s);
     if (e == cudaSuccess) e = launch_digit_matrices(A, B, (int)K, redo, s);
-    if (e == cudaSuccess) e = launch_digit_gemm(0, nullptr, (int)tiles, maps, A.out.ex, B.out.ex, o, redo, 152, s);
+    if (e == cudaSuccess) e = launch_digit_gemm(0, nullptr, nullptr, std::min(o.tiles, 152), maps, A.out.ex, B.out.ex, o, redo, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&state, redo, sizeof(int), cudaMemcpyDeviceToHost, s);
     // the buffer goes back when the stream is done with it, whatever failed
     const cudaError_t w = cudaStreamSynchronize(s);

@@ -292,7 +292,10 @@ __global__ void __launch_bounds__(128) stack_combine_f64_kernel(const TcCombJob*
                                                                 const double* __restrict__ coef,
                                                                 const double* __restrict__ t1,
                                                                 double* __restrict__ t2) {
-    stack_combine_job(jobs[blockIdx.x], terms, coef, t1, t2);
+    const TcCombJob j = jobs[blockIdx.x];  // a plan constant
+    dep_launch();
+    dep_wait();
+    stack_combine_job(j, terms, coef, t1, t2);
 }
 
 // The whole FP64 matvec in one launch, after a digit matvec that could not
@@ -318,6 +321,8 @@ __device__ __forceinline__ void cluster_barrier() {
 __global__ void __cluster_dims__(kRedoCtas, 1, 1) __launch_bounds__(ST)
     stack_redo_f64_kernel(const RedoArgs a, const double* __restrict__ x, double* __restrict__ y, int* redo) {
     __shared__ PieceTiles<false> sm;
+    dep_launch();
+    dep_wait();
     if (*(volatile int*)redo == 0) return;
     for (int i = blockIdx.x; i < a.n1; i += kRedoCtas) {
         __syncthreads();
@@ -458,12 +463,13 @@ struct F64Digits {
     DevBuf<__half> lq, rq, t2, xq;
     DevBuf<int32_t> lx, rx, tx, xx;  // exponents of their rows
     DevBuf<int32_t> kx;              // scales of the R stacks' columns
-    DevBuf<TcTile> tiles1, tiles3;
+    DevBuf<TcTile> tiles1, tiles3;   // dealt out to `sms` CTAs: begin1, begin3
+    DevBuf<int32_t> begin1, begin3;
     DevBuf<TcSplitJob> psi;
     DevBuf<DigitRows> rows;          // of T2
     DevBuf<int> redo;
     DigitMaps m1, m3;
-    int n1 = 0, n3 = 0, npsi = 0, nrows = 0, sms = 0;
+    int npsi = 0, nrows = 0, sms = 0;
     DigitStack stack(const DevBuf<__half>& q, const DevBuf<int32_t>& x) const { return {q.p, x.p, (int64_t)x.n}; }
 };
 
@@ -538,17 +544,23 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
         return e;
     };
     DevBuf<DigitRows> dl, dr, dc;
+    std::vector<TcTile> t1, t3;
+    std::vector<int32_t> b1, b3;
     cudaError_t e;
     int redo = 0, dev = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+        return e;
+    digit_schedule(C.tiles1x, d->sms, t1, b1);
+    digit_schedule(C.tiles3, d->sms, t3, b3);
     if ((e = stack(d->lq, d->lx, C.lq_rows)) != cudaSuccess || (e = stack(d->rq, d->rx, C.rq_rows)) != cudaSuccess ||
         (e = stack(d->t2, d->tx, C.t2q_rows)) != cudaSuccess || (e = stack(d->xq, d->xx, C.xq_rows)) != cudaSuccess ||
-        (e = d->kx.alloc((size_t)std::max(nk, 1))) != cudaSuccess || (e = d->tiles1.upload(C.tiles1x)) != cudaSuccess ||
-        (e = d->tiles3.upload(C.tiles3)) != cudaSuccess || (e = d->psi.upload(psi)) != cudaSuccess ||
+        (e = d->kx.alloc((size_t)std::max(nk, 1))) != cudaSuccess || (e = d->tiles1.upload(t1)) != cudaSuccess ||
+        (e = d->tiles3.upload(t3)) != cudaSuccess || (e = d->begin1.upload(b1)) != cudaSuccess ||
+        (e = d->begin3.upload(b3)) != cudaSuccess || (e = d->psi.upload(psi)) != cudaSuccess ||
         (e = d->rows.upload(trows)) != cudaSuccess || (e = d->redo.alloc(1)) != cudaSuccess ||
         (e = cudaMemset(d->redo.p, 0, sizeof(int))) != cudaSuccess || (e = dl.upload(lrows)) != cudaSuccess ||
-        (e = dr.upload(rrows)) != cudaSuccess || (e = dc.upload(rcols)) != cudaSuccess || (e = digit_setup()) != cudaSuccess ||
-        (e = cudaGetDevice(&dev)) != cudaSuccess ||
-        (e = cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+        (e = dr.upload(rrows)) != cudaSuccess || (e = dc.upload(rcols)) != cudaSuccess || (e = digit_setup()) != cudaSuccess)
         return e;
     if (!digit_maps(d->m1, d->stack(d->lq, d->lx), d->stack(d->xq, d->xx), err) ||
         !digit_maps(d->m3, d->stack(d->t2, d->tx), d->stack(d->rq, d->rx), err))
@@ -560,8 +572,6 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
             cudaSuccess ||
         (e = cudaMemcpy(&redo, d->redo.p, sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess)
         return e;
-    d->n1 = (int)C.tiles1x.size();
-    d->n3 = (int)C.tiles3.size();
     d->npsi = (int)psi.size();
     d->nrows = (int)trows.size();
     if (redo == 0) p.dg = std::move(d);
@@ -648,20 +658,20 @@ static cudaError_t digits_stage(F64Stack& p, const double* x, double* y, cudaStr
         o.out = p.t1.p;
         o.colbase = p.colbase.p;
         o.colstride = p.colstride.p;
-        return launch_digit_gemm(2, d.tiles1.p, d.n1, d.m1, d.lx.p, d.xx.p, o, d.redo.p, d.sms, s);
+        return launch_digit_gemm(2, d.tiles1.p, d.begin1.p, d.sms, d.m1, d.lx.p, d.xx.p, o, d.redo.p, s);
     }
     if (stage == 1) {
-        if (p.njobs > 0) stack_combine_f64_kernel<<<p.njobs, 128, 0, s>>>(p.jobs.p, p.terms.p, p.coef.p, p.t1.p, p.t2.p);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if (p.njobs > 0 && (e = launch_dependent(stack_combine_f64_kernel, p.njobs, 128, 0, s, p.jobs.p, p.terms.p, p.coef.p,
+                                                 p.t1.p, p.t2.p)) != cudaSuccess)
+            return e;
         return launch_digit_rows(d.rows.p, d.nrows, p.t2.p, d.kx.p, 1, d.stack(d.t2, d.tx), d.redo.p, s);
     }
     o.out = y;
     o.rowtab = p.yrow.p;
-    if ((e = launch_digit_gemm(1, d.tiles3.p, d.n3, d.m3, d.tx.p, d.rx.p, o, d.redo.p, d.sms, s)) != cudaSuccess) return e;
+    if ((e = launch_digit_gemm(1, d.tiles3.p, d.begin3.p, d.sms, d.m3, d.tx.p, d.rx.p, o, d.redo.p, s)) != cudaSuccess) return e;
     const RedoArgs a{p.pieces1.p, p.pieces3.p, p.segs.p, p.jobs.p, p.terms.p, p.coef.p,     p.lq.p, p.rq.p, p.xsrc.p,
                      p.colbase.p, p.yrow.p,    p.xstride.p, p.colstride.p, p.t1.p, p.t2.p, p.n1,   p.n3,   p.njobs};
-    stack_redo_f64_kernel<<<kRedoCtas, ST, 0, s>>>(a, x, y, d.redo.p);
-    return cudaGetLastError();
+    return launch_dependent(stack_redo_f64_kernel, kRedoCtas, ST, 0, s, a, x, y, d.redo.p);
 }
 
 cudaError_t f64stack_stage(F64Stack& p, const double* x, double* y, cudaStream_t s, int stage) {
