@@ -175,25 +175,28 @@ struct Sum {
 };
 constexpr int kCarryChunks = 64;  // chunks after which l is near its range
 
-// x * 2^t rounded to nearest even, on the integer pipes (the FP64 pipe does
+// x * 2^(e - kExpo) rounded to nearest, on the integer pipes (the FP64 pipe does
 // two operations a clock).  Free of branches, so that the columns of a row
-// overlap; *off is set where |x| < 2^32 or the result is subnormal or
-// overflows, which to_double_slow computes.
-__device__ __forceinline__ double to_double(int64_t x, int t, bool* off) {
+// overlap; *off is set where |x| < 2^32, which to_double_slow computes, as it
+// does where a tile's exponents come near the ends of the range (to_double
+// itself checks none).
+constexpr int kExpo = 1084;
+constexpr int kExpLow = 40, kExpHigh = 2040;  // for e in between it holds whatever x is
+__device__ __forceinline__ double to_double(int64_t x, int e, uint32_t* off) {
     const int32_t neg = (int32_t)((uint64_t)x >> 32) >> 31;
     const uint64_t u = (uint64_t)((x ^ (int64_t)neg) - (int64_t)neg);
     const uint32_t h = (uint32_t)(u >> 32), l = (uint32_t)u;
     // the leading bit to bit 62, so that rounding at bit 10 cannot carry out
     const int z = __clz(h) - 1;
     uint64_t q = ((uint64_t)__funnelshift_l(l, h, z) << 32) | (l << (z & 31));
-    q = (q + 0x1FFu + ((uint32_t)(q >> 10) & 1u)) >> 10;
-    const int e = t + 10 - z;  // the value is q * 2^e
-    const bool fast = h != 0 && (uint32_t)(e + 1073) < 2045u;
-    *off |= !fast && u != 0;
-    const uint32_t rh = ((uint32_t)(q >> 32) + ((uint32_t)(e + 1074) << 20)) | ((uint32_t)neg & 0x80000000u);
-    return fast ? __hiloint2double((int)rh, (int)(uint32_t)q) : 0.0;
+    q = (q + 0x200u) >> 10;
+    const bool zero = h == 0;
+    *off |= zero ? l : 0u;
+    const uint32_t rh = ((uint32_t)(q >> 32) + ((uint32_t)(e - z) << 20)) | ((uint32_t)neg & 0x80000000u);
+    return zero ? 0.0 : __hiloint2double((int)rh, (int)(uint32_t)q);
 }
-__device__ __noinline__ double to_double_slow(int64_t x, int t) {
+__device__ __noinline__ double to_double_slow(int64_t x, int e) {
+    int t = e - kExpo;
     uint64_t u = x < 0 ? 0 - (uint64_t)x : (uint64_t)x;
     if (u == 0) return 0.0;
     // drop the bits below the result's last place, 2^-1074 at the least
@@ -201,7 +204,7 @@ __device__ __noinline__ double to_double_slow(int64_t x, int t) {
     if (drop > 0) {
         const int d = min(drop, 63);
         const uint64_t half = 1ull << (d - 1), rest = u & ((1ull << d) - 1);
-        u = drop > 64 ? 0 : (u >> d) + (rest + ((u >> d) & 1) > half);
+        u = drop > 64 ? 0 : (u >> d) + (rest >= half);  // ties away from zero, as in to_double
         t += drop;
     }
     const double r = u == 0 ? 0.0 : t > 1000 ? INFINITY : ldexp((double)(long long)u, t);
@@ -371,7 +374,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
                     ea = exa[t.a_row + row0 + lane];
                     if (MODE == 1) rows = om.rowtab[t.out_off + row0 + lane];
                 }
-                if (lane < nc) eb = exb[t.b_row + h * HN + col0 + lane];
+                eb = exb[t.b_row + h * HN + col0 + min(lane, nc - 1)];  // (a column past the tile's takes the last one's)
                 if (MODE == 2)
 #pragma unroll
                     for (int g = 0; g < WCOLS / SCOLS; ++g)
@@ -422,25 +425,26 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
             }
             const int u = max(0, 26 - __clz((int)bits));
             const uint32_t um = 1u << (24 - u);
-            ea += u + 8 - kExBias;
+            ea += u + 8 - kExBias + kExpo;
+            const int eb_lo = __reduce_min_sync(0xffffffffu, eb), eb_hi = __reduce_max_sync(0xffffffffu, eb);
+            const bool inside = ea + eb_lo >= kExpLow && ea + eb_hi <= kExpHigh;
             // eight columns at a time through shared memory: consecutive lanes
             // store consecutive columns
 #pragma unroll
             for (int g = 0; g < WCOLS / SCOLS; ++g) {
                 if (g * SCOLS >= nc) break;
-                bool off = false;
-                double val[SCOLS];
-#pragma unroll
-                for (int i = 0; i < SCOLS; ++i)
-                    val[i] = to_double(acc[g * SCOLS + i].whole(um, u), ea + __shfl_sync(0xffffffffu, eb, g * SCOLS + i), &off);
-                if (__any_sync(0xffffffffu, off && row0 + lane < t.m_valid)) {
-#pragma unroll
-                    for (int i = 0; i < SCOLS; ++i)
-                        val[i] = to_double_slow(acc[g * SCOLS + i].whole(um, u), ea + __shfl_sync(0xffffffffu, eb, g * SCOLS + i));
-                }
+                uint32_t off = inside ? 0u : 1u;
                 __syncwarp();
 #pragma unroll
-                for (int i = 0; i < SCOLS; ++i) sw[lane * ST_LD + i] = val[i];
+                for (int i = 0; i < SCOLS; ++i)
+                    sw[lane * ST_LD + i] =
+                        to_double(acc[g * SCOLS + i].whole(um, u), ea + __shfl_sync(0xffffffffu, eb, g * SCOLS + i), &off);
+                if (__any_sync(0xffffffffu, off != 0 && row0 + lane < t.m_valid)) {
+#pragma unroll
+                    for (int i = 0; i < SCOLS; ++i)
+                        sw[lane * ST_LD + i] =
+                            to_double_slow(acc[g * SCOLS + i].whole(um, u), ea + __shfl_sync(0xffffffffu, eb, g * SCOLS + i));
+                }
                 __syncwarp();
                 const int col = h * HN + col0 + g * SCOLS + cl;
                 if (MODE != 1 && g * SCOLS + cl >= nc) continue;

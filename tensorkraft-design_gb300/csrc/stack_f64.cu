@@ -460,17 +460,16 @@ bool stage3_pieces(const TcTables& C, std::vector<F64Piece>& out, std::vector<KS
 // The digit form of a stacked plan (digit_gemm.cu): the operand stacks as
 // digits, their tiles, and the rows to turn into digits on every matvec.
 struct F64Digits {
-    DevBuf<__half> lq, rq, t2, xq;
-    DevBuf<int32_t> lx, rx, tx, xx;  // exponents of their rows
-    DevBuf<int32_t> kx;              // scales of the R stacks' columns
-    DevBuf<TcTile> tiles1, tiles3;   // dealt out to `sms` CTAs: begin1, begin3
-    DevBuf<int32_t> begin1, begin3;
-    DevBuf<TcSplitJob> psi;
-    DevBuf<DigitRows> rows;          // of T2
-    DevBuf<int> redo;
+    DevBuf<unsigned char> mem;       // one allocation for all of it
+    DigitStack l, r, t2, x;
+    const int32_t* kx = nullptr;     // scales of the R stacks' columns
+    const TcTile *tiles1 = nullptr, *tiles3 = nullptr;   // dealt out to `sms` CTAs:
+    const int32_t *begin1 = nullptr, *begin3 = nullptr;
+    const TcSplitJob* psi = nullptr;
+    const DigitRows* rows = nullptr;  // of T2
+    int* redo = nullptr;
     DigitMaps m1, m3;
     int npsi = 0, nrows = 0, sms = 0;
-    DigitStack stack(const DevBuf<__half>& q, const DevBuf<int32_t>& x) const { return {q.p, x.p, (int64_t)x.n}; }
 };
 
 struct F64Stack {
@@ -535,42 +534,67 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
         if (seen.insert(-1 - t.b_row).second) digit_rows_of(rrows, t.b_row, t.n_valid, t.b_cs, t.kch, kx[base]);
         if (t.n0 == 0) digit_rows_of(trows, t.a_row, t.m_valid, t.a_cs, t.kch, kx[base]);
     }
-    auto stack = [](DevBuf<__half>& q, DevBuf<int32_t>& x, int64_t rows) {
-        const size_t n = (size_t)std::max<int64_t>(rows, 1);
-        cudaError_t e = q.alloc(n * kTcBK * kDigits);
-        if (e == cudaSuccess) e = x.alloc(n);
-        if (e == cudaSuccess) e = cudaMemset(q.p, 0, sizeof(__half) * q.n);
-        if (e == cudaSuccess) e = cudaMemset(x.p, 0, sizeof(int32_t) * x.n);
-        return e;
-    };
-    DevBuf<DigitRows> dl, dr, dc;
     std::vector<TcTile> t1, t3;
     std::vector<int32_t> b1, b3;
     cudaError_t e;
     int redo = 0, dev = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
-        (e = cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+        (e = cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
+        (e = digit_setup()) != cudaSuccess)
         return e;
     digit_schedule(C.tiles1x, d->sms, t1, b1);
     digit_schedule(C.tiles3, d->sms, t3, b3);
-    if ((e = stack(d->lq, d->lx, C.lq_rows)) != cudaSuccess || (e = stack(d->rq, d->rx, C.rq_rows)) != cudaSuccess ||
-        (e = stack(d->t2, d->tx, C.t2q_rows)) != cudaSuccess || (e = stack(d->xq, d->xx, C.xq_rows)) != cudaSuccess ||
-        (e = d->kx.alloc((size_t)std::max(nk, 1))) != cudaSuccess || (e = d->tiles1.upload(t1)) != cudaSuccess ||
-        (e = d->tiles3.upload(t3)) != cudaSuccess || (e = d->begin1.upload(b1)) != cudaSuccess ||
-        (e = d->begin3.upload(b3)) != cudaSuccess || (e = d->psi.upload(psi)) != cudaSuccess ||
-        (e = d->rows.upload(trows)) != cudaSuccess || (e = d->redo.alloc(1)) != cudaSuccess ||
-        (e = cudaMemset(d->redo.p, 0, sizeof(int))) != cudaSuccess || (e = dl.upload(lrows)) != cudaSuccess ||
-        (e = dr.upload(rrows)) != cudaSuccess || (e = dc.upload(rcols)) != cudaSuccess || (e = digit_setup()) != cudaSuccess)
+    // the tables first (one copy), then what the device writes
+    Blob blob;
+    auto table = [&](const auto& v) { return blob.add(v.data(), sizeof(v[0]) * v.size()); };
+    const size_t o_redo = blob.add(&redo, sizeof(redo)), o_t1 = table(t1), o_t3 = table(t3), o_b1 = table(b1),
+                 o_b3 = table(b3), o_psi = table(psi), o_rows = table(trows), o_l = table(lrows), o_r = table(rrows),
+                 o_c = table(rcols);
+    std::vector<unsigned char> host(blob.size());
+    blob.copy_to(host.data());
+    size_t total = blob.size();
+    auto take = [&](size_t n) {
+        const size_t at = (total + 1023) & ~(size_t)1023;
+        total = at + n;
+        return at;
+    };
+    struct Place {
+        DigitStack* s;
+        size_t q, x;
+    };
+    std::vector<Place> places;
+    for (auto [s, rows] : {std::pair<DigitStack*, int64_t>{&d->l, C.lq_rows}, {&d->r, C.rq_rows}, {&d->t2, C.t2q_rows},
+                           {&d->x, C.xq_rows}}) {
+        s->rows = std::max<int64_t>(rows, 1);
+        const size_t q = take(digit_stack_bytes(s->rows));
+        places.push_back({s, q, take(sizeof(int32_t) * (size_t)s->rows)});
+    }
+    const size_t o_kx = take(sizeof(int32_t) * (size_t)std::max(nk, 1));
+    if ((e = d->mem.alloc(total)) != cudaSuccess ||
+        (e = cudaMemcpy(d->mem.p, host.data(), host.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
         return e;
-    if (!digit_maps(d->m1, d->stack(d->lq, d->lx), d->stack(d->xq, d->xx), err) ||
-        !digit_maps(d->m3, d->stack(d->t2, d->tx), d->stack(d->rq, d->rx), err))
-        return cudaErrorInvalidValue;
-    if ((e = launch_digit_rows(dl.p, (int)lrows.size(), p.lq.p, nullptr, 1, d->stack(d->lq, d->lx), d->redo.p, 0)) !=
+    unsigned char* m = d->mem.p;
+    for (const Place& pl : places) {
+        pl.s->q = reinterpret_cast<__half*>(m + pl.q);
+        pl.s->ex = reinterpret_cast<int32_t*>(m + pl.x);
+    }
+    int32_t* kxd = reinterpret_cast<int32_t*>(m + o_kx);
+    d->kx = kxd;
+    d->tiles1 = reinterpret_cast<const TcTile*>(m + o_t1);
+    d->tiles3 = reinterpret_cast<const TcTile*>(m + o_t3);
+    d->begin1 = reinterpret_cast<const int32_t*>(m + o_b1);
+    d->begin3 = reinterpret_cast<const int32_t*>(m + o_b3);
+    d->psi = reinterpret_cast<const TcSplitJob*>(m + o_psi);
+    d->rows = reinterpret_cast<const DigitRows*>(m + o_rows);
+    d->redo = reinterpret_cast<int*>(m + o_redo);
+    if (!digit_maps(d->m1, d->l, d->x, err) || !digit_maps(d->m3, d->t2, d->r, err)) return cudaErrorInvalidValue;
+    if ((e = launch_digit_rows(reinterpret_cast<const DigitRows*>(m + o_l), (int)lrows.size(), p.lq.p, nullptr, 1, d->l,
+                               d->redo, 0)) != cudaSuccess ||
+        (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_c), (int)rcols.size(), p.rq.p, kxd, 0)) !=
             cudaSuccess ||
-        (e = launch_digit_columns(dc.p, (int)rcols.size(), p.rq.p, d->kx.p, 0)) != cudaSuccess ||
-        (e = launch_digit_rows(dr.p, (int)rrows.size(), p.rq.p, d->kx.p, -1, d->stack(d->rq, d->rx), d->redo.p, 0)) !=
-            cudaSuccess ||
-        (e = cudaMemcpy(&redo, d->redo.p, sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess)
+        (e = launch_digit_rows(reinterpret_cast<const DigitRows*>(m + o_r), (int)rrows.size(), p.rq.p, kxd, -1, d->r,
+                               d->redo, 0)) != cudaSuccess ||
+        (e = cudaMemcpy(&redo, d->redo, sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess)
         return e;
     d->npsi = (int)psi.size();
     d->nrows = (int)trows.size();
@@ -654,24 +678,24 @@ static cudaError_t digits_stage(F64Stack& p, const double* x, double* y, cudaStr
     cudaError_t e;
     DigitOut o{};
     if (stage == 0) {
-        if ((e = launch_digit_psi(d.psi.p, d.npsi, x, d.stack(d.xq, d.xx), d.redo.p, s)) != cudaSuccess) return e;
+        if ((e = launch_digit_psi(d.psi, d.npsi, x, d.x, d.redo, s)) != cudaSuccess) return e;
         o.out = p.t1.p;
         o.colbase = p.colbase.p;
         o.colstride = p.colstride.p;
-        return launch_digit_gemm(2, d.tiles1.p, d.begin1.p, d.sms, d.m1, d.lx.p, d.xx.p, o, d.redo.p, s);
+        return launch_digit_gemm(2, d.tiles1, d.begin1, d.sms, d.m1, d.l.ex, d.x.ex, o, d.redo, s);
     }
     if (stage == 1) {
         if (p.njobs > 0 && (e = launch_dependent(stack_combine_f64_kernel, p.njobs, 128, 0, s, p.jobs.p, p.terms.p, p.coef.p,
                                                  p.t1.p, p.t2.p)) != cudaSuccess)
             return e;
-        return launch_digit_rows(d.rows.p, d.nrows, p.t2.p, d.kx.p, 1, d.stack(d.t2, d.tx), d.redo.p, s);
+        return launch_digit_rows(d.rows, d.nrows, p.t2.p, d.kx, 1, d.t2, d.redo, s);
     }
     o.out = y;
     o.rowtab = p.yrow.p;
-    if ((e = launch_digit_gemm(1, d.tiles3.p, d.begin3.p, d.sms, d.m3, d.tx.p, d.rx.p, o, d.redo.p, s)) != cudaSuccess) return e;
+    if ((e = launch_digit_gemm(1, d.tiles3, d.begin3, d.sms, d.m3, d.t2.ex, d.r.ex, o, d.redo, s)) != cudaSuccess) return e;
     const RedoArgs a{p.pieces1.p, p.pieces3.p, p.segs.p, p.jobs.p, p.terms.p, p.coef.p,     p.lq.p, p.rq.p, p.xsrc.p,
                      p.colbase.p, p.yrow.p,    p.xstride.p, p.colstride.p, p.t1.p, p.t2.p, p.n1,   p.n3,   p.njobs};
-    return launch_dependent(stack_redo_f64_kernel, kRedoCtas, ST, 0, s, a, x, y, d.redo.p);
+    return launch_dependent(stack_redo_f64_kernel, kRedoCtas, ST, 0, s, a, x, y, d.redo);
 }
 
 cudaError_t f64stack_stage(F64Stack& p, const double* x, double* y, cudaStream_t s, int stage) {
