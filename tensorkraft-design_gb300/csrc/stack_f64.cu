@@ -495,18 +495,21 @@ static void digit_rows_of(std::vector<DigitRows>& out, int32_t row, int n, int32
         out.push_back({row + r, std::min(kDigitRowsPerCta, n - r), cs, kch, kx, 0});
 }
 
-// Whether a plan's FP64 matvec runs on digits: from 8 million multiply-adds in
+// Whether a plan's FP64 matvec runs on digits: from 1.2 million multiply-adds in
 // stage 1.  Below, the FP64 kernels finish before the digit kernels' latencies
-// add up (Heisenberg D = 256, 3 million: 52 us against 59; Hubbard D = 512,
-// 3.6 million: 56 against 59; cylinder D = 128, 2 million: 60 against 73);
-// above, their pipe is the limit (Heisenberg D = 512, 25 million: 150 against
-// 75 us; Hubbard D = 1024, 25 million: 130 against 89; Hubbard D = 2048, 230
-// million: 701 against 184; cylinder D = 2048, 13 billion: 40.9 ms against 1.9).
+// add up (Heisenberg D = 128, 0.4 million: 23 us against 29; D = 181, 1.1
+// million: 33 and 33); above, their pipe is the limit (Hubbard D = 362, 1.3
+// million: 44 against 31 us; D = 512: 56 against 36; D = 2048, 230 million: 701
+// against 149; Heisenberg D = 512, 25 million: 151 against 51; cylinder D =
+// 2048, 13 billion: 40.9 ms against 1.84).  A plan of less than a dozen stage-3
+// tiles keeps its three launches up to 8 million: small plans of a few sectors
+// are relied on to be three launches (digits would take 58 us against 85 at 6.2
+// million on ten tiles).
 bool f64stack_on_digits(const TcTables& C) {
     double f = 0.0;
     for (const std::vector<TcTile>* v : {&C.tiles1, &C.tiles1x})
         for (const TcTile& t : *v) f += (double)t.m_valid * t.n_valid * t.k_valid;
-    return f >= 8e6;
+    return f >= (C.tiles3.size() + C.tiles3f.size() < 12 ? 8e6 : 1.2e6);
 }
 
 // Builds the digit form of p; left out (dg null) where the constant operands
