@@ -549,23 +549,21 @@ __device__ __forceinline__ int exponent_of(double x, int k) {
     return zero ? kNoExponent : (e > 0 ? e : 12 - __clz((int)(hi | 1))) + k;
 }
 
-// One CTA per 64-wide chunk of a stack: the columns' exponents.
+// One CTA per 64-wide chunk of a stack (blockIdx.y, past the stack's last: nothing): the columns' exponents.
 __global__ void __launch_bounds__(256) digit_columns_kernel(const DigitRows* __restrict__ jobs,
                                                             const double* __restrict__ q64, int32_t* __restrict__ kx) {
     __shared__ uint32_t top[4][kTcBK];
     const DigitRows j = jobs[blockIdx.x];
-    const int k = threadIdx.x & 63, w = threadIdx.x >> 6;
-    for (int c = 0; c < j.kch; ++c) {
-        uint32_t mx = 0;
-        for (int r = w; r < j.n; r += 4) mx = max(mx, abs_hi(q64[(((int64_t)j.row + (int64_t)c * j.cs + r) << 6) + k]));
-        top[w][k] = mx;
-        __syncthreads();
-        if (w == 0) {
-            mx = max(max(top[0][k], top[1][k]), max(top[2][k], top[3][k]));
-            kx[j.kx + c * kTcBK + k] = mx >> 20 ? (int)(mx >> 20) - 1023 : 0;
-        }
-        __syncthreads();
-    }
+    const int k = threadIdx.x & 63, w = threadIdx.x >> 6, c = blockIdx.y;
+    if (c >= j.kch) return;
+    uint32_t mx = 0;
+#pragma unroll 4
+    for (int r = w; r < j.n; r += 4) mx = max(mx, abs_hi(q64[(((int64_t)j.row + (int64_t)c * j.cs + r) << 6) + k]));
+    top[w][k] = mx;
+    __syncthreads();
+    if (w != 0) return;
+    mx = max(max(top[0][k], top[1][k]), max(top[2][k], top[3][k]));
+    kx[j.kx + c * kTcBK + k] = mx >> 20 ? (int)(mx >> 20) - 1023 : 0;
 }
 
 // One warp per row of an FP64 stack (K-major 64-wide chunks): the row's
@@ -797,9 +795,11 @@ void digit_schedule(const std::vector<TcTile>& in, int ctas, std::vector<TcTile>
         return top;
     };
     // half-wide tiles read A twice, but two SMs share what one would do
+    // (with many tiles a CTA the whole ones come out as even)
     std::vector<TcTile> halves;
+    const bool try_halves = in.size() < 4 * (size_t)ctas;
     for (const TcTile& t : in)
-        for (int n = 0; n < t.n_valid; n += HN) {
+        for (int n = 0; try_halves && n < t.n_valid; n += HN) {
             TcTile q = t;
             q.b_row += n;
             q.n_valid = std::min(HN, t.n_valid - n);
@@ -808,7 +808,7 @@ void digit_schedule(const std::vector<TcTile>& in, int ctas, std::vector<TcTile>
             halves.push_back(q);
         }
     std::vector<int> whole_cta, half_cta;
-    const double whole = pack(in, whole_cta), half = pack(halves, half_cta);
+    const double whole = pack(in, whole_cta), half = try_halves ? pack(halves, half_cta) : whole;
     const std::vector<TcTile>& v = half < whole ? halves : in;
     const std::vector<int>& cta = half < whole ? half_cta : whole_cta;
     std::vector<std::vector<int>> of((size_t)ctas);
@@ -822,9 +822,10 @@ void digit_schedule(const std::vector<TcTile>& in, int ctas, std::vector<TcTile>
     }
 }
 
-cudaError_t launch_digit_columns(const DigitRows* jobs, int n_jobs, const double* q64, int32_t* kx, cudaStream_t s) {
-    if (n_jobs <= 0) return cudaSuccess;
-    digit_columns_kernel<<<n_jobs, 256, 0, s>>>(jobs, q64, kx);
+cudaError_t launch_digit_columns(const DigitRows* jobs, int n_jobs, int max_kch, const double* q64, int32_t* kx,
+                                 cudaStream_t s) {
+    if (n_jobs <= 0 || max_kch <= 0) return cudaSuccess;
+    digit_columns_kernel<<<dim3((unsigned)n_jobs, (unsigned)max_kch), 256, 0, s>>>(jobs, q64, kx);
     return cudaGetLastError();
 }
 

@@ -97,7 +97,8 @@ cudaError_t launch_digit_gemm(int mode, const TcTile* tiles, const int32_t* begi
 
 // Exponents of a stack's columns: kx[j.kx + k] = floor(log2 max |x|) over the
 // rows [row, row + n) of job j at k, 0 for a column of zeros.
-cudaError_t launch_digit_columns(const DigitRows* jobs, int n_jobs, const double* q64, int32_t* kx, cudaStream_t s);
+cudaError_t launch_digit_columns(const DigitRows* jobs, int n_jobs, int max_kch, const double* q64, int32_t* kx,
+                                 cudaStream_t s);
 // Digits of FP64 operand stacks (rows of 64 doubles per chunk), of
 // x 2^(sign * kx) where the job has scales.
 cudaError_t launch_digit_rows(const DigitRows* jobs, int n_jobs, const double* q64, const int32_t* kx, int sign,

@@ -28,6 +28,8 @@
 //     those rows), with no predicated-off FMA past a segment's end;
 //   - pieces are cut so that each holds at most a share of the stage's
 //     FMAs, and go out longest first.
+// The launches are chained by programmatic dependent launch: for small plans they
+// are most of the time (Heisenberg D = 64: 17.4 -> 10.9 us).
 // Every output sums its k in ascending order.
 //
 // Large real plans run the same stacks on the fp16 tensor cores instead
@@ -212,7 +214,10 @@ __global__ void __launch_bounds__(ST, 4) stack_gemm1_f64_kernel(const F64Piece* 
                                                                 const int32_t* __restrict__ colstride,
                                                                 double* __restrict__ t1, double* __restrict__ t1_im) {
     __shared__ PieceTiles<CPLX> sm;
-    stack_piece1<CPLX>(pieces[blockIdx.x], sm, segs, lq, lq_im, x, x_im, xsrc, xstride, colbase, colstride, t1, t1_im);
+    const F64Piece t = pieces[blockIdx.x];  // a plan constant
+    dep_launch();
+    dep_wait();
+    stack_piece1<CPLX>(t, sm, segs, lq, lq_im, x, x_im, xsrc, xstride, colbase, colstride, t1, t1_im);
 }
 
 // Stage 3: y = T2 stacks * R stacks^T (CPLX: both complex, planar).
@@ -268,7 +273,10 @@ __global__ void __launch_bounds__(ST, 4) stack_gemm3_f64_kernel(const F64Piece* 
                                                                 const int64_t* __restrict__ yrow,
                                                                 double* __restrict__ y, double* __restrict__ y_im) {
     __shared__ PieceTiles<CPLX> sm;
-    stack_piece3<CPLX>(pieces[blockIdx.x], sm, segs, t2, t2_im, rq, rq_im, yrow, y, y_im);
+    const F64Piece t = pieces[blockIdx.x];  // a plan constant
+    dep_launch();
+    dep_wait();
+    stack_piece3<CPLX>(t, sm, segs, t2, t2_im, rq, rq_im, yrow, y, y_im);
 }
 
 // T2 = sum coef * T1 for one combine job (rows r0 .. r0 + rows of a slab),
@@ -497,10 +505,10 @@ static void digit_rows_of(std::vector<DigitRows>& out, int32_t row, int n, int32
 
 // Whether a plan's FP64 matvec runs on digits: from 1.2 million multiply-adds in
 // stage 1.  Below, the FP64 kernels finish before the digit kernels' latencies
-// add up (Heisenberg D = 128, 0.4 million: 23 us against 29; D = 181, 1.1
-// million: 33 and 33); above, their pipe is the limit (Hubbard D = 362, 1.3
-// million: 44 against 31 us; D = 512: 56 against 36; D = 2048, 230 million: 701
-// against 149; Heisenberg D = 512, 25 million: 151 against 51; cylinder D =
+// add up (Heisenberg D = 128, 0.4 million: 17 us against 29; Hubbard D = 256,
+// 0.4 million: 31 against 28); above, their pipe is the limit (Hubbard D = 362,
+// 1.3 million: 38 against 31 us; D = 512: 50 against 36; D = 2048, 230 million:
+// 701 against 149; Heisenberg D = 512, 25 million: 151 against 51; cylinder D =
 // 2048, 13 billion: 40.9 ms against 1.84).  A plan of less than a dozen stage-3
 // tiles keeps its three launches up to 8 million: small plans of a few sectors
 // are relied on to be three launches (digits would take 58 us against 85 at 6.2
@@ -593,7 +601,7 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
     if (!digit_maps(d->m1, d->l, d->x, err) || !digit_maps(d->m3, d->t2, d->r, err)) return cudaErrorInvalidValue;
     if ((e = launch_digit_rows(reinterpret_cast<const DigitRows*>(m + o_l), (int)lrows.size(), p.lq.p, nullptr, 1, d->l,
                                d->redo, 0)) != cudaSuccess ||
-        (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_c), (int)rcols.size(), p.rq.p, kxd, 0)) !=
+        (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_c), (int)rcols.size(), C.max_kch3, p.rq.p, kxd, 0)) !=
             cudaSuccess ||
         (e = launch_digit_rows(reinterpret_cast<const DigitRows*>(m + o_r), (int)rrows.size(), p.rq.p, kxd, -1, d->r,
                                d->redo, 0)) != cudaSuccess ||
@@ -704,15 +712,15 @@ static cudaError_t digits_stage(F64Stack& p, const double* x, double* y, cudaStr
 cudaError_t f64stack_stage(F64Stack& p, const double* x, double* y, cudaStream_t s, int stage) {
     if (p.dg) return digits_stage(p, x, y, s, stage);
     if (stage == 0 && p.n1 > 0)
-        stack_gemm1_f64_kernel<false><<<p.n1, ST, 0, s>>>(p.pieces1.p, p.segs.p, p.lq.p, nullptr, x, nullptr,
-                                                          p.xsrc.p, p.xstride.p, p.colbase.p, p.colstride.p, p.t1.p,
-                                                          nullptr);
-    else if (stage == 1 && p.njobs > 0)
-        stack_combine_f64_kernel<<<p.njobs, 128, 0, s>>>(p.jobs.p, p.terms.p, p.coef.p, p.t1.p, p.t2.p);
-    else if (stage == 2 && p.n3 > 0)
-        stack_gemm3_f64_kernel<false><<<p.n3, ST, 0, s>>>(p.pieces3.p, p.segs.p, p.t2.p, nullptr, p.rq.p, nullptr,
-                                                          p.yrow.p, y, nullptr);
-    return cudaGetLastError();
+        return launch_dependent(stack_gemm1_f64_kernel<false>, p.n1, ST, 0, s, p.pieces1.p, p.segs.p, p.lq.p, nullptr, x,
+                                nullptr, p.xsrc.p, p.xstride.p, p.colbase.p, p.colstride.p, p.t1.p, nullptr);
+    if (stage == 1 && p.njobs > 0)
+        return launch_dependent(stack_combine_f64_kernel, p.njobs, 128, 0, s, p.jobs.p, p.terms.p, p.coef.p, p.t1.p,
+                                p.t2.p);
+    if (stage == 2 && p.n3 > 0)
+        return launch_dependent(stack_gemm3_f64_kernel<false>, p.n3, ST, 0, s, p.pieces3.p, p.segs.p, p.t2.p, nullptr,
+                                p.rq.p, nullptr, p.yrow.p, y, nullptr);
+    return cudaSuccess;
 }
 
 cudaError_t f64stack_apply(F64Stack& p, const double* x, double* y, cudaStream_t s) {
@@ -726,18 +734,20 @@ cudaError_t f64stack_apply(F64Stack& p, const double* x, double* y, cudaStream_t
 cudaError_t f64stack_apply_complex(F64Stack& p, const double* xr, const double* xi, double* yr, double* yi,
                                    cudaStream_t s) {
     if (!p.cplx) return cudaErrorInvalidValue;
+    cudaError_t e = cudaSuccess;
     if (p.n1 > 0)
-        stack_gemm1_f64_kernel<true><<<p.n1, ST, 0, s>>>(p.pieces1.p, p.segs.p, p.lq.p, p.lq_im.p, xr, xi, p.xsrc.p,
-                                                         p.xstride.p, p.colbase.p, p.colstride.p, p.t1.p, p.t1_im.p);
-    if (p.njobs > 0) {
-        // the W_i W_j coefficients are real: the combine acts on each part
-        stack_combine_f64_kernel<<<p.njobs, 128, 0, s>>>(p.jobs.p, p.terms.p, p.coef.p, p.t1.p, p.t2.p);
-        stack_combine_f64_kernel<<<p.njobs, 128, 0, s>>>(p.jobs.p, p.terms.p, p.coef.p, p.t1_im.p, p.t2_im.p);
-    }
-    if (p.n3 > 0)
-        stack_gemm3_f64_kernel<true><<<p.n3, ST, 0, s>>>(p.pieces3.p, p.segs.p, p.t2.p, p.t2_im.p, p.rq.p, p.rq_im.p,
-                                                         p.yrow.p, yr, yi);
-    return cudaGetLastError();
+        e = launch_dependent(stack_gemm1_f64_kernel<true>, p.n1, ST, 0, s, p.pieces1.p, p.segs.p, p.lq.p, p.lq_im.p, xr, xi,
+                             p.xsrc.p, p.xstride.p, p.colbase.p, p.colstride.p, p.t1.p, p.t1_im.p);
+    // the W_i W_j coefficients are real: the combine acts on each part
+    if (e == cudaSuccess && p.njobs > 0)
+        e = launch_dependent(stack_combine_f64_kernel, p.njobs, 128, 0, s, p.jobs.p, p.terms.p, p.coef.p, p.t1.p, p.t2.p);
+    if (e == cudaSuccess && p.njobs > 0)
+        e = launch_dependent(stack_combine_f64_kernel, p.njobs, 128, 0, s, p.jobs.p, p.terms.p, p.coef.p, p.t1_im.p,
+                             p.t2_im.p);
+    if (e == cudaSuccess && p.n3 > 0)
+        e = launch_dependent(stack_gemm3_f64_kernel<true>, p.n3, ST, 0, s, p.pieces3.p, p.segs.p, p.t2.p, p.t2_im.p,
+                             p.rq.p, p.rq_im.p, p.yrow.p, yr, yi);
+    return e;
 }
 
 int f64stack_launches(const F64Stack& p) {
