@@ -208,7 +208,7 @@ tk_status tk_heff2_plan_footprint(const tk_env* env_l, const tk_env* env_r, cons
              8.0 * std::max<int64_t>(C.t1_total, 1) + 2.0 * (vb(C.tiles1) + vb(C.tiles3)) + vb(C.jobs) +
              vb(C.terms) + 8.0 * C.terms.size() + vb(C.yrow) + vb(C.t1col_base) + vb(C.t1col_stride) + vb(C.xsrc) +
              vb(C.xstride);
-        if (f64stack_on_digits(C)) {
+        if (f64stack_on_digits(C, false)) {
             // the same stacks and a psi copy as digits, an exponent a row
             double xrows = 0.0;
             for (const std::vector<TcTile>* v : {&C.tiles1, &C.tiles1x})

@@ -222,10 +222,27 @@ __device__ __forceinline__ TcTile tile_of(const TcTile* __restrict__ tiles, cons
     t.b_row = t.n0 = n0;
     t.b_cs = om.n;
     t.k_valid = om.k;
+    t.parts = 1;
     t.m_valid = min(kTcBM, om.m - m0);
     t.n_valid = min(kTcBN, om.n - n0);
     return t;
 }
+
+// The K of a tile: `parts` operands' K one after the other (two for complex
+// products), each from a chunk of its own; ring steps of KW, drained after at
+// most 64 k.
+struct KSteps {
+    int k, per, kch, total;  // K and ring steps of a part, chunks a part, ring steps
+    bool paired;             // two parts of one step each are drained together
+    __device__ __forceinline__ KSteps(const TcTile& t)
+        : k(t.k_valid), per((t.k_valid + KW - 1) / KW), kch((t.k_valid + kTcBK - 1) / kTcBK),
+          total(per * max(t.parts, 1)), paired(per == 1) {}
+    __device__ __forceinline__ int drains() const { return paired ? (total + 1) / 2 : total / max(per, 1) * kch; }
+    __device__ __forceinline__ bool first(int g) const { return paired ? (g & 1) == 0 : (g % per & 1) == 0; }
+    __device__ __forceinline__ bool last(int g) const {
+        return paired ? (g & 1) == 1 || g == total - 1 : (g % per & 1) == 1 || g % per == per - 1;
+    }
+};
 
 template <int MODE>
 __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* __restrict__ tiles,
@@ -287,14 +304,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
                 const int halves = t.n_valid > HN ? 2 : 1;
                 const int box = (t.m_valid + 31) >> 5;
                 const uint32_t bytes = kDigits * KW * 2 * (32 * box + HN * halves);
-                const int steps = (t.k_valid + KW - 1) / KW;
-                for (int q = 0; q < steps && ok; ++q, ++it) {
+                const KSteps ks(t);
+                for (int g = 0; g < ks.total && ok; ++g, ++it) {
+                    const int part = g / ks.per, q = g - part * ks.per;
                     const int st = it % kDigitRing;
                     uint8_t* base = smem + st * STAGE_BYTES;
                     if (it >= kDigitRing) ok = mbar_wait(&empty[st], (it / kDigitRing - 1) & 1, stop, redo);
                     if (!ok) break;
                     mbar_expect_tx(&full[st], bytes);
-                    const int x = (q & 1) * KW, c = q >> 1;
+                    const int x = (q & 1) * KW, c = part * ks.kch + (q >> 1);
                     tma_load_3d(base, &maps.a[box - 1], x, t.a_row + c * t.a_cs, &full[st]);
                     for (int h = 0; h < halves; ++h)
                         tma_load_3d(base + A_BYTES + h * H_BYTES, &maps.b, x, t.b_row + c * t.b_cs + HN * h, &full[st]);
@@ -312,10 +330,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
                 const TcTile t = tile_of<MODE>(tiles, om, ti);
                 const int halves = t.n_valid > HN ? 2 : 1;
                 const uint32_t astep = (uint32_t)((((t.m_valid + 31) >> 5) * 32) * KW * 2);
-                const int steps = (t.k_valid + KW - 1) / KW;
-                for (int q = 0; q < steps && ok; ++q, ++it) {
+                const KSteps k(t);
+                for (int g = 0; g < k.total && ok; ++g, ++it) {
+                    const int q = g % k.per;
                     const int st = it % kDigitRing;
-                    const bool first = (q & 1) == 0, last = (q & 1) == 1 || q == steps - 1;
+                    const bool first = k.first(g), last = k.last(g);
                     ok = mbar_wait(&full[st], (it / kDigitRing) & 1, stop, redo);
                     const uint32_t sa = smem_u32(smem + st * STAGE_BYTES);
                     const int ks = min(KW / 16, (t.k_valid - q * KW + 15) / 16);
@@ -386,7 +405,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
             Sum acc[WCOLS];
 #pragma unroll
             for (int i = 0; i < WCOLS; ++i) acc[i] = {0, 0};
-            const int chunks = (t.k_valid + kTcBK - 1) / kTcBK;
+            const int chunks = KSteps(t).drains();
             for (int c = 0; c < chunks && ok; ++c) {
                 ok = mbar_wait(&acc_full[buf], drains & 1, stop, redo);
                 ok = __all_sync(0xffffffffu, ok);
@@ -454,7 +473,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
                     step = pitch[g];
                     o = om.out + place[g] + (int64_t)(t.ldc + row0 + r0) * step;
                 } else if (MODE == 1) {
-                    o = om.out + t.n0 + col;
+                    // columns from `split` on are the imaginary part's
+                    const int at = t.n0 + col;
+                    o = t.split > 0 && at >= t.split ? om.out_im + (at - t.split) : om.out + at;
                 } else {
                     step = om.c_rs;
                     o = om.out + (int64_t)(t.n0 + col) * om.c_cs + (int64_t)(t.ldc + row0 + r0) * step;
@@ -540,6 +561,23 @@ __device__ __forceinline__ void put_digits(const DigitStack& o, int64_t row, int
     for (int j = 0; j < kDigits; ++j) p[j * (o.rows << 5)] = d[j];
 }
 
+// A complex operand's digits d + i f at chunk offsets c0 (first part) and c1.
+template <bool DUAL>
+__device__ __forceinline__ void put_complex(const DigitStack& o, int64_t row, int n_dual, int64_t c0, int64_t c1, int k,
+                                            const uint32_t* d, const uint32_t* f) {
+    put_digits(o, row + c0, k, d);
+    if (!DUAL) {
+        put_digits(o, row + c1, k, f);
+        return;
+    }
+    put_digits(o, row + n_dual + c0, k, f);
+    put_digits(o, row + n_dual + c1, k, d);
+    uint32_t m[kDigits];
+#pragma unroll
+    for (int j = 0; j < kDigits; ++j) m[j] = f[j] ^ 0x80008000u;
+    put_digits(o, row + c1, k, m);
+}
+
 // Exponent of x 2^k (below 1 for subnormals), kNoExponent for zero.
 constexpr int kNoExponent = -(1 << 20);
 __device__ __forceinline__ int exponent_of(double x, int k) {
@@ -551,14 +589,19 @@ __device__ __forceinline__ int exponent_of(double x, int k) {
 
 // One CTA per 64-wide chunk of a stack (blockIdx.y, past the stack's last: nothing): the columns' exponents.
 __global__ void __launch_bounds__(256) digit_columns_kernel(const DigitRows* __restrict__ jobs,
-                                                            const double* __restrict__ q64, int32_t* __restrict__ kx) {
+                                                            const double* __restrict__ q64,
+                                                            const double* __restrict__ q64_im, int32_t* __restrict__ kx) {
     __shared__ uint32_t top[4][kTcBK];
     const DigitRows j = jobs[blockIdx.x];
     const int k = threadIdx.x & 63, w = threadIdx.x >> 6, c = blockIdx.y;
     if (c >= j.kch) return;
     uint32_t mx = 0;
 #pragma unroll 4
-    for (int r = w; r < j.n; r += 4) mx = max(mx, abs_hi(q64[(((int64_t)j.row + (int64_t)c * j.cs + r) << 6) + k]));
+    for (int r = w; r < j.n; r += 4) {
+        const int64_t at = (((int64_t)j.row + (int64_t)c * j.cs + r) << 6) + k;
+        mx = max(mx, abs_hi(q64[at]));
+        if (q64_im) mx = max(mx, abs_hi(q64_im[at]));
+    }
     top[w][k] = mx;
     __syncthreads();
     if (w != 0) return;
@@ -616,6 +659,110 @@ __global__ void __launch_bounds__(32 * kDigitRowsPerCta) digit_rows_kernel(const
         if (c < j.kch) put(c, v[c]);
 #pragma unroll 2
     for (int c = kKeep; c < j.kch; ++c) put(c, at(c));
+}
+
+// The same for a complex operand (planar): the row's two parts on one grid, the
+// real part's chunks first, out row `to` + r (chunks `cs_out` apart).  DUAL (the
+// B operand of a product): row r holds (re | -im), row r + n_dual (im | re).
+template <bool DUAL>
+__global__ void __launch_bounds__(32 * kDigitRowsPerCta) digit_rows_complex_kernel(const DigitRowsC* __restrict__ jobs,
+                                                                                   const double* __restrict__ re,
+                                                                                   const double* __restrict__ im,
+                                                                                   const int32_t* __restrict__ kx,
+                                                                                   int sign, const DigitStack out,
+                                                                                   int* redo) {
+    const DigitRowsC j = jobs[blockIdx.x];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    dep_launch();
+    if (w >= j.n) return;
+    dep_wait();
+    const int64_t row = (int64_t)j.row + w, to = (int64_t)j.to + w;
+    auto at = [&](const double* q, int c) {
+        return reinterpret_cast<const double2*>(q + ((row + (int64_t)c * j.cs) << 6))[lane];
+    };
+    auto scale = [&](int c) {
+        if (j.kx < 0) return make_int2(0, 0);
+        const int2 k = reinterpret_cast<const int2*>(kx + j.kx + c * kTcBK)[lane];
+        return make_int2(sign * k.x, sign * k.y);
+    };
+    int mx = kNoExponent;
+    uint32_t hi = 0;
+#pragma unroll 2
+    for (int c = 0; c < j.kch; ++c) {
+        const double2 a = at(re, c), b = at(im, c);
+        const int2 k = scale(c);
+        hi = max(max(hi, max(abs_hi(a.x), abs_hi(a.y))), max(abs_hi(b.x), abs_hi(b.y)));
+        mx = max(max(mx, max(exponent_of(a.x, k.x), exponent_of(a.y, k.y))),
+                 max(exponent_of(b.x, k.x), exponent_of(b.y, k.y)));
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (hi >= 0x7FF00000u) atomicExch(redo, kDigitValue);
+    const int ex = mx == kNoExponent ? 1 : mx;
+    if (lane == 0) {
+        out.ex[to] = ex;
+        if (DUAL) out.ex[to + j.n_dual] = ex;
+    }
+    for (int c = 0; c < j.kch; ++c) {
+        const double2 a = at(re, c), b = at(im, c);
+        const int2 k = scale(c);
+        uint32_t d[kDigits], f[kDigits];
+        digits2(a.x, a.y, ex, d, k.x, k.y);
+        digits2(b.x, b.y, ex, f, k.x, k.y);
+        put_complex<DUAL>(out, to, j.n_dual, (int64_t)c * j.cs_out, (int64_t)(j.kch + c) * j.cs_out, 2 * lane, d, f);
+    }
+}
+
+// psi sub-blocks of a complex vector: digit_psi_kernel's work on both parts.
+__global__ void __launch_bounds__(256) digit_psi_complex_kernel(const DigitPsiC* __restrict__ jobs,
+                                                                const double* __restrict__ xr,
+                                                                const double* __restrict__ xi, const DigitStack out,
+                                                                int* redo) {
+    __shared__ uint32_t smax[32];
+    __shared__ double tr[32][kTcBK + 1], ti[32][kTcBK + 1];
+    const DigitPsiC j = jobs[blockIdx.x];
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const int nr = j.cols, K = j.rows, kch = (K + kTcBK - 1) / kTcBK;
+    const int64_t src = j.src + lane;
+    dep_launch();
+    if (tid < 32) smax[tid] = 0;
+    __syncthreads();
+    dep_wait();
+    uint32_t mx = 0;
+#pragma unroll 2
+    for (int k = w; k < K; k += 8) {
+        const int64_t o = src + (int64_t)k * j.pitch;
+        if (lane < nr) mx = max(mx, max(abs_hi(xr[o]), abs_hi(xi[o])));
+    }
+    atomicMax(&smax[lane], mx);
+    __syncthreads();
+    if (tid < nr) {
+        const int ex = row_exponent(smax[tid], redo);
+        out.ex[(int64_t)j.to + tid] = ex;
+        out.ex[(int64_t)j.to + j.n_dual + tid] = ex;
+        smax[tid] = (uint32_t)ex;
+    }
+    for (int c = 0; c < kch; ++c) {
+        const int k0 = c * kTcBK;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kTcBK / 8; ++i) {
+            const int k = k0 + w + i * 8;
+            const bool in = lane < nr && k < K;
+            const int64_t o = src + (int64_t)k * j.pitch;
+            tr[lane][k - k0] = in ? xr[o] : 0.0;
+            ti[lane][k - k0] = in ? xi[o] : 0.0;
+        }
+        __syncthreads();
+        const int kv = (min(kTcBK, K - k0) + 15) & ~15;  // whole 16-wide steps are multiplied
+        for (int r = w; r < nr; r += 8)
+            if (2 * lane < kv) {
+                uint32_t d[kDigits], f[kDigits];
+                digits2(tr[r][2 * lane], tr[r][2 * lane + 1], (int)smax[r], d);
+                digits2(ti[r][2 * lane], ti[r][2 * lane + 1], (int)smax[r], f);
+                put_complex<true>(out, (int64_t)j.to + r, j.n_dual, (int64_t)c * j.cs_out, (int64_t)(kch + c) * j.cs_out,
+                                  2 * lane, d, f);
+            }
+    }
 }
 
 // psi sub-blocks: 32 columns x all K rows by one CTA, lanes along the columns;
@@ -773,7 +920,7 @@ void digit_schedule(const std::vector<TcTile>& in, int ctas, std::vector<TcTile>
     // microseconds a tile holds its SM: the product per 64 k, then the ends
     // (measured on Hubbard D = 2048 and on dense products)
     auto cost = [](const TcTile& t) {
-        const double halves = t.n_valid > HN ? 2.0 : 1.0, k = std::ceil(t.k_valid / (double)KW) * 0.5;
+        const double halves = t.n_valid > HN ? 2.0 : 1.0, k = std::ceil(t.k_valid / (double)KW) * 0.5 * std::max(t.parts, 1);
         return 1.0 + k * (0.8 + 1.4 * halves) + 4.0 * t.m_valid * t.n_valid / (kTcBM * (double)kTcBN);
     };
     auto pack = [&](const std::vector<TcTile>& v, std::vector<int>& cta) {
@@ -822,10 +969,10 @@ void digit_schedule(const std::vector<TcTile>& in, int ctas, std::vector<TcTile>
     }
 }
 
-cudaError_t launch_digit_columns(const DigitRows* jobs, int n_jobs, int max_kch, const double* q64, int32_t* kx,
-                                 cudaStream_t s) {
+cudaError_t launch_digit_columns(const DigitRows* jobs, int n_jobs, int max_kch, const double* q64, const double* q64_im,
+                                 int32_t* kx, cudaStream_t s) {
     if (n_jobs <= 0 || max_kch <= 0) return cudaSuccess;
-    digit_columns_kernel<<<dim3((unsigned)n_jobs, (unsigned)max_kch), 256, 0, s>>>(jobs, q64, kx);
+    digit_columns_kernel<<<dim3((unsigned)n_jobs, (unsigned)max_kch), 256, 0, s>>>(jobs, q64, q64_im, kx);
     return cudaGetLastError();
 }
 
@@ -833,6 +980,20 @@ cudaError_t launch_digit_rows(const DigitRows* jobs, int n_jobs, const double* q
                               const DigitStack& out, int* redo, cudaStream_t s) {
     if (n_jobs <= 0) return cudaSuccess;
     return launch_dependent(digit_rows_kernel, n_jobs, 32 * kDigitRowsPerCta, 0, s, jobs, q64, kx, sign, out, redo);
+}
+
+cudaError_t launch_digit_rows_complex(const DigitRowsC* jobs, int n_jobs, const double* re, const double* im,
+                                      const int32_t* kx, int sign, bool dual, const DigitStack& out, int* redo,
+                                      cudaStream_t s) {
+    if (n_jobs <= 0) return cudaSuccess;
+    return launch_dependent(dual ? digit_rows_complex_kernel<true> : digit_rows_complex_kernel<false>, n_jobs,
+                            32 * kDigitRowsPerCta, 0, s, jobs, re, im, kx, sign, out, redo);
+}
+
+cudaError_t launch_digit_psi_complex(const DigitPsiC* jobs, int n_jobs, const double* xr, const double* xi,
+                                     const DigitStack& out, int* redo, cudaStream_t s) {
+    if (n_jobs <= 0) return cudaSuccess;
+    return launch_dependent(digit_psi_complex_kernel, n_jobs, 256, 0, s, jobs, xr, xi, out, redo);
 }
 
 cudaError_t launch_digit_matrices(const DigitMatrix& a, const DigitMatrix& b, int K, int* redo, cudaStream_t s) {

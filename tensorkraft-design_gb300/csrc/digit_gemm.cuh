@@ -56,6 +56,17 @@ inline size_t digit_stack_bytes(int64_t rows) { return (size_t)rows * kTcBK * kD
 struct DigitRows {
     int32_t row, n, cs, kch, kx, pad;
 };
+// The same of a complex stack: its digits go to rows to .. of a stack whose
+// chunks are cs_out rows apart (the imaginary part's chunks behind the real
+// part's), the second form of a B operand n_dual rows further.
+struct DigitRowsC {
+    int32_t row, n, cs, kch, kx, to, cs_out, n_dual;
+};
+// Columns [0, cols) at src of a psi sub-block (rows x pitch), as a B operand.
+struct DigitPsiC {
+    int64_t src;
+    int32_t rows, cols, pitch, to, cs_out, n_dual;
+};
 constexpr int kDigitRowsPerCta = 8;
 
 // Tensor maps of one product's operands: A in boxes of 32, 64, 96 or 128 rows
@@ -71,6 +82,7 @@ bool digit_maps(DigitMaps& m, const DigitStack& a, const DigitStack& b, std::str
 // single product whose tiles need no table).
 struct DigitOut {
     double* out;
+    double* out_im;  // mode 1, complex products: where a tile's columns from `split` on go
     const int64_t* rowtab;
     const int64_t* colbase;
     const int32_t* colstride;
@@ -97,12 +109,17 @@ cudaError_t launch_digit_gemm(int mode, const TcTile* tiles, const int32_t* begi
 
 // Exponents of a stack's columns: kx[j.kx + k] = floor(log2 max |x|) over the
 // rows [row, row + n) of job j at k, 0 for a column of zeros.
-cudaError_t launch_digit_columns(const DigitRows* jobs, int n_jobs, int max_kch, const double* q64, int32_t* kx,
-                                 cudaStream_t s);
+cudaError_t launch_digit_columns(const DigitRows* jobs, int n_jobs, int max_kch, const double* q64, const double* q64_im,
+                                 int32_t* kx, cudaStream_t s);
 // Digits of FP64 operand stacks (rows of 64 doubles per chunk), of
 // x 2^(sign * kx) where the job has scales.
 cudaError_t launch_digit_rows(const DigitRows* jobs, int n_jobs, const double* q64, const int32_t* kx, int sign,
                               const DigitStack& out, int* redo, cudaStream_t s);
+cudaError_t launch_digit_rows_complex(const DigitRowsC* jobs, int n_jobs, const double* re, const double* im,
+                                      const int32_t* kx, int sign, bool dual, const DigitStack& out, int* redo,
+                                      cudaStream_t s);
+cudaError_t launch_digit_psi_complex(const DigitPsiC* jobs, int n_jobs, const double* xr, const double* xi,
+                                     const DigitStack& out, int* redo, cudaStream_t s);
 // Digits of both operands of a dense product (*redo is set for operands that
 // one grid per row would hold less exactly than FP64): row r, k of K at
 // x[r * rs + k * ks], into stacks whose chunks are `rows` rows apart.

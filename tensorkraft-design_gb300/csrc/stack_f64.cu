@@ -316,33 +316,38 @@ struct RedoArgs {
     const KSeg* segs;
     const TcCombJob* jobs;
     const TcCombTerm* terms;
-    const double *coef, *lq, *rq;
+    const double *coef, *lq, *rq, *lq_im, *rq_im;
     const int64_t *xsrc, *colbase, *yrow;
     const int32_t *xstride, *colstride;
-    double *t1, *t2;
+    double *t1, *t2, *t1_im, *t2_im;
     int n1, n3, njobs;
 };
 __device__ __forceinline__ void cluster_barrier() {
     __threadfence();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+template <bool CPLX>
 __global__ void __cluster_dims__(kRedoCtas, 1, 1) __launch_bounds__(ST)
-    stack_redo_f64_kernel(const RedoArgs a, const double* __restrict__ x, double* __restrict__ y, int* redo) {
-    __shared__ PieceTiles<false> sm;
+    stack_redo_f64_kernel(const RedoArgs a, const double* __restrict__ x, const double* __restrict__ x_im,
+                          double* __restrict__ y, double* __restrict__ y_im, int* redo) {
+    __shared__ PieceTiles<CPLX> sm;
     dep_launch();
     dep_wait();
     if (*(volatile int*)redo == 0) return;
     for (int i = blockIdx.x; i < a.n1; i += kRedoCtas) {
         __syncthreads();
-        stack_piece1<false>(a.pieces1[i], sm, a.segs, a.lq, nullptr, x, nullptr, a.xsrc, a.xstride, a.colbase,
-                            a.colstride, a.t1, nullptr);
+        stack_piece1<CPLX>(a.pieces1[i], sm, a.segs, a.lq, a.lq_im, x, x_im, a.xsrc, a.xstride, a.colbase, a.colstride,
+                           a.t1, a.t1_im);
     }
     cluster_barrier();
-    for (int i = blockIdx.x; i < a.njobs; i += kRedoCtas) stack_combine_job(a.jobs[i], a.terms, a.coef, a.t1, a.t2);
+    for (int i = blockIdx.x; i < a.njobs; i += kRedoCtas) {
+        stack_combine_job(a.jobs[i], a.terms, a.coef, a.t1, a.t2);
+        if constexpr (CPLX) stack_combine_job(a.jobs[i], a.terms, a.coef, a.t1_im, a.t2_im);
+    }
     cluster_barrier();
     for (int i = blockIdx.x; i < a.n3; i += kRedoCtas) {
         __syncthreads();
-        stack_piece3<false>(a.pieces3[i], sm, a.segs, a.t2, nullptr, a.rq, nullptr, a.yrow, y, nullptr);
+        stack_piece3<CPLX>(a.pieces3[i], sm, a.segs, a.t2, a.t2_im, a.rq, a.rq_im, a.yrow, y, y_im);
     }
     cluster_barrier();
     if (blockIdx.x == 0 && threadIdx.x == 0) *redo = 0;
@@ -475,6 +480,11 @@ struct F64Digits {
     const int32_t *begin1 = nullptr, *begin3 = nullptr;
     const TcSplitJob* psi = nullptr;
     const DigitRows* rows = nullptr;  // of T2
+    // complex plans: the same jobs for planar operands, T1's column tables for both parts
+    const DigitPsiC* psi_c = nullptr;
+    const DigitRowsC* rows_c = nullptr;
+    const int64_t* colbase = nullptr;
+    const int32_t* colstride = nullptr;
     int* redo = nullptr;
     DigitMaps m1, m3;
     int npsi = 0, nrows = 0, sms = 0;
@@ -513,17 +523,164 @@ static void digit_rows_of(std::vector<DigitRows>& out, int32_t row, int n, int32
 // tiles keeps its three launches up to 8 million: small plans of a few sectors
 // are relied on to be three launches (digits would take 58 us against 85 at 6.2
 // million on ten tiles).
-bool f64stack_on_digits(const TcTables& C) {
+bool f64stack_on_digits(const TcTables& C, bool cplx) {
     double f = 0.0;
     for (const std::vector<TcTile>* v : {&C.tiles1, &C.tiles1x})
-        for (const TcTile& t : *v) f += (double)t.m_valid * t.n_valid * t.k_valid;
+        for (const TcTile& t : *v) f += (cplx ? 4.0 : 1.0) * t.m_valid * t.n_valid * t.k_valid;
     return f >= (C.tiles3.size() + C.tiles3f.size() < 12 ? 8e6 : 1.2e6);
+}
+
+// Room behind the tables for the digits and the column scales; the tables go up
+// in one copy, everything in one allocation.
+static cudaError_t digits_alloc(F64Digits& d, const Blob& blob, const int64_t (&rows)[4], int32_t nk, int32_t** kx) {
+    std::vector<unsigned char> host(blob.size());
+    blob.copy_to(host.data());
+    size_t total = blob.size(), q[4], x[4];
+    auto take = [&](size_t n) {
+        const size_t at = (total + 1023) & ~(size_t)1023;
+        total = at + n;
+        return at;
+    };
+    DigitStack* st[4] = {&d.l, &d.r, &d.t2, &d.x};
+    for (int i = 0; i < 4; ++i) {
+        st[i]->rows = std::max<int64_t>(rows[i], 1);
+        q[i] = take(digit_stack_bytes(st[i]->rows));
+        x[i] = take(sizeof(int32_t) * (size_t)st[i]->rows);
+    }
+    const size_t k = take(sizeof(int32_t) * (size_t)std::max(nk, 1));
+    cudaError_t e;
+    if ((e = d.mem.alloc(total)) != cudaSuccess ||
+        (e = cudaMemcpy(d.mem.p, host.data(), host.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
+        return e;
+    for (int i = 0; i < 4; ++i) {
+        st[i]->q = reinterpret_cast<__half*>(d.mem.p + q[i]);
+        st[i]->ex = reinterpret_cast<int32_t*>(d.mem.p + x[i]);
+    }
+    *kx = reinterpret_cast<int32_t*>(d.mem.p + k);
+    d.kx = *kx;
+    return cudaSuccess;
+}
+
+// The digit form of a complex plan: the same products on operands of two parts.
+// Row (A, T2): (re | im); column (psi, R): re (re | -im), im (im | re), the im
+// columns behind the re ones, so that one tile may hold both.
+static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::unique_ptr<F64Digits> d, std::string& err) {
+    struct Stack {
+        int32_t M = 0, N = 0, K = 0, kch = 0, a = INT32_MAX, b = INT32_MAX;  // rows, columns, K; first rows of A and B
+        int64_t out = INT64_MAX;  // first entry of the column table (stage 1) or row table (stage 3)
+    };
+    if (std::max({C.lq_rows, C.rq_rows, C.t2q_rows, C.xq_rows}) > INT32_MAX / 4) return cudaSuccess;  // 32-bit rows
+    std::map<int32_t, Stack> s1, s3;  // by the first row of the operand that names the stack
+    for (const std::vector<TcTile>* v : {&C.tiles1x, &C.tiles3})
+        for (const TcTile& t : *v) {
+            Stack& s = t.mode == 2 ? s1[t.a_row - t.ldc] : s3[t.b_row - t.n0];
+            s.M = t.a_cs, s.N = t.b_cs, s.K = t.k_valid, s.kch = t.kch;
+            s.a = std::min(s.a, t.a_row), s.b = std::min(s.b, t.b_row), s.out = std::min(s.out, t.out_off);
+        }
+    std::vector<TcTile> w1, w3, t1, t3;
+    std::vector<int32_t> b1, b3;
+    std::vector<DigitRowsC> lrows, rrows, trows;
+    std::vector<DigitRows> rcols;
+    std::vector<DigitPsiC> psi;
+    std::vector<int64_t> colbase(2 * C.t1col_base.size());
+    std::vector<int32_t> colstride(2 * C.t1col_stride.size());
+    const int64_t im = p.t1_im.p - p.t1.p;  // from T1's real part to its imaginary part
+    int32_t nk = 0;
+    auto rows = [](std::vector<DigitRowsC>& out, int32_t row, int n, int32_t cs, int32_t kch, int32_t kx, int32_t to,
+                   int32_t cs_out, int32_t n_dual) {
+        for (int r = 0; r < n; r += kDigitRowsPerCta)
+            out.push_back({row + r, std::min(kDigitRowsPerCta, n - r), cs, kch, kx, to + r, cs_out, n_dual});
+    };
+    auto tiles = [](std::vector<TcTile>& out, const Stack& s, int mode) {
+        for (int32_t m = 0; m < s.M; m += kTcBM)
+            for (int32_t n = 0; n < 2 * s.N; n += kTcBN) {
+                TcTile t{};
+                t.a_row = 2 * s.a + m, t.a_cs = s.M;
+                t.b_row = 4 * s.b + n, t.b_cs = 2 * s.N;
+                t.kch = s.kch, t.k_valid = s.K, t.parts = 2;
+                t.m_valid = std::min(kTcBM, s.M - m), t.n_valid = std::min(kTcBN, 2 * s.N - n);
+                t.mode = mode;
+                t.ldc = m, t.n0 = n;
+                t.out_off = mode == 2 ? 2 * s.out + n : s.out + m;
+                t.split = mode == 1 ? s.N : 0;
+                out.push_back(t);
+            }
+    };
+    std::map<int32_t, const Stack*> by_psi;  // stage-1 stacks by their first psi row
+    for (const auto& [key, s] : s1) {
+        by_psi[s.b] = &s;
+        tiles(w1, s, 2);
+        rows(lrows, s.a, s.M, s.M, s.kch, -1, 2 * s.a, s.M, 0);
+        for (int32_t c = 0; c < s.N; ++c)
+            for (int h = 0; h < 2; ++h) {
+                colbase[(size_t)(2 * s.out + h * s.N + c)] = C.t1col_base[(size_t)(s.out + c)] + h * im;
+                colstride[(size_t)(2 * s.out + h * s.N + c)] = C.t1col_stride[(size_t)(s.out + c)];
+            }
+    }
+    for (const TcSplitJob& j : C.split) {
+        if (j.a0 != 0) continue;
+        auto it = by_psi.upper_bound(j.xrow);
+        if (it == by_psi.begin()) {
+            err = "digit operands: psi sub-block outside every stack";
+            return cudaErrorInvalidValue;
+        }
+        const Stack& s = *std::prev(it)->second;
+        psi.push_back({j.src + j.b0, j.rows, std::min(32, j.cols - j.b0), j.cols, 4 * s.b + (j.xrow - s.b) + j.b0, 2 * s.N,
+                       s.N});
+    }
+    for (const auto& [key, s] : s3) {
+        tiles(w3, s, 1);
+        rcols.push_back({s.b, s.N, s.N, s.kch, nk, 0});
+        rows(rrows, s.b, s.N, s.N, s.kch, nk, 4 * s.b, 2 * s.N, s.N);
+        rows(trows, s.a, s.M, s.M, s.kch, nk, 2 * s.a, s.M, 0);
+        nk += s.kch * kTcBK;
+    }
+    cudaError_t e;
+    int redo = 0, dev = 0;
+    int32_t* kx = nullptr;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
+        (e = digit_setup()) != cudaSuccess)
+        return e;
+    digit_schedule(w1, d->sms, t1, b1);
+    digit_schedule(w3, d->sms, t3, b3);
+    Blob blob;
+    auto table = [&](const auto& v) { return blob.add(v.data(), sizeof(v[0]) * v.size()); };
+    const size_t o_redo = blob.add(&redo, sizeof(redo)), o_t1 = table(t1), o_t3 = table(t3), o_b1 = table(b1),
+                 o_b3 = table(b3), o_psi = table(psi), o_rows = table(trows), o_l = table(lrows), o_r = table(rrows),
+                 o_c = table(rcols), o_cb = table(colbase), o_cs = table(colstride);
+    if ((e = digits_alloc(*d, blob, {2 * C.lq_rows, 4 * C.rq_rows, 2 * C.t2q_rows, 4 * C.xq_rows}, nk, &kx)) != cudaSuccess)
+        return e;
+    unsigned char* m = d->mem.p;
+    d->tiles1 = reinterpret_cast<const TcTile*>(m + o_t1);
+    d->tiles3 = reinterpret_cast<const TcTile*>(m + o_t3);
+    d->begin1 = reinterpret_cast<const int32_t*>(m + o_b1);
+    d->begin3 = reinterpret_cast<const int32_t*>(m + o_b3);
+    d->psi_c = reinterpret_cast<const DigitPsiC*>(m + o_psi);
+    d->rows_c = reinterpret_cast<const DigitRowsC*>(m + o_rows);
+    d->colbase = reinterpret_cast<const int64_t*>(m + o_cb);
+    d->colstride = reinterpret_cast<const int32_t*>(m + o_cs);
+    d->redo = reinterpret_cast<int*>(m + o_redo);
+    if (!digit_maps(d->m1, d->l, d->x, err) || !digit_maps(d->m3, d->t2, d->r, err)) return cudaErrorInvalidValue;
+    if ((e = launch_digit_rows_complex(reinterpret_cast<const DigitRowsC*>(m + o_l), (int)lrows.size(), p.lq.p, p.lq_im.p,
+                                       nullptr, 1, false, d->l, d->redo, 0)) != cudaSuccess ||
+        (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_c), (int)rcols.size(), C.max_kch3, p.rq.p,
+                                  p.rq_im.p, kx, 0)) != cudaSuccess ||
+        (e = launch_digit_rows_complex(reinterpret_cast<const DigitRowsC*>(m + o_r), (int)rrows.size(), p.rq.p, p.rq_im.p,
+                                       kx, -1, true, d->r, d->redo, 0)) != cudaSuccess ||
+        (e = cudaMemcpy(&redo, d->redo, sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess)
+        return e;
+    d->npsi = (int)psi.size();
+    d->nrows = (int)trows.size();
+    if (redo == 0) p.dg = std::move(d);
+    return cudaSuccess;
 }
 
 // Builds the digit form of p; left out (dg null) where the constant operands
 // hold infinities or NaNs.
 static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& err) {
     std::unique_ptr<F64Digits> d(new F64Digits);
+    if (p.cplx) return digits_create_complex(C, p, std::move(d), err);
     std::vector<DigitRows> lrows, rrows, trows, rcols;
     std::vector<TcSplitJob> psi;
     for (const TcSplitJob& j : C.split)
@@ -561,36 +718,9 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
     const size_t o_redo = blob.add(&redo, sizeof(redo)), o_t1 = table(t1), o_t3 = table(t3), o_b1 = table(b1),
                  o_b3 = table(b3), o_psi = table(psi), o_rows = table(trows), o_l = table(lrows), o_r = table(rrows),
                  o_c = table(rcols);
-    std::vector<unsigned char> host(blob.size());
-    blob.copy_to(host.data());
-    size_t total = blob.size();
-    auto take = [&](size_t n) {
-        const size_t at = (total + 1023) & ~(size_t)1023;
-        total = at + n;
-        return at;
-    };
-    struct Place {
-        DigitStack* s;
-        size_t q, x;
-    };
-    std::vector<Place> places;
-    for (auto [s, rows] : {std::pair<DigitStack*, int64_t>{&d->l, C.lq_rows}, {&d->r, C.rq_rows}, {&d->t2, C.t2q_rows},
-                           {&d->x, C.xq_rows}}) {
-        s->rows = std::max<int64_t>(rows, 1);
-        const size_t q = take(digit_stack_bytes(s->rows));
-        places.push_back({s, q, take(sizeof(int32_t) * (size_t)s->rows)});
-    }
-    const size_t o_kx = take(sizeof(int32_t) * (size_t)std::max(nk, 1));
-    if ((e = d->mem.alloc(total)) != cudaSuccess ||
-        (e = cudaMemcpy(d->mem.p, host.data(), host.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
-        return e;
+    int32_t* kxd = nullptr;
+    if ((e = digits_alloc(*d, blob, {C.lq_rows, C.rq_rows, C.t2q_rows, C.xq_rows}, nk, &kxd)) != cudaSuccess) return e;
     unsigned char* m = d->mem.p;
-    for (const Place& pl : places) {
-        pl.s->q = reinterpret_cast<__half*>(m + pl.q);
-        pl.s->ex = reinterpret_cast<int32_t*>(m + pl.x);
-    }
-    int32_t* kxd = reinterpret_cast<int32_t*>(m + o_kx);
-    d->kx = kxd;
     d->tiles1 = reinterpret_cast<const TcTile*>(m + o_t1);
     d->tiles3 = reinterpret_cast<const TcTile*>(m + o_t3);
     d->begin1 = reinterpret_cast<const int32_t*>(m + o_b1);
@@ -601,7 +731,7 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
     if (!digit_maps(d->m1, d->l, d->x, err) || !digit_maps(d->m3, d->t2, d->r, err)) return cudaErrorInvalidValue;
     if ((e = launch_digit_rows(reinterpret_cast<const DigitRows*>(m + o_l), (int)lrows.size(), p.lq.p, nullptr, 1, d->l,
                                d->redo, 0)) != cudaSuccess ||
-        (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_c), (int)rcols.size(), C.max_kch3, p.rq.p, kxd, 0)) !=
+        (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_c), (int)rcols.size(), C.max_kch3, p.rq.p, nullptr, kxd, 0)) !=
             cudaSuccess ||
         (e = launch_digit_rows(reinterpret_cast<const DigitRows*>(m + o_r), (int)rrows.size(), p.rq.p, kxd, -1, d->r,
                                d->redo, 0)) != cudaSuccess ||
@@ -675,12 +805,18 @@ tk_status f64stack_create(const TcTables& C, std::unique_ptr<F64Stack, F64StackD
     p->n1 = (int)p1.size();
     p->n3 = (int)p3.size();
     p->njobs = (int)C.jobs.size();
-    if (!p->cplx && f64stack_on_digits(C) && (e = digits_create(C, *p, err)) != cudaSuccess) {
+    if (f64stack_on_digits(C, p->cplx) && (e = digits_create(C, *p, err)) != cudaSuccess) {
         if (err.empty()) err = std::string("digit operands: ") + cudaGetErrorString(e);
         return e == cudaErrorMemoryAllocation ? TK_ERR_OOM : TK_ERR_CUDA;
     }
     out = std::move(p);
     return TK_OK;
+}
+
+static RedoArgs redo_args(const F64Stack& p) {
+    return RedoArgs{p.pieces1.p, p.pieces3.p, p.segs.p,  p.jobs.p,    p.terms.p,     p.coef.p, p.lq.p, p.rq.p, p.lq_im.p,
+                    p.rq_im.p,   p.xsrc.p,    p.colbase.p, p.yrow.p,  p.xstride.p, p.colstride.p, p.t1.p,   p.t2.p, p.t1_im.p,
+                    p.t2_im.p,   p.n1,        p.n3,      p.njobs};
 }
 
 // One stage of the digit matvec.
@@ -704,9 +840,34 @@ static cudaError_t digits_stage(F64Stack& p, const double* x, double* y, cudaStr
     o.out = y;
     o.rowtab = p.yrow.p;
     if ((e = launch_digit_gemm(1, d.tiles3, d.begin3, d.sms, d.m3, d.t2.ex, d.r.ex, o, d.redo, s)) != cudaSuccess) return e;
-    const RedoArgs a{p.pieces1.p, p.pieces3.p, p.segs.p, p.jobs.p, p.terms.p, p.coef.p,     p.lq.p, p.rq.p, p.xsrc.p,
-                     p.colbase.p, p.yrow.p,    p.xstride.p, p.colstride.p, p.t1.p, p.t2.p, p.n1,   p.n3,   p.njobs};
-    return launch_dependent(stack_redo_f64_kernel, kRedoCtas, ST, 0, s, a, x, y, d.redo);
+    return launch_dependent(stack_redo_f64_kernel<false>, kRedoCtas, ST, 0, s, redo_args(p), x, nullptr, y, nullptr,
+                            d.redo);
+}
+
+// The digit matvec on planar vectors.
+static cudaError_t digits_apply_complex(F64Stack& p, const double* xr, const double* xi, double* yr, double* yi,
+                                        cudaStream_t s) {
+    F64Digits& d = *p.dg;
+    cudaError_t e = launch_digit_psi_complex(d.psi_c, d.npsi, xr, xi, d.x, d.redo, s);
+    DigitOut o{};
+    o.out = p.t1.p;
+    o.colbase = d.colbase;
+    o.colstride = d.colstride;
+    if (e == cudaSuccess) e = launch_digit_gemm(2, d.tiles1, d.begin1, d.sms, d.m1, d.l.ex, d.x.ex, o, d.redo, s);
+    if (e == cudaSuccess && p.njobs > 0)
+        e = launch_dependent(stack_combine_f64_kernel, p.njobs, 128, 0, s, p.jobs.p, p.terms.p, p.coef.p, p.t1.p, p.t2.p);
+    if (e == cudaSuccess && p.njobs > 0)
+        e = launch_dependent(stack_combine_f64_kernel, p.njobs, 128, 0, s, p.jobs.p, p.terms.p, p.coef.p, p.t1_im.p,
+                             p.t2_im.p);
+    if (e == cudaSuccess)
+        e = launch_digit_rows_complex(d.rows_c, d.nrows, p.t2.p, p.t2_im.p, d.kx, 1, false, d.t2, d.redo, s);
+    o = DigitOut{};
+    o.out = yr;
+    o.out_im = yi;
+    o.rowtab = p.yrow.p;
+    if (e == cudaSuccess) e = launch_digit_gemm(1, d.tiles3, d.begin3, d.sms, d.m3, d.t2.ex, d.r.ex, o, d.redo, s);
+    if (e != cudaSuccess) return e;
+    return launch_dependent(stack_redo_f64_kernel<true>, kRedoCtas, ST, 0, s, redo_args(p), xr, xi, yr, yi, d.redo);
 }
 
 cudaError_t f64stack_stage(F64Stack& p, const double* x, double* y, cudaStream_t s, int stage) {
@@ -734,6 +895,7 @@ cudaError_t f64stack_apply(F64Stack& p, const double* x, double* y, cudaStream_t
 cudaError_t f64stack_apply_complex(F64Stack& p, const double* xr, const double* xi, double* yr, double* yi,
                                    cudaStream_t s) {
     if (!p.cplx) return cudaErrorInvalidValue;
+    if (p.dg) return digits_apply_complex(p, xr, xi, yr, yi, s);
     cudaError_t e = cudaSuccess;
     if (p.n1 > 0)
         e = launch_dependent(stack_gemm1_f64_kernel<true>, p.n1, ST, 0, s, p.pieces1.p, p.segs.p, p.lq.p, p.lq_im.p, xr, xi,

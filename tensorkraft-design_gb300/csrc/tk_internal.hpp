@@ -176,7 +176,10 @@ struct TcTile {
     int64_t out_off;         // mode 1: row-table index of m0; mode 2: column-table index of n0
     int32_t ldc, n0;         // mode 1: n0 = column offset added to the row table; mode 2: ldc = m0
     int32_t n_mma, k_valid;  // UMMA N (n_valid rounded up to 16, <= kTcBN); stage 1: K of the stack (D_A)
-    int32_t fill0, pad_;     // fused stage 3: chunk c's fill segments are fill_segs[fill_chunk[fill0 + c] ..)
+    int32_t fill0;           // fused stage 3: chunk c's fill segments are fill_segs[fill_chunk[fill0 + c] ..)
+    int32_t parts;           // digit products: operands whose K follow one another (0 and 1: one; complex: 2)
+    int32_t split;           // digit products, mode 1: first column of the imaginary part (0: none)
+    int32_t pad_;
 };
 // Fused stage 3 (the W_i W_j combine inside the stage-3 GEMM): a stage-3
 // stack of at most TcOptions::fuse_max_ntiles column tiles builds its A

@@ -89,8 +89,8 @@ struct F64Stack;
 struct F64StackDeleter {
     void operator()(F64Stack* p) const;
 };
-// Whether a real plan of these tables runs its FP64 matvec on digits (digit_gemm.cu).
-bool f64stack_on_digits(const TcTables& C);
+// Whether a plan of these tables runs its FP64 matvec on digits (digit_gemm.cu).
+bool f64stack_on_digits(const TcTables& C, bool cplx);
 tk_status f64stack_create(const TcTables& C, std::unique_ptr<F64Stack, F64StackDeleter>& out, std::string& err);
 // stage 0: T1 = L stacks * psi; 1: the W_i W_j combine into T2; 2: y = T2 * R stacks
 cudaError_t f64stack_stage(F64Stack& p, const double* x, double* y, cudaStream_t s, int stage);

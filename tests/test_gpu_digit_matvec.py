@@ -114,3 +114,49 @@ def test_digit_matvec_two_plans_on_two_streams(lib_built):
             p.apply(x, y, stream=s.cuda_stream)
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(alone, ys))
+
+
+def _complex_plan(p, rng, integers):
+    """A plan over complex environments (not Hermitian: the matvec does not need it)."""
+    from tk_gb300 import Heff2Plan, sweep
+
+    def dev(e):
+        im = rng.standard_normal(e.data.shape) * (e.data != 0.0)
+        z = e.data + 1j * im
+        if integers:
+            z = np.rint(4.0 * z.real) + 1j * np.rint(4.0 * z.imag)
+        return sweep.DeviceEnv.from_dense(p.kind, z, e.bra_idx, e.mpo_idx, e.ket_idx)
+
+    return Heff2Plan.from_device_envs_complex(dev(p.env_l), dev(p.env_r), p.w_i, p.w_j, p.flux)
+
+
+def _apply_complex(plan, x, schedule):
+    import torch
+
+    plan.set_schedule(schedule)
+    xr, xi = torch.from_numpy(x.real.copy()).cuda(), torch.from_numpy(x.imag.copy()).cuda()
+    yr, yi = torch.full_like(xr, float("nan")), torch.full_like(xr, float("nan"))
+    plan.apply_complex(xr, xi, yr, yi)
+    torch.cuda.synchronize()
+    return yr.cpu().numpy(), yi.cpu().numpy()
+
+
+# K of a part below 32 (its two parts drained together), below 64, of several chunks
+@pytest.mark.parametrize("name,D", [("heisenberg", 130), ("heisenberg", 401), ("hubbard", 400), ("cylinder", 257)])
+def test_digit_matvec_complex(lib_built, name, D):
+    p = _problem(name, D, lambda e, side: e)
+    rng = np.random.default_rng(D)
+    plan = _complex_plan(p, rng, True)
+    assert plan.launches() == 7
+    x = rng.integers(-9, 10, plan.block_dim) + 1j * rng.integers(-9, 10, plan.block_dim)
+    for got, want in zip(_apply_complex(plan, x, _abi.SCHED_STACKED), _apply_complex(plan, x, _abi.SCHED_GROUPED)):
+        assert np.array_equal(got, want)  # every sum is exact
+    plan = _complex_plan(p, rng, False)
+    x = rng.standard_normal(plan.block_dim) + 1j * rng.standard_normal(plan.block_dim)
+    got, want = _apply_complex(plan, x, _abi.SCHED_STACKED), _apply_complex(plan, x, _abi.SCHED_GROUPED)
+    assert rel_err(got[0] + 1j * got[1], want[0] + 1j * want[1]) < 64 * 2.0 ** -53
+    x[plan.block_dim // 2] = complex(np.inf, 1.0)
+    got, want = _apply_complex(plan, x, _abi.SCHED_STACKED), _apply_complex(plan, x, _abi.SCHED_GROUPED)
+    for g, w in zip(got, want):
+        assert np.array_equal(np.isfinite(g), np.isfinite(w)) and not np.isfinite(w).all()
+        assert rel_err(g[np.isfinite(w)], w[np.isfinite(w)]) < 1e-13
