@@ -422,7 +422,7 @@ extern "C" tk_status tk_heff2_launches(const tk_heff2_plan* plan, int32_t* per_a
     const tk_heff2_plan* p = plan;
     int n = 0;
     if (p->is_complex && p->schedule == TK_SCHED_STACKED) {
-        n = f64stack_launches(*p->f64s) + (p->n_jobs > 0);  // the combine runs once per part
+        n = f64stack_launches(*p->f64s);
     } else if (p->is_complex) {
         n = 4 * (p->g1.n_tiles > 0) + 2 * (p->n_jobs > 0) + 4 * (p->g3.n_tiles > 0);
     } else if (p->precision == TK_PREC_BF16X3) {

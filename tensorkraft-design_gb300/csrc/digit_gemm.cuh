@@ -26,9 +26,9 @@ constexpr int kDigitRing = 2;  // shared-memory stages of 32 K of a product
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class... P, class... A>
-cudaError_t launch_dependent(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+cudaError_t launch_dependent(void (*k)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
     cudaLaunchConfig_t c{};
-    c.gridDim = dim3(grid);
+    c.gridDim = grid;
     c.blockDim = dim3(block);
     c.dynamicSmemBytes = smem;
     c.stream = s;

@@ -299,11 +299,14 @@ __global__ void __launch_bounds__(128) stack_combine_f64_kernel(const TcCombJob*
                                                                 const TcCombTerm* __restrict__ terms,
                                                                 const double* __restrict__ coef,
                                                                 const double* __restrict__ t1,
-                                                                double* __restrict__ t2) {
+                                                                double* __restrict__ t2,
+                                                                const double* __restrict__ t1_im,
+                                                                double* __restrict__ t2_im) {
     const TcCombJob j = jobs[blockIdx.x];  // a plan constant
     dep_launch();
     dep_wait();
-    stack_combine_job(j, terms, coef, t1, t2);
+    // the W_i W_j coefficients are real: they act on each part (blockIdx.y)
+    stack_combine_job(j, terms, coef, blockIdx.y ? t1_im : t1, blockIdx.y ? t2_im : t2);
 }
 
 // The whole FP64 matvec in one launch, after a digit matvec that could not
@@ -813,6 +816,13 @@ tk_status f64stack_create(const TcTables& C, std::unique_ptr<F64Stack, F64StackD
     return TK_OK;
 }
 
+// T2 from T1, both parts of a complex plan in one launch.
+static cudaError_t combine_stage(const F64Stack& p, cudaStream_t s) {
+    if (p.njobs == 0) return cudaSuccess;
+    return launch_dependent(stack_combine_f64_kernel, dim3((unsigned)p.njobs, p.cplx ? 2u : 1u), 128, 0, s, p.jobs.p,
+                            p.terms.p, p.coef.p, p.t1.p, p.t2.p, p.t1_im.p, p.t2_im.p);
+}
+
 static RedoArgs redo_args(const F64Stack& p) {
     return RedoArgs{p.pieces1.p, p.pieces3.p, p.segs.p,  p.jobs.p,    p.terms.p,     p.coef.p, p.lq.p, p.rq.p, p.lq_im.p,
                     p.rq_im.p,   p.xsrc.p,    p.colbase.p, p.yrow.p,  p.xstride.p, p.colstride.p, p.t1.p,   p.t2.p, p.t1_im.p,
@@ -832,9 +842,7 @@ static cudaError_t digits_stage(F64Stack& p, const double* x, double* y, cudaStr
         return launch_digit_gemm(2, d.tiles1, d.begin1, d.sms, d.m1, d.l.ex, d.x.ex, o, d.redo, s);
     }
     if (stage == 1) {
-        if (p.njobs > 0 && (e = launch_dependent(stack_combine_f64_kernel, p.njobs, 128, 0, s, p.jobs.p, p.terms.p, p.coef.p,
-                                                 p.t1.p, p.t2.p)) != cudaSuccess)
-            return e;
+        if ((e = combine_stage(p, s)) != cudaSuccess) return e;
         return launch_digit_rows(d.rows, d.nrows, p.t2.p, d.kx, 1, d.t2, d.redo, s);
     }
     o.out = y;
@@ -854,11 +862,7 @@ static cudaError_t digits_apply_complex(F64Stack& p, const double* xr, const dou
     o.colbase = d.colbase;
     o.colstride = d.colstride;
     if (e == cudaSuccess) e = launch_digit_gemm(2, d.tiles1, d.begin1, d.sms, d.m1, d.l.ex, d.x.ex, o, d.redo, s);
-    if (e == cudaSuccess && p.njobs > 0)
-        e = launch_dependent(stack_combine_f64_kernel, p.njobs, 128, 0, s, p.jobs.p, p.terms.p, p.coef.p, p.t1.p, p.t2.p);
-    if (e == cudaSuccess && p.njobs > 0)
-        e = launch_dependent(stack_combine_f64_kernel, p.njobs, 128, 0, s, p.jobs.p, p.terms.p, p.coef.p, p.t1_im.p,
-                             p.t2_im.p);
+    if (e == cudaSuccess) e = combine_stage(p, s);
     if (e == cudaSuccess)
         e = launch_digit_rows_complex(d.rows_c, d.nrows, p.t2.p, p.t2_im.p, d.kx, 1, false, d.t2, d.redo, s);
     o = DigitOut{};
@@ -875,9 +879,7 @@ cudaError_t f64stack_stage(F64Stack& p, const double* x, double* y, cudaStream_t
     if (stage == 0 && p.n1 > 0)
         return launch_dependent(stack_gemm1_f64_kernel<false>, p.n1, ST, 0, s, p.pieces1.p, p.segs.p, p.lq.p, nullptr, x,
                                 nullptr, p.xsrc.p, p.xstride.p, p.colbase.p, p.colstride.p, p.t1.p, nullptr);
-    if (stage == 1 && p.njobs > 0)
-        return launch_dependent(stack_combine_f64_kernel, p.njobs, 128, 0, s, p.jobs.p, p.terms.p, p.coef.p, p.t1.p,
-                                p.t2.p);
+    if (stage == 1) return combine_stage(p, s);
     if (stage == 2 && p.n3 > 0)
         return launch_dependent(stack_gemm3_f64_kernel<false>, p.n3, ST, 0, s, p.pieces3.p, p.segs.p, p.t2.p, nullptr,
                                 p.rq.p, nullptr, p.yrow.p, y, nullptr);
@@ -900,12 +902,7 @@ cudaError_t f64stack_apply_complex(F64Stack& p, const double* xr, const double* 
     if (p.n1 > 0)
         e = launch_dependent(stack_gemm1_f64_kernel<true>, p.n1, ST, 0, s, p.pieces1.p, p.segs.p, p.lq.p, p.lq_im.p, xr, xi,
                              p.xsrc.p, p.xstride.p, p.colbase.p, p.colstride.p, p.t1.p, p.t1_im.p);
-    // the W_i W_j coefficients are real: the combine acts on each part
-    if (e == cudaSuccess && p.njobs > 0)
-        e = launch_dependent(stack_combine_f64_kernel, p.njobs, 128, 0, s, p.jobs.p, p.terms.p, p.coef.p, p.t1.p, p.t2.p);
-    if (e == cudaSuccess && p.njobs > 0)
-        e = launch_dependent(stack_combine_f64_kernel, p.njobs, 128, 0, s, p.jobs.p, p.terms.p, p.coef.p, p.t1_im.p,
-                             p.t2_im.p);
+    if (e == cudaSuccess) e = combine_stage(p, s);
     if (e == cudaSuccess && p.n3 > 0)
         e = launch_dependent(stack_gemm3_f64_kernel<true>, p.n3, ST, 0, s, p.pieces3.p, p.segs.p, p.t2.p, p.t2_im.p,
                              p.rq.p, p.rq_im.p, p.yrow.p, yr, yi);
