@@ -232,15 +232,15 @@ __device__ __forceinline__ TcTile tile_of(const TcTile* __restrict__ tiles, cons
 // products), each from a chunk of its own; ring steps of KW, drained after at
 // most 64 k.
 struct KSteps {
-    int k, per, kch, total;  // K and ring steps of a part, chunks a part, ring steps
-    bool paired;             // two parts of one step each are drained together
+    int parts, per, kch;  // ring steps and chunks a part
+    bool paired;          // two parts of one step each are drained together
     __device__ __forceinline__ KSteps(const TcTile& t)
-        : k(t.k_valid), per((t.k_valid + KW - 1) / KW), kch((t.k_valid + kTcBK - 1) / kTcBK),
-          total(per * max(t.parts, 1)), paired(per == 1) {}
-    __device__ __forceinline__ int drains() const { return paired ? (total + 1) / 2 : total / max(per, 1) * kch; }
-    __device__ __forceinline__ bool first(int g) const { return paired ? (g & 1) == 0 : (g % per & 1) == 0; }
-    __device__ __forceinline__ bool last(int g) const {
-        return paired ? (g & 1) == 1 || g == total - 1 : (g % per & 1) == 1 || g % per == per - 1;
+        : parts(max(t.parts, 1)), per((t.k_valid + KW - 1) / KW), kch((t.k_valid + kTcBK - 1) / kTcBK), paired(per == 1) {}
+    __device__ __forceinline__ int drains() const { return paired ? (parts + 1) >> 1 : parts * kch; }
+    // whether step q of part p is the first, the last one between two drains
+    __device__ __forceinline__ bool first(int p, int q) const { return ((paired ? p : q) & 1) == 0; }
+    __device__ __forceinline__ bool last(int p, int q) const {
+        return paired ? (p & 1) || p == parts - 1 : (q & 1) || q == per - 1;
     }
 };
 
@@ -305,8 +305,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
                 const int box = (t.m_valid + 31) >> 5;
                 const uint32_t bytes = kDigits * KW * 2 * (32 * box + HN * halves);
                 const KSteps ks(t);
-                for (int g = 0; g < ks.total && ok; ++g, ++it) {
-                    const int part = g / ks.per, q = g - part * ks.per;
+                for (int part = 0; part < ks.parts && ok; ++part)
+                for (int q = 0; q < ks.per && ok; ++q, ++it) {
                     const int st = it % kDigitRing;
                     uint8_t* base = smem + st * STAGE_BYTES;
                     if (it >= kDigitRing) ok = mbar_wait(&empty[st], (it / kDigitRing - 1) & 1, stop, redo);
@@ -331,10 +331,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
                 const int halves = t.n_valid > HN ? 2 : 1;
                 const uint32_t astep = (uint32_t)((((t.m_valid + 31) >> 5) * 32) * KW * 2);
                 const KSteps k(t);
-                for (int g = 0; g < k.total && ok; ++g, ++it) {
-                    const int q = g % k.per;
+                for (int part = 0; part < k.parts && ok; ++part)
+                for (int q = 0; q < k.per && ok; ++q, ++it) {
                     const int st = it % kDigitRing;
-                    const bool first = k.first(g), last = k.last(g);
+                    const bool first = k.first(part, q), last = k.last(part, q);
                     ok = mbar_wait(&full[st], (it / kDigitRing) & 1, stop, redo);
                     const uint32_t sa = smem_u32(smem + st * STAGE_BYTES);
                     const int ks = min(KW / 16, (t.k_valid - q * KW + 15) / 16);
@@ -712,104 +712,91 @@ __global__ void __launch_bounds__(32 * kDigitRowsPerCta) digit_rows_complex_kern
     }
 }
 
-// psi sub-blocks of a complex vector: digit_psi_kernel's work on both parts.
-__global__ void __launch_bounds__(256) digit_psi_complex_kernel(const DigitPsiC* __restrict__ jobs,
-                                                                const double* __restrict__ xr,
-                                                                const double* __restrict__ xi, const DigitStack out,
-                                                                int* redo) {
+// psi sub-blocks: up to CW columns x all K rows by one CTA, lanes along the
+// columns (CW = 8: four rows of them); a 64-wide chunk is turned in shared memory (`pitch` doubles a column,
+// odd).  A K of one chunk is read once (a complex Hubbard D = 512 vector: 17 -> 6
+// us against reading it twice).  CPLX: both parts of a complex vector, on one
+// grid.
+constexpr int PT = 256;
+template <bool CPLX, int CW>
+__global__ void __launch_bounds__(PT) digit_psi_kernel(const DigitPsi* __restrict__ jobs, const double* __restrict__ x,
+                                                       const double* __restrict__ xi, int pitch, const DigitStack out,
+                                                       int* redo) {
+    extern __shared__ double tile[];  // [CW][pitch], the imaginary part's behind it
     __shared__ uint32_t smax[32];
-    __shared__ double tr[32][kTcBK + 1], ti[32][kTcBK + 1];
-    const DigitPsiC j = jobs[blockIdx.x];
+    const DigitPsi j = jobs[blockIdx.x];
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int nr = j.cols, K = j.rows, kch = (K + kTcBK - 1) / kTcBK;
-    const int64_t src = j.src + lane;
+    double* tile_im = tile + CW * pitch;
+    const int col = lane % CW, kw = w * (32 / CW) + lane / CW;  // this thread's column, first k
+    constexpr int KS = PT / CW;                                 // k step of the CTA
+    const int64_t src = j.src + col;
     dep_launch();
     if (tid < 32) smax[tid] = 0;
     __syncthreads();
     dep_wait();
     uint32_t mx = 0;
-#pragma unroll 2
-    for (int k = w; k < K; k += 8) {
-        const int64_t o = src + (int64_t)k * j.pitch;
-        if (lane < nr) mx = max(mx, max(abs_hi(xr[o]), abs_hi(xi[o])));
+    // chunk c into shared memory, zeros to a whole 16-wide step (they are multiplied)
+    auto fetch = [&](int c) {
+        const int k0 = c * kTcBK, kv = (min(kTcBK, K - k0) + 15) & ~15;
+#pragma unroll 4
+        for (int k = kw; k < kv; k += KS) {
+            const bool in = col < nr && k0 + k < K;
+            const int64_t o = src + (int64_t)(k0 + k) * j.pitch;
+            const double v = in ? x[o] : 0.0;
+            tile[col * pitch + k] = v;
+            mx = max(mx, abs_hi(v));
+            if (CPLX) {
+                const double u = in ? xi[o] : 0.0;
+                tile_im[col * pitch + k] = u;
+                mx = max(mx, abs_hi(u));
+            }
+        }
+        return kv;
+    };
+    if (kch == 1) {
+        fetch(0);
+    } else {
+#pragma unroll 4
+        for (int k = kw; k < K; k += KS)
+            if (col < nr) {
+                const int64_t o = src + (int64_t)k * j.pitch;
+                mx = max(mx, abs_hi(x[o]));
+                if (CPLX) mx = max(mx, abs_hi(xi[o]));
+            }
     }
-    atomicMax(&smax[lane], mx);
+    atomicMax(&smax[col], mx);
     __syncthreads();
     if (tid < nr) {
         const int ex = row_exponent(smax[tid], redo);
         out.ex[(int64_t)j.to + tid] = ex;
-        out.ex[(int64_t)j.to + j.n_dual + tid] = ex;
+        if (CPLX) out.ex[(int64_t)j.to + j.n_dual + tid] = ex;
         smax[tid] = (uint32_t)ex;
     }
     for (int c = 0; c < kch; ++c) {
-        const int k0 = c * kTcBK;
         __syncthreads();
-#pragma unroll
-        for (int i = 0; i < kTcBK / 8; ++i) {
-            const int k = k0 + w + i * 8;
-            const bool in = lane < nr && k < K;
-            const int64_t o = src + (int64_t)k * j.pitch;
-            tr[lane][k - k0] = in ? xr[o] : 0.0;
-            ti[lane][k - k0] = in ? xi[o] : 0.0;
-        }
-        __syncthreads();
-        const int kv = (min(kTcBK, K - k0) + 15) & ~15;  // whole 16-wide steps are multiplied
-        for (int r = w; r < nr; r += 8)
-            if (2 * lane < kv) {
-                uint32_t d[kDigits], f[kDigits];
-                digits2(tr[r][2 * lane], tr[r][2 * lane + 1], (int)smax[r], d);
-                digits2(ti[r][2 * lane], ti[r][2 * lane + 1], (int)smax[r], f);
-                put_complex<true>(out, (int64_t)j.to + r, j.n_dual, (int64_t)c * j.cs_out, (int64_t)(kch + c) * j.cs_out,
-                                  2 * lane, d, f);
+        const int kv = kch == 1 ? (K + 15) & ~15 : fetch(c);
+        if (kch > 1) __syncthreads();
+        // rows and pairs of k over the threads
+        const int pairs = kv >> 1;
+        for (int e = tid; e < nr * pairs; e += PT) {
+            const int r = e / pairs, k = 2 * (e - r * pairs);
+            const double* v = tile + r * pitch + k;
+            uint32_t d[kDigits];
+            digits2(v[0], v[1], (int)smax[r], d);
+            if (CPLX) {
+                const double* u = tile_im + r * pitch + k;
+                uint32_t f[kDigits];
+                digits2(u[0], u[1], (int)smax[r], f);
+                put_complex<true>(out, (int64_t)j.to + r, j.n_dual, (int64_t)c * j.cs, (int64_t)(kch + c) * j.cs, k, d, f);
+            } else {
+                put_digits(out, (int64_t)j.to + r + (int64_t)c * j.cs, k, d);
             }
+        }
     }
 }
 
-// psi sub-blocks: 32 columns x all K rows by one CTA, lanes along the columns;
-// each 64-wide chunk is turned in shared memory.
 constexpr int BT = 256;
-__global__ void __launch_bounds__(BT) digit_psi_kernel(const TcSplitJob* __restrict__ jobs, const double* __restrict__ x,
-                                                       const DigitStack out, int* redo) {
-    __shared__ uint32_t smax[32];
-    __shared__ double tile[32][kTcBK + 1];
-    const TcSplitJob j = jobs[blockIdx.x];
-    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    const int nr = min(32, j.cols - j.b0), K = j.rows;
-    const double* src = x + j.src + j.b0 + lane;
-    const int64_t row = (int64_t)j.xrow + j.b0;
-    dep_launch();
-    if (tid < 32) smax[tid] = 0;
-    __syncthreads();
-    dep_wait();
-    uint32_t mx = 0;
-#pragma unroll 4
-    for (int k = w; k < K; k += BT / 32) mx = max(mx, lane < nr ? abs_hi(src[(int64_t)k * j.cols]) : 0u);
-    atomicMax(&smax[lane], mx);
-    __syncthreads();
-    if (tid < nr) {
-        const int ex = row_exponent(smax[tid], redo);
-        out.ex[row + tid] = ex;
-        smax[tid] = (uint32_t)ex;
-    }
-    for (int c = 0; c * kTcBK < K; ++c) {
-        const int k0 = c * kTcBK;
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < kTcBK / (BT / 32); ++i) {
-            const int k = k0 + w + i * (BT / 32);
-            tile[lane][k - k0] = lane < nr && k < K ? src[(int64_t)k * j.cols] : 0.0;
-        }
-        __syncthreads();
-        const int kv = (min(kTcBK, K - k0) + 15) & ~15;  // whole 16-wide steps are multiplied
-        for (int r = w; r < nr; r += BT / 32)
-            if (2 * lane < kv) {
-                uint32_t d[kDigits];
-                digits2(tile[r][2 * lane], tile[r][2 * lane + 1], (int)smax[r], d);
-                put_digits(out, row + r + (int64_t)c * j.cstride, 2 * lane, d);
-            }
-    }
-}
-
 // The two operands of a dense product, 32 rows x 64 k a CTA (the rows of A,
 // then those of B).  PASS 0 leaves every row's largest high word in ex (zeroed
 // before), PASS 1 writes the digits; lanes walk along the shorter stride.
@@ -990,12 +977,6 @@ cudaError_t launch_digit_rows_complex(const DigitRowsC* jobs, int n_jobs, const 
                             32 * kDigitRowsPerCta, 0, s, jobs, re, im, kx, sign, out, redo);
 }
 
-cudaError_t launch_digit_psi_complex(const DigitPsiC* jobs, int n_jobs, const double* xr, const double* xi,
-                                     const DigitStack& out, int* redo, cudaStream_t s) {
-    if (n_jobs <= 0) return cudaSuccess;
-    return launch_dependent(digit_psi_complex_kernel, n_jobs, 256, 0, s, jobs, xr, xi, out, redo);
-}
-
 cudaError_t launch_digit_matrices(const DigitMatrix& a, const DigitMatrix& b, int K, int* redo, cudaStream_t s) {
     const dim3 grid((unsigned)((a.rows + 31) / 32 + (b.rows + 31) / 32), (unsigned)((K + kTcBK - 1) / kTcBK));
     cudaError_t e;
@@ -1011,10 +992,14 @@ cudaError_t launch_digit_matrices(const DigitMatrix& a, const DigitMatrix& b, in
     return cudaGetLastError();
 }
 
-cudaError_t launch_digit_psi(const TcSplitJob* jobs, int n_jobs, const double* x, const DigitStack& out, int* redo,
-                             cudaStream_t s) {
+cudaError_t launch_digit_psi(const DigitPsi* jobs, int n_jobs, int cols, int max_k, const double* x, const double* x_im,
+                             const DigitStack& out, int* redo, cudaStream_t s) {
     if (n_jobs <= 0) return cudaSuccess;
-    return launch_dependent(digit_psi_kernel, n_jobs, BT, 0, s, jobs, x, out, redo);
+    const int pitch = ((std::min(max_k, kTcBK) + 15) & ~15) + 1;
+    const size_t smem = sizeof(double) * cols * pitch * (x_im ? 2 : 1);
+    auto* k = cols == 8 ? (x_im ? digit_psi_kernel<true, 8> : digit_psi_kernel<false, 8>)
+                        : (x_im ? digit_psi_kernel<true, 32> : digit_psi_kernel<false, 32>);
+    return launch_dependent(k, n_jobs, PT, smem, s, jobs, x, x_im, pitch, out, redo);
 }
 
 }  // namespace tk

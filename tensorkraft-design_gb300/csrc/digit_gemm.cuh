@@ -62,10 +62,11 @@ struct DigitRows {
 struct DigitRowsC {
     int32_t row, n, cs, kch, kx, to, cs_out, n_dual;
 };
-// Columns [0, cols) at src of a psi sub-block (rows x pitch), as a B operand.
-struct DigitPsiC {
+// Columns [0, cols) (at most 32) at src of a psi sub-block (rows x pitch), as
+// rows to .. of a B operand; complex vectors' second form n_dual rows further.
+struct DigitPsi {
     int64_t src;
-    int32_t rows, cols, pitch, to, cs_out, n_dual;
+    int32_t rows, cols, pitch, to, cs, n_dual;
 };
 constexpr int kDigitRowsPerCta = 8;
 
@@ -118,8 +119,6 @@ cudaError_t launch_digit_rows(const DigitRows* jobs, int n_jobs, const double* q
 cudaError_t launch_digit_rows_complex(const DigitRowsC* jobs, int n_jobs, const double* re, const double* im,
                                       const int32_t* kx, int sign, bool dual, const DigitStack& out, int* redo,
                                       cudaStream_t s);
-cudaError_t launch_digit_psi_complex(const DigitPsiC* jobs, int n_jobs, const double* xr, const double* xi,
-                                     const DigitStack& out, int* redo, cudaStream_t s);
 // Digits of both operands of a dense product (*redo is set for operands that
 // one grid per row would hold less exactly than FP64): row r, k of K at
 // x[r * rs + k * ks], into stacks whose chunks are `rows` rows apart.
@@ -131,9 +130,9 @@ struct DigitMatrix {
     float* square;  // a scratch value per row
 };
 cudaError_t launch_digit_matrices(const DigitMatrix& a, const DigitMatrix& b, int K, int* redo, cudaStream_t s);
-// Digits of the psi sub-blocks of TcSplitJob lists (jobs with a0 == 0 alone:
-// 32 columns of a sub-block each, all its rows).
-cudaError_t launch_digit_psi(const TcSplitJob* jobs, int n_jobs, const double* x, const DigitStack& out, int* redo,
-                             cudaStream_t s);
+// Digits of psi sub-blocks (jobs of at most `cols` columns, 32 or 8, and max_k
+// rows), of both parts with x_im.
+cudaError_t launch_digit_psi(const DigitPsi* jobs, int n_jobs, int cols, int max_k, const double* x, const double* x_im,
+                             const DigitStack& out, int* redo, cudaStream_t s);
 
 }  // namespace tk

@@ -295,6 +295,7 @@ __device__ __forceinline__ void stack_combine_job(const TcCombJob& j, const TcCo
     }
 }
 
+template <bool CPLX>
 __global__ void __launch_bounds__(128) stack_combine_f64_kernel(const TcCombJob* __restrict__ jobs,
                                                                 const TcCombTerm* __restrict__ terms,
                                                                 const double* __restrict__ coef,
@@ -306,7 +307,10 @@ __global__ void __launch_bounds__(128) stack_combine_f64_kernel(const TcCombJob*
     dep_launch();
     dep_wait();
     // the W_i W_j coefficients are real: they act on each part (blockIdx.y)
-    stack_combine_job(j, terms, coef, blockIdx.y ? t1_im : t1, blockIdx.y ? t2_im : t2);
+    if (!CPLX)
+        stack_combine_job(j, terms, coef, t1, t2);
+    else
+        stack_combine_job(j, terms, coef, blockIdx.y ? t1_im : t1, blockIdx.y ? t2_im : t2);
 }
 
 // The whole FP64 matvec in one launch, after a digit matvec that could not
@@ -481,16 +485,15 @@ struct F64Digits {
     const int32_t* kx = nullptr;     // scales of the R stacks' columns
     const TcTile *tiles1 = nullptr, *tiles3 = nullptr;   // dealt out to `sms` CTAs:
     const int32_t *begin1 = nullptr, *begin3 = nullptr;
-    const TcSplitJob* psi = nullptr;
+    const DigitPsi* psi = nullptr;
     const DigitRows* rows = nullptr;  // of T2
-    // complex plans: the same jobs for planar operands, T1's column tables for both parts
-    const DigitPsiC* psi_c = nullptr;
+    // complex plans: the same for planar operands, T1's column tables for both parts
     const DigitRowsC* rows_c = nullptr;
     const int64_t* colbase = nullptr;
     const int32_t* colstride = nullptr;
     int* redo = nullptr;
     DigitMaps m1, m3;
-    int npsi = 0, nrows = 0, sms = 0;
+    int npsi = 0, max_k = 0, psi_cols = 32, nrows = 0, sms = 0;
 };
 
 struct F64Stack {
@@ -531,6 +534,25 @@ bool f64stack_on_digits(const TcTables& C, bool cplx) {
     for (const std::vector<TcTile>* v : {&C.tiles1, &C.tiles1x})
         for (const TcTile& t : *v) f += (cplx ? 4.0 : 1.0) * t.m_valid * t.n_valid * t.k_valid;
     return f >= (C.tiles3.size() + C.tiles3f.size() < 12 ? 8e6 : 1.2e6);
+}
+
+// Where a K of several chunks leaves less than two 32-column jobs an SM, they are
+// cut to eight columns: a job reads its K twice, one load after the other
+// (Heisenberg D = 1024, 162 jobs: 10.1 -> 7.5 us).
+static void psi_jobs(std::vector<DigitPsi>& psi, F64Digits& d) {
+    for (const DigitPsi& j : psi) d.max_k = std::max(d.max_k, j.rows);
+    if (d.max_k <= kTcBK || psi.size() >= 304) return;
+    std::vector<DigitPsi> cut;
+    for (const DigitPsi& j : psi)
+        for (int c = 0; c < j.cols; c += 8) {
+            DigitPsi q = j;
+            q.src += c;
+            q.to += c;
+            q.cols = std::min(8, j.cols - c);
+            cut.push_back(q);
+        }
+    psi.swap(cut);
+    d.psi_cols = 8;
 }
 
 // Room behind the tables for the digits and the column scales; the tables go up
@@ -584,7 +606,7 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
     std::vector<int32_t> b1, b3;
     std::vector<DigitRowsC> lrows, rrows, trows;
     std::vector<DigitRows> rcols;
-    std::vector<DigitPsiC> psi;
+    std::vector<DigitPsi> psi;
     std::vector<int64_t> colbase(2 * C.t1col_base.size());
     std::vector<int32_t> colstride(2 * C.t1col_stride.size());
     const int64_t im = p.t1_im.p - p.t1.p;  // from T1's real part to its imaginary part
@@ -631,6 +653,7 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
         psi.push_back({j.src + j.b0, j.rows, std::min(32, j.cols - j.b0), j.cols, 4 * s.b + (j.xrow - s.b) + j.b0, 2 * s.N,
                        s.N});
     }
+    psi_jobs(psi, *d);
     for (const auto& [key, s] : s3) {
         tiles(w3, s, 1);
         rcols.push_back({s.b, s.N, s.N, s.kch, nk, 0});
@@ -659,7 +682,7 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
     d->tiles3 = reinterpret_cast<const TcTile*>(m + o_t3);
     d->begin1 = reinterpret_cast<const int32_t*>(m + o_b1);
     d->begin3 = reinterpret_cast<const int32_t*>(m + o_b3);
-    d->psi_c = reinterpret_cast<const DigitPsiC*>(m + o_psi);
+    d->psi = reinterpret_cast<const DigitPsi*>(m + o_psi);
     d->rows_c = reinterpret_cast<const DigitRowsC*>(m + o_rows);
     d->colbase = reinterpret_cast<const int64_t*>(m + o_cb);
     d->colstride = reinterpret_cast<const int32_t*>(m + o_cs);
@@ -685,9 +708,10 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
     std::unique_ptr<F64Digits> d(new F64Digits);
     if (p.cplx) return digits_create_complex(C, p, std::move(d), err);
     std::vector<DigitRows> lrows, rrows, trows, rcols;
-    std::vector<TcSplitJob> psi;
+    std::vector<DigitPsi> psi;
     for (const TcSplitJob& j : C.split)
-        if (j.a0 == 0) psi.push_back(j);
+        if (j.a0 == 0) psi.push_back({j.src + j.b0, j.rows, std::min(32, j.cols - j.b0), j.cols, j.xrow + j.b0, j.cstride, 0});
+    psi_jobs(psi, *d);
     std::set<int32_t> seen;
     for (const TcTile& t : C.tiles1x)
         if (seen.insert(t.a_row).second) digit_rows_of(lrows, t.a_row, t.m_valid, t.a_cs, t.kch, -1);
@@ -728,7 +752,7 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
     d->tiles3 = reinterpret_cast<const TcTile*>(m + o_t3);
     d->begin1 = reinterpret_cast<const int32_t*>(m + o_b1);
     d->begin3 = reinterpret_cast<const int32_t*>(m + o_b3);
-    d->psi = reinterpret_cast<const TcSplitJob*>(m + o_psi);
+    d->psi = reinterpret_cast<const DigitPsi*>(m + o_psi);
     d->rows = reinterpret_cast<const DigitRows*>(m + o_rows);
     d->redo = reinterpret_cast<int*>(m + o_redo);
     if (!digit_maps(d->m1, d->l, d->x, err) || !digit_maps(d->m3, d->t2, d->r, err)) return cudaErrorInvalidValue;
@@ -819,7 +843,8 @@ tk_status f64stack_create(const TcTables& C, std::unique_ptr<F64Stack, F64StackD
 // T2 from T1, both parts of a complex plan in one launch.
 static cudaError_t combine_stage(const F64Stack& p, cudaStream_t s) {
     if (p.njobs == 0) return cudaSuccess;
-    return launch_dependent(stack_combine_f64_kernel, dim3((unsigned)p.njobs, p.cplx ? 2u : 1u), 128, 0, s, p.jobs.p,
+    return launch_dependent(p.cplx ? stack_combine_f64_kernel<true> : stack_combine_f64_kernel<false>,
+                            dim3((unsigned)p.njobs, p.cplx ? 2u : 1u), 128, 0, s, p.jobs.p,
                             p.terms.p, p.coef.p, p.t1.p, p.t2.p, p.t1_im.p, p.t2_im.p);
 }
 
@@ -835,7 +860,7 @@ static cudaError_t digits_stage(F64Stack& p, const double* x, double* y, cudaStr
     cudaError_t e;
     DigitOut o{};
     if (stage == 0) {
-        if ((e = launch_digit_psi(d.psi, d.npsi, x, d.x, d.redo, s)) != cudaSuccess) return e;
+        if ((e = launch_digit_psi(d.psi, d.npsi, d.psi_cols, d.max_k, x, nullptr, d.x, d.redo, s)) != cudaSuccess) return e;
         o.out = p.t1.p;
         o.colbase = p.colbase.p;
         o.colstride = p.colstride.p;
@@ -856,7 +881,7 @@ static cudaError_t digits_stage(F64Stack& p, const double* x, double* y, cudaStr
 static cudaError_t digits_apply_complex(F64Stack& p, const double* xr, const double* xi, double* yr, double* yi,
                                         cudaStream_t s) {
     F64Digits& d = *p.dg;
-    cudaError_t e = launch_digit_psi_complex(d.psi_c, d.npsi, xr, xi, d.x, d.redo, s);
+    cudaError_t e = launch_digit_psi(d.psi, d.npsi, d.psi_cols, d.max_k, xr, xi, d.x, d.redo, s);
     DigitOut o{};
     o.out = p.t1.p;
     o.colbase = d.colbase;
