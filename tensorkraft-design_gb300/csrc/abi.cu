@@ -161,6 +161,7 @@ void tk_ctx_destroy(tk_ctx* ctx) {
         if (ctx->dev_scratch) cudaFree(ctx->dev_scratch);
         if (ctx->host_stage) cudaFreeHost(ctx->host_stage);
         for (auto& b : ctx->gemm_free) cudaFree(b.first);
+        if (ctx->scratch_pool) cudaMemPoolDestroy((cudaMemPool_t)ctx->scratch_pool);
         if (ctx->stream) cudaStreamDestroy((cudaStream_t)ctx->stream);
     }
     delete ctx;

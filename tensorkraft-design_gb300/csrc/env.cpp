@@ -16,7 +16,6 @@
 // The two-site start vector psi(s_i, s_j, a, b) = sum_c A_i(s_i, a, c) A_j(s_j, c, b)
 // in a plan's block layout is one more grouped GEMM.
 #include <algorithm>
-#include <map>
 #include <string>
 #include <vector>
 
@@ -27,6 +26,7 @@ namespace tk {
 void env_layout(int kind, const QIndex& bra, const QIndex& mpo, const QIndex& ket, EnvLayout& out) {
     out = EnvLayout();
     std::vector<std::pair<uint64_t, std::array<int, 3>>> kb;
+    kb.reserve((size_t)bra.n() * std::min(mpo.n(), ket.n()));
     for (int b = 0; b < bra.n(); ++b)
         for (int w = 0; w < mpo.n(); ++w) {
             // q(ket) = q(bra) - q(w)
@@ -126,6 +126,45 @@ int64_t site_sub(const Bst3& A, const std::vector<int>& ssec, const std::vector<
     return b + sloc[st] * A.legs[1].dim[l] * A.legs[2].dim[r];
 }
 
+// The non-zero entries of a site MPO W[s, s', wl, wr] by bra state and output
+// channel, in the order of (s, input channel): what a growth sums over.
+class MpoRows {
+public:
+    struct Entry {
+        int64_t s, w;
+        double c;
+    };
+    MpoRows(bool left, const std::vector<double>& wd, int64_t d, int64_t nwl, int64_t nwr)
+        : nout_(left ? nwr : nwl), nin_(left ? nwl : nwr), used_((size_t)(d * nin_), 0) {
+        start_.push_back(0);
+        for (int64_t sp = 0; sp < d; ++sp)
+            for (int64_t o = 0; o < nout_; ++o) {
+                for (int64_t s = 0; s < d; ++s)
+                    for (int64_t i = 0; i < nin_; ++i) {
+                        const double c = wd[((s * d + sp) * nwl + (left ? i : o)) * nwr + (left ? o : i)];
+                        if (c == 0.0) continue;
+                        entries_.push_back({s, i, c});
+                        used_[(size_t)(s * nin_ + i)] = 1;
+                    }
+                start_.push_back(entries_.size());
+            }
+    }
+    const Entry* begin(int64_t sp, int64_t o) const { return entries_.data() + start_[(size_t)(sp * nout_ + o)]; }
+    const Entry* end(int64_t sp, int64_t o) const { return entries_.data() + start_[(size_t)(sp * nout_ + o) + 1]; }
+    // whether ket state s meets any of the input channels [w0, w0 + n)
+    bool any(int64_t s, int64_t w0, int64_t n) const {
+        for (int64_t w = w0; w < w0 + n; ++w)
+            if (used_[(size_t)(s * nin_ + w)]) return true;
+        return false;
+    }
+
+private:
+    int64_t nout_, nin_;
+    std::vector<Entry> entries_;
+    std::vector<size_t> start_;
+    std::vector<char> used_;
+};
+
 bool finish(GrowTables& G, int64_t n_env, int64_t n_site, int64_t n_out, bool left, std::string& err) {
     gemm_lpt_order(G.g1, kEnvTileM, kEnvTileN);
     gemm_lpt_order(G.g3, kEnvTileM, kEnvTileN);
@@ -173,59 +212,71 @@ static tk_status build_grow_tables_body(bool left, const QIndex& env_bra, const 
     }
     std::vector<double> Wd;
     if (!mpo_dense(W, Wd, err)) return TK_ERR_SECTOR_MISMATCH;
-    const int64_t d = P.total, nwl = W.legs[2].total, nwr = W.legs[3].total;
-    auto wval = [&](int64_t s, int64_t so, int64_t wl, int64_t wr) { return Wd[((s * d + so) * nwl + wl) * nwr + wr]; };
+    const int64_t d = P.total;
     std::vector<int> ssec;
     std::vector<int64_t> sloc;
     state_map(P, ssec, sloc);
-    std::vector<int> win_sec, wout_sec;
-    std::vector<int64_t> win_loc, wout_loc;
+    std::vector<int> win_sec;
+    std::vector<int64_t> win_loc;
     state_map(w_in, win_sec, win_loc);
-    state_map(w_out, wout_sec, wout_loc);
+    const MpoRows wr(left, Wd, d, W.legs[2].total, W.legs[3].total);
     EnvLayout lin, lout;
     env_layout(kind, bond_in, w_in, bond_in, lin);
     env_layout(kind, bond_out, w_out, bond_out, lout);
     G.out_total = lout.total;
     G.in_total = lin.total;
     const int nbi = bond_in.n(), nwi = w_in.n();
-    std::vector<int64_t> in_blk((size_t)nbi * nwi * nbi, -1);
-    for (size_t k = 0; k < lin.tri.size(); ++k)
-        in_blk[((size_t)lin.tri[k][0] * nwi + lin.tri[k][1]) * nbi + lin.tri[k][2]] = lin.off[k];
+    // (bra, mpo) sectors of the input -> its block and ket sector; at most one ket sector fits
+    std::vector<int64_t> in_blk((size_t)nbi * nwi, -1);
+    std::vector<int> in_ket((size_t)nbi * nwi, -1);
+    for (size_t k = 0; k < lin.tri.size(); ++k) {
+        in_blk[(size_t)lin.tri[k][0] * nwi + lin.tri[k][1]] = lin.off[k];
+        in_ket[(size_t)lin.tri[k][0] * nwi + lin.tri[k][1]] = lin.tri[k][2];
+    }
     const int nl = QL.n();
+    auto stage1 = [&](const GemmSeg& sg, int64_t m, int64_t n) {
+        GemmTask tk{};
+        tk.M = (int32_t)m;
+        tk.N = (int32_t)n;
+        tk.c_off = G.t1_total; tk.c_rs = tk.N; tk.c_cs = 1;
+        tk.seg_begin = (int)G.g1.segs.size();
+        G.g1.segs.push_back(sg);
+        tk.seg_end = (int)G.g1.segs.size();
+        tk.alpha = 1.0; tk.beta = 0.0;
+        G.g1.flops += 2.0 * tk.M * tk.N * (double)sg.K;
+        G.g1.tasks.push_back(tk);
+        gemm_add_tiles(G.g1, (int)G.g1.tasks.size() - 1, kEnvTileM, kEnvTileN);
+        G.t1_total += m * n;
+    };
+    // A T2 block is named by (s', vs or w, ket sector of its output block) and
+    // the output block follows from two of these, so each is met once below
+    // and nothing has to be looked up.
 
     if (left) {
-        // stage 1: T1(s, A', ws)[(a', w)][b] = L(A', ws, A)[(a', w)][a] * A(s, A, B)[a][b], A = A' - q(ws)
-        std::map<std::array<int64_t, 3>, std::pair<int64_t, int>> t1;  // (s, A', ws) -> (offset, B)
+        // stage 1: T1(s, A', ws)[(a', w)][b] = L(A', ws, A)[(a', w)][a] * A(s, A, B)[a][b], A = A' - q(ws);
+        // only the (s, ws) that W couples to an output are formed
+        struct Part { int64_t off; int b; };
+        std::vector<Part> t1((size_t)d * nbi * nwi, Part{0, -1});
         for (int64_t s = 0; s < d; ++s)
             for (int ap = 0; ap < nbi; ++ap)
                 for (int ws = 0; ws < nwi; ++ws) {
-                    Qn qa = qn_fuse(kind, QL.q[ap], qn_dual(kind, w_in.q[ws]));
-                    int a = QL.find(qa);
-                    if (a < 0) continue;
-                    int64_t lo = in_blk[((size_t)ap * nwi + ws) * nbi + a];
+                    const int a = in_ket[(size_t)ap * nwi + ws];
+                    if (a < 0 || !wr.any(s, w_in.off[ws], w_in.dim[ws])) continue;
                     int b = -1;
-                    int64_t so = site_sub(A, ssec, sloc, s, a, &b);
-                    if (lo < 0 || so < 0) continue;
+                    const int64_t so = site_sub(A, ssec, sloc, s, a, &b);
+                    if (so < 0) continue;
                     GemmSeg sg{};
-                    sg.a_off = lo; sg.a_rs = (int32_t)QL.dim[a]; sg.a_cs = 1;
+                    sg.a_off = in_blk[(size_t)ap * nwi + ws]; sg.a_rs = (int32_t)QL.dim[a]; sg.a_cs = 1;
                     sg.b_off = so; sg.b_rs = (int32_t)QR.dim[b]; sg.b_cs = 1;
                     sg.K = (int32_t)QL.dim[a];
-                    GemmTask tk{};
-                    tk.M = (int32_t)(QL.dim[ap] * w_in.dim[ws]);
-                    tk.N = (int32_t)QR.dim[b];
-                    tk.c_off = G.t1_total; tk.c_rs = tk.N; tk.c_cs = 1;
-                    tk.seg_begin = (int)G.g1.segs.size();
-                    G.g1.segs.push_back(sg);
-                    tk.seg_end = (int)G.g1.segs.size();
-                    tk.alpha = 1.0; tk.beta = 0.0;
-                    G.g1.flops += 2.0 * tk.M * tk.N * (double)sg.K;
-                    G.g1.tasks.push_back(tk);
-                    gemm_add_tiles(G.g1, (int)G.g1.tasks.size() - 1, kEnvTileM, kEnvTileN);
-                    t1[{s, ap, ws}] = {G.t1_total, b};
-                    G.t1_total += (int64_t)tk.M * tk.N;
+                    t1[((size_t)s * nbi + ap) * nwi + ws] = {G.t1_total, b};
+                    stage1(sg, QL.dim[ap] * w_in.dim[ws], QR.dim[b]);
                 }
         // stages 2 and 3, per output block (B', vs, B)
-        std::map<std::array<int64_t, 4>, int64_t> t2;  // (s', A', vs, B) -> offset
+        std::vector<int> left_of((size_t)QR.n() * P.n());  // A' = B' - q(s')
+        for (int bp = 0; bp < QR.n(); ++bp)
+            for (int p = 0; p < P.n(); ++p)
+                left_of[(size_t)bp * P.n() + p] = QL.find(qn_fuse(kind, QR.q[bp], qn_dual(kind, P.q[p])));
         for (size_t k = 0; k < lout.tri.size(); ++k) {
             const int bp = lout.tri[k][0], vs = lout.tri[k][1], b = lout.tri[k][2];
             const int64_t dvs = w_out.dim[vs];
@@ -236,56 +287,45 @@ static tk_status build_grow_tables_body(bool left, const QIndex& env_bra, const 
             tk.seg_begin = (int)G.g3.segs.size();
             tk.alpha = 1.0; tk.beta = 0.0;
             for (int64_t sp = 0; sp < d; ++sp) {
-                // bra block (s', A', B'): A' = B' - q(s')
-                Qn qap = qn_fuse(kind, QR.q[bp], qn_dual(kind, P.q[ssec[sp]]));
-                int ap = QL.find(qap);
+                // bra block (s', A', B')
+                const int ap = left_of[(size_t)bp * P.n() + ssec[sp]];
                 if (ap < 0) continue;
                 int rb = -1;
-                int64_t bo = site_sub(A, ssec, sloc, sp, ap, &rb);
+                const int64_t bo = site_sub(A, ssec, sloc, sp, ap, &rb);
                 if (bo < 0 || rb != bp) continue;
-                std::array<int64_t, 4> key{sp, ap, vs, b};
-                auto it = t2.find(key);
-                if (it == t2.end()) {
-                    // T2(s', A', vs, B)[(a', v)][b] = sum_{s, w} W[s, s', w, v] T1(s, A', ws(w))[(a', w)][b]
-                    const int64_t base = G.t2_total;
-                    size_t job0 = G.jobs.size(), term0 = G.terms.size();
-                    for (int64_t vl = 0; vl < dvs; ++vl) {
-                        const int64_t v = w_out.off[vs] + vl;
-                        CombJob j{};
-                        j.rows = (int32_t)QL.dim[ap];
-                        j.cols = (int32_t)QR.dim[b];
-                        j.out_off = base + vl * QR.dim[b];
-                        j.out_rs = (int32_t)(dvs * QR.dim[b]);
-                        j.term_begin = (int32_t)G.terms.size();
-                        for (int64_t s = 0; s < d; ++s)
-                            for (int64_t w = 0; w < w_in.total; ++w) {
-                                const double c = wval(s, sp, left ? w : v, left ? v : w);
-                                if (c == 0.0) continue;
-                                auto t = t1.find({s, ap, win_sec[w]});
-                                if (t == t1.end() || t->second.second != b) continue;
-                                CombTerm ct{};
-                                ct.in_off = t->second.first + win_loc[w] * QR.dim[b];
-                                ct.in_rs = (int32_t)(w_in.dim[win_sec[w]] * QR.dim[b]);
-                                ct.coef = c;
-                                G.terms.push_back(ct);
-                                G.comb_flops += 2.0 * j.rows * j.cols;
-                            }
-                        j.term_end = (int32_t)G.terms.size();
-                        G.jobs.push_back(j);
+                // T2(s', A', vs, B)[(a', v)][b] = sum_{s, w} W[s, s', w, v] T1(s, A', ws(w))[(a', w)][b]
+                const int64_t base = G.t2_total;
+                const size_t job0 = G.jobs.size(), term0 = G.terms.size();
+                for (int64_t vl = 0; vl < dvs; ++vl) {
+                    CombJob j{};
+                    j.rows = (int32_t)QL.dim[ap];
+                    j.cols = (int32_t)QR.dim[b];
+                    j.out_off = base + vl * QR.dim[b];
+                    j.out_rs = (int32_t)(dvs * QR.dim[b]);
+                    j.term_begin = (int32_t)G.terms.size();
+                    for (const MpoRows::Entry* t = wr.begin(sp, w_out.off[vs] + vl); t != wr.end(sp, w_out.off[vs] + vl); ++t) {
+                        const int ws = win_sec[t->w];
+                        const Part& part = t1[((size_t)t->s * nbi + ap) * nwi + ws];
+                        if (part.b != b) continue;
+                        CombTerm ct{};
+                        ct.in_off = part.off + win_loc[t->w] * QR.dim[b];
+                        ct.in_rs = (int32_t)(w_in.dim[ws] * QR.dim[b]);
+                        ct.coef = t->c;
+                        G.terms.push_back(ct);
+                        G.comb_flops += 2.0 * j.rows * j.cols;
                     }
-                    if (G.terms.size() == term0) {  // nothing reaches this block
-                        G.jobs.resize(job0);
-                        t2[key] = -1;
-                        continue;
-                    }
-                    G.t2_total += QL.dim[ap] * dvs * QR.dim[b];
-                    it = t2.emplace(key, base).first;
+                    j.term_end = (int32_t)G.terms.size();
+                    G.jobs.push_back(j);
                 }
-                if (it->second < 0) continue;
+                if (G.terms.size() == term0) {  // nothing reaches this block
+                    G.jobs.resize(job0);
+                    continue;
+                }
+                G.t2_total += QL.dim[ap] * dvs * QR.dim[b];
                 // L'(B', vs, B)[b'][(v, b)] += A(s', A', B')^T[b'][a'] * T2[a'][(v, b)]
                 GemmSeg sg{};
                 sg.a_off = bo; sg.a_rs = 1; sg.a_cs = (int32_t)QR.dim[bp];
-                sg.b_off = it->second; sg.b_rs = tk.N; sg.b_cs = 1;
+                sg.b_off = base; sg.b_rs = tk.N; sg.b_cs = 1;
                 sg.K = (int32_t)QL.dim[ap];
                 G.g3.segs.push_back(sg);
                 G.g3.flops += 2.0 * tk.M * tk.N * (double)sg.K;
@@ -296,41 +336,41 @@ static tk_status build_grow_tables_body(bool left, const QIndex& env_bra, const 
             gemm_add_tiles(G.g3, (int)G.g3.tasks.size() - 1, kEnvTileM, kEnvTileN);
         }
     } else {
-        // stage 1: T1(s, A, v)[a][b'] = A(s, A, B)[a][b] * R(B', vs, B)[b'][v][b], B' = B + q(vs)
-        std::map<std::array<int64_t, 3>, std::pair<int64_t, int>> t1;  // (s, A, v) -> (offset, B')
+        // (mpo, ket) sectors of the input -> its bra sector
+        std::vector<int> in_bra((size_t)nwi * nbi, -1);
+        for (const auto& t : lin.tri) in_bra[(size_t)t[1] * nbi + t[2]] = t[0];
+        // stage 1: T1(s, A, v)[a][b'] = A(s, A, B)[a][b] * R(B', vs, B)[b'][v][b], B' = B + q(vs);
+        // only the (s, v) that W couples to an output are formed
+        struct Part { int64_t off; int bp; };
+        std::vector<Part> t1((size_t)d * nl * nwi, Part{0, -1});  // the first of the sector's formed v
+        std::vector<int> nth((size_t)d * w_in.total);             // (s, v) -> its place among them
+        for (int64_t s = 0; s < d; ++s)
+            for (int vs = 0, n = 0; vs < nwi; ++vs, n = 0)
+                for (int64_t v = w_in.off[vs]; v < w_in.off[vs] + w_in.dim[vs]; ++v) {
+                    nth[(size_t)s * w_in.total + v] = n;
+                    n += wr.any(s, v, 1);
+                }
         for (int64_t s = 0; s < d; ++s)
             for (int a = 0; a < nl; ++a) {
                 int b = -1;
-                int64_t so = site_sub(A, ssec, sloc, s, a, &b);
+                const int64_t so = site_sub(A, ssec, sloc, s, a, &b);
                 if (so < 0) continue;
                 for (int vs = 0; vs < nwi; ++vs) {
-                    int bp = QR.find(qn_fuse(kind, QR.q[b], w_in.q[vs]));
+                    const int bp = in_bra[(size_t)vs * nbi + b];
                     if (bp < 0) continue;
-                    int64_t ro = in_blk[((size_t)bp * nwi + vs) * nbi + b];
-                    if (ro < 0) continue;
+                    const int64_t ro = in_blk[(size_t)bp * nwi + vs];
+                    t1[((size_t)s * nl + a) * nwi + vs] = {G.t1_total, bp};
                     for (int64_t vl = 0; vl < w_in.dim[vs]; ++vl) {
+                        if (!wr.any(s, w_in.off[vs] + vl, 1)) continue;
                         GemmSeg sg{};
                         sg.a_off = so; sg.a_rs = (int32_t)QR.dim[b]; sg.a_cs = 1;
                         sg.b_off = ro + vl * QR.dim[b]; sg.b_rs = 1; sg.b_cs = (int32_t)(w_in.dim[vs] * QR.dim[b]);
                         sg.K = (int32_t)QR.dim[b];
-                        GemmTask tk{};
-                        tk.M = (int32_t)QL.dim[a];
-                        tk.N = (int32_t)QR.dim[bp];
-                        tk.c_off = G.t1_total; tk.c_rs = tk.N; tk.c_cs = 1;
-                        tk.seg_begin = (int)G.g1.segs.size();
-                        G.g1.segs.push_back(sg);
-                        tk.seg_end = (int)G.g1.segs.size();
-                        tk.alpha = 1.0; tk.beta = 0.0;
-                        G.g1.flops += 2.0 * tk.M * tk.N * (double)sg.K;
-                        G.g1.tasks.push_back(tk);
-                        gemm_add_tiles(G.g1, (int)G.g1.tasks.size() - 1, kEnvTileM, kEnvTileN);
-                        t1[{s, a, w_in.off[vs] + vl}] = {G.t1_total, bp};
-                        G.t1_total += (int64_t)tk.M * tk.N;
+                        stage1(sg, QL.dim[a], QR.dim[bp]);
                     }
                 }
             }
         // stages 2 and 3, per output block (A', ws, A) and channel state w
-        std::map<std::array<int64_t, 4>, int64_t> t2;  // (s', A, w, B') -> offset
         for (size_t k = 0; k < lout.tri.size(); ++k) {
             const int ap = lout.tri[k][0], ws = lout.tri[k][1], a = lout.tri[k][2];
             const int64_t dws = w_out.dim[ws];
@@ -344,46 +384,34 @@ static tk_status build_grow_tables_body(bool left, const QIndex& env_bra, const 
                 tk.alpha = 1.0; tk.beta = 0.0;
                 for (int64_t sp = 0; sp < d; ++sp) {
                     int bp = -1;
-                    int64_t bo = site_sub(A, ssec, sloc, sp, ap, &bp);  // bra block (s', A', B')
+                    const int64_t bo = site_sub(A, ssec, sloc, sp, ap, &bp);  // bra block (s', A', B')
                     if (bo < 0) continue;
-                    std::array<int64_t, 4> key{sp, a, w, bp};
-                    auto it = t2.find(key);
-                    if (it == t2.end()) {
-                        // T2(s', A, w, B')[a][b'] = sum_{s, v} W[s, s', w, v] T1(s, A, v)[a][b']
-                        CombJob j{};
-                        j.rows = (int32_t)QL.dim[a];
-                        j.cols = (int32_t)QR.dim[bp];
-                        j.out_off = G.t2_total;
-                        j.out_rs = j.cols;
-                        j.term_begin = (int32_t)G.terms.size();
-                        for (int64_t s = 0; s < d; ++s)
-                            for (int64_t v = 0; v < w_in.total; ++v) {
-                                const double c = wval(s, sp, w, v);
-                                if (c == 0.0) continue;
-                                auto t = t1.find({s, a, v});
-                                if (t == t1.end() || t->second.second != bp) continue;
-                                CombTerm ct{};
-                                ct.in_off = t->second.first;
-                                ct.in_rs = j.cols;
-                                ct.coef = c;
-                                G.terms.push_back(ct);
-                                G.comb_flops += 2.0 * j.rows * j.cols;
-                            }
-                        j.term_end = (int32_t)G.terms.size();
-                        if (j.term_end == j.term_begin) {
-                            t2[key] = -1;
-                            continue;
-                        }
-                        G.jobs.push_back(j);
-                        it = t2.emplace(key, G.t2_total).first;
-                        G.t2_total += (int64_t)j.rows * j.cols;
+                    // T2(s', A, w, B')[a][b'] = sum_{s, v} W[s, s', w, v] T1(s, A, v)[a][b']
+                    CombJob j{};
+                    j.rows = (int32_t)QL.dim[a];
+                    j.cols = (int32_t)QR.dim[bp];
+                    j.out_off = G.t2_total;
+                    j.out_rs = j.cols;
+                    j.term_begin = (int32_t)G.terms.size();
+                    for (const MpoRows::Entry* t = wr.begin(sp, w); t != wr.end(sp, w); ++t) {
+                        const Part& part = t1[((size_t)t->s * nl + a) * nwi + win_sec[t->w]];
+                        if (part.bp != bp) continue;
+                        CombTerm ct{};
+                        ct.in_off = part.off + (int64_t)nth[(size_t)t->s * w_in.total + t->w] * j.rows * j.cols;
+                        ct.in_rs = j.cols;
+                        ct.coef = t->c;
+                        G.terms.push_back(ct);
+                        G.comb_flops += 2.0 * j.rows * j.cols;
                     }
-                    if (it->second < 0) continue;
+                    j.term_end = (int32_t)G.terms.size();
+                    if (j.term_end == j.term_begin) continue;
+                    G.jobs.push_back(j);
                     // R'(A', ws, A)[a'][(w, a)] += A(s', A', B')[a'][b'] * T2[a][b']^T
                     GemmSeg sg{};
                     sg.a_off = bo; sg.a_rs = (int32_t)QR.dim[bp]; sg.a_cs = 1;
-                    sg.b_off = it->second; sg.b_rs = 1; sg.b_cs = (int32_t)QR.dim[bp];
+                    sg.b_off = G.t2_total; sg.b_rs = 1; sg.b_cs = (int32_t)QR.dim[bp];
                     sg.K = (int32_t)QR.dim[bp];
+                    G.t2_total += (int64_t)j.rows * j.cols;
                     G.g3.segs.push_back(sg);
                     G.g3.flops += 2.0 * tk.M * tk.N * (double)sg.K;
                 }

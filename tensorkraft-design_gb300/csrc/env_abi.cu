@@ -3,6 +3,7 @@
 // site and the two-site start vector (tables in env.cpp).
 #include <cuda_runtime.h>
 
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -29,57 +30,94 @@ struct Guard {
     }
 };
 
-// Stream-ordered scratch: allocated from the device's memory pool on the
-// call's stream and released on it, so nothing waits on the host.
-struct Scratch {
-    cudaStream_t s;
-    std::vector<void*> ptrs;
-    explicit Scratch(cudaStream_t st) : s(st) {}
-    ~Scratch() {
-        for (void* p : ptrs) cudaFreeAsync(p, s);
-    }
-    template <class T>
-    cudaError_t upload(const std::vector<T>& v, T** out) {
-        *out = nullptr;
-        if (v.empty()) return cudaSuccess;
-        cudaError_t e = alloc(v.size() * sizeof(T), (void**)out);
-        if (e != cudaSuccess) return e;
-        // pageable source: staged before the call returns
-        return cudaMemcpyAsync(*out, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s);
-    }
-    cudaError_t alloc(size_t bytes, void** out) {
-        cudaError_t e = cudaMallocAsync(out, std::max<size_t>(bytes, 16), s);
-        if (e == cudaSuccess) ptrs.push_back(*out);
-        return e;
-    }
-};
+// The context's memory pool, made on first use.  A device's default pool hands
+// its memory back to the system whenever the device is synchronised, so a call
+// after each synchronisation maps it anew; this one keeps up to kPoolKeep
+// between calls and goes with the context.  Null where none can be made: the
+// default pool serves then.
+constexpr uint64_t kPoolKeep = 256ull << 20;
 
-tk_status launch_table(Scratch& sc, const GemmTable& g, const double* A, const double* B, double* C) {
-    GemmTask* t = nullptr;
-    GemmSeg* sg = nullptr;
-    GemmTile* tl = nullptr;
-    cudaError_t e;
-    if ((e = sc.upload(g.tasks, &t)) != cudaSuccess) return cuda_fail("upload tables", e);
-    if ((e = sc.upload(g.segs, &sg)) != cudaSuccess) return cuda_fail("upload tables", e);
-    if ((e = sc.upload(g.tiles, &tl)) != cudaSuccess) return cuda_fail("upload tables", e);
-    if ((e = launch_gemm_f64(tl, (int)g.tiles.size(), t, sg, A, B, C, sc.s)) != cudaSuccess)
-        return cuda_fail("grouped gemm", e);
-    return TK_OK;
+cudaMemPool_t scratch_pool(tk_ctx* ctx) {
+    std::lock_guard<std::mutex> lock(ctx->pool_mutex);
+    if (!ctx->scratch_pool) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = ctx->device;
+        cudaMemPool_t pool = nullptr;
+        uint64_t keep = kPoolKeep;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) cudaGetLastError();
+        ctx->scratch_pool = pool;
+    }
+    return (cudaMemPool_t)ctx->scratch_pool;
 }
 
-// A GEMM table uploaded to stream-ordered scratch.
+// The tables and scratch of one call: one allocation, ordered on the call's
+// stream and released on it, and one upload, so that nothing waits on the host.
+class Scratch {
+public:
+    Scratch(cudaMemPool_t pool, cudaStream_t s) : pool_(pool), s_(s) {}
+    ~Scratch() {
+        if (base_) cudaFreeAsync(base_, s_);
+    }
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+    // lays a table out; the pointer is valid after commit()
+    template <class T>
+    void table(const std::vector<T>& v, const T** out) {
+        const size_t at = tables_.size(), bytes = v.size() * sizeof(T);
+        tables_.resize(at + (bytes + 15) / 16 * 16);
+        if (bytes) std::memcpy(tables_.data() + at, v.data(), bytes);
+        slots_.push_back({(const void**)out, at, bytes > 0});
+    }
+    cudaError_t commit(size_t doubles, double** work) {
+        *work = nullptr;
+        const size_t bytes = tables_.size() + sizeof(double) * doubles;
+        if (bytes == 0) return cudaSuccess;
+        cudaError_t e =
+            pool_ ? cudaMallocFromPoolAsync(&base_, bytes, pool_, s_) : cudaMallocAsync(&base_, bytes, s_);
+        if (e != cudaSuccess) {
+            base_ = nullptr;
+            return e;
+        }
+        for (const Slot& t : slots_) *t.out = t.any ? (char*)base_ + t.at : nullptr;
+        *work = (double*)((char*)base_ + tables_.size());
+        // pageable source: staged before the call returns
+        return tables_.empty() ? cudaSuccess
+                               : cudaMemcpyAsync(base_, tables_.data(), tables_.size(), cudaMemcpyHostToDevice, s_);
+    }
+
+private:
+    struct Slot {
+        const void** out;
+        size_t at;
+        bool any;
+    };
+    cudaMemPool_t pool_;
+    cudaStream_t s_;
+    void* base_ = nullptr;
+    std::vector<char> tables_;
+    std::vector<Slot> slots_;
+};
+
+// A GEMM table in a call's scratch.
 struct DevTable {
-    GemmTask* t = nullptr;
-    GemmSeg* sg = nullptr;
-    GemmTile* tl = nullptr;
+    const GemmTask* t = nullptr;
+    const GemmSeg* sg = nullptr;
+    const GemmTile* tl = nullptr;
     int n = 0;
-    tk_status upload(Scratch& sc, const GemmTable& g) {
-        cudaError_t e;
-        if ((e = sc.upload(g.tasks, &t)) != cudaSuccess || (e = sc.upload(g.segs, &sg)) != cudaSuccess ||
-            (e = sc.upload(g.tiles, &tl)) != cudaSuccess)
-            return cuda_fail("upload tables", e);
+    void put(Scratch& sc, const GemmTable& g) {
+        sc.table(g.tasks, &t);
+        sc.table(g.segs, &sg);
+        sc.table(g.tiles, &tl);
         n = (int)g.tiles.size();
-        return TK_OK;
+    }
+    cudaError_t run(const double* A, const double* B, double* C, cudaStream_t s) const {
+        return launch_gemm_f64(tl, n, t, sg, A, B, C, s);
     }
 };
 
@@ -130,37 +168,41 @@ tk_status grow(const char* name, bool left, tk_ctx* ctx, const tk_env* env, cons
         return TK_ERR_CUDA;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    Scratch sc(s);
+    Scratch sc(scratch_pool(ctx), s);
     cudaError_t e;
     const size_t parts = cplx ? 2 : 1;
-    double *t1 = nullptr, *t2 = nullptr;
-    if ((e = sc.alloc(sizeof(double) * parts * (size_t)G.t1_total, (void**)&t1)) != cudaSuccess)
-        return cuda_fail("scratch", e);
-    if ((e = sc.alloc(sizeof(double) * parts * (size_t)G.t2_total, (void**)&t2)) != cudaSuccess)
-        return cuda_fail("scratch", e);
+    DevTable g1, g3;
+    const CombJob* jobs = nullptr;
+    const CombTerm* terms = nullptr;
+    st = guard_host("environment growth tables", err, [&] {
+        g1.put(sc, G.g1);
+        g3.put(sc, G.g3);
+        sc.table(G.jobs, &jobs);
+        sc.table(G.terms, &terms);
+        return TK_OK;
+    });
+    if (st != TK_OK) {
+        set_error(std::string(name) + ": " + err);
+        return st;
+    }
+    double* t1 = nullptr;
+    if ((e = sc.commit(parts * (size_t)(G.t1_total + G.t2_total), &t1)) != cudaSuccess) return cuda_fail("scratch", e);
+    double* t2 = t1 + parts * (size_t)G.t1_total;
     if ((e = cudaMemsetAsync(out, 0, sizeof(double) * (size_t)G.out_total, s)) != cudaSuccess)
         return cuda_fail("cudaMemsetAsync", e);
     if (cplx && (e = cudaMemsetAsync(out_im, 0, sizeof(double) * (size_t)G.out_total, s)) != cudaSuccess)
         return cuda_fail("cudaMemsetAsync", e);
-    CombJob* jobs = nullptr;
-    CombTerm* terms = nullptr;
-    if ((e = sc.upload(G.jobs, &jobs)) != cudaSuccess) return cuda_fail("upload tables", e);
-    if ((e = sc.upload(G.terms, &terms)) != cudaSuccess) return cuda_fail("upload tables", e);
     if (!cplx) {
-        if (left)
-            st = launch_table(sc, G.g1, env->data, A.data, t1);
-        else
-            st = launch_table(sc, G.g1, A.data, env->data, t1);
-        if (st != TK_OK) return st;
+        if ((e = left ? g1.run(env->data, A.data, t1, s) : g1.run(A.data, env->data, t1, s)) != cudaSuccess)
+            return cuda_fail("grouped gemm", e);
         if ((e = launch_combine_f64(jobs, (int)G.jobs.size(), terms, t1, t2, s)) != cudaSuccess)
             return cuda_fail("combine", e);
-        return launch_table(sc, G.g3, A.data, t2, out);
+        if ((e = g3.run(A.data, t2, out, s)) != cudaSuccess) return cuda_fail("grouped gemm", e);
+        return TK_OK;
     }
     // complex: stage 1 without conjugation, stage 3 with the bra (site operand) conjugated
     double* t1i = t1 + G.t1_total;
     double* t2i = t2 + G.t2_total;
-    DevTable g1, g3;
-    if ((st = g1.upload(sc, G.g1)) != TK_OK || (st = g3.upload(sc, G.g3)) != TK_OK) return st;
     if (left)
         e = launch_gemm_c64(g1.tl, g1.n, g1.t, g1.sg, env->data, env_im, A.data, a_im, t1, t1i, false, s);
     else
@@ -338,9 +380,18 @@ tk_status tk_heff2_two_site_product_complex(tk_heff2_plan* plan, const tk_bst* a
     if ((e = cudaMemsetAsync(psi_re, 0, sizeof(double) * n, s)) != cudaSuccess ||
         (e = cudaMemsetAsync(psi_im, 0, sizeof(double) * n, s)) != cudaSuccess)
         return cuda_fail("cudaMemsetAsync", e);
-    Scratch sc(s);
+    Scratch sc(nullptr, s);
     DevTable g;
-    if ((st = g.upload(sc, gt)) != TK_OK) return st;
+    double* none = nullptr;
+    st = guard_host("two-site product tables", err, [&] {
+        g.put(sc, gt);
+        return TK_OK;
+    });
+    if (st != TK_OK) {
+        set_error("tk_heff2_two_site_product_complex: " + err);
+        return st;
+    }
+    if ((e = sc.commit(0, &none)) != cudaSuccess) return cuda_fail("upload tables", e);
     if ((e = launch_gemm_c64(g.tl, g.n, g.t, g.sg, Ai.data, a_i_im, Aj.data, a_j_im, psi_re, psi_im, false, s)) !=
         cudaSuccess)
         return cuda_fail("grouped gemm", e);
@@ -359,8 +410,8 @@ tk_status tk_heff2_two_site_product(tk_heff2_plan* plan, const tk_bst* a_i, cons
         set_error("tk_heff2_two_site_product: " + err);
         return TK_ERR_INVALID_ARG;
     }
-    GemmTable g;
-    tk_status st = build_product_tables(plan->host, Ai, Aj, g, err);
+    GemmTable gt;
+    tk_status st = build_product_tables(plan->host, Ai, Aj, gt, err);
     if (st != TK_OK) {
         set_error("tk_heff2_two_site_product: " + err);
         return st;
@@ -374,8 +425,20 @@ tk_status tk_heff2_two_site_product(tk_heff2_plan* plan, const tk_bst* a_i, cons
     cudaError_t e;
     if ((e = cudaMemsetAsync(psi_dev, 0, sizeof(double) * (size_t)plan->host.total, s)) != cudaSuccess)
         return cuda_fail("cudaMemsetAsync", e);
-    Scratch sc(s);
-    return launch_table(sc, g, Ai.data, Aj.data, psi_dev);
+    Scratch sc(nullptr, s);
+    DevTable g;
+    double* none = nullptr;
+    st = guard_host("two-site product tables", err, [&] {
+        g.put(sc, gt);
+        return TK_OK;
+    });
+    if (st != TK_OK) {
+        set_error("tk_heff2_two_site_product: " + err);
+        return st;
+    }
+    if ((e = sc.commit(0, &none)) != cudaSuccess) return cuda_fail("upload tables", e);
+    if ((e = g.run(Ai.data, Aj.data, psi_dev, s)) != cudaSuccess) return cuda_fail("grouped gemm", e);
+    return TK_OK;
 }
 
 }  // extern "C"

@@ -31,6 +31,9 @@ struct tk_ctx {
     // device buffers of finished tk_gemm_f64 calls, for the next ones (linalg.cu)
     std::mutex gemm_mutex;
     std::vector<std::pair<void*, size_t>> gemm_free;
+    // cudaMemPool_t of the environment growths' tables and scratch (env_abi.cu)
+    std::mutex pool_mutex;
+    void* scratch_pool = nullptr;
 };
 
 namespace tk {

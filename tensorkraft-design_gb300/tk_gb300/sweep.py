@@ -68,6 +68,15 @@ def env_layout(kind: int, bra: QIndex, mpo: QIndex, ket: QIndex):
     return keys, offs, tot.value
 
 
+def _env_size(kind: int, bond: QIndex, mpo: QIndex) -> int:
+    """Elements of the environment on `bond` and `mpo` (tk_env_layout's total alone)."""
+    m = _Marshal()
+    b, w = m.qindex(bond), m.qindex(mpo)
+    n, tot = C.c_int64(0), C.c_int64(0)
+    check(_abi.load().tk_env_layout(kind, C.byref(b), C.byref(w), C.byref(b), C.byref(n), None, None, C.byref(tot)))
+    return tot.value
+
+
 class DeviceEnv:
     """Block-sparse environment (bra, mpo, ket) in the canonical layout, device data."""
 
@@ -213,7 +222,7 @@ def _grow(left: bool, env: DeviceEnv, A: SiteTensor, W, stream=None, device: int
     e, a, w = env.marshal(m), A.marshal(m), m.bst(W)
     bond = A.legs[2] if left else A.legs[1]
     wl = W.indices[3] if left else W.indices[2]
-    _, _, total = env_layout(A.kind, bond, wl, bond)
+    total = _env_size(A.kind, bond, wl)
     out = torch.empty(max(total, 1), dtype=torch.float64, device=f"cuda:{device}")
     s = C.c_void_p(stream) if stream is not None else C.c_void_p(0)
     if not cplx:
