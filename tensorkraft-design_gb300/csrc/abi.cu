@@ -190,7 +190,7 @@ tk_status tk_heff2_plan_footprint(const tk_env* env_l, const tk_env* env_r, cons
     }
     std::string err;
     Heff2Tables H;
-    tk_status st = build_heff2_tables(*env_l, *env_r, *w_i, *w_j, psi_flux, kF64TileM, kF64TileN, H, err);
+    tk_status st = build_heff2_tables(*env_l, *env_r, *w_i, *w_j, psi_flux, H, err);
     if (st == TK_OK) st = ensure_tc_tables(H, err);  // the stack sizes of both precisions come from them
     if (st != TK_OK) {
         set_error("tk_heff2_plan_footprint: " + err);
@@ -272,7 +272,7 @@ tk_status tk::plan_create_impl(tk_ctx* ctx, const tk_env* env_l, const tk_env* e
         return TK_ERR_OOM;
     }
     std::string err;
-    tk_status st = build_heff2_tables(*env_l, *env_r, *w_i, *w_j, psi_flux, kF64TileM, kF64TileN, p->host, err,
+    tk_status st = build_heff2_tables(*env_l, *env_r, *w_i, *w_j, psi_flux, p->host, err,
                                       l_blocks, r_blocks);
     if (st != TK_OK) {
         set_error("tk_heff2_plan_create: " + err);

@@ -166,8 +166,8 @@ private:
 };
 
 bool finish(GrowTables& G, int64_t n_env, int64_t n_site, int64_t n_out, bool left, std::string& err) {
-    gemm_lpt_order(G.g1, kEnvTileM, kEnvTileN);
-    gemm_lpt_order(G.g3, kEnvTileM, kEnvTileN);
+    gemm_lpt_order(G.g1);
+    gemm_lpt_order(G.g3);
     if (G.g1.tiles.size() > (size_t)INT32_MAX || G.g3.tiles.size() > (size_t)INT32_MAX ||
         G.jobs.size() > (size_t)INT32_MAX || G.terms.size() > (size_t)INT32_MAX) {
         err = "environment tables exceed 32-bit index range";
@@ -245,7 +245,7 @@ static tk_status build_grow_tables_body(bool left, const QIndex& env_bra, const 
         tk.alpha = 1.0; tk.beta = 0.0;
         G.g1.flops += 2.0 * tk.M * tk.N * (double)sg.K;
         G.g1.tasks.push_back(tk);
-        gemm_add_tiles(G.g1, (int)G.g1.tasks.size() - 1, kEnvTileM, kEnvTileN);
+        gemm_add_tiles(G.g1, (int)G.g1.tasks.size() - 1);
         G.t1_total += m * n;
     };
     // A T2 block is named by (s', vs or w, ket sector of its output block) and
@@ -333,7 +333,7 @@ static tk_status build_grow_tables_body(bool left, const QIndex& env_bra, const 
             tk.seg_end = (int)G.g3.segs.size();
             if (tk.seg_end == tk.seg_begin) continue;  // stays zero
             G.g3.tasks.push_back(tk);
-            gemm_add_tiles(G.g3, (int)G.g3.tasks.size() - 1, kEnvTileM, kEnvTileN);
+            gemm_add_tiles(G.g3, (int)G.g3.tasks.size() - 1);
         }
     } else {
         // (mpo, ket) sectors of the input -> its bra sector
@@ -418,7 +418,7 @@ static tk_status build_grow_tables_body(bool left, const QIndex& env_bra, const 
                 tk.seg_end = (int)G.g3.segs.size();
                 if (tk.seg_end == tk.seg_begin) continue;
                 G.g3.tasks.push_back(tk);
-                gemm_add_tiles(G.g3, (int)G.g3.tasks.size() - 1, kEnvTileM, kEnvTileN);
+                gemm_add_tiles(G.g3, (int)G.g3.tasks.size() - 1);
             }
         }
     }
@@ -480,10 +480,10 @@ static tk_status build_product_tables_body(const Heff2Tables& H, const Bst3& Ai,
                 tk.alpha = 1.0; tk.beta = 0.0;
                 g.flops += 2.0 * tk.M * tk.N * (double)sg.K;
                 g.tasks.push_back(tk);
-                gemm_add_tiles(g, (int)g.tasks.size() - 1, kEnvTileM, kEnvTileN);
+                gemm_add_tiles(g, (int)g.tasks.size() - 1);
             }
     }
-    gemm_lpt_order(g, kEnvTileM, kEnvTileN);
+    gemm_lpt_order(g);
     if (!gemm_table_ok(g, Ai.total, Aj.total, H.total, "two-site product", err)) return TK_ERR_INVALID_ARG;
     return TK_OK;
 }

@@ -11,9 +11,6 @@
 #include "tk_env.hpp"
 #include "tk_plan.cuh"
 
-static_assert(tk::kEnvTileM == tk::kF64TileM && tk::kEnvTileN == tk::kF64TileN,
-              "environment tables are cut for the grouped FP64 GEMM tile");
-
 using namespace tk;
 
 namespace {

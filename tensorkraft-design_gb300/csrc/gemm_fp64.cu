@@ -1,13 +1,20 @@
 // gemm_fp64.cu -- FP64 sector-GEMM path of the two-site H_eff.
 //
-// grouped_gemm_f64: one CTA per output tile (64, 32 or 16 square, chosen per
-// task by the host so small sector blocks are not padded).  A tile's task is one
+// grouped_gemm_f64: one CTA per 16 x 16 output tile.  A tile's task is one
 // output block; its K dimension is a list of segments (one per contributing
 // sector pair), accumulated in registers, so every output element is written
 // exactly once and no atomics are needed.  Operand tiles are staged through
 // shared memory with the load mapping chosen per segment so that the
 // unit-stride direction of each operand is the one walked by consecutive
 // threads (coalesced for K-major and N-major operands alike).
+//
+// What bounds it is the FP64 pipe (1.2 TFLOP/s over the chip, so a 64 x 64 x 240
+// tile keeps one SM busy for a quarter of a millisecond), not the loads (1 byte a
+// multiply-add even at 16 x 16).  Hence the small edge: the pipe does hardly any
+// work for padding and the longest tile is short beside the whole.  With edges of
+// 64, 32 or 16 by task, the growth of an environment of 2 x 78 MFLOP (hubbard,
+// D = 2048) took 139 + 281 us, its pipe 2 x 105; with 16 everywhere
+// 82 + 85 us, its pipe 2 x 69.
 //
 // combine_f64: applies the fused two-site MPO W_ij between the two GEMM
 // stages, out = sum_t coef_t * in_t over equally shaped slabs.
@@ -21,125 +28,149 @@ namespace tk {
 
 namespace {
 
+constexpr int NT = 256;
 constexpr int BK = 16;
-constexpr int NT = 256;  // 16 x 16 threads
+constexpr int E = kF64Tile;
+constexpr int kSegs = 32;  // segments of a task kept in shared memory at a time
 
-// One E x E output tile (E = 64, 32 or 16): thread (tx, ty) owns the
-// (E/16) x (E/16) outputs (ty + 16 i, tx + 16 j); in a 16 x 16 tile the
-// threads are laid over the valid mv x nv outputs instead (thread t owns
-// (t / nv, t % nv)), so that a sector block of 13 x 13 keeps six warps
-// busy and leaves two idle rather than spreading its outputs over all eight.
-// Every output sums its segments in order and k ascending inside each, and
-// only the k < K of each segment are multiplied, whatever E and the mapping
-// are, so neither changes the result.  Warps without a valid output skip the
-// multiplications (the FP64 pipe is this GPU's bottleneck for these tiles).
-template <int E>
-__device__ __forceinline__ void gemm_tile(const GemmTile& tile, const GemmTask& task, const GemmSeg* __restrict__ segs,
-                                          const double* __restrict__ A, const double* __restrict__ B,
-                                          double* __restrict__ C, double (*As)[65], double (*Bs)[65], double amul,
-                                          int accumulate) {
-    constexpr int R = E / 16;
-    const int tid = threadIdx.x;
+__device__ __forceinline__ void store_out(const GemmTask& task, double* __restrict__ C, int gm, int gn, double acc,
+                                          double amul, int accumulate) {
+    double* c = C + task.c_off + (int64_t)gm * task.c_rs + (int64_t)gn * task.c_cs;
+    double v = amul * task.alpha * acc;
+    if (accumulate)
+        v += *c;
+    else if (task.beta != 0.0)
+        v += task.beta * *c;
+    *c = v;
+}
+
+// The threads are laid over the valid mv x nv outputs (thread t owns
+// (t / nv, t % nv)), so that a sector block of 13 x 13 keeps six warps busy and
+// leaves two idle rather than spreading its outputs over all eight.  Every
+// output sums its segments in order and k ascending inside each.  A step of k
+// past a segment's K is not issued: a predicated-off FMA holds the pipe as long
+// as a real one.  The next 16 k are on their way from memory while the present
+// ones are multiplied.
+__global__ void __launch_bounds__(NT, 6) grouped_gemm_f64_kernel(const GemmTile* __restrict__ tiles, int n_tiles,
+                                                                 const GemmTask* __restrict__ tasks,
+                                                                 const GemmSeg* __restrict__ segs,
+                                                                 const double* __restrict__ A,
+                                                                 const double* __restrict__ B,
+                                                                 double* __restrict__ C, double amul, int accumulate) {
+    __shared__ double As[2][BK][E + 1];
+    __shared__ double Bs[2][BK][E + 1];
+    __shared__ GemmSeg sseg[kSegs];
+    if ((int)blockIdx.x >= n_tiles) return;
+    const GemmTile tile = tiles[blockIdx.x];
+    const GemmTask& task = tasks[tile.task];
+    const int tid = threadIdx.x, lo = tid & 15, hi = tid >> 4;
     const int mv = min(E, task.M - tile.m0), nv = min(E, task.N - tile.n0);
-    int tx = tid & 15, ty = tid >> 4;
-    bool mine = true;
-    if (E == 16) {
-        mine = tid < mv * nv;
-        ty = mine ? tid / nv : 0;
-        tx = mine ? tid - ty * nv : 0;
-    } else {
-        mine = ty < mv && tx < nv;
+    const int seg_begin = task.seg_begin, seg_end = task.seg_end;
+    const bool mine = tid < mv * nv;
+    const int ty = mine ? tid / nv : 0, tx = mine ? tid - ty * nv : 0;
+    const bool warp_busy = (tid & ~31) < mv * nv;
+    double acc = 0.0;
+    int p = 0;
+    for (int s0 = seg_begin; s0 < seg_end; s0 += kSegs) {
+        const int ns = min(kSegs, seg_end - s0);
+        // the last reads of the batch before lie ahead of that batch's last barrier
+        for (int i = tid; i < ns; i += NT) sseg[i] = segs[s0 + i];
+        __syncthreads();
+        double va, vb;
+        auto fetch = [&](const GemmSeg& sg, int k0) {
+            const bool ak = sg.a_cs == 1, bn = sg.b_cs == 1;
+            const int am = ak ? hi : lo, ka = k0 + (ak ? lo : hi);
+            const int bc = bn ? lo : hi, kb = k0 + (bn ? hi : lo);
+            va = am < mv && ka < sg.K ? A[sg.a_off + (int64_t)(tile.m0 + am) * sg.a_rs + (int64_t)ka * sg.a_cs] : 0.0;
+            vb = bc < nv && kb < sg.K ? B[sg.b_off + (int64_t)kb * sg.b_rs + (int64_t)(tile.n0 + bc) * sg.b_cs] : 0.0;
+        };
+        int s = 0, k0 = 0;
+        fetch(sseg[0], 0);
+        while (s < ns) {
+            const bool ak = sseg[s].a_cs == 1, bn = sseg[s].b_cs == 1;
+            const int K = sseg[s].K, kl = min(BK, K - k0);
+            As[p][ak ? lo : hi][ak ? hi : lo] = va;
+            Bs[p][bn ? hi : lo][bn ? lo : hi] = vb;
+            __syncthreads();
+            k0 += BK;
+            if (k0 >= K) {
+                ++s;
+                k0 = 0;
+            }
+            if (s < ns) fetch(sseg[s], k0);
+            if (warp_busy) {
+                if (kl == BK) {
+#pragma unroll
+                    for (int k = 0; k < BK; ++k) acc = fma(As[p][k][ty], Bs[p][k][tx], acc);
+                } else {
+#pragma unroll 1
+                    for (int k = 0; k < kl; ++k) acc = fma(As[p][k][ty], Bs[p][k][tx], acc);
+                }
+            }
+            p ^= 1;
+        }
     }
-    const bool warp_busy = __any_sync(0xffffffffu, mine);
+    if (mine) store_out(task, C, tile.m0 + ty, tile.n0 + tx, acc, amul, accumulate);
+}
+
+// 64 x 64 tiles of one dense product, where 16 x 16 ones would not fit the
+// caller's table: thread (tx, ty) owns the outputs (ty + 16 i, tx + 16 j).
+__global__ void __launch_bounds__(NT) wide_gemm_f64_kernel(const GemmTile* __restrict__ tiles, int n_tiles,
+                                                           const GemmTask* __restrict__ tasks,
+                                                           const GemmSeg* __restrict__ segs,
+                                                           const double* __restrict__ A, const double* __restrict__ B,
+                                                           double* __restrict__ C) {
+    constexpr int W = kF64WideTile, R = W / 16;
+    __shared__ double As[BK][W + 1];
+    __shared__ double Bs[BK][W + 1];
+    if ((int)blockIdx.x >= n_tiles) return;
+    const GemmTile tile = tiles[blockIdx.x];
+    const GemmTask task = tasks[tile.task];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     double acc[R][R];
 #pragma unroll
     for (int i = 0; i < R; ++i)
 #pragma unroll
         for (int j = 0; j < R; ++j) acc[i][j] = 0.0;
-
     for (int s = task.seg_begin; s < task.seg_end; ++s) {
         const GemmSeg sg = segs[s];
         for (int k0 = 0; k0 < sg.K; k0 += BK) {
-            // A tile: E x BK
 #pragma unroll
-            for (int r = 0; r < (E * BK) / NT; ++r) {
-                int e = tid + r * NT;
-                int m, k;
-                if (sg.a_cs == 1) { k = e % BK; m = e / BK; } else { m = e % E; k = e / E; }
-                int gm = tile.m0 + m, gk = k0 + k;
-                double v = 0.0;
-                if (gm < task.M && gk < sg.K) v = A[sg.a_off + (int64_t)gm * sg.a_rs + (int64_t)gk * sg.a_cs];
-                As[k][m] = v;
-            }
-            // B tile: BK x E
-#pragma unroll
-            for (int r = 0; r < (BK * E) / NT; ++r) {
-                int e = tid + r * NT;
-                int k, n;
-                if (sg.b_cs == 1) { n = e % E; k = e / E; } else { k = e % BK; n = e / BK; }
-                int gn = tile.n0 + n, gk = k0 + k;
-                double v = 0.0;
-                if (gn < task.N && gk < sg.K) v = B[sg.b_off + (int64_t)gk * sg.b_rs + (int64_t)gn * sg.b_cs];
-                Bs[k][n] = v;
+            for (int r = 0; r < (W * BK) / NT; ++r) {
+                const int e = tid + r * NT;
+                const bool ak = sg.a_cs == 1, bn = sg.b_cs == 1;
+                const int m = ak ? e / BK : e % W, ka = ak ? e % BK : e / W;
+                const int n = bn ? e % W : e / BK, kb = bn ? e / W : e % BK;
+                const int gm = tile.m0 + m, gn = tile.n0 + n;
+                As[ka][m] = gm < task.M && k0 + ka < sg.K
+                                ? A[sg.a_off + (int64_t)gm * sg.a_rs + (int64_t)(k0 + ka) * sg.a_cs] : 0.0;
+                Bs[kb][n] = gn < task.N && k0 + kb < sg.K
+                                ? B[sg.b_off + (int64_t)(k0 + kb) * sg.b_rs + (int64_t)gn * sg.b_cs] : 0.0;
             }
             __syncthreads();
-            const int kl = min(BK, sg.K - k0);  // k past the segment's K would add zero products
-            if (warp_busy) {
+            const int kl = min(BK, sg.K - k0);
+#pragma unroll 4
+            for (int k = 0; k < kl; ++k) {
+                double a[R], b[R];
 #pragma unroll
-                for (int k = 0; k < BK; ++k) {
-                    if (k < kl) {
-                        double a[R], b[R];
+                for (int i = 0; i < R; ++i) a[i] = As[k][ty + 16 * i];
 #pragma unroll
-                        for (int i = 0; i < R; ++i) a[i] = As[k][ty + 16 * i];
+                for (int j = 0; j < R; ++j) b[j] = Bs[k][tx + 16 * j];
 #pragma unroll
-                        for (int j = 0; j < R; ++j) b[j] = Bs[k][tx + 16 * j];
+                for (int i = 0; i < R; ++i)
 #pragma unroll
-                        for (int i = 0; i < R; ++i)
-#pragma unroll
-                            for (int j = 0; j < R; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-                    }
-                }
+                    for (int j = 0; j < R; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
             }
             __syncthreads();
         }
     }
-    if (!mine) return;
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-        int gm = tile.m0 + ty + 16 * i;
-        if (gm >= task.M) continue;
+    for (int i = 0; i < R; ++i)
 #pragma unroll
         for (int j = 0; j < R; ++j) {
-            int gn = tile.n0 + tx + 16 * j;
-            if (gn >= task.N) continue;
-            double* c = C + task.c_off + (int64_t)gm * task.c_rs + (int64_t)gn * task.c_cs;
-            double v = amul * task.alpha * acc[i][j];
-            if (accumulate)
-                v += *c;
-            else if (task.beta != 0.0)
-                v += task.beta * *c;
-            *c = v;
+            const int gm = tile.m0 + ty + 16 * i, gn = tile.n0 + tx + 16 * j;
+            if (gm < task.M && gn < task.N) store_out(task, C, gm, gn, acc[i][j], 1.0, 0);
         }
-    }
-}
-
-__global__ void __launch_bounds__(NT) grouped_gemm_f64_kernel(const GemmTile* __restrict__ tiles, int n_tiles,
-                                                              const GemmTask* __restrict__ tasks,
-                                                              const GemmSeg* __restrict__ segs,
-                                                              const double* __restrict__ A,
-                                                              const double* __restrict__ B,
-                                                              double* __restrict__ C, double amul, int accumulate) {
-    __shared__ double As[BK][65];
-    __shared__ double Bs[BK][65];
-    const int tile_id = blockIdx.x;
-    if (tile_id >= n_tiles) return;
-    const GemmTile tile = tiles[tile_id];
-    const GemmTask task = tasks[tile.task];
-    switch (tile.cls) {  // block-uniform
-    case 1: gemm_tile<32>(tile, task, segs, A, B, C, As, Bs, amul, accumulate); break;
-    case 2: gemm_tile<16>(tile, task, segs, A, B, C, As, Bs, amul, accumulate); break;
-    default: gemm_tile<64>(tile, task, segs, A, B, C, As, Bs, amul, accumulate); break;
-    }
 }
 
 __global__ void __launch_bounds__(256) combine_f64_kernel(const CombJob* __restrict__ jobs,
@@ -177,6 +208,13 @@ cudaError_t launch_gemm_f64(const GemmTile* tiles, int n_tiles, const GemmTask* 
                             bool accumulate) {
     if (n_tiles <= 0) return cudaSuccess;
     grouped_gemm_f64_kernel<<<n_tiles, NT, 0, s>>>(tiles, n_tiles, tasks, segs, A, B, C, amul, accumulate ? 1 : 0);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_wide_gemm_f64(const GemmTile* tiles, int n_tiles, const GemmTask* tasks, const GemmSeg* segs,
+                                 const double* A, const double* B, double* C, cudaStream_t s) {
+    if (n_tiles <= 0) return cudaSuccess;
+    wide_gemm_f64_kernel<<<n_tiles, NT, 0, s>>>(tiles, n_tiles, tasks, segs, A, B, C);
     return cudaGetLastError();
 }
 

@@ -6,14 +6,16 @@
 
 namespace tk {
 
-// FP64 grouped segmented GEMM over a tile list (one CTA per 64x64 tile).
-constexpr int kF64TileM = 64;
-constexpr int kF64TileN = 64;
+// FP64 grouped segmented GEMM over a list of kF64Tile-square tiles, one CTA each.
 // C = amul * alpha * A B (+ beta C, or + C when `accumulate`), per task.
 cudaError_t launch_gemm_f64(const GemmTile* tiles, int n_tiles, const GemmTask* tasks, const GemmSeg* segs,
                             const double* A, const double* B, double* C, cudaStream_t s, double amul = 1.0,
                             bool accumulate = false);
-// The same tables on planar complex operands (four launches): C = A B, or
+// Plain dense products over a list of kF64WideTile-square tiles.
+constexpr int kF64WideTile = 64;
+cudaError_t launch_wide_gemm_f64(const GemmTile* tiles, int n_tiles, const GemmTask* tasks, const GemmSeg* segs,
+                                 const double* A, const double* B, double* C, cudaStream_t s);
+// The tables of launch_gemm_f64 on planar complex operands (four launches): C = A B, or
 // conj(A) B with conj_a; the tasks must overwrite their output (beta = 0).
 cudaError_t launch_gemm_c64(const GemmTile* tiles, int n_tiles, const GemmTask* tasks, const GemmSeg* segs,
                             const double* Ar, const double* Ai, const double* Br, const double* Bi, double* Cr,

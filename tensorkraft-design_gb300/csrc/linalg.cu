@@ -77,7 +77,6 @@ struct Scratch {
         if (e_ != cudaSuccess) return fail(#op, e_);  \
     } while (0)
 
-void tiles_for(GemmTable& g, int task) { bsgemm_tiles_for(g, task); }
 
 // A device buffer for one tk_gemm_f64 call.  The call waits for its stream
 // before it gives the buffer back, so any thread's next call on the context
@@ -260,7 +259,7 @@ tk_status tk_gemm_f64(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* 
         g.segs.push_back(s);
     }
     g.tasks.push_back(t);
-    tiles_for(g, 0);
+    gemm_add_tiles(g, 0);
     Scratch sc;
     GemmTask* dt; GemmSeg* ds; GemmTile* dl;
     CK(sc.put(g.tasks, &dt));
@@ -465,7 +464,7 @@ tk_status tk_spmv_f64(tk_ctx* ctx, const tk_bst* a_abi, const double* x, double*
         }
         t.seg_end = (int)g.segs.size();
         g.tasks.push_back(t);
-        tiles_for(g, (int)g.tasks.size() - 1);
+        gemm_add_tiles(g, (int)g.tasks.size() - 1);
     }
     // Row sectors without blocks are zero.
     for (int r = 0; r < A.legs[0].n(); ++r) {
@@ -476,7 +475,7 @@ tk_status tk_spmv_f64(tk_ctx* ctx, const tk_bst* a_abi, const double* x, double*
         t.alpha = 1.0; t.beta = 0.0;
         t.seg_begin = t.seg_end = (int)g.segs.size();
         g.tasks.push_back(t);
-        tiles_for(g, (int)g.tasks.size() - 1);
+        gemm_add_tiles(g, (int)g.tasks.size() - 1);
     }
     if (rows == 0) return TK_OK;
     int dev = ctx ? ctx->device : 0;

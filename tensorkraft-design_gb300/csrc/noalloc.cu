@@ -53,7 +53,7 @@ std::mutex g_setup_mutex;
 unsigned char* g_scratch_ptr[kMaxDevices] = {};
 
 // Writes the GEMM's task, its single K segment and the tile list into the scratch.
-__global__ void fill_gemm_tables_kernel(tk::GemmTask task, tk::GemmSeg seg, int ntile_n, int ntiles,
+__global__ void fill_gemm_tables_kernel(tk::GemmTask task, tk::GemmSeg seg, int edge, int ntile_n, int ntiles,
                                         unsigned char* scratch) {
     tk::GemmTask* t = reinterpret_cast<tk::GemmTask*>(scratch);
     tk::GemmSeg* s = reinterpret_cast<tk::GemmSeg*>(scratch + 128);
@@ -63,7 +63,7 @@ __global__ void fill_gemm_tables_kernel(tk::GemmTask task, tk::GemmSeg seg, int 
         *s = seg;
     }
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntiles; i += gridDim.x * blockDim.x)
-        tiles[i] = tk::GemmTile{0, (i / ntile_n) * tk::kF64TileM, (i % ntile_n) * tk::kF64TileN, 0};
+        tiles[i] = tk::GemmTile{0, (i / ntile_n) * edge, (i % ntile_n) * edge, 0};
 }
 
 tk_status fail(const std::string& msg, tk_status code) {
@@ -85,12 +85,16 @@ extern "C" tk_status tk_gemm_f64_noalloc(tk_ctx* ctx, double alpha, const tk_mat
         std::llabs(a->col_stride) > lim || std::llabs(b->row_stride) > lim || std::llabs(b->col_stride) > lim ||
         std::llabs(c->row_stride) > lim || std::llabs(c->col_stride) > lim)
         return fail("tk_gemm_f64_noalloc: dimensions or strides exceed 32 bits", TK_ERR_UNSUPPORTED);
-    const int64_t ntm = (c->rows + tk::kF64TileM - 1) / tk::kF64TileM;
-    const int64_t ntn = (c->cols + tk::kF64TileN - 1) / tk::kF64TileN;
+    int edge = tk::kF64WideTile;
+    int64_t ntm = (c->rows + edge - 1) / edge, ntn = (c->cols + edge - 1) / edge;
     if (ntm * ntn > kNoallocMaxTiles)
         return fail("tk_gemm_f64_noalloc: output needs " + std::to_string(ntm * ntn) + " 64x64 tiles, more than the " +
                         std::to_string(kNoallocMaxTiles) + " the 1 MiB no-allocation scratch holds; use tk_gemm_f64",
                     TK_ERR_INVALID_ARG);
+    // the grouped kernel's 16 x 16 tiles while the scratch holds their list (outputs
+    // up to 4096 x 4096): small outputs fill the GPU, and padding costs least
+    const int64_t sm = (c->rows + tk::kF64Tile - 1) / tk::kF64Tile, sn = (c->cols + tk::kF64Tile - 1) / tk::kF64Tile;
+    if (sm * sn <= kNoallocMaxTiles) edge = tk::kF64Tile, ntm = sm, ntn = sn;
     const int dev = ctx ? ctx->device : 0;
     if (dev < 0 || dev >= kMaxDevices) return fail("tk_gemm_f64_noalloc: device index out of range", TK_ERR_INVALID_ARG);
     int prev = -1;
@@ -137,12 +141,14 @@ extern "C" tk_status tk_gemm_f64_noalloc(tk_ctx* ctx, double alpha, const tk_mat
     const int ntiles = (int)(ntm * ntn);
     cudaStream_t s = (cudaStream_t)stream;
     const int fill_blocks = (ntiles + 255) / 256;
-    fill_gemm_tables_kernel<<<fill_blocks, 256, 0, s>>>(task, seg, (int)ntn, ntiles, scratch);
+    fill_gemm_tables_kernel<<<fill_blocks, 256, 0, s>>>(task, seg, edge, (int)ntn, ntiles, scratch);
     if ((e = cudaGetLastError()) != cudaSuccess)
         return fail(std::string("tk_gemm_f64_noalloc: table fill launch: ") + cudaGetErrorString(e), TK_ERR_CUDA);
-    e = tk::launch_gemm_f64(reinterpret_cast<const tk::GemmTile*>(scratch + kNoallocHeader), ntiles,
-                            reinterpret_cast<const tk::GemmTask*>(scratch),
-                            reinterpret_cast<const tk::GemmSeg*>(scratch + 128), a->data, b->data, c->data, s);
+    const auto* tiles = reinterpret_cast<const tk::GemmTile*>(scratch + kNoallocHeader);
+    const auto* dtask = reinterpret_cast<const tk::GemmTask*>(scratch);
+    const auto* dseg = reinterpret_cast<const tk::GemmSeg*>(scratch + 128);
+    e = edge == tk::kF64Tile ? tk::launch_gemm_f64(tiles, ntiles, dtask, dseg, a->data, b->data, c->data, s)
+                             : tk::launch_wide_gemm_f64(tiles, ntiles, dtask, dseg, a->data, b->data, c->data, s);
     if (e != cudaSuccess) return fail(std::string("tk_gemm_f64_noalloc: GEMM launch: ") + cudaGetErrorString(e), TK_ERR_CUDA);
     return TK_OK;
 }

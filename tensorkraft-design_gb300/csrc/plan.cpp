@@ -262,36 +262,13 @@ void enumerate4(int kind, const QIndex* legs, const Qn& flux, std::vector<std::a
 
 }  // namespace
 
-static void add_tiles(GemmTable& g, int task_id, int tile_m, int tile_n, const std::vector<int64_t>&) {
-    gemm_add_tiles(g, task_id, tile_m, tile_n);
-}
-
-int gemm_tile_class(int M, int N) {
-    // square tiles of edge 64 >> cls; cost = tiles x (area + a fixed per-tile share)
-    int best = 0;
-    double best_cost = 0.0;
-    for (int cls = 0; cls < kGemmTileClasses; ++cls) {
-        const int e = 64 >> cls;
-        const double cost = (double)((M + e - 1) / e) * ((N + e - 1) / e) * ((double)e * e + 256.0);
-        if (cls == 0 || cost < best_cost) {
-            best = cls;
-            best_cost = cost;
-        }
-    }
-    return best;
-}
-
-void gemm_add_tiles(GemmTable& g, int task_id, int tile_m, int tile_n) {
+void gemm_add_tiles(GemmTable& g, int task_id) {
     const GemmTask& t = g.tasks[task_id];
-    const int cls = (tile_m == 64 && tile_n == 64) ? gemm_tile_class(t.M, t.N) : 0;
-    const int e = 64 >> cls;
-    for (int m0 = 0; m0 < t.M; m0 += e)
-        for (int n0 = 0; n0 < t.N; n0 += e) g.tiles.push_back({task_id, m0, n0, cls});
+    for (int m0 = 0; m0 < t.M; m0 += kF64Tile)
+        for (int n0 = 0; n0 < t.N; n0 += kF64Tile) g.tiles.push_back({task_id, m0, n0, 0});
 }
 
-static void lpt_order(GemmTable& g, int tile_m, int tile_n) { gemm_lpt_order(g, tile_m, tile_n); }
-
-void gemm_lpt_order(GemmTable& g, int tile_m, int tile_n) {
+void gemm_lpt_order(GemmTable& g) {
     // Cost of a tile = (rows) x (cols) x (total K); heaviest first, equal costs
     // in their order.  The costs are whole numbers of few bits, so a counting
     // sort by 11-bit digits takes two or three passes (2,317 tiles: 0.25 ms by
@@ -308,8 +285,8 @@ void gemm_lpt_order(GemmTable& g, int tile_m, int tile_n) {
     for (size_t i = 0; i < key.size(); ++i) {
         const GemmTile& x = g.tiles[i];
         const GemmTask& t = g.tasks[x.task];
-        const int64_t rm = std::min(std::min(tile_m, 64 >> x.cls), t.M - x.m0);
-        const int64_t rn = std::min(std::min(tile_n, 64 >> x.cls), t.N - x.n0);
+        const int64_t rm = std::min(kF64Tile, t.M - x.m0);
+        const int64_t rn = std::min(kF64Tile, t.N - x.n0);
         key[i] = {(ktot[x.task] + 1) * rm * rn, (uint32_t)i};
         top = std::max(top, key[i].cost);
     }
@@ -337,7 +314,6 @@ void gemm_lpt_order(GemmTable& g, int tile_m, int tile_n) {
 bool gemm_table_ok(const GemmTable& g, int64_t na, int64_t nb, int64_t nc, const char* name, std::string& err) {
         for (const GemmTile& tl : g.tiles) {
             if (tl.task < 0 || (size_t)tl.task >= g.tasks.size()) { err = std::string(name) + ": tile task"; return false; }
-            if (tl.cls < 0 || tl.cls >= kGemmTileClasses) { err = std::string(name) + ": tile class"; return false; }
             const GemmTask& t = g.tasks[tl.task];
             if (tl.m0 < 0 || tl.m0 >= t.M || tl.n0 < 0 || tl.n0 >= t.N) { err = std::string(name) + ": tile origin"; return false; }
         }
@@ -975,7 +951,7 @@ static tk_status build_tc_tables(Heff2Tables& T, const TcSource& X, const TcOpti
 }
 
 static tk_status build_heff2_tables_body(const tk_env& envL, const tk_env& envR, const tk_bst& wi_abi,
-                                         const tk_bst& wj_abi, const int32_t* psi_flux, int tile_m, int tile_n,
+                                         const tk_bst& wj_abi, const int32_t* psi_flux,
                                          Heff2Tables& T, std::string& err, const double* l_blocks,
                                          const double* r_blocks) {
     Bst4 wi, wj;
@@ -1205,7 +1181,7 @@ static tk_status build_heff2_tables_body(const tk_env& envL, const tk_env& envR,
                     T1I(p, ap, ws, b) = off;
                     off += (int64_t)tk.M * tk.N;
                     T.g1.tasks.push_back(tk);
-                    add_tiles(T.g1, (int)T.g1.tasks.size() - 1, tile_m, tile_n, ks);
+                    gemm_add_tiles(T.g1, (int)T.g1.tasks.size() - 1);
                 }
     T.t1_total = off;
 
@@ -1323,7 +1299,7 @@ static tk_status build_heff2_tables_body(const tk_env& envL, const tk_env& envR,
                 tk.alpha = 1.0; tk.beta = 0.0;
                 for (int64_t k : ks) T.g3.flops += 2.0 * tk.M * tk.N * (double)k;
                 T.g3.tasks.push_back(tk);
-                add_tiles(T.g3, (int)T.g3.tasks.size() - 1, tile_m, tile_n, ks);
+                gemm_add_tiles(T.g3, (int)T.g3.tasks.size() - 1);
             }
     // --- split-precision regrouping (tensor-core stacks) ---------------------
     {
@@ -1338,8 +1314,8 @@ static tk_status build_heff2_tables_body(const tk_env& envL, const tk_env& envR,
         X->wl_loc = wl_loc;
         T.tcsrc = X;  // the split tables themselves are built on first use (ensure_tc_tables)
     }
-    lpt_order(T.g1, tile_m, tile_n);
-    lpt_order(T.g3, tile_m, tile_n);
+    gemm_lpt_order(T.g1);
+    gemm_lpt_order(T.g3);
     // Algorithmic bytes: psi in, y out, the block-sparse L, R and W_ij terms, FP64.
     T.alg_bytes = 8.0 * (2.0 * (double)T.total + (double)T.lbuf.size() + (double)T.rbuf.size() + (double)nterms);
     // Index ranges must fit the kernels' 32-bit strides and counts.
@@ -1433,10 +1409,10 @@ extern "C" void tk_debug_fail_host_alloc(int32_t countdown) {
 namespace tk {
 
 tk_status build_heff2_tables(const tk_env& envL, const tk_env& envR, const tk_bst& wi_abi, const tk_bst& wj_abi,
-                             const int32_t* psi_flux, int tile_m, int tile_n, Heff2Tables& T, std::string& err,
+                             const int32_t* psi_flux, Heff2Tables& T, std::string& err,
                              const double* l_blocks, const double* r_blocks) {
     return guard_host("sector tables", err, [&] {
-        return build_heff2_tables_body(envL, envR, wi_abi, wj_abi, psi_flux, tile_m, tile_n, T, err, l_blocks, r_blocks);
+        return build_heff2_tables_body(envL, envR, wi_abi, wj_abi, psi_flux, T, err, l_blocks, r_blocks);
     });
 }
 

@@ -8,10 +8,6 @@
 
 namespace tk {
 
-// Output tile of the grouped FP64 GEMM kernel these tables feed (64 x 64).
-constexpr int kEnvTileM = 64;
-constexpr int kEnvTileN = 64;
-
 // Rank-3 MPS site tensor (s, a_L, a_R) with q(s) + q(a_L) = q(a_R): block of
 // (physical sector, left sector) -> element offset (row-major (s, a, b)) and
 // its right sector.  `data` is a device pointer, never read on the host.

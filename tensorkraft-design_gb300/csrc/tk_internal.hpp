@@ -107,12 +107,11 @@ struct GemmTask {
     int32_t seg_begin, seg_end;
     double alpha, beta;
 };
-// A tile is a square of edge 64 >> cls (cls 0: 64, 1: 32, 2: 16), chosen per
-// task so small sector blocks are not padded to 64 x 64.
+// A tile is the square of edge kF64Tile at (m0, n0) of its task's output.
+constexpr int kF64Tile = 16;
 struct GemmTile {
-    int32_t task, m0, n0, cls;
+    int32_t task, m0, n0, pad;
 };
-constexpr int kGemmTileClasses = 3;
 // Channel combine (W_i*W_j applied between the two GEMM stages):
 //   out[out_off + r*out_rs + c] = sum_t coef_t * in[in_off_t + r*in_rs_t + c]
 struct CombJob {
@@ -137,14 +136,10 @@ struct GemmTable {
     std::vector<GemmTile> tiles;
     double flops = 0.0;
 };
-// Tile class of an M x N task: the edge (64, 32 or 16) with the least
-// padded area plus a fixed per-tile share.
-int gemm_tile_class(int M, int N);
-// Appends the output tiles of task `task_id`; with tile_m = tile_n = 64 the
-// edge comes from gemm_tile_class, otherwise 64 x 64 tiles.
-void gemm_add_tiles(GemmTable& g, int task_id, int tile_m, int tile_n);
+// Appends the output tiles of task `task_id`.
+void gemm_add_tiles(GemmTable& g, int task_id);
 // Orders tiles heaviest first (rows x cols x total K), stable.
-void gemm_lpt_order(GemmTable& g, int tile_m, int tile_n);
+void gemm_lpt_order(GemmTable& g);
 // Every operand and output access of a table checked against buffer sizes.
 bool gemm_table_ok(const GemmTable& g, int64_t na, int64_t nb, int64_t nc, const char* name, std::string& err);
 bool comb_table_ok(const std::vector<CombJob>& jobs, const std::vector<CombTerm>& terms, int64_t n_in, int64_t n_out,
@@ -368,7 +363,7 @@ tk_status guard_host(const char* what, std::string& err, F&& build) {
 // l_blocks / r_blocks (host copies of environments in the canonical block
 // layout of env_layout) the environments' dense data are not read.
 tk_status build_heff2_tables(const tk_env& L, const tk_env& R, const tk_bst& wi, const tk_bst& wj,
-                             const int32_t* psi_flux, int tile_m, int tile_n, Heff2Tables& out,
+                             const int32_t* psi_flux, Heff2Tables& out,
                              std::string& err, const double* l_blocks = nullptr, const double* r_blocks = nullptr);
 
 // Canonical block layout of a block-sparse environment (bra, mpo, ket): every
