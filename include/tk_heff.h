@@ -411,15 +411,10 @@ tk_status tk_gemm_f64(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* 
  * No counterpart in the reference.  tk_gemm_f64 for callers that cannot
  * allocate device memory at call time (a sweep running out of a pre-sized
  * arena, a runtime that only hands over memory it manages, latency-bound
- * loops): same arguments and result, but the kernel's tile tables live in a
- * fixed 1 MiB device array inside the library instead of per-call
- * cudaMalloc'd buffers, so nothing is allocated or freed and the call does
- * not synchronise (stream-ordered on `stream`).  At most 65 520 64x64 output
- * tiles per call; larger calls return TK_ERR_INVALID_ARG.  The first call on
- * a device looks up the array's address (make it before any stream capture);
- * that address is cached for the process, so the entry point must not be
- * used again after cudaDeviceReset.  Calls share the array: calls on
- * different streams that overlap on the GPU race on it.
+ * loops): same arguments and result, always by the FP64 kernel, whose task is
+ * passed by value, so nothing is allocated or freed and the call does not
+ * synchronise (stream-ordered on `stream`).  Outputs of at most 65 520 64x64
+ * squares; larger calls return TK_ERR_INVALID_ARG.
  */
 tk_status tk_gemm_f64_noalloc(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* b,
                               double beta, tk_mat_mut* c, void* stream);

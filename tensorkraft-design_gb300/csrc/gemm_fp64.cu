@@ -18,11 +18,15 @@
 //
 // combine_f64: applies the fused two-site MPO W_ij between the two GEMM
 // stages, out = sum_t coef_t * in_t over equally shaped slabs.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "kernels.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace tk {
 
@@ -113,64 +117,64 @@ __global__ void __launch_bounds__(NT, 6) grouped_gemm_f64_kernel(const GemmTile*
     if (mine) store_out(task, C, tile.m0 + ty, tile.n0 + tx, acc, amul, accumulate);
 }
 
-// 64 x 64 tiles of one dense product, where 16 x 16 ones would not fit the
-// caller's table: thread (tx, ty) owns the outputs (ty + 16 i, tx + 16 j).
-__global__ void __launch_bounds__(NT) wide_gemm_f64_kernel(const GemmTile* __restrict__ tiles, int n_tiles,
-                                                           const GemmTask* __restrict__ tasks,
-                                                           const GemmSeg* __restrict__ segs,
-                                                           const double* __restrict__ A, const double* __restrict__ B,
-                                                           double* __restrict__ C) {
-    constexpr int W = kF64WideTile, R = W / 16;
-    __shared__ double As[BK][W + 1];
-    __shared__ double Bs[BK][W + 1];
-    if ((int)blockIdx.x >= n_tiles) return;
-    const GemmTile tile = tiles[blockIdx.x];
-    const GemmTask task = tasks[tile.task];
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    double acc[R][R];
+// One dense product C = alpha A B + beta C, its task and segment passed by
+// value (no tables, no upload).  `split` CTAs of a cluster share a tile's K and
+// the first sums their parts in order through distributed shared memory: a
+// 16 x 16 x 2048 tile alone takes one SM 160 us, and with 49 such tiles
+// (100 x 100 x 2000) two thirds of the SMs have nothing to do.
+__global__ void __launch_bounds__(NT, 6) dense_gemm_f64_kernel(const GemmTask task, const GemmSeg sg, int ntn,
+                                                               int split, const double* __restrict__ A,
+                                                               const double* __restrict__ B,
+                                                               double* __restrict__ C) {
+    __shared__ double As[2][BK][E + 1];
+    __shared__ double Bs[2][BK][E + 1];
+    __shared__ double part[NT];
+    const int tile = blockIdx.x / split, rank = blockIdx.x % split;
+    const int m0 = tile / ntn * E, n0 = tile % ntn * E;
+    const int tid = threadIdx.x, lo = tid & 15, hi = tid >> 4;
+    const int mv = min(E, task.M - m0), nv = min(E, task.N - n0);
+    const bool mine = tid < mv * nv;
+    const int ty = mine ? tid / nv : 0, tx = mine ? tid - ty * nv : 0;
+    const bool warp_busy = (tid & ~31) < mv * nv;
+    const bool ak = sg.a_cs == 1, bn = sg.b_cs == 1;
+    const int am = ak ? hi : lo, ka = ak ? lo : hi, bc = bn ? lo : hi, kb = bn ? hi : lo;
+    const double* pa = A + (int64_t)(m0 + am) * sg.a_rs;
+    const double* pb = B + (int64_t)(n0 + bc) * sg.b_cs;
+    const int64_t per = ((int64_t)sg.K + BK * split - 1) / (BK * split) * BK;  // k of each CTA
+    const int64_t k_end = min((int64_t)sg.K, per * (rank + 1));
+    double acc = 0.0, va, vb;
+    auto fetch = [&](int64_t k0) {
+        va = am < mv && k0 + ka < k_end ? pa[(k0 + ka) * sg.a_cs] : 0.0;
+        vb = bc < nv && k0 + kb < k_end ? pb[(k0 + kb) * sg.b_rs] : 0.0;
+    };
+    int p = 0;
+    int64_t k0 = per * rank;
+    fetch(k0);
+    for (; k0 < k_end; k0 += BK, p ^= 1) {
+        As[p][ka][am] = va;
+        Bs[p][kb][bc] = vb;
+        __syncthreads();
+        fetch(k0 + BK);
+        if (warp_busy) {
+            if (k_end - k0 >= BK) {
 #pragma unroll
-    for (int i = 0; i < R; ++i)
-#pragma unroll
-        for (int j = 0; j < R; ++j) acc[i][j] = 0.0;
-    for (int s = task.seg_begin; s < task.seg_end; ++s) {
-        const GemmSeg sg = segs[s];
-        for (int k0 = 0; k0 < sg.K; k0 += BK) {
-#pragma unroll
-            for (int r = 0; r < (W * BK) / NT; ++r) {
-                const int e = tid + r * NT;
-                const bool ak = sg.a_cs == 1, bn = sg.b_cs == 1;
-                const int m = ak ? e / BK : e % W, ka = ak ? e % BK : e / W;
-                const int n = bn ? e % W : e / BK, kb = bn ? e / W : e % BK;
-                const int gm = tile.m0 + m, gn = tile.n0 + n;
-                As[ka][m] = gm < task.M && k0 + ka < sg.K
-                                ? A[sg.a_off + (int64_t)gm * sg.a_rs + (int64_t)(k0 + ka) * sg.a_cs] : 0.0;
-                Bs[kb][n] = gn < task.N && k0 + kb < sg.K
-                                ? B[sg.b_off + (int64_t)(k0 + kb) * sg.b_rs + (int64_t)gn * sg.b_cs] : 0.0;
+                for (int k = 0; k < BK; ++k) acc = fma(As[p][k][ty], Bs[p][k][tx], acc);
+            } else {
+                const int kl = (int)(k_end - k0);
+#pragma unroll 1
+                for (int k = 0; k < kl; ++k) acc = fma(As[p][k][ty], Bs[p][k][tx], acc);
             }
-            __syncthreads();
-            const int kl = min(BK, sg.K - k0);
-#pragma unroll 4
-            for (int k = 0; k < kl; ++k) {
-                double a[R], b[R];
-#pragma unroll
-                for (int i = 0; i < R; ++i) a[i] = As[k][ty + 16 * i];
-#pragma unroll
-                for (int j = 0; j < R; ++j) b[j] = Bs[k][tx + 16 * j];
-#pragma unroll
-                for (int i = 0; i < R; ++i)
-#pragma unroll
-                    for (int j = 0; j < R; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-            }
-            __syncthreads();
         }
     }
-#pragma unroll
-    for (int i = 0; i < R; ++i)
-#pragma unroll
-        for (int j = 0; j < R; ++j) {
-            const int gm = tile.m0 + ty + 16 * i, gn = tile.n0 + tx + 16 * j;
-            if (gm < task.M && gn < task.N) store_out(task, C, gm, gn, acc[i][j], 1.0, 0);
-        }
+    if (split > 1) {
+        cg::cluster_group cluster = cg::this_cluster();
+        part[tid] = acc;
+        cluster.sync();
+        if (rank == 0)
+            for (int r = 1; r < split; ++r) acc += cluster.map_shared_rank(part, r)[tid];
+        cluster.sync();  // the parts are there until they are read
+    }
+    if (mine && rank == 0) store_out(task, C, m0 + ty, n0 + tx, acc, 1.0, 0);
 }
 
 __global__ void __launch_bounds__(256) combine_f64_kernel(const CombJob* __restrict__ jobs,
@@ -211,11 +215,42 @@ cudaError_t launch_gemm_f64(const GemmTile* tiles, int n_tiles, const GemmTask* 
     return cudaGetLastError();
 }
 
-cudaError_t launch_wide_gemm_f64(const GemmTile* tiles, int n_tiles, const GemmTask* tasks, const GemmSeg* segs,
-                                 const double* A, const double* B, double* C, cudaStream_t s) {
-    if (n_tiles <= 0) return cudaSuccess;
-    wide_gemm_f64_kernel<<<n_tiles, NT, 0, s>>>(tiles, n_tiles, tasks, segs, A, B, C);
-    return cudaGetLastError();
+double dense_gemm_f64_plan(int64_t M, int64_t N, int64_t K, int* split) {
+    // 85 ns a k for a tile on its SM's pipe; the SM with the most tiles counts.
+    // A share has at least 64 k.  Eight shares against one: 16 x 16 x 2048 28 us
+    // against 175, 100 x 100 x 2000 61 against 171, 200 x 200 x 1000 93 against 139;
+    // with the chip full (2048 x 32 x 2048) 241 against 274.
+    const double tiles = (double)((M + E - 1) / E) * ((N + E - 1) / E);
+    double best = 0.0;
+    for (int s = 1; s <= 8; s *= 2) {
+        if (s > 1 && K < 64 * s) break;
+        const double per = (double)((K + (int64_t)BK * s - 1) / ((int64_t)BK * s) * BK);
+        const double t = std::ceil(tiles * s / 152.0) * per * 85e-9 + (s > 1 ? 2e-6 : 0.0);
+        if (s == 1 || t < 0.9 * best) {
+            best = t;
+            if (split) *split = s;
+        }
+    }
+    return best + 8e-6;
+}
+
+cudaError_t launch_dense_gemm_f64(const GemmTask& task, const GemmSeg& seg, const double* A, const double* B,
+                                  double* C, cudaStream_t s) {
+    int split = 1;
+    dense_gemm_f64_plan(task.M, task.N, seg.K, &split);
+    const int64_t ntn = (task.N + (int64_t)E - 1) / E, ntm = (task.M + (int64_t)E - 1) / E;
+    if (ntm * ntn * split > INT32_MAX) return cudaErrorInvalidConfiguration;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)split;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(ntm * ntn * split));
+    cfg.blockDim = dim3(NT);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = split > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, dense_gemm_f64_kernel, task, seg, (int)ntn, split, A, B, C);
 }
 
 cudaError_t launch_gemm_c64(const GemmTile* tiles, int n_tiles, const GemmTask* tasks, const GemmSeg* segs,

@@ -11,10 +11,11 @@ namespace tk {
 cudaError_t launch_gemm_f64(const GemmTile* tiles, int n_tiles, const GemmTask* tasks, const GemmSeg* segs,
                             const double* A, const double* B, double* C, cudaStream_t s, double amul = 1.0,
                             bool accumulate = false);
-// Plain dense products over a list of kF64WideTile-square tiles.
-constexpr int kF64WideTile = 64;
-cudaError_t launch_wide_gemm_f64(const GemmTile* tiles, int n_tiles, const GemmTask* tasks, const GemmSeg* segs,
-                                 const double* A, const double* B, double* C, cudaStream_t s);
+// One dense product of M x K by K x N, without tables: the estimated time in
+// seconds, with the CTAs that share a tile's K in *split; and the launch.
+double dense_gemm_f64_plan(int64_t M, int64_t N, int64_t K, int* split = nullptr);
+cudaError_t launch_dense_gemm_f64(const GemmTask& task, const GemmSeg& seg, const double* A, const double* B,
+                                  double* C, cudaStream_t s);
 // The tables of launch_gemm_f64 on planar complex operands (four launches): C = A B, or
 // conj(A) B with conj_a; the tasks must overwrite their output (beta = 0).
 cudaError_t launch_gemm_c64(const GemmTile* tiles, int n_tiles, const GemmTask* tasks, const GemmSeg* segs,

@@ -196,16 +196,18 @@ tk_status gemm_digits(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* 
 }
 
 // The faster of the two kernels for a product.  The digits cost 45 us however
-// small it is (128^3: 33 us against 15 for the FP64 kernel, 256^3: 40 against
-// 42), then 4 us for 64 k of as many 128 x 64 tiles as there are SMs and 6 us
-// for the tiles' ends (100 x 100 x 2000: 145 us against 158); the FP64 kernel
-// runs near its pipe's 1.2 TFLOP/s when it is large (2048^3: 15 ms against
-// 0.56 ms).  Digits of more than 2 GB are not laid out.
+// small it is, then 4 us for 64 k of as many 128 x 64 tiles as there are SMs and
+// 6 us for the tiles' ends; the FP64 kernel's estimate is its own.  Whole calls,
+// digits against FP64 kernel: 300^3 73 us against 76, 512 x 512 x 128 61 against
+// 77, 2048 x 64 x 300 74 against 95, 400^3 76 against 147, 2048 x 32 x 2048 151
+// against 251, 2048^3 0.62 ms against 14.6; on the other side 256^3 and
+// 200 x 200 x 1000 stay with the FP64 kernel (54 and 110 us, digits 67 and 115 by
+// the estimate).  Digits of more than 2 GB are not laid out.
 bool gemm_on_digits(int64_t M, int64_t N, int64_t K) {
     if (K <= 0 || (double)(M + N) * (K + kTcBK) * kDigits * 2.0 > 2147483648.0) return false;
     const double tiles = (double)((M + kTcBM - 1) / kTcBM) * ((N + kTcBN - 1) / kTcBN);
     const double waves = std::ceil(tiles / 152.0), kch = (double)((K + kTcBK - 1) / kTcBK);
-    return 45e-6 + waves * (6e-6 + 4e-6 * kch) < 2.0 * M * N * K / 1.2e12;
+    return 45e-6 + waves * (6e-6 + 4e-6 * kch) < dense_gemm_f64_plan(M, N, K);
 }
 
 }  // namespace
@@ -240,7 +242,6 @@ tk_status tk_gemm_f64(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* 
         const tk_status st = gemm_digits(ctx, alpha, a, b, beta, c, s, &done);
         if (st != TK_OK || done) return st;
     }
-    GemmTable g;
     GemmTask t{};
     t.M = (int32_t)a->rows;
     t.N = (int32_t)b->cols;
@@ -249,24 +250,11 @@ tk_status tk_gemm_f64(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* 
     t.c_cs = (int32_t)c->col_stride;
     t.alpha = alpha;
     t.beta = beta;
-    t.seg_begin = 0;
-    t.seg_end = a->cols > 0 ? 1 : 0;
-    if (a->cols > 0) {
-        GemmSeg s{};
-        s.a_off = 0; s.a_rs = (int32_t)a->row_stride; s.a_cs = (int32_t)a->col_stride;
-        s.b_off = 0; s.b_rs = (int32_t)b->row_stride; s.b_cs = (int32_t)b->col_stride;
-        s.K = (int32_t)a->cols;
-        g.segs.push_back(s);
-    }
-    g.tasks.push_back(t);
-    gemm_add_tiles(g, 0);
-    Scratch sc;
-    GemmTask* dt; GemmSeg* ds; GemmTile* dl;
-    CK(sc.put(g.tasks, &dt));
-    CK(sc.put(g.segs, &ds));
-    CK(sc.put(g.tiles, &dl));
-    CK(launch_gemm_f64(dl, (int)g.tiles.size(), dt, ds, a->data, b->data, c->data, s));
-    // The task tables are freed on return; finish the launch first.
+    GemmSeg sg{};
+    sg.a_rs = (int32_t)a->row_stride; sg.a_cs = (int32_t)a->col_stride;
+    sg.b_rs = (int32_t)b->row_stride; sg.b_cs = (int32_t)b->col_stride;
+    sg.K = (int32_t)a->cols;
+    CK(launch_dense_gemm_f64(t, sg, a->data, b->data, c->data, s));
     CK(cudaStreamSynchronize(s));
     return TK_OK;
 }
