@@ -17,7 +17,7 @@
 //
 // The kernel is persistent and warp-specialised, one CTA per SM: one thread
 // moves operands by TMA (32 k of all digits of 128 + 64 rows: 84 KB, a ring of
-// two), one issues tcgen05.mma, eight warps drain the accumulators.  The
+// two), one warp issues tcgen05.mma, eight warps drain the accumulators.  The
 // digits of 32 B rows lie one after the other in shared memory and the levels
 // 32 columns apart in TMEM, so digit i of A meets digits 0 .. 6 - i of B in
 // ONE instruction (N = 32 (7 - i)) that lands on levels i .. 6: seven
@@ -118,17 +118,24 @@ __device__ __forceinline__ uint64_t sw64_desc(uint32_t saddr) {
 __device__ __forceinline__ uint32_t idesc_f16(int n) {
     return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTcBM >> 4) << 24);
 }
+// Called by a whole warp with the same arguments; one lane issues.  (Under a
+// branch on the lane the operands would be moved to uniform registers one by
+// one for each instruction, which takes longer than the instruction.)
 __device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
         "l"(a), "l"(b), "r"(idesc), "r"(accum)
         : "memory");
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
+        : "memory");
 }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -261,7 +268,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
     uint64_t* done = acc_empty + 2;
     uint32_t* tslot = (uint32_t*)(done + 1);
     volatile int* stop = (volatile int*)(tslot + 1);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
     dep_launch();
     if (threadIdx.x == 0) {
@@ -322,49 +329,53 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
             for (int i = max(0, it - kDigitRing); i < it; ++i) mbar_drain(&full[i % kDigitRing], (i / kDigitRing) & 1);
         }
     } else if (warp == EPI_WARPS + 1) {
-        if (lane == 0) {
-            int it = 0, unit = 0;
-            int drains[2] = {0, 0};
-            bool ok = run;
-            for (int ti = t_begin; ti < t_end && ok; ti += t_step) {
-                const TcTile t = tile_of<MODE>(tiles, om, ti);
-                const int halves = t.n_valid > HN ? 2 : 1;
-                const uint32_t astep = (uint32_t)((((t.m_valid + 31) >> 5) * 32) * KW * 2);
-                const KSteps k(t);
-                for (int part = 0; part < k.parts && ok; ++part)
-                for (int q = 0; q < k.per && ok; ++q, ++it) {
-                    const int st = it % kDigitRing;
-                    const bool first = k.first(part, q), last = k.last(part, q);
-                    ok = mbar_wait(&full[st], (it / kDigitRing) & 1, stop, redo);
-                    const uint32_t sa = smem_u32(smem + st * STAGE_BYTES);
-                    const int ks = min(KW / 16, (t.k_valid - q * KW + 15) / 16);
-                    for (int h = 0; h < halves && ok; ++h) {
-                        const int buf = (unit + h) & 1;
-                        if (first && drains[buf] > 0) ok = mbar_wait(&acc_empty[buf], (drains[buf] - 1) & 1, stop, redo);
-                        if (!ok) break;
-                        fence_after();
-                        const uint64_t b0 = sw64_desc(sa + A_BYTES + h * H_BYTES);
-                        const uint32_t d0 = tmem + buf * TMEM_HALF;
-                        for (int kk = 0; kk < ks; ++kk) {
-                            const uint64_t adv = (uint64_t)((kk * 32) >> 4);
-#pragma unroll
-                            for (int i = 0; i < kDigits; ++i)
-                                mma_f16(d0 + i * HN, sw64_desc(sa + i * astep) + adv, b0 + adv,
-                                        idesc_f16((kDigits - i) * HN), !(first && kk == 0 && i == 0));
-                        }
-                        if (last) {
-                            mma_commit(&acc_full[buf]);
-                            ++drains[buf];
-                        }
+        int it = 0, unit = 0;
+        uint32_t drained = 0, phase = 0;  // per accumulator: whether it was summed before, the parity to wait for
+        bool ok = run;
+        auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, stop, redo)) != 0; };
+        for (int ti = t_begin; ti < t_end && ok; ti += t_step) {
+            const TcTile t = tile_of<MODE>(tiles, om, ti);
+            const int halves = t.n_valid > HN ? 2 : 1;
+            const uint32_t astep = (uint32_t)((((t.m_valid + 31) >> 5) * 32) * KW * 2) >> 4;
+            const KSteps k(t);
+            for (int part = 0; part < k.parts && ok; ++part)
+            for (int q = 0; q < k.per && ok; ++q, ++it) {
+                const int st = it % kDigitRing;
+                const bool first = k.first(part, q), last = k.last(part, q);
+                ok = wait(&full[st], (it / kDigitRing) & 1);
+                const uint32_t sa = smem_u32(smem + st * STAGE_BYTES);
+                const uint64_t a0 = sw64_desc(sa);
+                const bool both = t.k_valid - q * KW > 16;  // 16-k steps of this stage
+                for (int h = 0; h < halves && ok; ++h) {
+                    const int buf = (unit + h) & 1;
+                    if (first && ((drained >> buf) & 1)) {
+                        ok = wait(&acc_empty[buf], (phase >> buf) & 1);
+                        phase ^= 1u << buf;
                     }
-                    mma_commit(&empty[st]);
+                    if (!ok) break;
+                    fence_after();
+                    const uint64_t b0 = sw64_desc(sa + A_BYTES + h * H_BYTES);
+                    const uint32_t d0 = tmem + buf * TMEM_HALF;
+#pragma unroll
+                    for (int kk = 0; kk < KW / 16; ++kk) {
+                        if (kk > 0 && !both) break;
+#pragma unroll
+                        for (int i = 0; i < kDigits; ++i)
+                            mma_f16(d0 + i * HN, a0 + i * astep + kk * 2, b0 + kk * 2, idesc_f16((kDigits - i) * HN),
+                                    i > 0 || kk > 0 || !first);
+                    }
+                    if (last) {
+                        mma_commit(&acc_full[buf]);
+                        drained |= 1u << buf;
+                    }
                 }
-                unit += halves;
+                mma_commit(&empty[st]);
             }
-            // no instruction is in flight when the accumulators are given back
-            mma_commit(done);
-            mbar_drain(done, 0);
+            unit += halves;
         }
+        // no instruction is in flight when the accumulators are given back
+        mma_commit(done);
+        mbar_drain(done, 0);
     } else {
         // warps 0-7 drain accumulator 0, warps 8-15 accumulator 1; warp % 4 is
         // the TMEM lane quarter, (warp / 4) % 2 the 16 of the half's 32 columns:
