@@ -86,6 +86,18 @@ __device__ __forceinline__ bool mbar_test(uint64_t* b, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+// mbar_test without its suspension: 60 clocks less where nothing is to be waited for.
+__device__ __forceinline__ bool mbar_done(uint64_t* b, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(b)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 // Bounded wait.  Once one wait of the CTA has run out (*stop), every later one
 // returns at once, so that all roles leave together.
 __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, volatile int* stop, int* redo) {
@@ -332,7 +344,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
         int it = 0, unit = 0;
         uint32_t drained = 0, phase = 0;  // per accumulator: whether it was summed before, the parity to wait for
         bool ok = run;
-        auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, stop, redo)) != 0; };
+        auto wait = [&](uint64_t* bar, uint32_t parity) {
+            return __all_sync(0xffffffffu, mbar_done(bar, parity)) ||
+                   __all_sync(0xffffffffu, mbar_wait(bar, parity, stop, redo));
+        };
         for (int ti = t_begin; ti < t_end && ok; ti += t_step) {
             const TcTile t = tile_of<MODE>(tiles, om, ti);
             const int halves = t.n_valid > HN ? 2 : 1;
@@ -356,13 +371,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
                     fence_after();
                     const uint64_t b0 = sw64_desc(sa + A_BYTES + h * H_BYTES);
                     const uint32_t d0 = tmem + buf * TMEM_HALF;
+                    // the second step goes backwards, so that wide instructions are the
+                    // ones in the queue (two or three deep) during the next wait
 #pragma unroll
                     for (int kk = 0; kk < KW / 16; ++kk) {
                         if (kk > 0 && !both) break;
 #pragma unroll
-                        for (int i = 0; i < kDigits; ++i)
+                        for (int j = 0; j < kDigits; ++j) {
+                            const int i = kk == 0 ? j : kDigits - 1 - j;
                             mma_f16(d0 + i * HN, a0 + i * astep + kk * 2, b0 + kk * 2, idesc_f16((kDigits - i) * HN),
                                     i > 0 || kk > 0 || !first);
+                        }
                     }
                     if (last) {
                         mma_commit(&acc_full[buf]);
