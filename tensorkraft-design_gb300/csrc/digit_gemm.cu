@@ -554,15 +554,20 @@ __device__ __forceinline__ int row_exponent(uint32_t max_hi, int* redo) {
 }
 // x 2^k on its row's grid, rounded to nearest, plus 128 in each of the six
 // low bytes: byte j is then digit 6 - j plus 128, the upper 16 bits digit 0.
+__device__ __noinline__ uint64_t shifted_up(uint64_t m, int n) { return n > 63 ? 0 : m << n; }
 __device__ __forceinline__ uint64_t on_grid(double x, int ex, int k = 0) {
     const uint64_t b = (uint64_t)__double_as_longlong(x);
     const int e = (int)(b >> 52) & 0x7FF;
-    uint64_t m = (b & 0xFFFFFFFFFFFFFull) << 4;
-    if (e) m |= 1ull << 56;
-    const int s = min(ex - max(e, 1) - k, 62);
-    m = s >= 0 ? (m + ((1ull << s) >> 1)) >> s : m << -s;
-    if ((int64_t)b < 0) m = 0 - m;
-    return m + 0x0000808080808080ull;
+    uint64_t m = (b & 0xFFFFFFFFFFFFFull) << 5;  // one bit more than the grid has, for the rounding
+    if (e) m |= 1ull << 57;
+    const int s = min(ex - max(e, 1) - k, 63);
+    if (__builtin_expect(s < 0, 0))  // (rows of subnormals or zeros alone)
+        m = shifted_up(m, -s);
+    else
+        m >>= s;
+    m = (m + 1) >> 1;
+    const uint64_t neg = (uint64_t)((int64_t)b >> 63);
+    return (m ^ neg) - neg + 0x0000808080808080ull;
 }
 // The digits of two neighbouring elements, as pairs of fp16.
 __device__ __forceinline__ void digits2(double x, double y, int ex, uint32_t* d, int kx = 0, int ky = 0) {
@@ -586,9 +591,9 @@ __device__ __forceinline__ void digits2(double x, double y, int ex, uint32_t* d,
     d[0] = half_of(top + 0x64006400u, 0x66006600u);  // minus 1536
 }
 __device__ __forceinline__ void put_digits(const DigitStack& o, int64_t row, int k, const uint32_t* d) {
-    uint32_t* p = reinterpret_cast<uint32_t*>(o.q) + (row << 5) + (k >> 1);
+    uint32_t* p = reinterpret_cast<uint32_t*>(o.q) + row * (kDigits * kTcBK / 2) + (k >> 1);
 #pragma unroll
-    for (int j = 0; j < kDigits; ++j) p[j * (o.rows << 5)] = d[j];
+    for (int j = 0; j < kDigits; ++j) p[j * (kTcBK / 2)] = d[j];
 }
 
 // A complex operand's digits d + i f at chunk offsets c0 (first part) and c1.
@@ -661,10 +666,17 @@ __global__ void __launch_bounds__(32 * kDigitRowsPerCta) digit_rows_kernel(const
     };
     double2 v[kKeep];
     int mx = kNoExponent;
-    uint32_t hi = 0;
+    uint32_t hi = 0, tiny = 0;  // tiny: whether there are subnormals
+    auto top1 = [&](double x, int k) {
+        const uint32_t h = abs_hi(x);
+        const int e = (int)(h >> 20);
+        hi = max(hi, h);
+        tiny |= e > 0 ? 0u : h | (uint32_t)__double2loint(x);
+        mx = max(mx, e > 0 ? e + k : kNoExponent);
+    };
     auto top = [&](const double2& u, const int2& k) {
-        hi = max(hi, max(abs_hi(u.x), abs_hi(u.y)));
-        mx = max(mx, max(exponent_of(u.x, k.x), exponent_of(u.y, k.y)));
+        top1(u.x, k.x);
+        top1(u.y, k.y);
     };
 #pragma unroll
     for (int c = 0; c < kKeep; ++c)
@@ -674,6 +686,13 @@ __global__ void __launch_bounds__(32 * kDigitRowsPerCta) digit_rows_kernel(const
         }
 #pragma unroll 4
     for (int c = kKeep; c < j.kch; ++c) top(at(c), scale(c));
+    if (__any_sync(0xffffffffu, tiny != 0)) {
+        for (int c = 0; c < j.kch; ++c) {
+            const double2 u = at(c);
+            const int2 k = scale(c);
+            mx = max(mx, max(exponent_of(u.x, k.x), exponent_of(u.y, k.y)));
+        }
+    }
     mx = __reduce_max_sync(0xffffffffu, mx);
     if (hi >= 0x7FF00000u) atomicExch(redo, kDigitValue);
     const int ex = mx == kNoExponent ? 1 : mx;
@@ -865,7 +884,9 @@ __global__ void __launch_bounds__(BT) digit_matrix_kernel(const DigitMatrix A, c
             digits2(u, v, sex[r], d);
             put_digits(m.out, r0 + r + (int64_t)blockIdx.y * m.rows, 2 * lane, d);
             // the row's squares, its largest element counting at most 1
-            const float a = (float)(int)(on_grid(u, sex[r]) >> 32) * 0x1p-25f, b = (float)(int)(on_grid(v, sex[r]) >> 32) * 0x1p-25f;
+            const float2 d0 = __half22float2(*reinterpret_cast<const __half2*>(&d[0]));
+            const float2 d1 = __half22float2(*reinterpret_cast<const __half2*>(&d[1]));
+            const float a = fmaf(d1.x, 0x1p-17f, d0.x * 0x1p-9f), b = fmaf(d1.y, 0x1p-17f, d0.y * 0x1p-9f);
             float sq = fmaf(a, a, b * b);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
@@ -904,7 +925,7 @@ bool digit_maps(DigitMaps& m, const DigitStack& a, const DigitStack& b, std::str
     auto make = [&](CUtensorMap* map, const DigitStack& s, int box_rows) {
         if (s.rows <= 0) return true;
         cuuint64_t dims[3] = {(cuuint64_t)kTcBK, (cuuint64_t)s.rows, (cuuint64_t)kDigits};
-        cuuint64_t strides[2] = {(cuuint64_t)kTcBK * 2, (cuuint64_t)s.rows * kTcBK * 2};
+        cuuint64_t strides[2] = {(cuuint64_t)kTcBK * 2 * kDigits, (cuuint64_t)kTcBK * 2};
         cuuint32_t box[3] = {(cuuint32_t)KW, (cuuint32_t)box_rows, (cuuint32_t)kDigits};
         cuuint32_t estr[3] = {1, 1, 1};
         CUresult r = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn)(

@@ -42,8 +42,8 @@ cudaError_t launch_dependent(void (*k)(P...), dim3 grid, unsigned block, size_t 
 #endif
 
 // A digit operand in the operand-stack layout (K-major 64-wide chunks, see
-// TcTables): plane j of `rows` rows of 64, and the biased exponent of every
-// row of chunk 0.
+// TcTables): `rows` rows of seven digits of 64 elements each, one after the
+// other, and the biased exponent of every row of chunk 0.
 struct DigitStack {
     __half* q = nullptr;
     int32_t* ex = nullptr;
