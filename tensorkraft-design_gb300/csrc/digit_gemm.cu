@@ -59,7 +59,9 @@ constexpr int NTHREADS = 32 * (EPI_WARPS + 2);
 constexpr int SCOLS = 8;                              // columns staged at a time for the stores
 constexpr int ST_LD = SCOLS + 1;
 constexpr int STORE_BYTES = 32 * ST_LD * 8;           // per drain warp
-constexpr int SMEM_BYTES = 1024 + kDigitRing * STAGE_BYTES + EPI_WARPS * STORE_BYTES + 256;
+constexpr int TILE_CACHE = 64;                        // tiles of a CTA kept in shared memory
+constexpr int SMEM_BYTES = 1024 + kDigitRing * STAGE_BYTES + EPI_WARPS * STORE_BYTES + TILE_CACHE * (int)sizeof(TcTile) + 256;
+static_assert(sizeof(TcTile) % 8 == 0 && SMEM_BYTES <= 227 * 1024, "tiles are copied as 8-byte words");
 constexpr int TMEM_ALLOC = 512, TMEM_HALF = 256;
 constexpr long WAIT_LIMIT = 1L << 24;
 
@@ -273,7 +275,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     double* store = (double*)(smem + kDigitRing * STAGE_BYTES);
-    uint64_t* full = (uint64_t*)(smem + kDigitRing * STAGE_BYTES + EPI_WARPS * STORE_BYTES);
+    TcTile* cache = (TcTile*)(smem + kDigitRing * STAGE_BYTES + EPI_WARPS * STORE_BYTES);
+    uint64_t* full = (uint64_t*)(cache + TILE_CACHE);
     uint64_t* empty = full + kDigitRing;
     uint64_t* acc_full = empty + kDigitRing;
     uint64_t* acc_empty = acc_full + 2;
@@ -301,6 +304,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    // this CTA's tiles: a run of the table, or every gridDim.x-th of the C grid.
+    // Its first tiles are copied (the table is the plan's, no kernel writes it):
+    // each role then starts a tile without waiting for its descriptor.
+    const int t_begin = MODE == 0 ? (int)blockIdx.x : begin[blockIdx.x];
+    const int t_end = MODE == 0 ? om.tiles : begin[blockIdx.x + 1];
+    const int t_step = MODE == 0 ? (int)gridDim.x : 1;
+    if (MODE != 0) {
+        const int n = min(t_end - t_begin, TILE_CACHE) * (int)(sizeof(TcTile) / 8);
+        for (int i = threadIdx.x; i < n; i += NTHREADS)
+            reinterpret_cast<uint64_t*>(cache)[i] = reinterpret_cast<const uint64_t*>(tiles + t_begin)[i];
+    }
+    auto tile_at = [&](int ti) {
+        return MODE != 0 && ti - t_begin < TILE_CACHE ? cache[ti - t_begin] : tile_of<MODE>(tiles, om, ti);
+    };
     dep_wait();
     if (threadIdx.x == 0) *stop = *(volatile int*)redo;  // an operand held an infinity or a NaN: another kernel computes this product
     fence_before();
@@ -309,17 +326,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
     const uint32_t tmem = *tslot;
     const bool run = *stop == 0;  // written before the barrier; a wait can only run out after it
     __syncthreads();
-    // this CTA's tiles: a run of the table, or every gridDim.x-th of the C grid
-    const int t_begin = MODE == 0 ? (int)blockIdx.x : begin[blockIdx.x];
-    const int t_end = MODE == 0 ? om.tiles : begin[blockIdx.x + 1];
-    const int t_step = MODE == 0 ? (int)gridDim.x : 1;
-
     if (warp == EPI_WARPS) {
         if (lane == 0) {
             int it = 0;
             bool ok = run;
             for (int ti = t_begin; ti < t_end && ok; ti += t_step) {
-                const TcTile t = tile_of<MODE>(tiles, om, ti);
+                const TcTile t = tile_at(ti);
                 const int halves = t.n_valid > HN ? 2 : 1;
                 const int box = (t.m_valid + 31) >> 5;
                 const uint32_t bytes = kDigits * KW * 2 * (32 * box + HN * halves);
@@ -349,7 +361,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
                    __all_sync(0xffffffffu, mbar_wait(bar, parity, stop, redo));
         };
         for (int ti = t_begin; ti < t_end && ok; ti += t_step) {
-            const TcTile t = tile_of<MODE>(tiles, om, ti);
+            const TcTile t = tile_at(ti);
             const int halves = t.n_valid > HN ? 2 : 1;
             const uint32_t astep = (uint32_t)((((t.m_valid + 31) >> 5) * 32) * KW * 2) >> 4;
             const KSteps k(t);
@@ -405,7 +417,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
         int drains = 0, unit = 0;
         bool ok = run;
         for (int ti = t_begin; ti < t_end && ok; ti += t_step) {
-            const TcTile t = tile_of<MODE>(tiles, om, ti);
+            const TcTile t = tile_at(ti);
             const int halves = t.n_valid > HN ? 2 : 1;
             const int h = (buf - unit) & 1;
             unit += halves;
