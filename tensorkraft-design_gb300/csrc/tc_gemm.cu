@@ -138,6 +138,26 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t adesc, uint64_t
         : "memory");
 }
 
+// The same by a whole warp with the same arguments, one lane of which issues:
+// under a branch on the lane every operand would be moved to uniform registers
+// one by one.
+__device__ __forceinline__ void warp_mma_bf16(uint32_t tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                              uint32_t accum) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum)
+        : "memory");
+}
+__device__ __forceinline__ void warp_mma_commit(uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
+        : "memory");
+}
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
@@ -252,7 +272,7 @@ __global__ void __launch_bounds__(128, 1) tc_gemm_kernel(const TcTile* __restric
     uint64_t* done = empty + NST;
     uint32_t* tslot = (uint32_t*)(done + 1);
     const TcTile t = tiles[blockIdx.x];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     grid_dep_launch();
 
     if (t.kch == 0) {  // no K: the tile is zero
@@ -339,12 +359,12 @@ __global__ void __launch_bounds__(128, 1) tc_gemm_kernel(const TcTile* __restric
             load_a(c, st, &full[s]);
             load_b(c, st, &full[s]);
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         // MMA issuer: three bf16 products per 16-wide K step
         const uint32_t idesc = make_idesc(t.n_mma);
         for (int c = 0; c < t.kch && ok; ++c) {
             const int s = c % NST;
-            ok = mbar_wait(&full[s], (c / NST) & 1, err, ERR_FULL_TIMEOUT);
+            ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (c / NST) & 1, err, ERR_FULL_TIMEOUT));
             if (!ok) break;
             fence_after();
             const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
@@ -353,13 +373,13 @@ __global__ void __launch_bounds__(128, 1) tc_gemm_kernel(const TcTile* __restric
 #pragma unroll
             for (int kk = 0; kk < kTcBK / 16; ++kk) {
                 const uint64_t adv = (uint64_t)((kk * 32) >> 4);  // 16 bf16 = 32 bytes along K
-                mma_bf16(tmem, ah + adv, bh + adv, idesc, (c | kk) != 0);
-                mma_bf16(tmem, ah + adv, bl + adv, idesc, 1u);
-                mma_bf16(tmem, al + adv, bh + adv, idesc, 1u);
+                warp_mma_bf16(tmem, ah + adv, bh + adv, idesc, (c | kk) != 0);
+                warp_mma_bf16(tmem, ah + adv, bl + adv, idesc, 1u);
+                warp_mma_bf16(tmem, al + adv, bh + adv, idesc, 1u);
             }
-            mma_commit(&empty[s]);
+            warp_mma_commit(&empty[s]);
         }
-        mma_commit(done);
+        warp_mma_commit(done);
     }
     __syncwarp();
     // epilogue: thread r owns accumulator row r (TMEM lane r)
