@@ -190,11 +190,12 @@ tk_status tk_heff2_set_precision(tk_heff2_plan* plan, int32_t precision);
  * 32 x 64 outputs that step over the stack columns their rows hold, so that
  * nearly every FP64 FMA issued is one of the product's own (complex plans:
  * the same pieces with complex FMAs on planar operands; the default of
- * complex plans too).  Large real plans run these stacks on the fp16 tensor
- * cores: every operand row as seven integer digits on one grid (to 2^-58 of
- * its largest element), multiplied exactly and each sum rounded once, with
- * the FP64 kernels standing by for vectors with infinities or NaNs.  Every
- * schedule computes the same sums to FP64 precision. */
+ * complex plans too).  Large plans, real and complex, run these stacks on
+ * the fp16 tensor cores: every operand row as seven integer digits on one
+ * grid (to 2^-58 of its largest element), multiplied exactly and each sum
+ * rounded once, with the FP64 kernels standing by for vectors with
+ * infinities or NaNs.  Every schedule computes the same sums to FP64
+ * precision. */
 #define TK_SCHED_GROUPED   0
 #define TK_SCHED_PER_BLOCK 1
 #define TK_SCHED_STACKED   2

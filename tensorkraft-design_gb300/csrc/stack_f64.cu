@@ -32,10 +32,11 @@
 // are most of the time (Heisenberg D = 64: 17.4 -> 10.9 us).
 // Every output sums its k in ascending order.
 //
-// Large real plans run the same stacks on the fp16 tensor cores instead
+// Large plans run the same stacks on the fp16 tensor cores instead
 // (digit_gemm.cu): digits of psi, T1 by digit products, the same combine,
-// digits of T2, y by digit products.  Hubbard D = 2048: 701 -> 184 us; cylinder
-// D = 2048: 40.9 -> 1.88 ms, relative error 2.6e-15 -> 1.5e-15.
+// digits of T2, y by digit products.  Hubbard D = 2048: 701 -> 142 us; cylinder
+// D = 2048: 40.9 -> 1.58 ms, relative error 2.6e-15 -> 1.5e-15; a complex plan
+// takes both parts as one K twice as long.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -523,9 +524,9 @@ static void digit_rows_of(std::vector<DigitRows>& out, int32_t row, int n, int32
 // stage 1.  Below, the FP64 kernels finish before the digit kernels' latencies
 // add up (Heisenberg D = 128, 0.4 million: 17 us against 29; Hubbard D = 256,
 // 0.4 million: 31 against 28); above, their pipe is the limit (Hubbard D = 362,
-// 1.3 million: 38 against 31 us; D = 512: 50 against 36; D = 2048, 230 million:
-// 701 against 149; Heisenberg D = 512, 25 million: 151 against 51; cylinder D =
-// 2048, 13 billion: 40.9 ms against 1.84).  A plan of less than a dozen stage-3
+// 1.3 million: 38 against 31 us; D = 512: 50 against 33; D = 2048, 230 million:
+// 701 against 142; Heisenberg D = 512, 25 million: 151 against 48; cylinder D =
+// 2048, 13 billion: 40.9 ms against 1.58).  A plan of less than a dozen stage-3
 // tiles keeps its three launches up to 8 million: small plans of a few sectors
 // are relied on to be three launches (digits would take 58 us against 85 at 6.2
 // million on ten tiles).

@@ -68,11 +68,12 @@ struct DevGemm {
         if ((e = segs.upload(g.segs)) != cudaSuccess) return e;
         if ((e = tiles.upload(g.tiles)) != cudaSuccess) return e;
         n_tiles = (int)g.tiles.size();
-        std::vector<GemmTile> by(g.tiles);
-        std::stable_sort(by.begin(), by.end(), [](const GemmTile& a, const GemmTile& b) { return a.task < b.task; });
         task_tile_begin.assign(g.tasks.size() + 1, 0);
-        for (const GemmTile& t : by) task_tile_begin[t.task + 1]++;
+        for (const GemmTile& t : g.tiles) task_tile_begin[t.task + 1]++;
         for (size_t i = 1; i < task_tile_begin.size(); ++i) task_tile_begin[i] += task_tile_begin[i - 1];
+        std::vector<GemmTile> by(g.tiles.size());  // in their order within a task
+        std::vector<int> next(task_tile_begin);
+        for (const GemmTile& t : g.tiles) by[next[t.task]++] = t;
         return tiles_by_task.upload(by);
     }
 };
