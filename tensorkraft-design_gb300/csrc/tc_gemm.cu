@@ -36,6 +36,7 @@
 #include <algorithm>
 #include <cstring>
 #include <string>
+#include <type_traits>
 
 #include "tc_gemm.cuh"
 #include "tk_plan.cuh"
@@ -1130,52 +1131,78 @@ __global__ void __launch_bounds__(kThreads, kThreads == 128 ? 12 : 16) combine_t
     const bool inl = nterm <= kTcCombInline;
     const bool resident = !inl && nterm <= TCH;
     if (resident && (int)threadIdx.x < nterm) st[threadIdx.x] = terms[j.term_begin + threadIdx.x];
-    // element threadIdx.x's (row, column) in the job, and one step of kThreads elements
-    const int dq = kThreads / j.cols, dr = kThreads - dq * j.cols;
-    int rl = (int)threadIdx.x / j.cols, cl = (int)threadIdx.x - rl * j.cols;
+    // pair threadIdx.x's (row, pair) in the job, and one step of kThreads pairs;
+    // a pair is the columns of an even k and the next (k0 odd: the first pair
+    // holds one column)
+    const int odd = j.k0 & 1, np = (odd + j.cols + 1) >> 1;
+    // (x + 1/2) / np in fp32: at least 1 / (2 np) from a whole number, x <= kThreads
+    const float inv = __fdividef(1.f, (float)np);
+    const int dq = (int)((kThreads + 0.5f) * inv), dr = kThreads - dq * np;
+    int rl = (int)((threadIdx.x + 0.5f) * inv), pl = (int)threadIdx.x - rl * np;
     grid_dep_wait();
     if (resident) __syncthreads();
     if (inl) {
         const float* src[kTcCombInline];
 #pragma unroll
         for (int q = 0; q < kTcCombInline; ++q) src[q] = t1 + j.inl[q].in_off;
-        for (int e0 = 0; e0 < n; e0 += U * kThreads) {
-            bool valid[U];
-            int r[U], c[U];
-            float acc[U], v[kTcCombInline][U];
+        const int n2 = j.rows * np;
+        // N pairs of a thread at a time: no slots that the whole block leaves empty
+        auto pairs = [&](auto count, int e0) {
+            constexpr int UP = decltype(count)::value;
+            bool lo[UP], hi[UP];
+            int r[UP], c[UP];
+            float v[kTcCombInline][UP][2];
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                valid[u] = e0 + u * kThreads + (int)threadIdx.x < n;
+            for (int u = 0; u < UP; ++u) {
+                const bool valid = e0 + u * kThreads + (int)threadIdx.x < n2;
                 r[u] = j.r0 + rl;
-                c[u] = cl;
-                acc[u] = 0.f;
-                cl += dr;
+                c[u] = 2 * pl - odd;
+                lo[u] = valid && c[u] >= 0;
+                hi[u] = valid && c[u] + 1 < j.cols;
+                pl += dr;
                 rl += dq;
-                if (cl >= j.cols) {
-                    cl -= j.cols;
+                if (pl >= np) {
+                    pl -= np;
                     ++rl;
                 }
             }
 #pragma unroll
             for (int q = 0; q < kTcCombInline; ++q)
 #pragma unroll
-                for (int u = 0; u < U; ++u)
-                    v[q][u] = (q < nterm && valid[u]) ? __ldg(src[q] + t1_off<kWide>(r[u], j.inl[q].in_rs, c[u])) : 0.f;
-#pragma unroll
-            for (int q = 0; q < kTcCombInline; ++q)
-                if (q < nterm)
-#pragma unroll
-                    for (int u = 0; u < U; ++u) acc[u] = fmaf(j.inl[q].coef, v[q][u], acc[u]);
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (valid[u]) {
-                    const int k = j.k0 + c[u];
-                    const int64_t idx = ((int64_t)(j.t2row + (k >> 6) * j.cstride + r[u]) << 6) + (k & 63);
-                    const __nv_bfloat16 h = __float2bfloat16_rn(acc[u]);
-                    th[idx] = h;
-                    tl[idx] = __float2bfloat16_rn(acc[u] - __bfloat162float(h));
+                for (int u = 0; u < UP; ++u) {
+                    const float* p = src[q] + t1_off<kWide>(r[u], j.inl[q].in_rs, c[u]);
+                    v[q][u][0] = (q < nterm && lo[u]) ? __ldg(p) : 0.f;
+                    v[q][u][1] = (q < nterm && hi[u]) ? __ldg(p + 1) : 0.f;
                 }
-        }
+#pragma unroll
+            for (int u = 0; u < UP; ++u) {
+                float x = 0.f, y = 0.f;
+#pragma unroll
+                for (int q = 0; q < kTcCombInline; ++q)
+                    if (q < nterm) {
+                        x = fmaf(j.inl[q].coef, v[q][u][0], x);
+                        y = fmaf(j.inl[q].coef, v[q][u][1], y);
+                    }
+                const int k = j.k0 + c[u];
+                const int64_t idx = ((int64_t)(j.t2row + (k >> 6) * j.cstride + r[u]) << 6) + (k & 63);
+                const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+                const __nv_bfloat162 l =
+                    __floats2bfloat162_rn(x - __low2float(h), y - __high2float(h));
+                if (lo[u] && hi[u]) {
+                    *reinterpret_cast<__nv_bfloat162*>(th + idx) = h;
+                    *reinterpret_cast<__nv_bfloat162*>(tl + idx) = l;
+                } else if (lo[u]) {
+                    th[idx] = __low2bfloat16(h);
+                    tl[idx] = __low2bfloat16(l);
+                } else if (hi[u]) {
+                    th[idx + 1] = __high2bfloat16(h);
+                    tl[idx + 1] = __high2bfloat16(l);
+                }
+            }
+        };
+        int e0 = 0;
+        for (; e0 + kThreads < n2; e0 += U / 2 * kThreads) pairs(std::integral_constant<int, U / 2>{}, e0);
+        if (e0 < n2) pairs(std::integral_constant<int, 1>{}, e0);
         return;
     }
     for (int e0 = 0; e0 < n; e0 += U * kThreads) {  // block-uniform trip count
