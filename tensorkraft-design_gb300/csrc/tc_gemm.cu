@@ -1097,30 +1097,51 @@ __global__ void __launch_bounds__(kSplitThreads) split_psi_kernel(const TcSplitJ
     }
 }
 
-constexpr int kCombThreads = 128;  // combine: threads per job
+// Combine: threads per job, 128, or 64 where `combine_narrow` says so.  A thread's
+// set-up is most of what it issues, so half the threads issue less (at twenty
+// CTAs an SM: 16, 18 and 22 are 2 to 10 % slower), but a job of more than 256
+// elements then takes two passes.  That pays where jobs are small, or so many
+// that no CTA waits alone.  Split matvec in us, 64 against 128 threads (jobs,
+// elements a job): Hubbard D = 128 (4,024, 4) 13.4 / 14.6, D = 2048 (15,384, 254)
+// 46.7 / 48.0, cylinder D = 2048 (49,278, 523) 273 / 281, D = 64 (1,924, 5) 13.1 /
+// 13.7; Heisenberg D = 128 (230, 108) 14.5 / 13.1, cylinder D = 128 (1,988, 39)
+// 22.6 / 19.3, D = 512 (5,540, 292) 43.1 / 40.9, D = 1024 (17,078, 378) 93.6 / 91.0.
+constexpr int kCombThreads = 128;
+bool combine_narrow(const std::vector<TcCombJob>& jobs) {
+    double elems = 0.0, most = 0.0;
+    for (const TcCombJob& j : jobs) {
+        elems += (double)j.rows * j.cols;
+        most = std::max(most, (double)j.rows * j.cols);
+    }
+    const double n = (double)jobs.size(), mean = elems / std::max(n, 1.0);
+    return most <= 256.0 || (mean <= 256.0 && n >= 4000.0) || n >= 32768.0;
+}
 
 // W_i W_j channel combine: T1 (fp32) -> stage-3 A operand, bf16 hi/lo.  One
 // CTA per job (rows [r0, r0 + rows) of one output slab, at most
 // kTcCombMaxElems elements unless a single row is longer).  A job of at most
 // kTcCombInline terms (most of them: a channel pair reached from one or two
 // others) reads its terms from its own descriptor; longer term lists are
-// staged in shared memory.  Each thread owns U elements, so a thread has
+// staged in shared memory.  Each thread owns U elements at a time, so it has
 // TU x U independent T1 loads in flight before the first use.  Elements run
 // in row-major order, contiguous in T1 and in the operand chunk.  The kernel
-// is bound by its instruction issue: a thread walks its elements (tid, tid +
-// 128, ...) by one precomputed quotient and remainder of 128 instead of a
-// division per element, and (kWide false: T1 below 2^31 elements) forms
-// its T1 and operand offsets in 32 bits.
+// is bound by its instruction issue: with terms of its descriptor a job is
+// walked in pairs of columns (one address, conversion and store for two), by
+// one precomputed quotient and remainder of kThreads pairs instead of a
+// division each, and (kWide false: T1 below 2^31 elements) forms its T1 and
+// operand offsets in 32 bits.  Warp instructions on Hubbard / cylinder D = 2048:
+// one element at a time 19.4 / 82 million, pairs 16.7 / 67.
 template <bool kWide>
 __device__ __forceinline__ int64_t t1_off(int r, int rs, int c) {
     return kWide ? (int64_t)r * rs + c : (int64_t)(r * rs + c);
 }
 
 template <bool kWide, int kThreads = kCombThreads, int U = 4>
-__global__ void __launch_bounds__(kThreads, kThreads == 128 ? 12 : 16) combine_tc_kernel(
+__global__ void __launch_bounds__(kThreads, kThreads == 128 ? 12 : U == 4 ? 20 : 16) combine_tc_kernel(
     const TcCombJob* __restrict__ jobs, const TcCombTerm* __restrict__ terms, const float* __restrict__ t1,
     __nv_bfloat16* __restrict__ th, __nv_bfloat16* __restrict__ tl) {
     constexpr int TU = 2, TCH = 64;
+    static_assert(kThreads >= TCH, "one thread stages a term");
     __shared__ TcCombTerm st[TCH];
     const TcCombJob j = jobs[blockIdx.x];
     grid_dep_launch();
@@ -1492,6 +1513,7 @@ struct TcPlan {
     bool p1 = false;                    // stage 1 as the persistent kernel (TcOptions::stage1_persistent)
     bool narrow1 = false;               // stage 1 in 32-wide K chunks (TcOptions::stage1_narrow)
     int p1_ctas = 0;                    // its resident CTAs per SM x SMs
+    bool comb_narrow = false;           // the combine takes 64 threads a job (combine_narrow)
     bool t1_wide = false;               // T1 holds 2^31 elements or more (64-bit combine offsets)
     __nv_bfloat16 *lh = nullptr, *ll = nullptr, *rh = nullptr, *rl = nullptr;
     __nv_bfloat16 *th = nullptr, *tl = nullptr;
@@ -1568,6 +1590,7 @@ tk_status tc_plan_create(const Heff2Tables& host, const double*, const double*,
     p->n3 = (int)C.tiles3.size();
     p->n3f = (int)C.tiles3f.size();
     p->t1_wide = C.t1_total > INT32_MAX;
+    p->comb_narrow = combine_narrow(C.jobs);
     p->nsplit = (int)C.split.size();
     p->njobs = (int)C.jobs.size();
     p->nst1 = C.max_kch1 <= 1 ? 1 : 2;
@@ -1720,6 +1743,9 @@ cudaError_t tc_apply_stage(TcPlan& tc, const Heff2Tables&, const CombJob*, int, 
                        tc.th, tc.tl);
         else if (tc.njobs > 0 && tc.comb_form == 3)
             launch_pdl(tc.t1_wide ? combine_tc_kernel<true, 64, 8> : combine_tc_kernel<false, 64, 8>, tc.njobs, 64, 0,
+                       s, (const TcCombJob*)tc.jobs, (const TcCombTerm*)tc.terms, (const float*)tc.t1, tc.th, tc.tl);
+        else if (tc.njobs > 0 && tc.comb_narrow)
+            launch_pdl(tc.t1_wide ? combine_tc_kernel<true, 64, 4> : combine_tc_kernel<false, 64, 4>, tc.njobs, 64, 0,
                        s, (const TcCombJob*)tc.jobs, (const TcCombTerm*)tc.terms, (const float*)tc.t1, tc.th, tc.tl);
         else if (tc.njobs > 0)
             launch_pdl(tc.t1_wide ? combine_tc_kernel<true> : combine_tc_kernel<false>, tc.njobs, kCombThreads, 0, s,
