@@ -166,7 +166,6 @@ struct OrthArgs {
     double* partial = nullptr;
     unsigned* bar = nullptr;  // [0] arrivals, [1] CTAs done, [2] set when a wait ran out
 };
-constexpr int KT = 512;
 constexpr long kBarrierPolls = 1L << 22;
 
 // acc[j] = sum over i of V_j[i] w[i], j < MJ; with W also *ww = sum of w[i]^2.
@@ -198,6 +197,7 @@ __device__ __forceinline__ void dot_chunk_of(int mj, const double* V, int64_t ld
 }
 
 // (Two CTAs fit an SM, so that two solvers on two streams can run at once.)
+template <int KT>
 __global__ void __launch_bounds__(KT, 2) orthogonalise_kernel(const OrthArgs a) {
     extern __shared__ double sm[];
     double* red = sm;                 // [MCH][KT]
@@ -216,6 +216,7 @@ __global__ void __launch_bounds__(KT, 2) orthogonalise_kernel(const OrthArgs a) 
         for (int j = 0; j < MCH; ++j)
             if (j < mj) red[j * KT + tid] = acc[j];
         __syncthreads();
+        static_assert(KT / 32 >= MCH, "a warp per sum");
         if (warp < mj) {
             double s[4] = {};
 #pragma unroll
@@ -386,16 +387,27 @@ __global__ void __launch_bounds__(KT, 2) orthogonalise_kernel(const OrthArgs a) 
     }
 }
 
+// Vectors of at most two elements a thread of 256 take CTAs of 256: a block's sums
+// cost the FP64 pipe in proportion to its threads, and longer vectors need 512
+// for their loads.  Davidson, 12 steps, 256 against 512 threads: n = 1,148 1.06 ms
+// against 1.16, 10 thousand 1.24 / 1.34, 62 thousand 1.90 / 1.94; expm at 15
+// thousand 0.90 / 0.96; Lanczos at 398 thousand 3.04 / 2.95 the other way round.
+constexpr int64_t kShortVector = 2 * 256 * 152;
 cudaError_t launch_orthogonalise(OrthArgs a, cudaStream_t s) {
     int dev = 0, sms = 0;
     cudaError_t e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
         return e;
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((a.n + KT - 1) / KT, std::min(sms, RG / 2)));
-    void* args[] = {&a};
-    return cudaLaunchCooperativeKernel((const void*)orthogonalise_kernel, dim3(grid), dim3(KT), args,
-                                       sizeof(double) * (MCH * KT + a.m + 2), s);
+    auto launch = [&](const void* kernel, int threads) {
+        const int64_t blocks = (a.n + threads - 1) / threads;
+        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(blocks, std::min(sms, RG / 2)));
+        void* args[] = {&a};
+        return cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args,
+                                           sizeof(double) * (MCH * threads + a.m + 2), s);
+    };
+    return a.n <= kShortVector ? launch((const void*)orthogonalise_kernel<256>, 256)
+                               : launch((const void*)orthogonalise_kernel<512>, 512);
 }
 
 inline int vgrid(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 16)); }
