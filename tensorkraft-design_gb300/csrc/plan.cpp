@@ -332,6 +332,16 @@ bool gemm_table_ok(const GemmTable& g, int64_t na, int64_t nb, int64_t nc, const
         return true;
 }
 
+bool combine_narrow(const std::vector<TcCombJob>& jobs) {
+    double elems = 0.0, most = 0.0;
+    for (const TcCombJob& j : jobs) {
+        elems += (double)j.rows * j.cols;
+        most = std::max(most, (double)j.rows * j.cols);
+    }
+    const double n = (double)jobs.size(), mean = elems / std::max(n, 1.0);
+    return most <= 256.0 || (mean <= 256.0 && n >= 4000.0) || n >= 32768.0;
+}
+
 bool comb_table_ok(const std::vector<CombJob>& jobs, const std::vector<CombTerm>& terms, int64_t n_in, int64_t n_out,
                    std::string& err) {
     for (const CombJob& j : jobs) {

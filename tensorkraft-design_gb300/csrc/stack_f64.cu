@@ -297,7 +297,7 @@ __device__ __forceinline__ void stack_combine_job(const TcCombJob& j, const TcCo
 }
 
 template <bool CPLX>
-__global__ void __launch_bounds__(128) stack_combine_f64_kernel(const TcCombJob* __restrict__ jobs,
+__global__ void __launch_bounds__(256) stack_combine_f64_kernel(const TcCombJob* __restrict__ jobs,
                                                                 const TcCombTerm* __restrict__ terms,
                                                                 const double* __restrict__ coef,
                                                                 const double* __restrict__ t1,
@@ -508,7 +508,7 @@ struct F64Stack {
     DevBuf<TcCombTerm> terms;
     DevBuf<int64_t> yrow, colbase, xsrc;
     DevBuf<int32_t> colstride, xstride;
-    int n1 = 0, n3 = 0, njobs = 0;
+    int n1 = 0, n3 = 0, njobs = 0, comb_threads = 0;
     double bytes[3] = {0.0, 0.0, 0.0};  // per stage, without the psi / y vectors
 };
 
@@ -833,6 +833,11 @@ tk_status f64stack_create(const TcTables& C, std::unique_ptr<F64Stack, F64StackD
     p->n1 = (int)p1.size();
     p->n3 = (int)p3.size();
     p->njobs = (int)C.jobs.size();
+    // Threads a combine job, whole matvecs in us at 256 / 128: Heisenberg D = 256
+    // 32.8 / 35.8, D = 1024 89.1 / 91.1, cylinder D = 128 42.5 / 46.3, D = 512
+    // 126 / 131; the other way round (combine_narrow) Hubbard D = 2048 145 / 142,
+    // cylinder D = 64 17.4 / 17.0, D = 2048 1,599 / 1,580.
+    p->comb_threads = combine_narrow(C.jobs) ? 128 : 256;
     if (f64stack_on_digits(C, p->cplx) && (e = digits_create(C, *p, err)) != cudaSuccess) {
         if (err.empty()) err = std::string("digit operands: ") + cudaGetErrorString(e);
         return e == cudaErrorMemoryAllocation ? TK_ERR_OOM : TK_ERR_CUDA;
@@ -845,7 +850,7 @@ tk_status f64stack_create(const TcTables& C, std::unique_ptr<F64Stack, F64StackD
 static cudaError_t combine_stage(const F64Stack& p, cudaStream_t s) {
     if (p.njobs == 0) return cudaSuccess;
     return launch_dependent(p.cplx ? stack_combine_f64_kernel<true> : stack_combine_f64_kernel<false>,
-                            dim3((unsigned)p.njobs, p.cplx ? 2u : 1u), 128, 0, s, p.jobs.p,
+                            dim3((unsigned)p.njobs, p.cplx ? 2u : 1u), (unsigned)p.comb_threads, 0, s, p.jobs.p,
                             p.terms.p, p.coef.p, p.t1.p, p.t2.p, p.t1_im.p, p.t2_im.p);
 }
 

@@ -1107,15 +1107,6 @@ __global__ void __launch_bounds__(kSplitThreads) split_psi_kernel(const TcSplitJ
 // 13.7; Heisenberg D = 128 (230, 108) 14.5 / 13.1, cylinder D = 128 (1,988, 39)
 // 22.6 / 19.3, D = 512 (5,540, 292) 43.1 / 40.9, D = 1024 (17,078, 378) 93.6 / 91.0.
 constexpr int kCombThreads = 128;
-bool combine_narrow(const std::vector<TcCombJob>& jobs) {
-    double elems = 0.0, most = 0.0;
-    for (const TcCombJob& j : jobs) {
-        elems += (double)j.rows * j.cols;
-        most = std::max(most, (double)j.rows * j.cols);
-    }
-    const double n = (double)jobs.size(), mean = elems / std::max(n, 1.0);
-    return most <= 256.0 || (mean <= 256.0 && n >= 4000.0) || n >= 32768.0;
-}
 
 // W_i W_j channel combine: T1 (fp32) -> stage-3 A operand, bf16 hi/lo.  One
 // CTA per job (rows [r0, r0 + rows) of one output slab, at most

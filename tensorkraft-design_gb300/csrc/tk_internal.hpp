@@ -216,6 +216,9 @@ struct TcCombJob {
     TcCombTerm inl[kTcCombInline];  // terms[term_begin .. term_end) when there are at most kTcCombInline
 };
 constexpr int kTcCombMaxElems = 512;
+// Whether a list of combine jobs gets fewer threads a job: none is large, or they
+// are many and small, or very many.
+bool combine_narrow(const std::vector<TcCombJob>& jobs);
 constexpr int kTcPsiPieces = 8;
 struct TcTables {
     int64_t lq_rows = 0, rq_rows = 0, xq_rows = 0, t2q_rows = 0, t1_total = 0;
