@@ -836,8 +836,9 @@ tk_status f64stack_create(const TcTables& C, std::unique_ptr<F64Stack, F64StackD
     // Threads a combine job, whole matvecs in us at 256 / 128: Heisenberg D = 256
     // 32.8 / 35.8, D = 1024 89.1 / 91.1, cylinder D = 128 42.5 / 46.3, D = 512
     // 126 / 131; the other way round (combine_narrow) Hubbard D = 2048 145 / 142,
-    // cylinder D = 64 17.4 / 17.0, D = 2048 1,599 / 1,580.
-    p->comb_threads = combine_narrow(C.jobs) ? 128 : 256;
+    // cylinder D = 64 17.4 / 17.0, and from 16 thousand jobs on: cylinder D = 1150
+    // 508 / 497, D = 2048 1,599 / 1,580 (D = 1024, 17 thousand: 331 / 332).
+    p->comb_threads = combine_narrow(C.jobs) || C.jobs.size() >= 16384 ? 128 : 256;
     if (f64stack_on_digits(C, p->cplx) && (e = digits_create(C, *p, err)) != cudaSuccess) {
         if (err.empty()) err = std::string("digit operands: ") + cudaGetErrorString(e);
         return e == cudaErrorMemoryAllocation ? TK_ERR_OOM : TK_ERR_CUDA;
