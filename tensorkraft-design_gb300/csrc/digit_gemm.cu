@@ -860,11 +860,37 @@ __global__ void __launch_bounds__(PT) digit_psi_kernel(const DigitPsi* __restric
 }
 
 constexpr int BT = 256;
+// The high word of |x|, 1 for what has none of its own: zero only for zero.
+__device__ __forceinline__ uint32_t abs_top(double x) {
+    const uint32_t hi = abs_hi(x);
+    return hi == 0 && __double2loint(x) != 0 ? 1u : hi;
+}
+// Whether x lies on the grid of digits 0 .. 3 of a row with exponent ex: its lowest bit at
+// 2^(ex - 1055) or above.
+__device__ __forceinline__ bool in_four_digits(double x, int ex) {
+    const uint64_t b = (uint64_t)__double_as_longlong(x);
+    const int e = (int)(b >> 52) & 0x7FF;
+    const uint64_t m = (b & 0xFFFFFFFFFFFFFull) | (e ? 1ull << 52 : 0);
+    return m == 0 || max(e, 1) + __ffsll((long long)m) - 1 >= ex + 20;
+}
+// |x| 2^-e in fp32, rounded down (e by its biased form ex: |x| < 2^(ex - 1022))
+__device__ __forceinline__ float below_one(double x, int ex) {
+    const uint32_t hi = abs_hi(x);
+    const int e = (int)(hi >> 20) - ex + 126;
+    const uint32_t m = ((hi & 0xFFFFFu) << 3) | ((uint32_t)__double2loint(x) >> 29);
+    return hi >> 20 && e > 0 ? __uint_as_float(((uint32_t)e << 23) | m) : 0.0f;
+}
+// The k's of a product that digit_gate_kernel looks at: kGate of them, or all.
+constexpr int kGate = kDigitSamples;
+__host__ __device__ __forceinline__ int gate_k(int s, int K) { return K > kGate ? (int)((int64_t)s * K / kGate) : s; }
 // The two operands of a dense product, 32 rows x 64 k a CTA (the rows of A,
-// then those of B).  PASS 0 leaves every row's largest high word in ex (zeroed
-// before), PASS 1 writes the digits; lanes walk along the shorter stride.
+// then those of B).  PASS 0 leaves every row's largest high word in top (zeroed
+// before), PASS 1 writes the exponents, the digits and the gate's samples, and sets
+// *wide where an element is not on the grid of four digits; lanes walk along the
+// shorter stride.
 template <int PASS>
-__global__ void __launch_bounds__(BT) digit_matrix_kernel(const DigitMatrix A, const DigitMatrix B, int K, int* redo) {
+__global__ void __launch_bounds__(BT) digit_matrix_kernel(const DigitMatrix A, const DigitMatrix B, int K, int* wide,
+                                                          int* redo) {
     __shared__ double tile[32][kTcBK + 1];
     __shared__ int sex[32];
     const int na = (A.rows + 31) / 32;
@@ -875,7 +901,8 @@ __global__ void __launch_bounds__(BT) digit_matrix_kernel(const DigitMatrix A, c
     const double* x = m.x + r0 * m.rs + k0 * m.ks;
     auto fetch = [&](int r, int k) { return r < nr && k0 + k < K ? x[r * m.rs + k * m.ks] : 0.0; };
     if (PASS == 1 && tid < nr) {
-        sex[tid] = row_exponent((uint32_t)m.out.ex[r0 + tid], redo);
+        sex[tid] = row_exponent(m.top[r0 + tid], redo);
+        if (blockIdx.y == 0) m.out.ex[r0 + tid] = sex[tid];
     }
     if ((m.rs < 0 ? -m.rs : m.rs) < (m.ks < 0 ? -m.ks : m.ks)) {
 #pragma unroll
@@ -888,41 +915,78 @@ __global__ void __launch_bounds__(BT) digit_matrix_kernel(const DigitMatrix A, c
         }
     }
     __syncthreads();
+    bool four = true;
+    // which samples this lane's two k are (-1: none), and whether *wide still needs a look
+    int at[2] = {-1, -1};
+    bool look = false;
+    if (PASS == 1) {
+        look = *(volatile int*)wide == 0;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int k = k0 + 2 * lane + i, s = K > kGate ? (int)(((int64_t)k * kGate + K - 1) / K) : k;
+            if (k < K && s < kGate && gate_k(s, K) == k) at[i] = s;
+        }
+    }
     for (int r = w; r < nr; r += BT / 32) {
         if (PASS == 0) {
-            const uint32_t mx = __reduce_max_sync(0xffffffffu, max(abs_hi(tile[r][lane]), abs_hi(tile[r][lane + 32])));
-            if (lane == 0) atomicMax(m.out.ex + r0 + r, (int)mx);
+            const uint32_t mx = __reduce_max_sync(0xffffffffu, max(abs_top(tile[r][lane]), abs_top(tile[r][lane + 32])));
+            if (lane == 0) atomicMax(m.top + r0 + r, mx);
         } else {
             const double u = tile[r][2 * lane], v = tile[r][2 * lane + 1];
             uint32_t d[kDigits];
             digits2(u, v, sex[r], d);
             put_digits(m.out, r0 + r + (int64_t)blockIdx.y * m.rows, 2 * lane, d);
-            // the row's squares, its largest element counting at most 1
-            const float2 d0 = __half22float2(*reinterpret_cast<const __half2*>(&d[0]));
-            const float2 d1 = __half22float2(*reinterpret_cast<const __half2*>(&d[1]));
-            const float a = fmaf(d1.x, 0x1p-17f, d0.x * 0x1p-9f), b = fmaf(d1.y, 0x1p-17f, d0.y * 0x1p-9f);
-            float sq = fmaf(a, a, b * b);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-            if (lane == 0) atomicAdd(m.square + r0 + r, sq);
+            if (look) four = four && in_four_digits(u, sex[r]) && in_four_digits(v, sex[r]);
+            if (at[0] >= 0) m.sample[(int64_t)at[0] * m.rows + r0 + r] = below_one(u, sex[r]);
+            if (at[1] >= 0) m.sample[(int64_t)at[1] * m.rows + r0 + r] = below_one(v, sex[r]);
         }
     }
+    if (PASS == 1 && __syncthreads_or(!four) && tid == 0) atomicExch(wide, 1);
 }
-// The largest high word of every row becomes its exponent.  A row far from
-// flat has no place on one grid: with P = K 2^(2 e) / sum x^2, the digits' error
-// is about 2^-59 sqrt(P_a P_b / K) of ||a|| ||b||, an FP64 chain's 2^-53
-// sqrt(K / 12) of sqrt(sum a^2 b^2), about ||a|| ||b|| / sqrt(K); so a row whose P
-// exceeds 64 sqrt(K / 12) (a normal one has up to 110, and P <= 4 K) sends the
-// product to the FP64 pipe.
-__global__ void digit_exponent_kernel(const DigitMatrix A, const DigitMatrix B, float least, int* redo) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    for (int o = 0; o < 2; ++o) {
-        const DigitMatrix& m = o ? B : A;
-        if (i >= m.rows) continue;
-        const uint32_t hi = (uint32_t)m.out.ex[i];
-        m.out.ex[i] = row_exponent(hi, redo);
-        if (hi != 0 && m.square[i] < least) atomicExch(redo, kDigitValue);
+
+// Whether the digits hold a dense product as exactly as an FP64 chain of K steps
+// does, output by output.  They leave out at most half a unit of each element's grid,
+// 2^(e - 58), and the products of digits i + j > 6, 6.03 x 2^-60 2^(ea + eb) a k:
+//   |error| <= K 2^-56.1 2^(ea + eb),
+// the chain's bound is K 2^-53 sum |a_k b_k|.  So an output with
+//   sum |a_k b_k| >= 2^-3 2^(ea + eb)
+// has the smaller bound on digits.  The sum over kGate of the k, evenly spaced, is a
+// lower bound of it and enough for operands without structure (N(0, 1): about 0.6 at
+// 64 k, the least of a million outputs 0.27); where one output falls below, *redo
+// sends the product to the FP64 pipe.  Rows of zeros, and operands whose elements all
+// lie in four digits, have no error at all.  (A statement on the rows alone will not
+// do: sum |a_k b_k| depends on where the large elements of both meet.)
+// 64 x 64 outputs a CTA in fp32; at 2048^3 it takes 21 us and the call 515 us (507 without).
+__global__ void __launch_bounds__(BT) digit_gate_kernel(const DigitMatrix A, const DigitMatrix B, int K, const int* wide,
+                                                        int* redo) {
+    __shared__ __align__(16) float sa[kGate][64], sb[kGate][64];
+    if (*wide == 0) return;
+    const int tid = threadIdx.x, ks = min(K, kGate);
+    const int m0 = (int)blockIdx.y * 64, n0 = (int)blockIdx.x * 64;
+    for (int i = tid; i < 64 * ks; i += BT) {
+        const int r = i & 63, k = i >> 6;
+        sa[k][r] = m0 + r < A.rows ? A.sample[(int64_t)k * A.rows + m0 + r] : 0.0f;
+        sb[k][r] = n0 + r < B.rows ? B.sample[(int64_t)k * B.rows + n0 + r] : 0.0f;
     }
+    __syncthreads();
+    const int tx = (tid & 15) * 4, ty = (tid >> 4) * 4;
+    float acc[4][4] = {};
+    for (int k = 0; k < ks; ++k) {
+        const float4 a = *reinterpret_cast<const float4*>(&sa[k][ty]), b = *reinterpret_cast<const float4*>(&sb[k][tx]);
+        const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+    }
+    bool bad = false;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            bad |= m0 + ty + i < A.rows && n0 + tx + j < B.rows && acc[i][j] < 0.125f && A.top[m0 + ty + i] != 0 &&
+                   B.top[n0 + tx + j] != 0;
+    if (__syncthreads_or(bad) && tid == 0) atomicExch(redo, kDigitValue);
 }
 
 }  // namespace
@@ -1042,18 +1106,11 @@ cudaError_t launch_digit_rows_complex(const DigitRowsC* jobs, int n_jobs, const 
                             32 * kDigitRowsPerCta, 0, s, jobs, re, im, kx, sign, out, redo);
 }
 
-cudaError_t launch_digit_matrices(const DigitMatrix& a, const DigitMatrix& b, int K, int* redo, cudaStream_t s) {
+cudaError_t launch_digit_matrices(const DigitMatrix& a, const DigitMatrix& b, int K, int* wide, int* redo, cudaStream_t s) {
     const dim3 grid((unsigned)((a.rows + 31) / 32 + (b.rows + 31) / 32), (unsigned)((K + kTcBK - 1) / kTcBK));
-    cudaError_t e;
-    if ((e = cudaMemsetAsync(a.out.ex, 0, sizeof(int32_t) * a.rows, s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(b.out.ex, 0, sizeof(int32_t) * b.rows, s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(a.square, 0, sizeof(float) * a.rows, s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(b.square, 0, sizeof(float) * b.rows, s)) != cudaSuccess)
-        return e;
-    digit_matrix_kernel<0><<<grid, BT, 0, s>>>(a, b, K, redo);
-    digit_matrix_kernel<1><<<grid, BT, 0, s>>>(a, b, K, redo);
-    digit_exponent_kernel<<<(std::max(a.rows, b.rows) + 255) / 256, 256, 0, s>>>(
-        a, b, std::sqrt(12.0f * (float)K) / 64.0f, redo);
+    digit_matrix_kernel<0><<<grid, BT, 0, s>>>(a, b, K, wide, redo);
+    digit_matrix_kernel<1><<<grid, BT, 0, s>>>(a, b, K, wide, redo);
+    digit_gate_kernel<<<dim3((unsigned)((b.rows + 63) / 64), (unsigned)((a.rows + 63) / 64)), BT, 0, s>>>(a, b, K, wide, redo);
     return cudaGetLastError();
 }
 

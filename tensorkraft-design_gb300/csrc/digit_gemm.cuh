@@ -119,17 +119,19 @@ cudaError_t launch_digit_rows(const DigitRows* jobs, int n_jobs, const double* q
 cudaError_t launch_digit_rows_complex(const DigitRowsC* jobs, int n_jobs, const double* re, const double* im,
                                       const int32_t* kx, int sign, bool dual, const DigitStack& out, int* redo,
                                       cudaStream_t s);
-// Digits of both operands of a dense product (*redo is set for operands that
-// one grid per row would hold less exactly than FP64): row r, k of K at
-// x[r * rs + k * ks], into stacks whose chunks are `rows` rows apart.
+// Digits of both operands of a dense product (*redo is set where an output might be
+// less exact than by an FP64 chain): row r, k of K at x[r * rs + k * ks], into stacks
+// whose chunks are `rows` rows apart.  `top` and *wide start at zero.
 struct DigitMatrix {
     const double* x;
     int64_t rs, ks;
     int rows;
     DigitStack out;
-    float* square;  // a scratch value per row
+    uint32_t* top;  // scratch: a value a row,
+    float* sample;  // 64 values a row
 };
-cudaError_t launch_digit_matrices(const DigitMatrix& a, const DigitMatrix& b, int K, int* redo, cudaStream_t s);
+constexpr int kDigitSamples = 64;
+cudaError_t launch_digit_matrices(const DigitMatrix& a, const DigitMatrix& b, int K, int* wide, int* redo, cudaStream_t s);
 // Digits of psi sub-blocks (jobs of at most `cols` columns, 32 or 8, and max_k
 // rows), of both parts with x_im.
 cudaError_t launch_digit_psi(const DigitPsi* jobs, int n_jobs, int cols, int max_k, const double* x, const double* x_im,

@@ -132,25 +132,26 @@ struct GemmBuffer {
 };
 
 // The dense product on the fp16 tensor cores (digit_gemm.cu).  *done is left
-// false where the FP64 kernel is to run instead: operands that one grid per
-// row would hold less exactly, and no memory for the digits.
+// false where the FP64 kernel is to run instead: an output that might be less
+// exact on digits, and no memory for them.
 tk_status gemm_digits(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* b, double beta, tk_mat_mut* c,
                       cudaStream_t s, bool* done) {
     *done = false;
     const int64_t M = a->rows, N = b->cols, K = a->cols, kch = (K + kTcBK - 1) / kTcBK;
-    DigitMatrix A{a->data, a->row_stride, a->col_stride, (int)M, {}, nullptr};
-    DigitMatrix B{b->data, b->col_stride, b->row_stride, (int)N, {}, nullptr};
+    DigitMatrix A{a->data, a->row_stride, a->col_stride, (int)M, {}, nullptr, nullptr};
+    DigitMatrix B{b->data, b->col_stride, b->row_stride, (int)N, {}, nullptr, nullptr};
     A.out.rows = M * kch;
     B.out.rows = N * kch;
-    size_t total = 256;
+    size_t total = 256;  // the flags
     auto take = [&](size_t n) {
         const size_t at = total;
         total += (n + 255) & ~(size_t)255;
         return at;
     };
-    const size_t qa = take(digit_stack_bytes(A.out.rows)), qb = take(digit_stack_bytes(B.out.rows));
+    const size_t ta = take(sizeof(uint32_t) * M), tb = take(sizeof(uint32_t) * N), zeroed = total;
     const size_t ea = take(sizeof(int32_t) * M), eb = take(sizeof(int32_t) * N);
-    const size_t sa = take(sizeof(float) * M), sb = take(sizeof(float) * N);
+    const size_t sa = take(sizeof(float) * kDigitSamples * M), sb = take(sizeof(float) * kDigitSamples * N);
+    const size_t qa = take(digit_stack_bytes(A.out.rows)), qb = take(digit_stack_bytes(B.out.rows));
     GemmBuffer buf(ctx, total);
     if (!buf.p) return TK_OK;
     unsigned char* p = static_cast<unsigned char*>(buf.p);
@@ -159,8 +160,10 @@ tk_status gemm_digits(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* 
     B.out.q = reinterpret_cast<__half*>(p + qb);
     A.out.ex = reinterpret_cast<int32_t*>(p + ea);
     B.out.ex = reinterpret_cast<int32_t*>(p + eb);
-    A.square = reinterpret_cast<float*>(p + sa);
-    B.square = reinterpret_cast<float*>(p + sb);
+    A.top = reinterpret_cast<uint32_t*>(p + ta);
+    B.top = reinterpret_cast<uint32_t*>(p + tb);
+    A.sample = reinterpret_cast<float*>(p + sa);
+    B.sample = reinterpret_cast<float*>(p + sb);
     DigitMaps maps;
     std::string err;
     if (!digit_maps(maps, A.out, B.out, err)) {
@@ -179,8 +182,8 @@ tk_status gemm_digits(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* 
     o.tiles = (int)(((M + kTcBM - 1) / kTcBM) * ((N + kTcBN - 1) / kTcBN));
     int state = 0;
     cudaError_t e = digit_setup();
-    if (e == cudaSuccess) e = cudaMemsetAsync(redo, 0, sizeof(int), s);
-    if (e == cudaSuccess) e = launch_digit_matrices(A, B, (int)K, redo, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, zeroed, s);
+    if (e == cudaSuccess) e = launch_digit_matrices(A, B, (int)K, redo + 1, redo, s);
     if (e == cudaSuccess) e = launch_digit_gemm(0, nullptr, nullptr, std::min(o.tiles, 152), maps, A.out.ex, B.out.ex, o, redo, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&state, redo, sizeof(int), cudaMemcpyDeviceToHost, s);
     // the buffer goes back when the stream is done with it, whatever failed
