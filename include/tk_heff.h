@@ -134,7 +134,10 @@ tk_status tk_heff2_plan_footprint(const tk_env* env_l, const tk_env* env_r, cons
  * next call on, the countdown-th host-allocation checkpoint of the plan-table
  * builders, or the countdown-th device allocation made for a plan, fails as
  * if memory were exhausted (counted from 1; 0 disarms).  The failing call
- * returns TK_ERR_OOM and releases what it had allocated. */
+ * returns TK_ERR_OOM and releases what it had allocated.  A device countdown
+ * of -v, 0 < v < 256, fails nothing: until disarmed, every device allocation
+ * made for a plan starts out filled with bytes v (memory that another program
+ * or plan has left). */
 void tk_debug_fail_host_alloc(int32_t countdown);
 void tk_debug_fail_device_alloc(int32_t countdown);
 

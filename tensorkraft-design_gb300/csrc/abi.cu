@@ -124,7 +124,7 @@ extern "C" {
 int32_t tk_version(void) { return 1; }
 
 void tk_debug_fail_device_alloc(int32_t countdown) {
-    g_fail_device_alloc.store(countdown > 0 ? countdown : 0, std::memory_order_relaxed);
+    g_fail_device_alloc.store(countdown > -256 ? countdown : 0, std::memory_order_relaxed);
 }
 
 const char* tk_last_error(void) { return g_last_error.c_str(); }

@@ -479,12 +479,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
             }
             if (!ok || !mine) continue;
             // s 2^24 + l in 64 bits, for the whole row less the u low bits that the
-            // row's largest sum leaves no room for (it then has 62 of its own)
+            // row's largest sum leaves no room for (it then has 62 of its own); of the
+            // tile's columns only: the others' operand rows belong to other tiles or to
+            // nobody, and must not decide how these are rounded
             uint32_t bits = 0;
 #pragma unroll
             for (int i = 0; i < WCOLS; ++i) {
                 const int32_t hi = (int32_t)(acc[i].s >> 32);
-                bits |= (uint32_t)(hi ^ (hi >> 31));
+                if (i < nc) bits |= (uint32_t)(hi ^ (hi >> 31));
             }
             const int u = max(0, 26 - __clz((int)bits));
             const uint32_t um = 1u << (24 - u);

@@ -584,7 +584,9 @@ static cudaError_t digits_alloc(F64Digits& d, const Blob& blob, const int64_t (&
     }
     *kx = reinterpret_cast<int32_t*>(d.mem.p + k);
     d.kx = *kx;
-    return cudaSuccess;
+    // digit_psi_kernel writes a column's k up to a multiple of 16; a product's boxes of
+    // 32 rows take in more of neighbouring columns (outputs that nothing uses)
+    return cudaMemset(d.x.q, 0, digit_stack_bytes(d.x.rows));
 }
 
 // The digit form of a complex plan: the same products on operands of two parts.

@@ -15,7 +15,8 @@ namespace tk {
 
 // Device allocations of a plan.  With a countdown armed by
 // tk_debug_fail_device_alloc, the countdown-th allocation fails as if the
-// device were out of memory (test hook for the TK_ERR_OOM paths).
+// device were out of memory (test hook for the TK_ERR_OOM paths); a negative one
+// fills every allocation with a byte.
 extern std::atomic<int> g_fail_device_alloc;
 inline cudaError_t dev_malloc(void** p, size_t bytes) {
     int c = g_fail_device_alloc.load(std::memory_order_relaxed);
@@ -25,7 +26,8 @@ inline cudaError_t dev_malloc(void** p, size_t bytes) {
         *p = nullptr;
         return cudaErrorMemoryAllocation;
     }
-    return cudaMalloc(p, bytes);
+    const cudaError_t e = cudaMalloc(p, bytes);
+    return e == cudaSuccess && c < 0 ? cudaMemset(*p, -c, bytes) : e;
 }
 
 template <class T>
