@@ -561,6 +561,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
 // ---------------------------------------------------------------- digits
 
 __device__ __forceinline__ uint32_t abs_hi(double x) { return (uint32_t)__double2hiint(x) & 0x7FFFFFFFu; }
+// The high word of |x|, 1 for what has none of its own: zero only for zero.
+__device__ __forceinline__ uint32_t abs_top(double x) {
+    const uint32_t hi = abs_hi(x);
+    return hi == 0 && __double2loint(x) != 0 ? 1u : hi;
+}
 // Biased exponent of a row whose largest element has these high bits (below 1
 // for a row of subnormals).
 __device__ __forceinline__ int row_exponent(uint32_t max_hi, int* redo) {
@@ -638,6 +643,12 @@ __device__ __forceinline__ int exponent_of(double x, int k) {
     return zero ? kNoExponent : (e > 0 ? e : 12 - __clz((int)(hi | 1))) + k;
 }
 
+// Scale of a column of zeros: what the other operand holds at that k is multiplied
+// by zeros, so it must neither set its row's exponent nor take up its digits.
+constexpr int kDeadColumn = -4096;
+// A row's exponent; one with nothing but dead columns counts as zeros.
+__device__ __forceinline__ int scaled_row_exponent(int mx) { return mx < kDeadColumn / 2 ? 1 : mx; }
+
 // One CTA per 64-wide chunk of a stack (blockIdx.y, past the stack's last: nothing): the columns' exponents.
 __global__ void __launch_bounds__(256) digit_columns_kernel(const DigitRows* __restrict__ jobs,
                                                             const double* __restrict__ q64,
@@ -650,14 +661,14 @@ __global__ void __launch_bounds__(256) digit_columns_kernel(const DigitRows* __r
 #pragma unroll 4
     for (int r = w; r < j.n; r += 4) {
         const int64_t at = (((int64_t)j.row + (int64_t)c * j.cs + r) << 6) + k;
-        mx = max(mx, abs_hi(q64[at]));
-        if (q64_im) mx = max(mx, abs_hi(q64_im[at]));
+        mx = max(mx, abs_top(q64[at]));
+        if (q64_im) mx = max(mx, abs_top(q64_im[at]));
     }
     top[w][k] = mx;
     __syncthreads();
     if (w != 0) return;
     mx = max(max(top[0][k], top[1][k]), max(top[2][k], top[3][k]));
-    kx[j.kx + c * kTcBK + k] = mx >> 20 ? (int)(mx >> 20) - 1023 : 0;
+    kx[j.kx + c * kTcBK + k] = mx == 0 ? kDeadColumn : (mx >> 20 ? (int)(mx >> 20) : 12 - __clz((int)mx)) - 1023;
 }
 
 // One warp per row of an FP64 stack (K-major 64-wide chunks): the row's
@@ -711,7 +722,7 @@ __global__ void __launch_bounds__(32 * kDigitRowsPerCta) digit_rows_kernel(const
     }
     mx = __reduce_max_sync(0xffffffffu, mx);
     if (hi >= 0x7FF00000u) atomicExch(redo, kDigitValue);
-    const int ex = mx == kNoExponent ? 1 : mx;
+    const int ex = scaled_row_exponent(mx);
     if (lane == 0) out.ex[row] = ex;
     auto put = [&](int c, const double2& u) {
         const int2 k = scale(c);
@@ -762,7 +773,7 @@ __global__ void __launch_bounds__(32 * kDigitRowsPerCta) digit_rows_complex_kern
     }
     mx = __reduce_max_sync(0xffffffffu, mx);
     if (hi >= 0x7FF00000u) atomicExch(redo, kDigitValue);
-    const int ex = mx == kNoExponent ? 1 : mx;
+    const int ex = scaled_row_exponent(mx);
     if (lane == 0) {
         out.ex[to] = ex;
         if (DUAL) out.ex[to + j.n_dual] = ex;
@@ -862,11 +873,6 @@ __global__ void __launch_bounds__(PT) digit_psi_kernel(const DigitPsi* __restric
 }
 
 constexpr int BT = 256;
-// The high word of |x|, 1 for what has none of its own: zero only for zero.
-__device__ __forceinline__ uint32_t abs_top(double x) {
-    const uint32_t hi = abs_hi(x);
-    return hi == 0 && __double2loint(x) != 0 ? 1u : hi;
-}
 // Whether x lies on the grid of digits 0 .. 3 of a row with exponent ex: its lowest bit at
 // 2^(ex - 1055) or above.
 __device__ __forceinline__ bool in_four_digits(double x, int ex) {

@@ -109,7 +109,7 @@ cudaError_t launch_digit_gemm(int mode, const TcTile* tiles, const int32_t* begi
                               const int32_t* exa, const int32_t* exb, const DigitOut& out, int* redo, cudaStream_t s);
 
 // Exponents of a stack's columns: kx[j.kx + k] = floor(log2 max |x|) over the
-// rows [row, row + n) of job j at k, 0 for a column of zeros.
+// rows [row, row + n) of job j at k; far below any of them for a column of zeros.
 cudaError_t launch_digit_columns(const DigitRows* jobs, int n_jobs, int max_kch, const double* q64, const double* q64_im,
                                  int32_t* kx, cudaStream_t s);
 // Digits of FP64 operand stacks (rows of 64 doubles per chunk), of

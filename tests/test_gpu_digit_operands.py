@@ -1,10 +1,11 @@
 """Operands of the FP64 matvec on digits (csrc/stack_f64.cu, csrc/digit_gemm.cu): what lies behind
-them in memory."""
+them in memory, and columns of R that are zero or subnormal."""
 import numpy as np
 import pytest
 
+from helpers import rel_err
 from test_gpu_digit_matvec import _apply, _apply_complex, _complex_plan, _problem
-from tk_gb300 import _abi
+from tk_gb300 import Environment, _abi
 
 pytestmark = pytest.mark.gpu
 
@@ -37,3 +38,56 @@ def test_complex_result_does_not_depend_on_unwritten_memory(stale, name, D):
     stale(True)
     got = _apply_complex(_complex_plan(p, np.random.default_rng(D), False), x, _abi.SCHED_STACKED)
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+def _right_sector(key, nc):
+    """Charges of leg 3 of a packed block key (8 bits of two's complement a component)."""
+    q = [(int(key) >> (8 * (3 * nc + c))) & 255 for c in range(nc)]
+    return tuple(v - 256 if v > 127 else v for v in q)
+
+
+# ket states of R that no operator connects, and states connected by subnormal elements alone, with large
+# amplitudes in psi: they add nothing, or nothing that counts, to the result
+@pytest.mark.parametrize("scale,boost", [(0.0, 2.0 ** 30), (2.0 ** -1060, 2.0 ** 900)])
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("name,D", [("heisenberg", 401), ("hubbard", 700), ("cylinder", 257)])
+def test_vanishing_columns_of_r_cost_the_others_no_digits(lib_built, name, D, cplx, scale, boost):
+    def change(e, side):
+        if side == 0:
+            return e
+        d = e.data.copy()
+        d[:, :, ::5] *= scale
+        return Environment(d, e.bra_idx, e.mpo_idx, e.ket_idx)
+
+    p = _problem(name, D, change)
+    rng = np.random.default_rng(D)
+    plan = _complex_plan(p, rng, False) if cplx else p.plan()
+    if cplx:  # (imaginary parts are drawn where the real part is not zero: scaled here as well)
+        from tk_gb300 import Heff2Plan, sweep
+
+        def dev(e, side):
+            im = rng.standard_normal(e.data.shape) * (e.data != 0.0)
+            if side:
+                im[:, :, ::5] *= scale
+            return sweep.DeviceEnv.from_dense(p.kind, e.data + 1j * im, e.bra_idx, e.mpo_idx, e.ket_idx)
+
+        plan = Heff2Plan.from_device_envs_complex(dev(p.env_l, 0), dev(p.env_r, 1), p.w_i, p.w_j, p.flux)
+    assert plan.launches() == 6
+    ket = p.env_r.ket_idx
+    nc = len(ket.sectors[0][0])
+    first, at = {}, 0
+    for q, n in ket.sectors:
+        first[tuple(q)] = (at, n)
+        at += n
+    x = rng.standard_normal(plan.block_dim) + (1j * rng.standard_normal(plan.block_dim) if cplx else 0.0)
+    keys, offs = plan.blocks()
+    for key, a, b in zip(keys, offs, list(offs[1:]) + [plan.block_dim]):
+        o, n = first[_right_sector(key, nc)]
+        cols = (o + np.arange(n)) % 5 == 0
+        x[a:b].reshape(-1, n)[:, cols] *= boost
+    if cplx:
+        got, want = ([np.concatenate(_apply_complex(plan, x, s))] for s in (_abi.SCHED_STACKED, _abi.SCHED_GROUPED))
+    else:
+        got, want = ([_apply(plan, x, s)] for s in (_abi.SCHED_STACKED, _abi.SCHED_GROUPED))
+    assert np.isfinite(want[0]).all() and np.linalg.norm(want[0]) < 2.0 ** 40
+    assert rel_err(got[0], want[0]) < 64 * 2.0 ** -53
