@@ -652,23 +652,25 @@ __device__ __forceinline__ int scaled_row_exponent(int mx) { return mx < kDeadCo
 // One CTA per 64-wide chunk of a stack (blockIdx.y, past the stack's last: nothing): the columns' exponents.
 __global__ void __launch_bounds__(256) digit_columns_kernel(const DigitRows* __restrict__ jobs,
                                                             const double* __restrict__ q64,
-                                                            const double* __restrict__ q64_im, int32_t* __restrict__ kx) {
-    __shared__ uint32_t top[4][kTcBK];
+                                                            const double* __restrict__ q64_im,
+                                                            const int32_t* __restrict__ ex, int32_t* __restrict__ kx) {
+    __shared__ int top[4][kTcBK];
     const DigitRows j = jobs[blockIdx.x];
     const int k = threadIdx.x & 63, w = threadIdx.x >> 6, c = blockIdx.y;
     if (c >= j.kch) return;
-    uint32_t mx = 0;
+    int mx = kNoExponent;
 #pragma unroll 4
     for (int r = w; r < j.n; r += 4) {
         const int64_t at = (((int64_t)j.row + (int64_t)c * j.cs + r) << 6) + k;
-        mx = max(mx, abs_top(q64[at]));
-        if (q64_im) mx = max(mx, abs_top(q64_im[at]));
+        const int by = ex ? -ex[j.ex0 + r] : -1023;
+        mx = max(mx, exponent_of(q64[at], by));
+        if (q64_im) mx = max(mx, exponent_of(q64_im[at], by));
     }
     top[w][k] = mx;
     __syncthreads();
     if (w != 0) return;
     mx = max(max(top[0][k], top[1][k]), max(top[2][k], top[3][k]));
-    kx[j.kx + c * kTcBK + k] = mx == 0 ? kDeadColumn : (mx >> 20 ? (int)(mx >> 20) : 12 - __clz((int)mx)) - 1023;
+    kx[j.kx + c * kTcBK + k] = mx == kNoExponent ? kDeadColumn : mx;
 }
 
 // One warp per row of an FP64 stack (K-major 64-wide chunks): the row's
@@ -796,10 +798,10 @@ __global__ void __launch_bounds__(32 * kDigitRowsPerCta) digit_rows_complex_kern
 constexpr int PT = 256;
 template <bool CPLX, int CW>
 __global__ void __launch_bounds__(PT) digit_psi_kernel(const DigitPsi* __restrict__ jobs, const double* __restrict__ x,
-                                                       const double* __restrict__ xi, int pitch, const DigitStack out,
-                                                       int* redo) {
+                                                       const double* __restrict__ xi, const int32_t* __restrict__ kx,
+                                                       int pitch, const DigitStack out, int* redo) {
     extern __shared__ double tile[];  // [CW][pitch], the imaginary part's behind it
-    __shared__ uint32_t smax[32];
+    __shared__ int smax[32], scale[kTcBK];
     const DigitPsi j = jobs[blockIdx.x];
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int nr = j.cols, K = j.rows, kch = (K + kTcBK - 1) / kTcBK;
@@ -807,11 +809,21 @@ __global__ void __launch_bounds__(PT) digit_psi_kernel(const DigitPsi* __restric
     const int col = lane % CW, kw = w * (32 / CW) + lane / CW;  // this thread's column, first k
     constexpr int KS = PT / CW;                                 // k step of the CTA
     const int64_t src = j.src + col;
+    const int32_t* sk = kx + j.kx;  // (a plan constant)
     dep_launch();
-    if (tid < 32) smax[tid] = 0;
+    if (tid < 32) smax[tid] = kNoExponent;
+    if (tid < kTcBK) scale[tid] = sk[tid];
     __syncthreads();
     dep_wait();
-    uint32_t mx = 0;
+    int mx = kNoExponent;
+    uint32_t hi = 0, tiny = 0;  // tiny: whether there are subnormals
+    auto look = [&](double v, int s) {
+        const uint32_t h = abs_hi(v);
+        const int e = (int)(h >> 20);
+        hi = max(hi, h);
+        tiny |= e > 0 ? 0u : h | (uint32_t)__double2loint(v);
+        mx = max(mx, e > 0 ? e + s : kNoExponent);
+    };
     // chunk c into shared memory, zeros to a whole 16-wide step (they are multiplied)
     auto fetch = [&](int c) {
         const int k0 = c * kTcBK, kv = (min(kTcBK, K - k0) + 15) & ~15;
@@ -821,11 +833,11 @@ __global__ void __launch_bounds__(PT) digit_psi_kernel(const DigitPsi* __restric
             const int64_t o = src + (int64_t)(k0 + k) * j.pitch;
             const double v = in ? x[o] : 0.0;
             tile[col * pitch + k] = v;
-            mx = max(mx, abs_hi(v));
+            if (kch == 1) look(v, scale[k]);
             if (CPLX) {
                 const double u = in ? xi[o] : 0.0;
                 tile_im[col * pitch + k] = u;
-                mx = max(mx, abs_hi(u));
+                if (kch == 1) look(u, scale[k]);
             }
         }
         return kv;
@@ -837,33 +849,45 @@ __global__ void __launch_bounds__(PT) digit_psi_kernel(const DigitPsi* __restric
         for (int k = kw; k < K; k += KS)
             if (col < nr) {
                 const int64_t o = src + (int64_t)k * j.pitch;
-                mx = max(mx, abs_hi(x[o]));
-                if (CPLX) mx = max(mx, abs_hi(xi[o]));
+                const int s = sk[k];
+                look(x[o], s);
+                if (CPLX) look(xi[o], s);
             }
     }
+    if (tiny) {
+        for (int k = kw; k < K; k += KS) {  // (col < nr, or it would have seen zeros)
+            const int64_t o = src + (int64_t)k * j.pitch;
+            mx = max(mx, exponent_of(x[o], sk[k]));
+            if (CPLX) mx = max(mx, exponent_of(xi[o], sk[k]));
+        }
+    }
     atomicMax(&smax[col], mx);
+    if (hi >= 0x7FF00000u) atomicExch(redo, kDigitValue);
     __syncthreads();
     if (tid < nr) {
-        const int ex = row_exponent(smax[tid], redo);
+        const int ex = scaled_row_exponent(smax[tid]);
         out.ex[(int64_t)j.to + tid] = ex;
         if (CPLX) out.ex[(int64_t)j.to + j.n_dual + tid] = ex;
-        smax[tid] = (uint32_t)ex;
+        smax[tid] = ex;
     }
     for (int c = 0; c < kch; ++c) {
         __syncthreads();
         const int kv = kch == 1 ? (K + 15) & ~15 : fetch(c);
-        if (kch > 1) __syncthreads();
+        if (kch > 1) {
+            if (tid < kTcBK) scale[tid] = sk[c * kTcBK + tid];
+            __syncthreads();
+        }
         // rows and pairs of k over the threads
         const int pairs = kv >> 1;
         for (int e = tid; e < nr * pairs; e += PT) {
             const int r = e / pairs, k = 2 * (e - r * pairs);
             const double* v = tile + r * pitch + k;
             uint32_t d[kDigits];
-            digits2(v[0], v[1], (int)smax[r], d);
+            digits2(v[0], v[1], smax[r], d, scale[k], scale[k + 1]);
             if (CPLX) {
                 const double* u = tile_im + r * pitch + k;
                 uint32_t f[kDigits];
-                digits2(u[0], u[1], (int)smax[r], f);
+                digits2(u[0], u[1], smax[r], f, scale[k], scale[k + 1]);
                 put_complex<true>(out, (int64_t)j.to + r, j.n_dual, (int64_t)c * j.cs, (int64_t)(kch + c) * j.cs, k, d, f);
             } else {
                 put_digits(out, (int64_t)j.to + r + (int64_t)c * j.cs, k, d);
@@ -1094,9 +1118,9 @@ void digit_schedule(const std::vector<TcTile>& in, int ctas, std::vector<TcTile>
 }
 
 cudaError_t launch_digit_columns(const DigitRows* jobs, int n_jobs, int max_kch, const double* q64, const double* q64_im,
-                                 int32_t* kx, cudaStream_t s) {
+                                 const int32_t* ex, int32_t* kx, cudaStream_t s) {
     if (n_jobs <= 0 || max_kch <= 0) return cudaSuccess;
-    digit_columns_kernel<<<dim3((unsigned)n_jobs, (unsigned)max_kch), 256, 0, s>>>(jobs, q64, q64_im, kx);
+    digit_columns_kernel<<<dim3((unsigned)n_jobs, (unsigned)max_kch), 256, 0, s>>>(jobs, q64, q64_im, ex, kx);
     return cudaGetLastError();
 }
 
@@ -1123,13 +1147,13 @@ cudaError_t launch_digit_matrices(const DigitMatrix& a, const DigitMatrix& b, in
 }
 
 cudaError_t launch_digit_psi(const DigitPsi* jobs, int n_jobs, int cols, int max_k, const double* x, const double* x_im,
-                             const DigitStack& out, int* redo, cudaStream_t s) {
+                             const int32_t* kx, const DigitStack& out, int* redo, cudaStream_t s) {
     if (n_jobs <= 0) return cudaSuccess;
     const int pitch = ((std::min(max_k, kTcBK) + 15) & ~15) + 1;
     const size_t smem = sizeof(double) * cols * pitch * (x_im ? 2 : 1);
     auto* k = cols == 8 ? (x_im ? digit_psi_kernel<true, 8> : digit_psi_kernel<false, 8>)
                         : (x_im ? digit_psi_kernel<true, 32> : digit_psi_kernel<false, 32>);
-    return launch_dependent(k, n_jobs, PT, smem, s, jobs, x, x_im, pitch, out, redo);
+    return launch_dependent(k, n_jobs, PT, smem, s, jobs, x, x_im, kx, pitch, out, redo);
 }
 
 }  // namespace tk

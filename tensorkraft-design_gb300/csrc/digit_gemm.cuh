@@ -52,9 +52,10 @@ struct DigitStack {
 inline size_t digit_stack_bytes(int64_t rows) { return (size_t)rows * kTcBK * kDigits * sizeof(__half); }
 
 // Rows [row, row + n) of a stack whose chunks are `cs` rows apart; `kx` >= 0:
-// the index of the power-of-two scales of its k (launch_digit_columns).
+// the index of the power-of-two scales of its k (launch_digit_columns); `ex0`
+// >= 0: row 0's exponent in the table that launch_digit_columns gets.
 struct DigitRows {
-    int32_t row, n, cs, kch, kx, pad;
+    int32_t row, n, cs, kch, kx, ex0;
 };
 // The same of a complex stack: its digits go to rows to .. of a stack whose
 // chunks are cs_out rows apart (the imaginary part's chunks behind the real
@@ -64,9 +65,10 @@ struct DigitRowsC {
 };
 // Columns [0, cols) (at most 32) at src of a psi sub-block (rows x pitch), as
 // rows to .. of a B operand; complex vectors' second form n_dual rows further.
+// `kx`: the index of the scales of its k.
 struct DigitPsi {
     int64_t src;
-    int32_t rows, cols, pitch, to, cs, n_dual;
+    int32_t rows, cols, pitch, to, cs, n_dual, kx, pad;
 };
 constexpr int kDigitRowsPerCta = 8;
 
@@ -109,9 +111,10 @@ cudaError_t launch_digit_gemm(int mode, const TcTile* tiles, const int32_t* begi
                               const int32_t* exa, const int32_t* exb, const DigitOut& out, int* redo, cudaStream_t s);
 
 // Exponents of a stack's columns: kx[j.kx + k] = floor(log2 max |x|) over the
-// rows [row, row + n) of job j at k; far below any of them for a column of zeros.
+// rows [row, row + n) of job j at k (with exponents of rows: of x by its row's
+// largest); far below any of them for a column of zeros.
 cudaError_t launch_digit_columns(const DigitRows* jobs, int n_jobs, int max_kch, const double* q64, const double* q64_im,
-                                 int32_t* kx, cudaStream_t s);
+                                 const int32_t* ex, int32_t* kx, cudaStream_t s);
 // Digits of FP64 operand stacks (rows of 64 doubles per chunk), of
 // x 2^(sign * kx) where the job has scales.
 cudaError_t launch_digit_rows(const DigitRows* jobs, int n_jobs, const double* q64, const int32_t* kx, int sign,
@@ -133,8 +136,8 @@ struct DigitMatrix {
 constexpr int kDigitSamples = 64;
 cudaError_t launch_digit_matrices(const DigitMatrix& a, const DigitMatrix& b, int K, int* wide, int* redo, cudaStream_t s);
 // Digits of psi sub-blocks (jobs of at most `cols` columns, 32 or 8, and max_k
-// rows), of both parts with x_im.
+// rows) times 2^kx, of both parts with x_im.
 cudaError_t launch_digit_psi(const DigitPsi* jobs, int n_jobs, int cols, int max_k, const double* x, const double* x_im,
-                             const DigitStack& out, int* redo, cudaStream_t s);
+                             const int32_t* kx, const DigitStack& out, int* redo, cudaStream_t s);
 
 }  // namespace tk

@@ -483,7 +483,7 @@ bool stage3_pieces(const TcTables& C, std::vector<F64Piece>& out, std::vector<KS
 struct F64Digits {
     DevBuf<unsigned char> mem;       // one allocation for all of it
     DigitStack l, r, t2, x;
-    const int32_t* kx = nullptr;     // scales of the R stacks' columns
+    const int32_t* kx = nullptr;     // scales of the R and L stacks' columns
     const TcTile *tiles1 = nullptr, *tiles3 = nullptr;   // dealt out to `sms` CTAs:
     const int32_t *begin1 = nullptr, *begin3 = nullptr;
     const DigitPsi* psi = nullptr;
@@ -517,7 +517,7 @@ void F64StackDeleter::operator()(F64Stack* p) const { delete p; }
 // The rows of a stack, kDigitRowsPerCta a job.
 static void digit_rows_of(std::vector<DigitRows>& out, int32_t row, int n, int32_t cs, int32_t kch, int32_t kx) {
     for (int r = 0; r < n; r += kDigitRowsPerCta)
-        out.push_back({row + r, std::min(kDigitRowsPerCta, n - r), cs, kch, kx, 0});
+        out.push_back({row + r, std::min(kDigitRowsPerCta, n - r), cs, kch, kx, -1});
 }
 
 // Whether a plan's FP64 matvec runs on digits: from 1.2 million multiply-adds in
@@ -596,6 +596,7 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
     struct Stack {
         int32_t M = 0, N = 0, K = 0, kch = 0, a = INT32_MAX, b = INT32_MAX;  // rows, columns, K; first rows of A and B
         int64_t out = INT64_MAX;  // first entry of the column table (stage 1) or row table (stage 3)
+        int32_t kx = 0;           // stage 1: scales of its k
     };
     if (std::max({C.lq_rows, C.rq_rows, C.t2q_rows, C.xq_rows}) > INT32_MAX / 4) return cudaSuccess;  // 32-bit rows
     std::map<int32_t, Stack> s1, s3;  // by the first row of the operand that names the stack
@@ -608,7 +609,7 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
     std::vector<TcTile> w1, w3, t1, t3;
     std::vector<int32_t> b1, b3;
     std::vector<DigitRowsC> lrows, rrows, trows;
-    std::vector<DigitRows> rcols;
+    std::vector<DigitRows> rcols, lcols;
     std::vector<DigitPsi> psi;
     std::vector<int64_t> colbase(2 * C.t1col_base.size());
     std::vector<int32_t> colstride(2 * C.t1col_stride.size());
@@ -635,10 +636,15 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
             }
     };
     std::map<int32_t, const Stack*> by_psi;  // stage-1 stacks by their first psi row
-    for (const auto& [key, s] : s1) {
+    int kch1 = 0;
+    for (auto& [key, s] : s1) {
         by_psi[s.b] = &s;
         tiles(w1, s, 2);
-        rows(lrows, s.a, s.M, s.M, s.kch, -1, 2 * s.a, s.M, 0);
+        s.kx = nk;
+        nk += s.kch * kTcBK;
+        kch1 = std::max(kch1, s.kch);
+        lcols.push_back({s.a, s.M, s.M, s.kch, s.kx, 2 * s.a});
+        rows(lrows, s.a, s.M, s.M, s.kch, s.kx, 2 * s.a, s.M, 0);
         for (int32_t c = 0; c < s.N; ++c)
             for (int h = 0; h < 2; ++h) {
                 colbase[(size_t)(2 * s.out + h * s.N + c)] = C.t1col_base[(size_t)(s.out + c)] + h * im;
@@ -654,12 +660,12 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
         }
         const Stack& s = *std::prev(it)->second;
         psi.push_back({j.src + j.b0, j.rows, std::min(32, j.cols - j.b0), j.cols, 4 * s.b + (j.xrow - s.b) + j.b0, 2 * s.N,
-                       s.N});
+                       s.N, s.kx, 0});
     }
     psi_jobs(psi, *d);
     for (const auto& [key, s] : s3) {
         tiles(w3, s, 1);
-        rcols.push_back({s.b, s.N, s.N, s.kch, nk, 0});
+        rcols.push_back({s.b, s.N, s.N, s.kch, nk, -1});
         rows(rrows, s.b, s.N, s.N, s.kch, nk, 4 * s.b, 2 * s.N, s.N);
         rows(trows, s.a, s.M, s.M, s.kch, nk, 2 * s.a, s.M, 0);
         nk += s.kch * kTcBK;
@@ -677,7 +683,7 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
     auto table = [&](const auto& v) { return blob.add(v.data(), sizeof(v[0]) * v.size()); };
     const size_t o_redo = blob.add(&redo, sizeof(redo)), o_t1 = table(t1), o_t3 = table(t3), o_b1 = table(b1),
                  o_b3 = table(b3), o_psi = table(psi), o_rows = table(trows), o_l = table(lrows), o_r = table(rrows),
-                 o_c = table(rcols), o_cb = table(colbase), o_cs = table(colstride);
+                 o_c = table(rcols), o_lc = table(lcols), o_cb = table(colbase), o_cs = table(colstride);
     if ((e = digits_alloc(*d, blob, {2 * C.lq_rows, 4 * C.rq_rows, 2 * C.t2q_rows, 4 * C.xq_rows}, nk, &kx)) != cudaSuccess)
         return e;
     unsigned char* m = d->mem.p;
@@ -691,10 +697,16 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
     d->colstride = reinterpret_cast<const int32_t*>(m + o_cs);
     d->redo = reinterpret_cast<int*>(m + o_redo);
     if (!digit_maps(d->m1, d->l, d->x, err) || !digit_maps(d->m3, d->t2, d->r, err)) return cudaErrorInvalidValue;
-    if ((e = launch_digit_rows_complex(reinterpret_cast<const DigitRowsC*>(m + o_l), (int)lrows.size(), p.lq.p, p.lq_im.p,
-                                       nullptr, 1, false, d->l, d->redo, 0)) != cudaSuccess ||
+    // (L's rows without scales first, for their exponents)
+    if ((e = cudaMemset(kx, 0, sizeof(int32_t) * (size_t)nk)) != cudaSuccess ||
+        (e = launch_digit_rows_complex(reinterpret_cast<const DigitRowsC*>(m + o_l), (int)lrows.size(), p.lq.p, p.lq_im.p,
+                                       kx, -1, false, d->l, d->redo, 0)) != cudaSuccess ||
+        (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_lc), (int)lcols.size(), kch1, p.lq.p, p.lq_im.p,
+                                  d->l.ex, kx, 0)) != cudaSuccess ||
+        (e = launch_digit_rows_complex(reinterpret_cast<const DigitRowsC*>(m + o_l), (int)lrows.size(), p.lq.p, p.lq_im.p,
+                                       kx, -1, false, d->l, d->redo, 0)) != cudaSuccess ||
         (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_c), (int)rcols.size(), C.max_kch3, p.rq.p,
-                                  p.rq_im.p, kx, 0)) != cudaSuccess ||
+                                  p.rq_im.p, nullptr, kx, 0)) != cudaSuccess ||
         (e = launch_digit_rows_complex(reinterpret_cast<const DigitRowsC*>(m + o_r), (int)rrows.size(), p.rq.p, p.rq_im.p,
                                        kx, -1, true, d->r, d->redo, 0)) != cudaSuccess ||
         (e = cudaMemcpy(&redo, d->redo, sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess)
@@ -710,23 +722,44 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
 static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& err) {
     std::unique_ptr<F64Digits> d(new F64Digits);
     if (p.cplx) return digits_create_complex(C, p, std::move(d), err);
-    std::vector<DigitRows> lrows, rrows, trows, rcols;
+    std::vector<DigitRows> lrows, rrows, trows, rcols, lcols;
     std::vector<DigitPsi> psi;
-    for (const TcSplitJob& j : C.split)
-        if (j.a0 == 0) psi.push_back({j.src + j.b0, j.rows, std::min(32, j.cols - j.b0), j.cols, j.xrow + j.b0, j.cstride, 0});
-    psi_jobs(psi, *d);
     std::set<int32_t> seen;
-    for (const TcTile& t : C.tiles1x)
-        if (seen.insert(t.a_row).second) digit_rows_of(lrows, t.a_row, t.m_valid, t.a_cs, t.kch, -1);
+    int32_t nk = 0;
+    int kch1 = 0;
+    // stage 1: the columns of L on scales of their own, which psi takes up.  What
+    // a column has in its rows counts by the rows' largest elements, so that one
+    // channel of great magnitude does not set the scales of the others.
+    std::map<int32_t, int32_t> kx1;  // stack (its first psi row) -> scales
+    for (const TcTile& t : C.tiles1x) {
+        if (kx1.insert({t.b_row - t.n0, nk}).second) {
+            const int32_t a = t.a_row - t.ldc;
+            lcols.push_back({a, t.a_cs, t.a_cs, t.kch, nk, a});
+            nk += t.kch * kTcBK;
+            kch1 = std::max(kch1, t.kch);
+        }
+        if (seen.insert(t.a_row).second)
+            digit_rows_of(lrows, t.a_row, t.m_valid, t.a_cs, t.kch, kx1[t.b_row - t.n0]);
+    }
+    for (const TcSplitJob& j : C.split) {
+        if (j.a0 != 0) continue;
+        auto it = kx1.upper_bound(j.xrow);
+        if (it == kx1.begin()) {
+            err = "digit operands: psi sub-block outside every stack";
+            return cudaErrorInvalidValue;
+        }
+        psi.push_back({j.src + j.b0, j.rows, std::min(32, j.cols - j.b0), j.cols, j.xrow + j.b0, j.cstride, 0,
+                       std::prev(it)->second, 0});
+    }
+    psi_jobs(psi, *d);
     // stage 3: the columns of R on scales of their own, which T2 takes up, so
     // that no channel's magnitude (an energy against an identity) costs the
     // others digits
     std::map<int32_t, int32_t> kx;  // stack (row of its first R row) -> scales
-    int32_t nk = 0;
     for (const TcTile& t : C.tiles3) {
         const int32_t base = t.b_row - t.n0;
         if (kx.insert({base, nk}).second) {
-            rcols.push_back({base, t.b_cs, t.b_cs, t.kch, nk, 0});
+            rcols.push_back({base, t.b_cs, t.b_cs, t.kch, nk, -1});
             nk += t.kch * kTcBK;
         }
         if (seen.insert(-1 - t.b_row).second) digit_rows_of(rrows, t.b_row, t.n_valid, t.b_cs, t.kch, kx[base]);
@@ -747,7 +780,7 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
     auto table = [&](const auto& v) { return blob.add(v.data(), sizeof(v[0]) * v.size()); };
     const size_t o_redo = blob.add(&redo, sizeof(redo)), o_t1 = table(t1), o_t3 = table(t3), o_b1 = table(b1),
                  o_b3 = table(b3), o_psi = table(psi), o_rows = table(trows), o_l = table(lrows), o_r = table(rrows),
-                 o_c = table(rcols);
+                 o_c = table(rcols), o_lc = table(lcols);
     int32_t* kxd = nullptr;
     if ((e = digits_alloc(*d, blob, {C.lq_rows, C.rq_rows, C.t2q_rows, C.xq_rows}, nk, &kxd)) != cudaSuccess) return e;
     unsigned char* m = d->mem.p;
@@ -759,10 +792,16 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
     d->rows = reinterpret_cast<const DigitRows*>(m + o_rows);
     d->redo = reinterpret_cast<int*>(m + o_redo);
     if (!digit_maps(d->m1, d->l, d->x, err) || !digit_maps(d->m3, d->t2, d->r, err)) return cudaErrorInvalidValue;
-    if ((e = launch_digit_rows(reinterpret_cast<const DigitRows*>(m + o_l), (int)lrows.size(), p.lq.p, nullptr, 1, d->l,
+    // (L's rows without scales first, for their exponents)
+    if ((e = cudaMemset(kxd, 0, sizeof(int32_t) * (size_t)nk)) != cudaSuccess ||
+        (e = launch_digit_rows(reinterpret_cast<const DigitRows*>(m + o_l), (int)lrows.size(), p.lq.p, kxd, -1, d->l,
                                d->redo, 0)) != cudaSuccess ||
-        (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_c), (int)rcols.size(), C.max_kch3, p.rq.p, nullptr, kxd, 0)) !=
-            cudaSuccess ||
+        (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_lc), (int)lcols.size(), kch1, p.lq.p, nullptr,
+                                  d->l.ex, kxd, 0)) != cudaSuccess ||
+        (e = launch_digit_rows(reinterpret_cast<const DigitRows*>(m + o_l), (int)lrows.size(), p.lq.p, kxd, -1, d->l,
+                               d->redo, 0)) != cudaSuccess ||
+        (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_c), (int)rcols.size(), C.max_kch3, p.rq.p, nullptr,
+                                  nullptr, kxd, 0)) != cudaSuccess ||
         (e = launch_digit_rows(reinterpret_cast<const DigitRows*>(m + o_r), (int)rrows.size(), p.rq.p, kxd, -1, d->r,
                                d->redo, 0)) != cudaSuccess ||
         (e = cudaMemcpy(&redo, d->redo, sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess)
@@ -869,7 +908,7 @@ static cudaError_t digits_stage(F64Stack& p, const double* x, double* y, cudaStr
     cudaError_t e;
     DigitOut o{};
     if (stage == 0) {
-        if ((e = launch_digit_psi(d.psi, d.npsi, d.psi_cols, d.max_k, x, nullptr, d.x, d.redo, s)) != cudaSuccess) return e;
+        if ((e = launch_digit_psi(d.psi, d.npsi, d.psi_cols, d.max_k, x, nullptr, d.kx, d.x, d.redo, s)) != cudaSuccess) return e;
         o.out = p.t1.p;
         o.colbase = p.colbase.p;
         o.colstride = p.colstride.p;
@@ -890,7 +929,7 @@ static cudaError_t digits_stage(F64Stack& p, const double* x, double* y, cudaStr
 static cudaError_t digits_apply_complex(F64Stack& p, const double* xr, const double* xi, double* yr, double* yi,
                                         cudaStream_t s) {
     F64Digits& d = *p.dg;
-    cudaError_t e = launch_digit_psi(d.psi, d.npsi, d.psi_cols, d.max_k, xr, xi, d.x, d.redo, s);
+    cudaError_t e = launch_digit_psi(d.psi, d.npsi, d.psi_cols, d.max_k, xr, xi, d.kx, d.x, d.redo, s);
     DigitOut o{};
     o.out = p.t1.p;
     o.colbase = d.colbase;

@@ -91,3 +91,53 @@ def test_vanishing_columns_of_r_cost_the_others_no_digits(lib_built, name, D, cp
         got, want = ([_apply(plan, x, s)] for s in (_abi.SCHED_STACKED, _abi.SCHED_GROUPED))
     assert np.isfinite(want[0]).all() and np.linalg.norm(want[0]) < 2.0 ** 40
     assert rel_err(got[0], want[0]) < 64 * 2.0 ** -53
+
+
+def _left_sector(key, nc):
+    q = [(int(key) >> (8 * (2 * nc + c))) & 255 for c in range(nc)]
+    return tuple(v - 256 if v > 127 else v for v in q)
+
+
+# the same for L's ket states; and ket states on scales of their own (2^-20 .. 2^20, taken back in psi),
+# which a stack's rows must not see
+@pytest.mark.parametrize("kind", ["zero", "subnormal", "scales"])
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("name,D", [("heisenberg", 401), ("hubbard", 700), ("cylinder", 257), ("cylinder", 500)])
+def test_uneven_columns_of_l_cost_no_digits(lib_built, name, D, cplx, kind):
+    from tk_gb300 import Heff2Plan, sweep
+
+    p = _problem(name, D, lambda e, side: e)
+    rng = np.random.default_rng(D)
+    n = p.env_l.data.shape[2]
+    if kind == "scales":
+        left = np.exp2(rng.integers(-20, 21, n).astype(float))
+        back = 1.0 / left
+    else:
+        left, back = np.ones(n), np.ones(n)
+        left[::5], back[::5] = (0.0, 2.0 ** 30) if kind == "zero" else (2.0 ** -1060, 2.0 ** 900)
+    if cplx:
+        def dev(e, s):
+            z = e.data + 1j * rng.standard_normal(e.data.shape) * (e.data != 0.0)
+            re, im = z.real * s, z.imag * s
+            return sweep.DeviceEnv.from_dense(p.kind, re + 1j * im, e.bra_idx, e.mpo_idx, e.ket_idx)
+
+        plan = Heff2Plan.from_device_envs_complex(dev(p.env_l, left), dev(p.env_r, np.ones(p.env_r.data.shape[2])), p.w_i, p.w_j, p.flux)
+    else:
+        e = p.env_l
+        plan = type(p)(p.kind, Environment(e.data * left, e.bra_idx, e.mpo_idx, e.ket_idx), p.env_r, p.w_i, p.w_j, p.flux, p.name).plan()
+    assert plan.launches() == 6
+    first, at = {}, 0
+    for q, m in p.env_l.ket_idx.sectors:
+        first[tuple(q)] = (at, m)
+        at += m
+    nr = dict((tuple(q), m) for q, m in p.env_r.ket_idx.sectors)
+    nc = len(p.env_l.ket_idx.sectors[0][0])
+    x = rng.standard_normal(plan.block_dim) + (1j * rng.standard_normal(plan.block_dim) if cplx else 0.0)
+    keys, offs = plan.blocks()
+    for key, a, b in zip(keys, offs, list(offs[1:]) + [plan.block_dim]):
+        o, m = first[_left_sector(key, nc)]
+        x[a:b].reshape(-1, m, nr[_right_sector(key, nc)])[:] *= back[o:o + m, None]
+    run = (lambda s: np.concatenate(_apply_complex(plan, x, s))) if cplx else (lambda s: _apply(plan, x, s))
+    got, want = run(_abi.SCHED_STACKED), run(_abi.SCHED_GROUPED)
+    assert np.isfinite(want).all() and np.linalg.norm(want) < 2.0 ** 40
+    assert rel_err(got, want) < 64 * 2.0 ** -53
