@@ -718,7 +718,8 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
 }
 
 // Builds the digit form of p; left out (dg null) where the constant operands
-// hold infinities or NaNs.
+// hold infinities or NaNs, and (cudaErrorMemoryAllocation) where there is no
+// memory for it.
 static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& err) {
     std::unique_ptr<F64Digits> d(new F64Digits);
     if (p.cplx) return digits_create_complex(C, p, std::move(d), err);
@@ -881,8 +882,12 @@ tk_status f64stack_create(const TcTables& C, std::unique_ptr<F64Stack, F64StackD
     // 508 / 497, D = 2048 1,599 / 1,580 (D = 1024, 17 thousand: 331 / 332).
     p->comb_threads = combine_narrow(C.jobs) || C.jobs.size() >= 16384 ? 128 : 256;
     if (f64stack_on_digits(C, p->cplx) && (e = digits_create(C, *p, err)) != cudaSuccess) {
-        if (err.empty()) err = std::string("digit operands: ") + cudaGetErrorString(e);
-        return e == cudaErrorMemoryAllocation ? TK_ERR_OOM : TK_ERR_CUDA;
+        // without memory for the digits (7/4 of the stacks' bytes) the FP64 kernels run
+        if (e != cudaErrorMemoryAllocation) {
+            if (err.empty()) err = std::string("digit operands: ") + cudaGetErrorString(e);
+            return TK_ERR_CUDA;
+        }
+        cudaGetLastError();
     }
     out = std::move(p);
     return TK_OK;

@@ -1,0 +1,44 @@
+"""The FP64 kernels behind the matvec on digits (csrc/stack_f64.cu): a plan without memory for the digits."""
+import numpy as np
+import pytest
+
+from helpers import rel_err
+from test_gpu_digit_matvec import _apply, _apply_complex, _complex_plan, _problem
+from tk_gb300 import TkError, _abi
+
+pytestmark = pytest.mark.gpu
+
+
+def _plan_without_its_last_allocation(make):
+    """The plan made while the last allocation of its creation, the digits', finds no memory."""
+    lib = _abi.load()
+    try:
+        n = 0
+        while True:  # allocations of a creation: the countdown that none reaches
+            n += 1
+            lib.tk_debug_fail_device_alloc(n)
+            try:
+                plan = make()
+            except TkError as e:
+                assert e.status == 3  # TK_ERR_OOM
+                continue
+            return plan, n
+    finally:
+        lib.tk_debug_fail_device_alloc(0)
+
+
+@pytest.mark.parametrize("name,D", [("hubbard", 700), ("cylinder", 257)])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_plan_without_memory_for_digits_runs_in_fp64(lib_built, name, D, cplx):
+    p = _problem(name, D, lambda e, side: e)
+    make = (lambda: _complex_plan(p, np.random.default_rng(3), False)) if cplx else p.plan
+    assert make().launches() == 6
+    plan, _ = _plan_without_its_last_allocation(make)
+    assert plan.launches() == 3
+    x = np.random.default_rng(2).standard_normal(plan.block_dim)
+    if cplx:
+        got, want = (np.concatenate(_apply_complex(plan, x * (1 + 0.5j), s)) for s in (_abi.SCHED_STACKED, _abi.SCHED_GROUPED))
+    else:
+        got, want = (_apply(plan, x, s) for s in (_abi.SCHED_STACKED, _abi.SCHED_GROUPED))
+    assert rel_err(got, want) < 1e-14
+    assert make().launches() == 6  # nothing is left armed
