@@ -316,9 +316,15 @@ __global__ void __launch_bounds__(256) stack_combine_f64_kernel(const TcCombJob*
 
 // The whole FP64 matvec in one launch, after a digit matvec that could not
 // stand: *redo set by an operand with infinities or NaNs, or by a bounded wait
-// that ran out.  One cluster of eight CTAs, so that its stages can wait for one
-// another; otherwise it ends at once (launched behind every digit matvec).
-constexpr int kRedoCtas = 8;
+// that ran out.  Otherwise it ends at once (launched behind every digit matvec).
+// Its CTAs, as many as the GPU holds, take each stage's work from a queue; a stage
+// starts when the one before it is done.  A CTA waits only with nothing in hand,
+// for work that running CTAs have taken, so not all CTAs need be on the GPU at
+// once.  (As one cluster of eight CTAs, with the cluster's barrier between the
+// stages, cylinder D = 1000 took 225 ms, as the FP64 launches 8.1.)
+struct RedoQueue {
+    unsigned next[3], done[2], left, late;
+};
 struct RedoArgs {
     const F64Piece *pieces1, *pieces3;
     const KSeg* segs;
@@ -328,37 +334,88 @@ struct RedoArgs {
     const int64_t *xsrc, *colbase, *yrow;
     const int32_t *xstride, *colstride;
     double *t1, *t2, *t1_im, *t2_im;
+    RedoQueue* queue;
     int n1, n3, njobs;
 };
-__device__ __forceinline__ void cluster_barrier() {
-    __threadfence();
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+constexpr int kRedoCtasPerSm = 2;         // 9.2 ms, with 4: 8.3, but each digit matvec 0.7 us more
+constexpr int kRedoJobs = 8;              // combine jobs taken at a time
+constexpr unsigned kRedoPolls = 1u << 24;  // without progress of the others, some ten seconds
 template <bool CPLX>
-__global__ void __cluster_dims__(kRedoCtas, 1, 1) __launch_bounds__(ST)
+__global__ void __launch_bounds__(ST, kRedoCtasPerSm)
     stack_redo_f64_kernel(const RedoArgs a, const double* __restrict__ x, const double* __restrict__ x_im,
                           double* __restrict__ y, double* __restrict__ y_im, int* redo) {
     __shared__ PieceTiles<CPLX> sm;
+    __shared__ int item;
     dep_launch();
     dep_wait();
     if (*(volatile int*)redo == 0) return;
-    for (int i = blockIdx.x; i < a.n1; i += kRedoCtas) {
+    RedoQueue& q = *a.queue;
+    const int tid = threadIdx.x;
+    // the next of n items of stage s, -1 when all are taken
+    auto take = [&](int s, int n) {
         __syncthreads();
+        if (tid == 0) item = (int)atomicAdd(&q.next[s], 1u);
+        __syncthreads();
+        return item < n ? item : -1;
+    };
+    auto finish = [&](int s) {
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) atomicAdd(&q.done[s], 1u);
+    };
+    // until all n items of stage s are done; false when the others stand still
+    auto wait = [&](int s, int n) {
+        __syncthreads();
+        if (tid == 0) {
+            unsigned seen = 0, last = 0, polls = 0;
+            while (true) {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&q.done[s]) : "memory");
+                if (seen >= (unsigned)n || ++polls > kRedoPolls) break;
+                if (seen != last) polls = 0;
+                last = seen;
+                __nanosleep(200);
+            }
+            item = seen >= (unsigned)n;
+            if (!item) atomicExch(&q.late, 1u);
+        }
+        __syncthreads();
+        return item != 0;
+    };
+    const int batches = (a.njobs + kRedoJobs - 1) / kRedoJobs;
+    for (int i; (i = take(0, a.n1)) >= 0; finish(0))
         stack_piece1<CPLX>(a.pieces1[i], sm, a.segs, a.lq, a.lq_im, x, x_im, a.xsrc, a.xstride, a.colbase, a.colstride,
                            a.t1, a.t1_im);
+    if (wait(0, a.n1)) {
+        for (int i; (i = take(1, batches)) >= 0; finish(1))
+            for (int j = i * kRedoJobs; j < min(a.njobs, (i + 1) * kRedoJobs); ++j) {
+                stack_combine_job(a.jobs[j], a.terms, a.coef, a.t1, a.t2);
+                if constexpr (CPLX) stack_combine_job(a.jobs[j], a.terms, a.coef, a.t1_im, a.t2_im);
+            }
+        if (wait(1, batches))
+            for (int i; (i = take(2, a.n3)) >= 0;)
+                stack_piece3<CPLX>(a.pieces3[i], sm, a.segs, a.t2, a.t2_im, a.rq, a.rq_im, a.yrow, y, y_im);
     }
-    cluster_barrier();
-    for (int i = blockIdx.x; i < a.njobs; i += kRedoCtas) {
-        stack_combine_job(a.jobs[i], a.terms, a.coef, a.t1, a.t2);
-        if constexpr (CPLX) stack_combine_job(a.jobs[i], a.terms, a.coef, a.t1_im, a.t2_im);
+    // the last CTA leaves the queue as it found it; if a wait ran out, nothing of y stands
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) item = atomicAdd(&q.left, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!item) return;
+    __threadfence();
+    if (*(volatile unsigned*)&q.late)
+        for (int i = 0; i < a.n3; ++i) {
+            const F64Piece t = a.pieces3[i];
+            for (int e = tid; e < t.m_valid * t.n_valid; e += ST) {
+                const int64_t o = a.yrow[t.out_off + e / t.n_valid] + t.n0 + e % t.n_valid;
+                y[o] = NAN;
+                if constexpr (CPLX) y_im[o] = NAN;
+            }
+        }
+    __syncthreads();
+    if (tid == 0) {
+        q = RedoQueue{};
+        *redo = 0;
     }
-    cluster_barrier();
-    for (int i = blockIdx.x; i < a.n3; i += kRedoCtas) {
-        __syncthreads();
-        stack_piece3<CPLX>(a.pieces3[i], sm, a.segs, a.t2, a.t2_im, a.rq, a.rq_im, a.yrow, y, y_im);
-    }
-    cluster_barrier();
-    if (blockIdx.x == 0 && threadIdx.x == 0) *redo = 0;
 }
 
 double seg_len(const std::vector<KSeg>& segs, int32_t s0, int32_t n) {
@@ -493,6 +550,7 @@ struct F64Digits {
     const int64_t* colbase = nullptr;
     const int32_t* colstride = nullptr;
     int* redo = nullptr;
+    RedoQueue* queue = nullptr;
     DigitMaps m1, m3;
     int npsi = 0, max_k = 0, psi_cols = 32, nrows = 0, sms = 0;
 };
@@ -681,7 +739,8 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
     digit_schedule(w3, d->sms, t3, b3);
     Blob blob;
     auto table = [&](const auto& v) { return blob.add(v.data(), sizeof(v[0]) * v.size()); };
-    const size_t o_redo = blob.add(&redo, sizeof(redo)), o_t1 = table(t1), o_t3 = table(t3), o_b1 = table(b1),
+    const RedoQueue queue{};
+    const size_t o_redo = blob.add(&redo, sizeof(redo)), o_q = blob.add(&queue, sizeof(queue)), o_t1 = table(t1), o_t3 = table(t3), o_b1 = table(b1),
                  o_b3 = table(b3), o_psi = table(psi), o_rows = table(trows), o_l = table(lrows), o_r = table(rrows),
                  o_c = table(rcols), o_lc = table(lcols), o_cb = table(colbase), o_cs = table(colstride);
     if ((e = digits_alloc(*d, blob, {2 * C.lq_rows, 4 * C.rq_rows, 2 * C.t2q_rows, 4 * C.xq_rows}, nk, &kx)) != cudaSuccess)
@@ -696,6 +755,7 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
     d->colbase = reinterpret_cast<const int64_t*>(m + o_cb);
     d->colstride = reinterpret_cast<const int32_t*>(m + o_cs);
     d->redo = reinterpret_cast<int*>(m + o_redo);
+    d->queue = reinterpret_cast<RedoQueue*>(m + o_q);
     if (!digit_maps(d->m1, d->l, d->x, err) || !digit_maps(d->m3, d->t2, d->r, err)) return cudaErrorInvalidValue;
     // (L's rows without scales first, for their exponents)
     if ((e = cudaMemset(kx, 0, sizeof(int32_t) * (size_t)nk)) != cudaSuccess ||
@@ -779,7 +839,8 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
     // the tables first (one copy), then what the device writes
     Blob blob;
     auto table = [&](const auto& v) { return blob.add(v.data(), sizeof(v[0]) * v.size()); };
-    const size_t o_redo = blob.add(&redo, sizeof(redo)), o_t1 = table(t1), o_t3 = table(t3), o_b1 = table(b1),
+    const RedoQueue queue{};
+    const size_t o_redo = blob.add(&redo, sizeof(redo)), o_q = blob.add(&queue, sizeof(queue)), o_t1 = table(t1), o_t3 = table(t3), o_b1 = table(b1),
                  o_b3 = table(b3), o_psi = table(psi), o_rows = table(trows), o_l = table(lrows), o_r = table(rrows),
                  o_c = table(rcols), o_lc = table(lcols);
     int32_t* kxd = nullptr;
@@ -792,6 +853,7 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
     d->psi = reinterpret_cast<const DigitPsi*>(m + o_psi);
     d->rows = reinterpret_cast<const DigitRows*>(m + o_rows);
     d->redo = reinterpret_cast<int*>(m + o_redo);
+    d->queue = reinterpret_cast<RedoQueue*>(m + o_q);
     if (!digit_maps(d->m1, d->l, d->x, err) || !digit_maps(d->m3, d->t2, d->r, err)) return cudaErrorInvalidValue;
     // (L's rows without scales first, for their exponents)
     if ((e = cudaMemset(kxd, 0, sizeof(int32_t) * (size_t)nk)) != cudaSuccess ||
@@ -904,7 +966,15 @@ static cudaError_t combine_stage(const F64Stack& p, cudaStream_t s) {
 static RedoArgs redo_args(const F64Stack& p) {
     return RedoArgs{p.pieces1.p, p.pieces3.p, p.segs.p,  p.jobs.p,    p.terms.p,     p.coef.p, p.lq.p, p.rq.p, p.lq_im.p,
                     p.rq_im.p,   p.xsrc.p,    p.colbase.p, p.yrow.p,  p.xstride.p, p.colstride.p, p.t1.p,   p.t2.p, p.t1_im.p,
-                    p.t2_im.p,   p.n1,        p.n3,      p.njobs};
+                    p.t2_im.p,   p.dg->queue, p.n1,      p.n3,       p.njobs};
+}
+
+// The stand-by: at most kRedoCtasPerSm CTAs an SM, fewer where a stage has not so much work.
+template <bool CPLX>
+static cudaError_t launch_redo(const F64Stack& p, const double* x, const double* x_im, double* y, double* y_im,
+                               cudaStream_t s) {
+    const int ctas = std::min(kRedoCtasPerSm * p.dg->sms, std::max({p.n1, p.n3, 1}));
+    return launch_dependent(stack_redo_f64_kernel<CPLX>, ctas, ST, 0, s, redo_args(p), x, x_im, y, y_im, p.dg->redo);
 }
 
 // One stage of the digit matvec.
@@ -926,8 +996,7 @@ static cudaError_t digits_stage(F64Stack& p, const double* x, double* y, cudaStr
     o.out = y;
     o.rowtab = p.yrow.p;
     if ((e = launch_digit_gemm(1, d.tiles3, d.begin3, d.sms, d.m3, d.t2.ex, d.r.ex, o, d.redo, s)) != cudaSuccess) return e;
-    return launch_dependent(stack_redo_f64_kernel<false>, kRedoCtas, ST, 0, s, redo_args(p), x, nullptr, y, nullptr,
-                            d.redo);
+    return launch_redo<false>(p, x, nullptr, y, nullptr, s);
 }
 
 // The digit matvec on planar vectors.
@@ -949,7 +1018,7 @@ static cudaError_t digits_apply_complex(F64Stack& p, const double* xr, const dou
     o.rowtab = p.yrow.p;
     if (e == cudaSuccess) e = launch_digit_gemm(1, d.tiles3, d.begin3, d.sms, d.m3, d.t2.ex, d.r.ex, o, d.redo, s);
     if (e != cudaSuccess) return e;
-    return launch_dependent(stack_redo_f64_kernel<true>, kRedoCtas, ST, 0, s, redo_args(p), xr, xi, yr, yi, d.redo);
+    return launch_redo<true>(p, xr, xi, yr, yi, s);
 }
 
 cudaError_t f64stack_stage(F64Stack& p, const double* x, double* y, cudaStream_t s, int stage) {

@@ -1,10 +1,11 @@
-"""The FP64 kernels behind the matvec on digits (csrc/stack_f64.cu): a plan without memory for the digits."""
+"""The FP64 kernels behind the matvec on digits (csrc/stack_f64.cu): a plan without memory for the digits,
+and the time of a vector that digits cannot hold."""
 import numpy as np
 import pytest
 
 from helpers import rel_err
 from test_gpu_digit_matvec import _apply, _apply_complex, _complex_plan, _problem
-from tk_gb300 import TkError, _abi
+from tk_gb300 import Environment, TkError, _abi
 
 pytestmark = pytest.mark.gpu
 
@@ -42,3 +43,36 @@ def test_plan_without_memory_for_digits_runs_in_fp64(lib_built, name, D, cplx):
         got, want = (_apply(plan, x, s) for s in (_abi.SCHED_STACKED, _abi.SCHED_GROUPED))
     assert rel_err(got, want) < 1e-14
     assert make().launches() == 6  # nothing is left armed
+
+
+def _time(plan, x):
+    import torch
+
+    xd = torch.from_numpy(x).cuda()
+    yd = torch.empty_like(xd)
+    best = float("inf")
+    for _ in range(6):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        plan.apply(xd, yd, stream=torch.cuda.current_stream().cuda_stream)
+        b.record()
+        torch.cuda.synchronize()
+        best = min(best, a.elapsed_time(b))
+    return best
+
+
+def test_nonfinite_vector_costs_about_an_fp64_matvec(lib_built):
+    """Against a plan that keeps the FP64 kernels (its environment holds an infinity): the same work on
+    the same pipe, which the whole GPU has to share in."""
+    p = _problem("cylinder", 1000, lambda e, side: e)
+    plan = p.plan()
+    assert plan.launches() == 6
+    e = p.env_r.data.copy()
+    e[tuple(np.argwhere(e != 0.0)[7])] = np.inf
+    q = type(p)(p.kind, p.env_l, Environment(e, p.env_r.bra_idx, p.env_r.mpo_idx, p.env_r.ket_idx), p.w_i, p.w_j, p.flux, p.name)
+    fp64 = q.plan()
+    assert fp64.launches() == 3
+    x = np.random.default_rng(1).standard_normal(plan.block_dim)
+    bad = x.copy()
+    bad[plan.block_dim // 2] = np.nan
+    assert _time(plan, bad) < 2.0 * _time(fp64, x)
