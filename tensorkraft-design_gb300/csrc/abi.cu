@@ -13,6 +13,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -43,6 +44,23 @@ tk_status ctx_stream(tk_ctx* ctx, void** out) {
     }
     *out = ctx->stream;
     return TK_OK;
+}
+
+// The live contexts, for release_scratch.
+static std::mutex g_contexts_mutex;
+static std::vector<tk_ctx*> g_contexts;
+
+void release_scratch() {
+    std::lock_guard<std::mutex> all(g_contexts_mutex);
+    for (tk_ctx* ctx : g_contexts) {
+        {
+            std::lock_guard<std::mutex> lock(ctx->gemm_mutex);
+            for (auto& b : ctx->gemm_free) cudaFree(b.first);
+            ctx->gemm_free.clear();
+        }
+        std::lock_guard<std::mutex> lock(ctx->pool_mutex);
+        if (ctx->scratch_pool && cudaMemPoolTrimTo((cudaMemPool_t)ctx->scratch_pool, 0) != cudaSuccess) cudaGetLastError();
+    }
 }
 
 tk_status ctx_dev_scratch(tk_ctx* ctx, size_t bytes, void** out) {
@@ -148,12 +166,24 @@ tk_status tk_ctx_create(int32_t device, tk_ctx** out) {
         return TK_ERR_OOM;
     }
     c->device = device;
+    try {
+        std::lock_guard<std::mutex> all(g_contexts_mutex);
+        g_contexts.push_back(c);
+    } catch (const std::bad_alloc&) {
+        delete c;
+        set_error("tk_ctx_create: host allocation failed");
+        return TK_ERR_OOM;
+    }
     *out = c;
     return TK_OK;
 }
 
 void tk_ctx_destroy(tk_ctx* ctx) {
     if (!ctx) return;
+    {
+        std::lock_guard<std::mutex> all(g_contexts_mutex);
+        g_contexts.erase(std::remove(g_contexts.begin(), g_contexts.end(), ctx), g_contexts.end());
+    }
     ctx_release_solver(ctx);
     {
         DeviceGuard g(ctx->device);

@@ -78,10 +78,12 @@ struct Scratch {
     } while (0)
 
 
-// A device buffer for one tk_gemm_f64 call.  The call waits for its stream
-// before it gives the buffer back, so any thread's next call on the context
-// may take it; at most kGemmKeep bytes stay with the context.
-constexpr size_t kGemmKeep = (size_t)1 << 30;
+// A device buffer for one tk_gemm_f64 call; null where there is no memory (the
+// caller takes another path).  The call waits for its stream before it gives the
+// buffer back, so any thread's next call on the context may take it; at most
+// kGemmKeep bytes stay with the context (the digits of 4096^3), until memory runs
+// out (release_scratch).
+constexpr size_t kGemmKeep = (size_t)512 << 20;
 struct GemmBuffer {
     tk_ctx* ctx;
     void* p = nullptr;
@@ -99,8 +101,8 @@ struct GemmBuffer {
                 return;
             }
         }
-        if (cudaMalloc(&p, bytes) != cudaSuccess) {
-            cudaGetLastError();  // the caller takes another path
+        if (dev_malloc(&p, bytes) != cudaSuccess) {
+            cudaGetLastError();
             p = nullptr;
         }
         n = bytes;
@@ -129,6 +131,8 @@ struct GemmBuffer {
         }
         cudaFree(p);
     }
+    GemmBuffer(const GemmBuffer&) = delete;
+    GemmBuffer& operator=(const GemmBuffer&) = delete;
 };
 
 // The dense product on the fp16 tensor cores (digit_gemm.cu).  *done is left

@@ -13,20 +13,29 @@
 
 namespace tk {
 
+// Gives back the device memory that contexts keep between calls and no call uses.
+void release_scratch();
+
 // Device allocations of a plan.  With a countdown armed by
 // tk_debug_fail_device_alloc, the countdown-th allocation fails as if the
 // device were out of memory (test hook for the TK_ERR_OOM paths); a negative one
 // fills every allocation with a byte.
 extern std::atomic<int> g_fail_device_alloc;
 inline cudaError_t dev_malloc(void** p, size_t bytes) {
+    *p = nullptr;
     int c = g_fail_device_alloc.load(std::memory_order_relaxed);
     while (c > 0 && !g_fail_device_alloc.compare_exchange_weak(c, c - 1)) {
     }
     if (c == 1) {
-        *p = nullptr;
+        release_scratch();
         return cudaErrorMemoryAllocation;
     }
-    const cudaError_t e = cudaMalloc(p, bytes);
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {  // once more without what the contexts keep
+        cudaGetLastError();
+        release_scratch();
+        e = cudaMalloc(p, bytes);
+    }
     return e == cudaSuccess && c < 0 ? cudaMemset(*p, -c, bytes) : e;
 }
 
