@@ -55,6 +55,9 @@ def test_product_without_memory_for_digits_runs_in_fp64(lib_built):
     assert not np.array_equal(_run(A, B, "tk_gemm_f64"), want)  # on digits
     try:
         _refuse(1)
+        with pytest.raises(TkError):  # the context's idle buffers go
+            small_problem("hubbard", 48).plan()
+        _refuse(1)
         got = _run(A, B, "tk_gemm_f64")
     finally:
         _refuse(0)
