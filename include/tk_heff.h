@@ -396,6 +396,7 @@ tk_status tk_expm_krylov(tk_heff2_plan* plan, const tk_expm_cfg* cfg, double alp
  * LinAlgBackend::gemm (tk-linalg/src/traits.rs:114-121) on device memory:
  * C = alpha*op(A)*op(B) + beta*C with element strides as in MatRef/MatMut
  * (tk-core/src/matview.rs:12-33).  `is_conjugated` is a no-op for f64.
+ * After an error in the CUDA calls or kernels C's contents are unspecified.
  */
 typedef struct {
     const double* data;

@@ -756,7 +756,10 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
     d->colstride = reinterpret_cast<const int32_t*>(m + o_cs);
     d->redo = reinterpret_cast<int*>(m + o_redo);
     d->queue = reinterpret_cast<RedoQueue*>(m + o_q);
-    if (!digit_maps(d->m1, d->l, d->x, err) || !digit_maps(d->m3, d->t2, d->r, err)) return cudaErrorInvalidValue;
+    if (!digit_maps(d->m1, d->l, d->x, err) || !digit_maps(d->m3, d->t2, d->r, err)) {
+        err.clear();
+        return cudaSuccess;
+    }
     // (L's rows without scales first, for their exponents)
     if ((e = cudaMemset(kx, 0, sizeof(int32_t) * (size_t)nk)) != cudaSuccess ||
         (e = launch_digit_rows_complex(reinterpret_cast<const DigitRowsC*>(m + o_l), (int)lrows.size(), p.lq.p, p.lq_im.p,
@@ -778,7 +781,7 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
 }
 
 // Builds the digit form of p; left out (dg null) where the constant operands
-// hold infinities or NaNs, and (cudaErrorMemoryAllocation) where there is no
+// hold infinities or NaNs, without tensor maps, and (cudaErrorMemoryAllocation) where there is no
 // memory for it.
 static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& err) {
     std::unique_ptr<F64Digits> d(new F64Digits);
@@ -854,7 +857,10 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
     d->rows = reinterpret_cast<const DigitRows*>(m + o_rows);
     d->redo = reinterpret_cast<int*>(m + o_redo);
     d->queue = reinterpret_cast<RedoQueue*>(m + o_q);
-    if (!digit_maps(d->m1, d->l, d->x, err) || !digit_maps(d->m3, d->t2, d->r, err)) return cudaErrorInvalidValue;
+    if (!digit_maps(d->m1, d->l, d->x, err) || !digit_maps(d->m3, d->t2, d->r, err)) {
+        err.clear();
+        return cudaSuccess;
+    }
     // (L's rows without scales first, for their exponents)
     if ((e = cudaMemset(kxd, 0, sizeof(int32_t) * (size_t)nk)) != cudaSuccess ||
         (e = launch_digit_rows(reinterpret_cast<const DigitRows*>(m + o_l), (int)lrows.size(), p.lq.p, kxd, -1, d->l,
