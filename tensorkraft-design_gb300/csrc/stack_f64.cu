@@ -633,6 +633,10 @@ static cudaError_t digits_alloc(F64Digits& d, const Blob& blob, const int64_t (&
     }
     const size_t k = take(sizeof(int32_t) * (size_t)std::max(nk, 1));
     cudaError_t e;
+    // at most half of what is free: the solvers' vectors and other plans come later
+    size_t free_bytes = 0, all = 0;
+    if ((e = cudaMemGetInfo(&free_bytes, &all)) != cudaSuccess) return e;
+    if (total > free_bytes / 2) return cudaErrorMemoryAllocation;
     if ((e = d.mem.alloc(total)) != cudaSuccess ||
         (e = cudaMemcpy(d.mem.p, host.data(), host.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
         return e;
