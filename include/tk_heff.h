@@ -283,7 +283,8 @@ tk_status tk_heff2_autotune(tk_heff2_plan* plan, int32_t reps, int32_t use_cache
  * (L x psi GEMMs), stage 2 (W_i W_j combine) and stage 3 (x R GEMMs) to
  * ms[0..2], the algorithmic flops of each stage to flops[0..2] and its
  * compulsory global-memory bytes (operands read once, results written once,
- * in the precision the plan runs) to bytes[0..2]; flops/bytes may be NULL.
+ * in the precision the plan runs; large FP64 plans also write and read the
+ * digits of psi and of T2) to bytes[0..2]; flops/bytes may be NULL.
  * In split precision the W_i W_j combine of narrow stage-3 stacks runs inside
  * the stage-3 kernel; stage 2 then covers only the wide stacks' combine (0 ms
  * and 0 bytes when there are none) and stage 3 the rest, T1 reads included. */

@@ -961,6 +961,15 @@ tk_status f64stack_create(const TcTables& C, std::unique_ptr<F64Stack, F64StackD
         }
         cudaGetLastError();
     }
+    if (p->dg) {  // operands of two bytes a digit; those of psi and T2 written and read on top
+        double psi = 0.0;
+        for (const TcSplitJob& j : C.split)
+            if (j.a0 == 0 && j.b0 == 0) psi += (double)j.rows * j.cols;
+        constexpr double d = 2.0 * kDigits;
+        p->bytes[0] = d * (stack_elems(p1, true) + 2.0 * psi) + 8.0 * (double)C.t1_total;
+        p->bytes[1] += (8.0 + d) * t2_elems;
+        p->bytes[2] = d * (t2_elems + stack_elems(p3, false));
+    }
     out = std::move(p);
     return TK_OK;
 }

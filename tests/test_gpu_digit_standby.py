@@ -45,6 +45,22 @@ def test_plan_without_memory_for_digits_runs_in_fp64(lib_built, name, D, cplx):
     assert make().launches() == 6  # nothing is left armed
 
 
+def test_profile_counts_the_bytes_of_digits(lib_built):
+    """Against the same plan without digits: fourteen bytes an operand element for eight."""
+    import torch
+
+    p = _problem("cylinder", 257, lambda e, side: e)
+    plan = p.plan()
+    fp64, _ = _plan_without_its_last_allocation(p.plan)
+    x = torch.from_numpy(np.random.default_rng(2).standard_normal(plan.block_dim)).cuda()
+    y = torch.empty_like(x)
+    (_, fl, by), (_, fl64, by64) = plan.profile(x, y, reps=1), fp64.profile(x, y, reps=1)
+    vec = 8.0 * plan.block_dim
+    assert list(fl) == list(fl64)
+    assert by[2] - vec == 14.0 / 8.0 * (by64[2] - vec)
+    assert by[0] > by64[0] + 28.0 * plan.block_dim / 2 and by[1] > by64[1]
+
+
 def _time(plan, x):
     import torch
 
