@@ -141,3 +141,45 @@ def test_uneven_columns_of_l_cost_no_digits(lib_built, name, D, cplx, kind):
     got, want = run(_abi.SCHED_STACKED), run(_abi.SCHED_GROUPED)
     assert np.isfinite(want).all() and np.linalg.norm(want) < 2.0 ** 40
     assert rel_err(got, want) < 64 * 2.0 ** -53
+
+
+# a converged state in mixed canonical form: identity channels in both environments, amplitudes that fall
+# from 1 to 1e-8 along both bonds inside every sector
+@pytest.mark.parametrize("name,D", [("heisenberg", 401), ("hubbard", 700), ("cylinder", 257)])
+def test_rows_of_a_graded_state_beside_identity_channels(lib_built, name, D):
+    """Digits hold rows and columns to 2^-58 of their largest element, so the promise is by norm, as for the
+    eigensolvers: the result to a few 2^-53, and each of its rows to the bound of an FP64 chain (2 K 2^-53)
+    on the row's largest sum of magnitudes, K the terms of an output."""
+    def change(e, side):
+        d = e.data.copy()
+        w = 0 if side == 0 else d.shape[1] - 1
+        d[:, w, :] = np.eye(d.shape[0])
+        return Environment(d, e.bra_idx, e.mpo_idx, e.ket_idx)
+
+    p = _problem(name, D, change)
+    plan = p.plan()
+    assert plan.launches() == 6
+    fall = [{tuple(q): np.logspace(0, -8, n) for q, n in e.ket_idx.sectors} for e in (p.env_l, p.env_r)]
+    nc = len(p.env_l.ket_idx.sectors[0][0])
+    x = np.random.default_rng(D).standard_normal(plan.block_dim)
+    keys, offs = plan.blocks()
+    blocks = [(a, b, _left_sector(k, nc), _right_sector(k, nc)) for k, a, b in zip(keys, offs, list(offs[1:]) + [plan.block_dim])]
+    for a, b, ql, qr in blocks:
+        x[a:b].reshape(-1, len(fall[0][ql]), len(fall[1][qr]))[:] *= fall[0][ql][:, None] * fall[1][qr]
+    got, want = _apply(plan, x, _abi.SCHED_STACKED), _apply(plan, x, _abi.SCHED_GROUPED)
+    assert rel_err(got, want) < 64 * 2.0 ** -53
+
+    def absolute(t):
+        out = type(t).__new__(type(t))
+        out.__dict__.update(t.__dict__)
+        out.blocks = {k: np.abs(v) for k, v in t.blocks.items()}
+        return out
+
+    q = type(p)(p.kind, *(Environment(np.abs(e.data), e.bra_idx, e.mpo_idx, e.ket_idx) for e in (p.env_l, p.env_r)),
+                absolute(p.w_i), absolute(p.w_j), p.flux, p.name)
+    mags = _apply(q.plan(), np.abs(x), _abi.SCHED_GROUPED)
+    K = p.env_l.data.shape[1] * (p.env_l.data.shape[2] + p.env_r.data.shape[2])
+    for a, b, ql, qr in blocks:
+        n = len(fall[1][qr])
+        err, row = np.abs(got - want)[a:b].reshape(-1, n).max(1), mags[a:b].reshape(-1, n).max(1)
+        assert (err <= 2 * K * 2.0 ** -53 * row).all()
