@@ -897,13 +897,18 @@ __global__ void __launch_bounds__(PT) digit_psi_kernel(const DigitPsi* __restric
 }
 
 constexpr int BT = 256;
-// Whether x lies on the grid of digits 0 .. 3 of a row with exponent ex: its lowest bit at
-// 2^(ex - 1055) or above.
+// Whether x lies on the grid of digits 0 .. 3 of a row with exponent ex: its lowest
+// bit at 2^(ex - 1055) or above.
 __device__ __forceinline__ bool in_four_digits(double x, int ex) {
     const uint64_t b = (uint64_t)__double_as_longlong(x);
     const int e = (int)(b >> 52) & 0x7FF;
     const uint64_t m = (b & 0xFFFFFFFFFFFFFull) | (e ? 1ull << 52 : 0);
     return m == 0 || max(e, 1) + __ffsll((long long)m) - 1 >= ex + 20;
+}
+// Whether x may have bits below its row's grid.
+__device__ __forceinline__ bool below_grid(double x, int ex) {
+    const uint32_t hi = abs_hi(x);
+    return (int)(hi >> 20) < ex - 4 && (hi | (uint32_t)__double2loint(x)) != 0;
 }
 // |x| 2^-e in fp32, rounded down (e by its biased form ex: |x| < 2^(ex - 1022))
 __device__ __forceinline__ float below_one(double x, int ex) {
@@ -917,9 +922,10 @@ constexpr int kGate = kDigitSamples;
 __host__ __device__ __forceinline__ int gate_k(int s, int K) { return K > kGate ? (int)((int64_t)s * K / kGate) : s; }
 // The two operands of a dense product, 32 rows x 64 k a CTA (the rows of A,
 // then those of B).  PASS 0 leaves every row's largest high word in top (zeroed
-// before), PASS 1 writes the exponents, the digits and the gate's samples, and sets
-// *wide where an element is not on the grid of four digits; lanes walk along the
-// shorter stride.
+// before), PASS 1 writes the exponents, the digits and the gate's samples, and finds
+// whether an element is not on the grid of four digits (*wide) and, for a K of one
+// chunk, the most elements of a row that may be off its grid (*inexact, zeroed before);
+// lanes walk along the shorter stride.
 template <int PASS>
 __global__ void __launch_bounds__(BT) digit_matrix_kernel(const DigitMatrix A, const DigitMatrix B, int K, int* wide,
                                                           int* redo) {
@@ -947,10 +953,9 @@ __global__ void __launch_bounds__(BT) digit_matrix_kernel(const DigitMatrix A, c
         }
     }
     __syncthreads();
-    bool four = true;
-    // which samples this lane's two k are (-1: none), and whether *wide still needs a look
-    int at[2] = {-1, -1};
-    bool look = false;
+    uint32_t off = 0;  // elements off the grid, a byte for each of the warp's four rows
+    bool four = true, look = false;  // look: whether *wide is still open
+    int at[2] = {-1, -1};            // which samples this lane's two k are (-1: none)
     if (PASS == 1) {
         look = *(volatile int*)wide == 0;
 #pragma unroll
@@ -969,20 +974,32 @@ __global__ void __launch_bounds__(BT) digit_matrix_kernel(const DigitMatrix A, c
             digits2(u, v, sex[r], d);
             put_digits(m.out, r0 + r + (int64_t)blockIdx.y * m.rows, 2 * lane, d);
             if (look) four = four && in_four_digits(u, sex[r]) && in_four_digits(v, sex[r]);
+            if (K <= kTcBK) off |= (uint32_t)(below_grid(u, sex[r]) + below_grid(v, sex[r])) << (r - w);
             if (at[0] >= 0) m.sample[(int64_t)at[0] * m.rows + r0 + r] = below_one(u, sex[r]);
             if (at[1] >= 0) m.sample[(int64_t)at[1] * m.rows + r0 + r] = below_one(v, sex[r]);
         }
     }
-    if (PASS == 1 && __syncthreads_or(!four) && tid == 0) atomicExch(wide, 1);
+    if (PASS == 1) {
+        if (__syncthreads_or(!four) && tid == 0) atomicExch(wide, 1);
+        if (K <= kTcBK) {
+            static_assert(32 / (BT / 32) == 4 && BT / 32 == 8, "rows w, w + 8, w + 16, w + 24: bytes 0 .. 3");
+            off = __reduce_add_sync(0xffffffffu, off);
+            if (lane == 0)
+                atomicMax(m.inexact, (int)max(max(off & 255u, (off >> 8) & 255u), max((off >> 16) & 255u, off >> 24)));
+        }
+    }
 }
 
 // Whether the digits hold a dense product as exactly as an FP64 chain of K steps
-// does, output by output.  They leave out at most half a unit of each element's grid,
-// 2^(e - 58), and the products of digits i + j > 6, 6.03 x 2^-60 2^(ea + eb) a k:
-//   |error| <= K 2^-56.1 2^(ea + eb),
-// the chain's bound is K 2^-53 sum |a_k b_k|.  So an output with
-//   sum |a_k b_k| >= 2^-3 2^(ea + eb)
-// has the smaller bound on digits.  The sum over kGate of the k, evenly spaced, is a
+// does, output by output.  They leave out half a unit, 2^(e - 58), of an element that
+// is not on its row's grid (shares f_a and f_b of the two rows' k) and the products of
+// digits i + j > 6, 6.03 x 2^-60 2^(ea + eb) a k:
+//   |error| <= (2^-58 (f_a + f_b) + 0.052 x 2^-53) K 2^(ea + eb)
+// with the roundings of the sums, where the chain's bound is K 2^-53 sum |a_k b_k|.  So
+// an output with
+//   sum |a_k b_k| >= ((f_a + f_b) / 32 + 0.052) 2^(ea + eb)
+// has the smaller bound on digits (f = 1 where K is longer than a chunk: there the sums
+// are far above it).  The sum over kGate of the k, evenly spaced, is a
 // lower bound of it and enough for operands without structure (N(0, 1): about 0.6 at
 // 64 k, the least of a million outputs 0.27); where one output falls below, *redo
 // sends the product to the FP64 pipe.  Rows of zeros, and operands whose elements all
@@ -1012,11 +1029,12 @@ __global__ void __launch_bounds__(BT) digit_gate_kernel(const DigitMatrix A, con
             for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
     }
     bool bad = false;
+    const float least = (K <= kTcBK ? (float)(*A.inexact + *B.inexact) / (32.0f * (float)K) : 0.0625f) + 0.052f;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            bad |= m0 + ty + i < A.rows && n0 + tx + j < B.rows && acc[i][j] < 0.125f && A.top[m0 + ty + i] != 0 &&
+            bad |= m0 + ty + i < A.rows && n0 + tx + j < B.rows && acc[i][j] < least && A.top[m0 + ty + i] != 0 &&
                    B.top[n0 + tx + j] != 0;
     if (__syncthreads_or(bad) && tid == 0) atomicExch(redo, kDigitValue);
 }

@@ -124,14 +124,15 @@ cudaError_t launch_digit_rows_complex(const DigitRowsC* jobs, int n_jobs, const 
                                       cudaStream_t s);
 // Digits of both operands of a dense product (*redo is set where an output might be
 // less exact than by an FP64 chain): row r, k of K at x[r * rs + k * ks], into stacks
-// whose chunks are `rows` rows apart.  `top` and *wide start at zero.
+// whose chunks are `rows` rows apart.  `top`, *inexact and *wide start at zero.
 struct DigitMatrix {
     const double* x;
     int64_t rs, ks;
     int rows;
     DigitStack out;
     uint32_t* top;  // scratch: a value a row,
-    float* sample;  // 64 values a row
+    int* inexact;   // one value,
+    float* sample;  // kDigitSamples values a row
 };
 constexpr int kDigitSamples = 64;
 cudaError_t launch_digit_matrices(const DigitMatrix& a, const DigitMatrix& b, int K, int* wide, int* redo, cudaStream_t s);

@@ -142,8 +142,8 @@ tk_status gemm_digits(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* 
                       cudaStream_t s, bool* done) {
     *done = false;
     const int64_t M = a->rows, N = b->cols, K = a->cols, kch = (K + kTcBK - 1) / kTcBK;
-    DigitMatrix A{a->data, a->row_stride, a->col_stride, (int)M, {}, nullptr, nullptr};
-    DigitMatrix B{b->data, b->col_stride, b->row_stride, (int)N, {}, nullptr, nullptr};
+    DigitMatrix A{a->data, a->row_stride, a->col_stride, (int)M, {}, nullptr, nullptr, nullptr};
+    DigitMatrix B{b->data, b->col_stride, b->row_stride, (int)N, {}, nullptr, nullptr, nullptr};
     A.out.rows = M * kch;
     B.out.rows = N * kch;
     size_t total = 256;  // the flags
@@ -166,6 +166,8 @@ tk_status gemm_digits(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* 
     B.out.ex = reinterpret_cast<int32_t*>(p + eb);
     A.top = reinterpret_cast<uint32_t*>(p + ta);
     B.top = reinterpret_cast<uint32_t*>(p + tb);
+    A.inexact = redo + 2;
+    B.inexact = redo + 3;
     A.sample = reinterpret_cast<float*>(p + sa);
     B.sample = reinterpret_cast<float*>(p + sb);
     DigitMaps maps;

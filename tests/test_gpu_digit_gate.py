@@ -76,7 +76,7 @@ def test_uneven_operands_take_the_fp64_kernel(lib_built, what, make, arg):
     assert np.array_equal(got, _run(A, B, "tk_gemm_f64_noalloc"))
 
 
-@pytest.mark.parametrize("M,N,K", [(512, 512, 512), (300, 700, 1000), (600, 1000, 64), (1030, 1025, 19), (2050, 1090, 65)])
+@pytest.mark.parametrize("M,N,K", [(512, 512, 512), (300, 700, 1000), (600, 1000, 64), (1030, 1025, 19), (2050, 1090, 65), (2048, 2048, 17)])
 @pytest.mark.parametrize("kind", ["normal", "uniform", "integers"])
 def test_even_operands_stay_on_digits(lib_built, M, N, K, kind):
     """Also with rows and columns of zeros, whose products are exact on any grid."""

@@ -25,11 +25,22 @@ def _refuse(n):
     _abi.load().tk_debug_fail_device_alloc(n)
 
 
+def _refused_plan():
+    """A plan whose first allocation finds no memory: the contexts' idle buffers are released."""
+    try:
+        _refuse(1)
+        with pytest.raises(TkError):
+            small_problem("hubbard", 48).plan()
+    finally:
+        _refuse(0)
+
+
 def test_kept_memory_is_bounded_and_given_back(lib_built):
     rng = np.random.default_rng(1)
     context(0)
     A, B = rng.standard_normal((300, 300)), rng.standard_normal((300, 300))
     _run(A, B, "tk_gemm_f64")  # module and pool are there
+    _refused_plan()  # (what earlier tests left with the context goes)
     before = _used()
     big = rng.standard_normal((5000, 5000))  # 708 MB of digits
     _run(big, big, "tk_gemm_f64")
@@ -38,12 +49,7 @@ def test_kept_memory_is_bounded_and_given_back(lib_built):
     _run(mid, mid, "tk_gemm_f64")
     kept = _used()
     assert kept - before >= 100 * MiB  # (else there is nothing to give back)
-    try:
-        _refuse(1)
-        with pytest.raises(TkError):
-            small_problem("hubbard", 48).plan()
-    finally:
-        _refuse(0)
+    _refused_plan()
     assert _used() <= kept - 100 * MiB
     assert np.isfinite(_run(mid, mid, "tk_gemm_f64")).all()
 
@@ -53,10 +59,8 @@ def test_product_without_memory_for_digits_runs_in_fp64(lib_built):
     A, B = rng.standard_normal((512, 300)), rng.standard_normal((300, 640))
     want = _run(A, B, "tk_gemm_f64_noalloc")
     assert not np.array_equal(_run(A, B, "tk_gemm_f64"), want)  # on digits
+    _refused_plan()
     try:
-        _refuse(1)
-        with pytest.raises(TkError):  # the context's idle buffers go
-            small_problem("hubbard", 48).plan()
         _refuse(1)
         got = _run(A, B, "tk_gemm_f64")
     finally:
