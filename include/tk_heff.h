@@ -194,11 +194,14 @@ tk_status tk_heff2_set_precision(tk_heff2_plan* plan, int32_t precision);
  * nearly every FP64 FMA issued is one of the product's own (complex plans:
  * the same pieces with complex FMAs on planar operands; the default of
  * complex plans too).  Large plans, real and complex, run these stacks on
- * the fp16 tensor cores: every operand row as seven integer digits on one
- * grid (to 2^-58 of its largest element), multiplied exactly and each sum
- * rounded once, with the FP64 kernels standing by for vectors with
- * infinities or NaNs.  Every schedule computes the same sums to FP64
- * precision. */
+ * the fp16 tensor cores where there is memory for it: every operand row as
+ * seven integer digits on one grid (to 2^-58 of its largest element),
+ * multiplied exactly and each sum rounded once, with the FP64 kernels
+ * standing by for vectors with infinities or NaNs.  Every schedule computes
+ * the same sums.  On digits the result has FP64 precision by norm, as
+ * eigensolvers need it; an output that is small beside its row's others can
+ * have fewer right digits than an FP64 chain gives.  GROUPED and PER_BLOCK
+ * sum every output in FP64 multiply-adds. */
 #define TK_SCHED_GROUPED   0
 #define TK_SCHED_PER_BLOCK 1
 #define TK_SCHED_STACKED   2
@@ -420,7 +423,7 @@ tk_status tk_gemm_f64(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* 
  * loops): same arguments and result, always by the FP64 kernel, whose task is
  * passed by value, so nothing is allocated or freed and the call does not
  * synchronise (stream-ordered on `stream`).  Outputs of at most 65 520 64x64
- * squares; larger calls return TK_ERR_INVALID_ARG.
+ * squares (a limit of the interface); larger calls return TK_ERR_INVALID_ARG.
  */
 tk_status tk_gemm_f64_noalloc(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* b,
                               double beta, tk_mat_mut* c, void* stream);

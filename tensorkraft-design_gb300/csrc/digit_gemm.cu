@@ -10,14 +10,18 @@
 // with a leading digit, at most 2^16 each, and s - 1 of at most 2^14; level 0
 // one of 2^18), so fp32 accumulation is exact; after 64 k the seven sums are
 // added to an integer sum per output, and the result is rounded to FP64
-// once.  What is left out (levels 7 and up, at most 2^-64 of row maximum times
-// column maximum per k) lies three bits below the result's own rounding, and
-// each digit sum is that much finer than an FP64 element of the row's largest
-// magnitude: see the accuracy test for the error against exact sums.
+// once.  Left out are, of an element, what lies below half a unit of its row's
+// grid, 2^(e - 58) (nothing for the elements within five binary orders of the
+// row's largest), and the levels 7 and up, at most 6.03 x 2^-60 2^(ea + eb) a k.
+// So an output's error goes by the largest elements of its row and column: by
+// norm it is smaller than that of an FP64 chain, but an output that is small
+// because its row and column are large at different k has fewer right digits.
+// Dense products are checked output by output (digit_gate_kernel); the matvec
+// brings the columns of its constant operands to even magnitudes.
 //
 // The kernel is persistent and warp-specialised, one CTA per SM: one thread
 // moves operands by TMA (32 k of all digits of 128 + 64 rows: 84 KB, a ring of
-// two), one warp issues tcgen05.mma, eight warps drain the accumulators.  The
+// two), one warp issues tcgen05.mma, sixteen warps drain the accumulators.  The
 // digits of 32 B rows lie one after the other in shared memory and the levels
 // 32 columns apart in TMEM, so digit i of A meets digits 0 .. 6 - i of B in
 // ONE instruction (N = 32 (7 - i)) that lands on levels i .. 6: seven
@@ -26,7 +30,7 @@
 // while the other is summed.
 //
 // Measured (2048^3, N(0, 1) operands): product 0.40 ms (1.2 PFLOP/s of fp16,
-// 0.63 of the measured peak), the call 0.51 ms, against 14.6 ms for the FP64
+// 0.63 of the measured peak), the call 0.52 ms, against 14.6 ms for the FP64
 // kernel, whose pipe is at its limit; relative error 4.9e-17 against 5.8e-16
 // at K = 300.  The 28 instructions of a stage take 1935 clocks alone (1792
 // ideal) and 2790 here; leaving the loads out changes nothing, leaving the

@@ -203,12 +203,14 @@ tk_status gemm_digits(tk_ctx* ctx, double alpha, const tk_mat* a, const tk_mat* 
 
 // The faster of the two kernels for a product.  The digits cost 45 us however
 // small it is, then 4 us for 64 k of as many 128 x 64 tiles as there are SMs and
-// 6 us for the tiles' ends; the FP64 kernel's estimate is its own.  Whole calls,
-// digits against FP64 kernel: 300^3 73 us against 76, 512 x 512 x 128 61 against
-// 77, 2048 x 64 x 300 74 against 95, 400^3 76 against 147, 2048 x 32 x 2048 151
-// against 251, 2048^3 0.62 ms against 14.6; on the other side 256^3 and
-// 200 x 200 x 1000 stay with the FP64 kernel (54 and 110 us, digits 67 and 115 by
-// the estimate).  Digits of more than 2 GB are not laid out.
+// 6 us for the tiles' ends (estimates, 10 to 15 % above what large products take);
+// the FP64 kernel's estimate is its own.  Whole calls, digits against FP64 kernel:
+// 200 x 200 x 1000 97 us against 98, 300^3 67 against 71, 512 x 512 x 128 56
+// against 71, 2048 x 64 x 300 69 against 90, 400^3 69 against 142, 2048 x 32 x
+// 2048 143 against 245, 2048^3 0.51 ms against 13.9; on the other side 256^3 and
+// 512 x 512 x 64 stay with the FP64 kernel (53 and 48 us).  Operands that the gate
+// refuses have cost 50 us and the digits' passes when the FP64 kernel starts.
+// Digits of more than 2 GB are not laid out.
 bool gemm_on_digits(int64_t M, int64_t N, int64_t K) {
     if (K <= 0 || (double)(M + N) * (K + kTcBK) * kDigits * 2.0 > 2147483648.0) return false;
     const double tiles = (double)((M + kTcBM - 1) / kTcBM) * ((N + kTcBN - 1) / kTcBN);

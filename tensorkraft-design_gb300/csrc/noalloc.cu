@@ -11,9 +11,9 @@
 // index (dense_gemm_f64_kernel), so nothing is allocated, freed or copied.
 //
 // Limits and rules:
-//   * outputs of at most kNoallocMaxTiles 64x64 squares (about 16k x 16k), the
-//     size of the table that the call once kept in a fixed device array; larger
-//     calls are rejected with TK_ERR_INVALID_ARG;
+//   * outputs of at most kNoallocMaxTiles 64x64 squares (about 16k x 16k): a limit
+//     of the interface, from the table that the call once kept in a fixed device
+//     array; larger calls are rejected with TK_ERR_INVALID_ARG;
 //   * the call is stream-ordered and does not synchronise: C is complete when
 //     the stream reaches the end of the call's work.
 #include <cuda_runtime.h>
@@ -51,8 +51,8 @@ extern "C" tk_status tk_gemm_f64_noalloc(tk_ctx* ctx, double alpha, const tk_mat
         return fail("tk_gemm_f64_noalloc: dimensions or strides exceed 32 bits", TK_ERR_UNSUPPORTED);
     const int64_t ntm = (c->rows + 63) / 64, ntn = (c->cols + 63) / 64;
     if (ntm * ntn > kNoallocMaxTiles)
-        return fail("tk_gemm_f64_noalloc: output needs " + std::to_string(ntm * ntn) + " 64x64 tiles, more than the " +
-                        std::to_string(kNoallocMaxTiles) + " the 1 MiB no-allocation scratch holds; use tk_gemm_f64",
+        return fail("tk_gemm_f64_noalloc: output of " + std::to_string(ntm * ntn) + " 64x64 squares, more than the " +
+                        std::to_string(kNoallocMaxTiles) + " this call takes (its former no-allocation scratch); use tk_gemm_f64",
                     TK_ERR_INVALID_ARG);
     const int dev = ctx ? ctx->device : 0;
     if (dev < 0 || dev >= kMaxDevices) return fail("tk_gemm_f64_noalloc: device index out of range", TK_ERR_INVALID_ARG);

@@ -34,9 +34,13 @@
 //
 // Large plans run the same stacks on the fp16 tensor cores instead
 // (digit_gemm.cu): digits of psi, T1 by digit products, the same combine,
-// digits of T2, y by digit products.  Hubbard D = 2048: 701 -> 142 us; cylinder
-// D = 2048: 40.9 -> 1.58 ms, relative error 2.6e-15 -> 1.5e-15; a complex plan
-// takes both parts as one K twice as long.
+// digits of T2, y by digit products.  Hubbard D = 2048: 701 -> 143 us; cylinder
+// D = 2048: 40.9 -> 1.60 ms, relative error 2.6e-15 -> 1.5e-15; a complex plan
+// takes both parts as one K twice as long.  The columns of L and R, and with them
+// psi's and T2's elements at that k, are scaled by powers of two to even
+// magnitudes: ket states that are empty or on scales of their own would cost the
+// others digits (1 % of the matvec; without L's, ket scales of 2^-20 .. 2^20 left
+// a relative error of 2e-6).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -583,8 +587,8 @@ static void digit_rows_of(std::vector<DigitRows>& out, int32_t row, int n, int32
 // add up (Heisenberg D = 128, 0.4 million: 17 us against 29; Hubbard D = 256,
 // 0.4 million: 31 against 28); above, their pipe is the limit (Hubbard D = 362,
 // 1.3 million: 38 against 31 us; D = 512: 50 against 33; D = 2048, 230 million:
-// 701 against 142; Heisenberg D = 512, 25 million: 151 against 48; cylinder D =
-// 2048, 13 billion: 40.9 ms against 1.58).  A plan of less than a dozen stage-3
+// 701 against 143; Heisenberg D = 512, 25 million: 151 against 48; cylinder D =
+// 2048, 13 billion: 40.9 ms against 1.60).  A plan of less than a dozen stage-3
 // tiles keeps its three launches up to 8 million: small plans of a few sectors
 // are relied on to be three launches (digits would take 58 us against 85 at 6.2
 // million on ten tiles).
