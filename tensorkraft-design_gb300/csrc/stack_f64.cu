@@ -512,20 +512,25 @@ bool stage3_pieces(const TcTables& C, std::vector<F64Piece>& out, std::vector<KS
             if (a[i].kb != b[i].kb || a[i].ke != b[i].ke) return false;
         return true;
     };
+    // a bra sector without blocks of R has tiles without K: no rows of T2 are theirs
+    const std::vector<KSeg> none;
+    auto row_of = [&](const TcTile& t, int m) -> const std::vector<KSeg>& {
+        return t.kch > 0 ? rowk[(size_t)t.a_row + m] : none;
+    };
     double total = 0.0;
     for (const TcTile& t : C.tiles3)
-        for (int m = 0; m < t.m_valid; ++m) total += (double)t.n_valid * klen(rowk[(size_t)t.a_row + m]);
+        for (int m = 0; m < t.m_valid; ++m) total += (double)t.n_valid * klen(row_of(t, m));
     const double target = std::max(1.0, total / (152.0 * 16.0));
     for (const TcTile& t : C.tiles3) {
         int m = 0;
         while (m < t.m_valid) {
-            const std::vector<KSeg>& ks = rowk[(size_t)t.a_row + m];
+            const std::vector<KSeg>& ks = row_of(t, m);
             if (!ks.empty() && (ks.front().kb < 0 || ks.back().ke > t.k_valid)) {
                 err = "stacked FP64 stage-3 row reaches past its stack's K";
                 return false;
             }
             int e = m + 1;
-            while (e < t.m_valid && same(rowk[(size_t)t.a_row + e], ks)) ++e;
+            while (e < t.m_valid && same(row_of(t, e), ks)) ++e;
             // rows no combine job writes get a piece without segments: it stores zeros
             const int32_t s0 = (int32_t)segs.size();
             segs.insert(segs.end(), ks.begin(), ks.end());
@@ -666,13 +671,23 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
     };
     if (std::max({C.lq_rows, C.rq_rows, C.t2q_rows, C.xq_rows}) > INT32_MAX / 4) return cudaSuccess;  // 32-bit rows
     std::map<int32_t, Stack> s1, s3;  // by the first row of the operand that names the stack
+    std::vector<TcTile> w3;
     for (const std::vector<TcTile>* v : {&C.tiles1x, &C.tiles3})
         for (const TcTile& t : *v) {
+            if (t.kch == 0) {  // zeros, in either part: no operands; the second tile's columns all lie behind the split
+                TcTile z = t;
+                z.a_row = z.b_row = 0;
+                w3.push_back(z);
+                z.n0 += 1;
+                z.split = 1;
+                w3.push_back(z);
+                continue;
+            }
             Stack& s = t.mode == 2 ? s1[t.a_row - t.ldc] : s3[t.b_row - t.n0];
             s.M = t.a_cs, s.N = t.b_cs, s.K = t.k_valid, s.kch = t.kch;
             s.a = std::min(s.a, t.a_row), s.b = std::min(s.b, t.b_row), s.out = std::min(s.out, t.out_off);
         }
-    std::vector<TcTile> w1, w3, t1, t3;
+    std::vector<TcTile> w1, t1, t3;
     std::vector<int32_t> b1, b3;
     std::vector<DigitRowsC> lrows, rrows, trows;
     std::vector<DigitRows> rcols, lcols;
@@ -829,6 +844,7 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
     // others digits
     std::map<int32_t, int32_t> kx;  // stack (row of its first R row) -> scales
     for (const TcTile& t : C.tiles3) {
+        if (t.kch == 0) continue;  // zeros, without operands
         const int32_t base = t.b_row - t.n0;
         if (kx.insert({base, nk}).second) {
             rcols.push_back({base, t.b_cs, t.b_cs, t.kch, nk, -1});
