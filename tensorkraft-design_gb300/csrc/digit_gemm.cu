@@ -647,9 +647,6 @@ __device__ __forceinline__ int exponent_of(double x, int k) {
     return zero ? kNoExponent : (e > 0 ? e : 12 - __clz((int)(hi | 1))) + k;
 }
 
-// Scale of a column of zeros: what the other operand holds at that k is multiplied
-// by zeros, so it must neither set its row's exponent nor take up its digits.
-constexpr int kDeadColumn = -4096;
 // A row's exponent; one with nothing but dead columns counts as zeros.
 __device__ __forceinline__ int scaled_row_exponent(int mx) { return mx < kDeadColumn / 2 ? 1 : mx; }
 
@@ -669,9 +666,10 @@ __global__ void __launch_bounds__(kColumnRows * kTcBK) digit_columns_kernel(cons
 #pragma unroll 4
     for (int r = w; r < j.n; r += kColumnRows) {
         const int64_t at = (((int64_t)j.row + (int64_t)c * j.cs + r) << 6) + k;
-        const int by = ex ? -ex[j.ex0 + r] : -1023;
-        mx = max(mx, exponent_of(q64[at], by));
-        if (q64_im) mx = max(mx, exponent_of(q64_im[at], by));
+        const int unit = ex ? ex[j.ex0 + r] : 1023;
+        if (unit == kNoGain) continue;
+        mx = max(mx, exponent_of(q64[at], -unit));
+        if (q64_im) mx = max(mx, exponent_of(q64_im[at], -unit));
     }
     top[w][k] = mx;
     __syncthreads();

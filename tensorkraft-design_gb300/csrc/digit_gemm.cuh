@@ -111,8 +111,11 @@ cudaError_t launch_digit_gemm(int mode, const TcTile* tiles, const int32_t* begi
                               const int32_t* exa, const int32_t* exb, const DigitOut& out, int* redo, cudaStream_t s);
 
 // Exponents of a stack's columns: kx[j.kx + k] = floor(log2 max |x|) over the
-// rows [row, row + n) of job j at k (with exponents of rows: of x by its row's
-// largest); far below any of them for a column of zeros.
+// rows [row, row + n) of job j at k, of x 2^(1023 - ex[j.ex0 + r]) with a table ex
+// (leaving out rows of kNoGain); kDeadColumn for a column of zeros, far below the others:
+// what the other operand holds at that k is multiplied by zeros, so it must neither set
+// its row's exponent nor take up its digits.
+constexpr int kNoGain = INT32_MIN, kDeadColumn = -8192;
 cudaError_t launch_digit_columns(const DigitRows* jobs, int n_jobs, int max_kch, const double* q64, const double* q64_im,
                                  const int32_t* ex, int32_t* kx, cudaStream_t s);
 // Digits of FP64 operand stacks (rows of 64 doubles per chunk), of

@@ -627,7 +627,7 @@ static tk_status build_tc_tables(Heff2Tables& T, const TcSource& X, const TcOpti
         auto kchunks = [&](int64_t K) { return (int32_t)((K + BK - 1) / BK); };
         std::vector<StackCopy> lcopy, rcopy;
         // T1 pieces: key (p, A', ws, B) -> (offset of channel-0 row, row stride per a')
-        struct Piece { uint64_t key; int64_t off; int32_t rs; };
+        struct Piece { uint64_t key; int64_t off; int32_t rs, row; };  // row: of the L stacks
         std::vector<Piece> pieces;
         auto pkey = [&](int64_t p, int ap, int ws, int b) -> uint64_t {
             return (((uint64_t)p * nA + ap) * nWL + ws) * nB + b;
@@ -737,7 +737,8 @@ static tk_status build_tc_tables(Heff2Tables& T, const TcSource& X, const TcOpti
                     const int64_t DB = QB.dim[xp[jx].second];
                     // channel-0 row of the slab, row stride per a' = dws rows of D_B
                     pieces.push_back({pkey(xp[jx].first, lp[i].first, lp[i].second, xp[jx].second),
-                                      t1off + xcol[jx] * rows + lrow[i] * DB, (int32_t)(WL.dim[lp[i].second] * DB)});
+                                      t1off + xcol[jx] * rows + lrow[i] * DB, (int32_t)(WL.dim[lp[i].second] * DB),
+                                      (int32_t)(lb + lrow[i])});
                 }
             t1off += rows * cols;
         }
@@ -788,6 +789,7 @@ static tk_status build_tc_tables(Heff2Tables& T, const TcSource& X, const TcOpti
             std::vector<Slab> slabs;
             std::vector<TcCombTerm> sterms;
             std::vector<double> scoef;  // the same coefficients in FP64
+            std::vector<int32_t> srow;  // the L row of a term's first row
             for (size_t i = 0; i < yp.size(); ++i) {
                 int64_t po = yp[i].first;
                 int ap = yp[i].second;
@@ -810,6 +812,7 @@ static tk_status build_tc_tables(Heff2Tables& T, const TcSource& X, const TcOpti
                                 ct.coef = (float)tm.c;
                                 sterms.push_back(ct);
                                 scoef.push_back(tm.c);
+                                srow.push_back((int32_t)(it->row + wl_loc[tm.wl]));
                             }
                         }
                         sl.te = (int32_t)sterms.size();
@@ -828,6 +831,7 @@ static tk_status build_tc_tables(Heff2Tables& T, const TcSource& X, const TcOpti
                     j.term_begin = (int32_t)C.terms.size();
                     C.terms.insert(C.terms.end(), sterms.begin() + sl.tb, sterms.begin() + sl.te);
                     C.term_coef64.insert(C.term_coef64.end(), scoef.begin() + sl.tb, scoef.begin() + sl.te);
+                    C.term_row.insert(C.term_row.end(), srow.begin() + sl.tb, srow.begin() + sl.te);
                     j.term_end = (int32_t)C.terms.size();
                     for (int q = 0; q < kTcCombInline && j.term_begin + q < j.term_end; ++q)
                         j.inl[q] = C.terms[j.term_begin + q];

@@ -45,6 +45,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <map>
 #include <memory>
 #include <set>
@@ -660,6 +661,46 @@ static cudaError_t digits_alloc(F64Digits& d, const Blob& blob, const int64_t (&
     return cudaMemset(d.x.q, 0, digit_stack_bytes(d.x.rows));
 }
 
+// What a row of an L stack can come to in the result: the largest coefficient times
+// column of R that the combine's terms give a row of T1 (binary exponents, kNoGain
+// where no term reads it), as launch_digit_columns takes it for that row's unit.
+// The scales of L's columns go by it: with psi's element at k on 2^kx, where some
+// row's L 2^gain reaches 2^kx, the largest scaled element of a psi column does reach
+// the result at full size, and no row's error can come to more than 2^-58 of it.
+// (By the rows' own sizes instead, a channel that is large but hardly counts at the k
+// where psi is large left relative errors up to 2e-7.)  kx3: exponents of R's columns;
+// stack3: a stack-3 tile's first row of T2 -> its scales.
+static std::vector<int32_t> row_gains(const TcTables& C, const std::map<int32_t, int32_t>& stack3,
+                                      const std::vector<int32_t>& kx3) {
+    const std::vector<std::pair<int32_t, int32_t>> stacks(stack3.begin(), stack3.end());
+    std::vector<int32_t> gain((size_t)C.lq_rows, kNoGain);
+    int32_t slab = -1, r = 0;  // the jobs of a slab have its terms in common
+    for (const TcCombJob& j : C.jobs) {
+        if (j.term_begin != slab) {
+            slab = j.term_begin;
+            const auto st = std::upper_bound(stacks.begin(), stacks.end(), j.t2row,
+                                             [](int32_t v, const auto& x) { return v < x.first; });
+            const int32_t* k = kx3.data() + std::prev(st)->second + j.k0;
+            r = *std::max_element(k, k + j.cols);
+        }
+        if (r <= kDeadColumn) continue;
+        for (int t = j.term_begin; t < j.term_end; ++t) {
+            const double c = C.term_coef64[(size_t)t];
+            if (c == 0.0) continue;
+            uint64_t bits;
+            std::memcpy(&bits, &c, sizeof(bits));
+            const int32_t g = (int32_t)((bits >> 52) & 0x7FF) - 1023 + r, step = C.terms[(size_t)t].in_rs / j.cols;
+            int32_t* x = gain.data() + C.term_row[(size_t)t] + (int64_t)j.r0 * step;
+            // (a slab's rows are all raised together)
+            if (*x >= g) continue;
+            for (int i = 0; i < j.rows; ++i) x[(int64_t)i * step] = g;
+        }
+    }
+    for (int32_t& g : gain)
+        if (g != kNoGain) g = 1023 - g;  // the unit of a row's exponents
+    return gain;
+}
+
 // The digit form of a complex plan: the same products on operands of two parts.
 // Row (A, T2): (re | im); column (psi, R): re (re | -im), im (im | re), the im
 // columns behind the re ones, so that one tile may hold both.
@@ -718,13 +759,14 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
     };
     std::map<int32_t, const Stack*> by_psi;  // stage-1 stacks by their first psi row
     int kch1 = 0;
+    std::map<int32_t, int32_t> stack3;  // first row of T2 -> scales
     for (auto& [key, s] : s1) {
         by_psi[s.b] = &s;
         tiles(w1, s, 2);
         s.kx = nk;
         nk += s.kch * kTcBK;
         kch1 = std::max(kch1, s.kch);
-        lcols.push_back({s.a, s.M, s.M, s.kch, s.kx, 2 * s.a});
+        lcols.push_back({s.a, s.M, s.M, s.kch, s.kx, s.a});
         rows(lrows, s.a, s.M, s.M, s.kch, s.kx, 2 * s.a, s.M, 0);
         for (int32_t c = 0; c < s.N; ++c)
             for (int h = 0; h < 2; ++h) {
@@ -747,6 +789,7 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
     for (const auto& [key, s] : s3) {
         tiles(w3, s, 1);
         rcols.push_back({s.b, s.N, s.N, s.kch, nk, -1});
+        stack3[s.a] = nk;
         rows(rrows, s.b, s.N, s.N, s.kch, nk, 4 * s.b, 2 * s.N, s.N);
         rows(trows, s.a, s.M, s.M, s.kch, nk, 2 * s.a, s.M, 0);
         nk += s.kch * kTcBK;
@@ -783,16 +826,18 @@ static cudaError_t digits_create_complex(const TcTables& C, F64Stack& p, std::un
         err.clear();
         return cudaSuccess;
     }
-    // (L's rows without scales first, for their exponents)
+    std::vector<int32_t> kx3((size_t)std::max(nk, 1)), gain;
     if ((e = cudaMemset(kx, 0, sizeof(int32_t) * (size_t)nk)) != cudaSuccess ||
-        (e = launch_digit_rows_complex(reinterpret_cast<const DigitRowsC*>(m + o_l), (int)lrows.size(), p.lq.p, p.lq_im.p,
-                                       kx, -1, false, d->l, d->redo, 0)) != cudaSuccess ||
+        (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_c), (int)rcols.size(), C.max_kch3, p.rq.p,
+                                  p.rq_im.p, nullptr, kx, 0)) != cudaSuccess ||
+        (e = cudaMemcpy(kx3.data(), kx, sizeof(int32_t) * (size_t)nk, cudaMemcpyDeviceToHost)) != cudaSuccess)
+        return e;
+    gain = row_gains(C, stack3, kx3);
+    if ((e = cudaMemcpy(d->l.ex, gain.data(), sizeof(int32_t) * gain.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_lc), (int)lcols.size(), kch1, p.lq.p, p.lq_im.p,
                                   d->l.ex, kx, 0)) != cudaSuccess ||
         (e = launch_digit_rows_complex(reinterpret_cast<const DigitRowsC*>(m + o_l), (int)lrows.size(), p.lq.p, p.lq_im.p,
                                        kx, -1, false, d->l, d->redo, 0)) != cudaSuccess ||
-        (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_c), (int)rcols.size(), C.max_kch3, p.rq.p,
-                                  p.rq_im.p, nullptr, kx, 0)) != cudaSuccess ||
         (e = launch_digit_rows_complex(reinterpret_cast<const DigitRowsC*>(m + o_r), (int)rrows.size(), p.rq.p, p.rq_im.p,
                                        kx, -1, true, d->r, d->redo, 0)) != cudaSuccess ||
         (e = cudaMemcpy(&redo, d->redo, sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess)
@@ -814,9 +859,7 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
     std::set<int32_t> seen;
     int32_t nk = 0;
     int kch1 = 0;
-    // stage 1: the columns of L on scales of their own, which psi takes up.  What
-    // a column has in its rows counts by the rows' largest elements, so that one
-    // channel of great magnitude does not set the scales of the others.
+    // stage 1: the columns of L on scales of their own (row_gains), which psi takes up
     std::map<int32_t, int32_t> kx1;  // stack (its first psi row) -> scales
     for (const TcTile& t : C.tiles1x) {
         if (kx1.insert({t.b_row - t.n0, nk}).second) {
@@ -842,7 +885,7 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
     // stage 3: the columns of R on scales of their own, which T2 takes up, so
     // that no channel's magnitude (an energy against an identity) costs the
     // others digits
-    std::map<int32_t, int32_t> kx;  // stack (row of its first R row) -> scales
+    std::map<int32_t, int32_t> kx, stack3;  // stack (its first row of R, a tile's first row of T2) -> scales
     for (const TcTile& t : C.tiles3) {
         if (t.kch == 0) continue;  // zeros, without operands
         const int32_t base = t.b_row - t.n0;
@@ -852,6 +895,7 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
         }
         if (seen.insert(-1 - t.b_row).second) digit_rows_of(rrows, t.b_row, t.n_valid, t.b_cs, t.kch, kx[base]);
         if (t.n0 == 0) digit_rows_of(trows, t.a_row, t.m_valid, t.a_cs, t.kch, kx[base]);
+        stack3[t.a_row] = kx[base];
     }
     std::vector<TcTile> t1, t3;
     std::vector<int32_t> b1, b3;
@@ -885,16 +929,18 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
         err.clear();
         return cudaSuccess;
     }
-    // (L's rows without scales first, for their exponents)
+    std::vector<int32_t> kx3((size_t)std::max(nk, 1)), gain;
     if ((e = cudaMemset(kxd, 0, sizeof(int32_t) * (size_t)nk)) != cudaSuccess ||
-        (e = launch_digit_rows(reinterpret_cast<const DigitRows*>(m + o_l), (int)lrows.size(), p.lq.p, kxd, -1, d->l,
-                               d->redo, 0)) != cudaSuccess ||
+        (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_c), (int)rcols.size(), C.max_kch3, p.rq.p, nullptr,
+                                  nullptr, kxd, 0)) != cudaSuccess ||
+        (e = cudaMemcpy(kx3.data(), kxd, sizeof(int32_t) * (size_t)nk, cudaMemcpyDeviceToHost)) != cudaSuccess)
+        return e;
+    gain = row_gains(C, stack3, kx3);
+    if ((e = cudaMemcpy(d->l.ex, gain.data(), sizeof(int32_t) * gain.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_lc), (int)lcols.size(), kch1, p.lq.p, nullptr,
                                   d->l.ex, kxd, 0)) != cudaSuccess ||
         (e = launch_digit_rows(reinterpret_cast<const DigitRows*>(m + o_l), (int)lrows.size(), p.lq.p, kxd, -1, d->l,
                                d->redo, 0)) != cudaSuccess ||
-        (e = launch_digit_columns(reinterpret_cast<const DigitRows*>(m + o_c), (int)rcols.size(), C.max_kch3, p.rq.p, nullptr,
-                                  nullptr, kxd, 0)) != cudaSuccess ||
         (e = launch_digit_rows(reinterpret_cast<const DigitRows*>(m + o_r), (int)rrows.size(), p.rq.p, kxd, -1, d->r,
                                d->redo, 0)) != cudaSuccess ||
         (e = cudaMemcpy(&redo, d->redo, sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess)

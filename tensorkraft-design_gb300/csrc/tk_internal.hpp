@@ -226,6 +226,7 @@ struct TcTables {
     std::vector<double> lq64, rq64;                    // the same stacks in FP64 (stacked FP64 schedule)
     std::vector<double> lq64_im, rq64_im;              // their imaginary parts (complex environments)
     std::vector<double> term_coef64;                   // FP64 coefficients of `terms`
+    std::vector<int32_t> term_row;                     // the L stacks' row of a term's row 0 (its row r: in_rs / cols r further)
     std::vector<TcTile> tiles1, tiles3;
     std::vector<TcTile> tiles1x;       // stage-1 tiles of tall stacks (B operand from the split copy)
     // psi in kTcPsiPieces pieces at block boundaries x_cut[0] = 0 < ... <

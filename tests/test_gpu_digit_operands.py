@@ -183,3 +183,78 @@ def test_rows_of_a_graded_state_beside_identity_channels(lib_built, name, D):
         n = len(fall[1][qr])
         err, row = np.abs(got - want)[a:b].reshape(-1, n).max(1), mags[a:b].reshape(-1, n).max(1)
         assert (err <= 2 * K * 2.0 ** -53 * row).all()
+
+
+def _structured(e, rng):
+    """An environment with some of: channels, bra and ket states on scales of 2^-20 .. 2^20, nine elements in
+    ten left out, groups of states with couplings of 1e-10, an identity channel; and the ket scales."""
+    d = e.data.copy()
+    nb, nw, nk = d.shape
+    ket = np.ones(nk)
+    pick = rng.random(6)
+    if pick[0] < 0.4:
+        d *= np.exp2(rng.integers(-20, 21, nw).astype(float))[None, :, None]
+    if pick[1] < 0.4:
+        d *= np.exp2(rng.integers(-20, 21, nb).astype(float))[:, None, None]
+    if pick[2] < 0.6:
+        ket = np.exp2(rng.integers(-20, 21, nk).astype(float))
+        d *= ket
+    if pick[3] < 0.3:
+        d *= rng.random(d.shape) < 0.1
+    if pick[4] < 0.3:
+        g = rng.integers(0, 3, nb)
+        d *= np.where(g[:, None, None] == g[None, None, :], 1.0, 1e-10)
+    if pick[5] < 0.4:
+        d[:, rng.integers(2) * (nw - 1), :] = np.eye(nb)
+    return Environment(d, e.bra_idx, e.mpo_idx, e.ket_idx), ket
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("seed", range(24))
+def test_norm_error_of_structured_environments(lib_built, seed, cplx):
+    """The difference from FP64 chains, in the 2-norm, against what they promise themselves: 2 K 2^-53 of
+    the sums of magnitudes, K the terms of an output."""
+    from tk_gb300 import Heff2Plan, sweep
+
+    rng = np.random.default_rng(seed)
+    p = _problem(*[("heisenberg", 401), ("cylinder", 257), ("hubbard", 700)][seed % 3], lambda e, side: e)
+    (el, kl), (er, kr) = _structured(p.env_l, rng), _structured(p.env_r, rng)
+
+    def absolute(t):
+        out = type(t).__new__(type(t))
+        out.__dict__.update(t.__dict__)
+        out.blocks = {k: np.abs(v) for k, v in t.blocks.items()}
+        return out
+
+    def turned(e):
+        return sweep.DeviceEnv.from_dense(p.kind, e.data * np.exp(2j * np.pi * rng.random(e.data.shape)), e.bra_idx, e.mpo_idx, e.ket_idx)
+
+    q = type(p)(p.kind, el, er, p.w_i, p.w_j, p.flux, p.name)
+    plan = Heff2Plan.from_device_envs_complex(turned(el), turned(er), p.w_i, p.w_j, p.flux) if cplx else q.plan()
+    nc = len(el.ket_idx.sectors[0][0])
+    first, at = {}, 0
+    legs = []
+    for e, scale in ((el, kl), (er, kr)):
+        n = len(scale)
+        # taken back, left alone, falling, on scales of its own
+        f = [1.0 / scale, np.ones(n), None, np.exp2(rng.integers(-20, 21, n).astype(float))][rng.integers(4)]
+        if f is None:
+            f = np.concatenate([np.logspace(0, -8, m) for _, m in e.ket_idx.sectors])
+        first, at = {}, 0
+        for c, m in e.ket_idx.sectors:
+            first[tuple(c)] = f[at:at + m]
+            at += m
+        legs.append(first)
+    x = rng.standard_normal(plan.block_dim)
+    keys, offs = plan.blocks()
+    for key, a, b in zip(keys, offs, list(offs[1:]) + [plan.block_dim]):
+        fl, fr = legs[0][_left_sector(key, nc)], legs[1][_right_sector(key, nc)]
+        x[a:b].reshape(-1, len(fl), len(fr))[:] *= fl[:, None] * fr
+    z = x * np.exp(2j * np.pi * rng.random(len(x))) if cplx else x
+    run = (lambda s: np.concatenate(_apply_complex(plan, z, s))) if cplx else (lambda s: _apply(plan, z, s))
+    got, want = run(_abi.SCHED_STACKED), run(_abi.SCHED_GROUPED)
+    mags = type(p)(p.kind, *(Environment(np.abs(e.data), e.bra_idx, e.mpo_idx, e.ket_idx) for e in (el, er)),
+                   absolute(p.w_i), absolute(p.w_j), p.flux, p.name)
+    size = np.linalg.norm(_apply(mags.plan(), np.abs(x), _abi.SCHED_GROUPED))
+    K = el.data.shape[1] * (max(m for _, m in el.ket_idx.sectors) + max(m for _, m in er.ket_idx.sectors))
+    assert np.linalg.norm(got - want) <= 2 * K * 2.0 ** -53 * size
