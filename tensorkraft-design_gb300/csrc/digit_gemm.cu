@@ -17,7 +17,7 @@
 // norm it is smaller than that of an FP64 chain, but an output that is small
 // because its row and column are large at different k has fewer right digits.
 // Dense products are checked output by output (digit_gate_kernel); the matvec
-// brings the columns of its constant operands to even magnitudes.
+// scales its operands' k so that its result is held by norm (stack_f64.cu).
 //
 // The kernel is persistent and warp-specialised, one CTA per SM: one thread
 // moves operands by TMA (32 k of all digits of 128 + 64 rows: 84 KB, a ring of
