@@ -438,10 +438,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) digit_gemm_kernel(const TcTile* _
             int32_t pitch[WCOLS / SCOLS] = {};
             if (mine) {
                 if (row0 + lane < t.m_valid) {
-                    if (t.k_valid > 0) ea = exa[t.a_row + row0 + lane];  // (a tile without K has no operands: zeros)
+                    ea = exa[t.a_row + row0 + lane];
                     if (MODE == 1) rows = om.rowtab[t.out_off + row0 + lane];
                 }
-                if (t.k_valid > 0) eb = exb[t.b_row + h * HN + col0 + min(lane, nc - 1)];  // (a column past the tile's takes the last one's)
+                eb = exb[t.b_row + h * HN + col0 + min(lane, nc - 1)];  // (a column past the tile's takes the last one's)
                 if (MODE == 2)
 #pragma unroll
                     for (int g = 0; g < WCOLS / SCOLS; ++g)

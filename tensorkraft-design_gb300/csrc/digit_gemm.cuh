@@ -43,7 +43,9 @@ cudaError_t launch_dependent(void (*k)(P...), dim3 grid, unsigned block, size_t 
 
 // A digit operand in the operand-stack layout (K-major 64-wide chunks, see
 // TcTables): `rows` rows of seven digits of 64 elements each, one after the
-// other, and the biased exponent of every row of chunk 0.
+// other, and the biased exponent of every row of chunk 0 (kTcBM entries more, for
+// tiles without K: they have no rows, a_row = b_row = 0, and their sums are zeros
+// whatever the exponents).
 struct DigitStack {
     __half* q = nullptr;
     int32_t* ex = nullptr;

@@ -641,7 +641,7 @@ static cudaError_t digits_alloc(F64Digits& d, const Blob& blob, const int64_t (&
     for (int i = 0; i < 4; ++i) {
         st[i]->rows = std::max<int64_t>(rows[i], 1);
         q[i] = take(digit_stack_bytes(st[i]->rows));
-        x[i] = take(sizeof(int32_t) * (size_t)st[i]->rows);
+        x[i] = take(sizeof(int32_t) * (size_t)(st[i]->rows + kTcBM));
     }
     const size_t k = take(sizeof(int32_t) * (size_t)std::max(nk, 1));
     cudaError_t e;
@@ -888,8 +888,12 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
     // that no channel's magnitude (an energy against an identity) costs the
     // others digits
     std::map<int32_t, int32_t> kx, stack3;  // stack (its first row of R, a tile's first row of T2) -> scales
-    for (const TcTile& t : C.tiles3) {
-        if (t.kch == 0) continue;  // zeros, without operands
+    std::vector<TcTile> w3(C.tiles3);
+    for (TcTile& t : w3) {
+        if (t.kch == 0) {  // zeros, without operands
+            t.a_row = t.b_row = 0;
+            continue;
+        }
         const int32_t base = t.b_row - t.n0;
         if (kx.insert({base, nk}).second) {
             rcols.push_back({base, t.b_cs, t.b_cs, t.kch, nk, -1});
@@ -908,7 +912,7 @@ static cudaError_t digits_create(const TcTables& C, F64Stack& p, std::string& er
         (e = digit_setup()) != cudaSuccess)
         return e;
     digit_schedule(C.tiles1x, d->sms, t1, b1);
-    digit_schedule(C.tiles3, d->sms, t3, b3);
+    digit_schedule(w3, d->sms, t3, b3);
     // the tables first (one copy), then what the device writes
     Blob blob;
     auto table = [&](const auto& v) { return blob.add(v.data(), sizeof(v[0]) * v.size()); };
